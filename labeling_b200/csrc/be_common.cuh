@@ -114,29 +114,6 @@ __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p)
     return *reinterpret_cast<const volatile uint32_t *>(p);
 }
 
-// Foreground bits of four packed pixels: bit k = byte k > thr.
-__device__ __forceinline__ uint32_t fg4(uint32_t w, uint32_t thr4)
-{
-    uint32_t m = __vcmpgtu4(w, thr4) & 0x01010101u;
-    return (m * 0x10204080u) >> 28;
-}
-
-// Foreground bits of 16 pixels held in a uint4 (bit k = pixel k).
-__device__ __forceinline__ uint32_t fg16(uint4 v, uint32_t thr4)
-{
-    return fg4(v.x, thr4) | (fg4(v.y, thr4) << 4) | (fg4(v.z, thr4) << 8) | (fg4(v.w, thr4) << 12);
-}
-
-// Spread the 8 bit-pairs of a 16-bit word into the low two bits of 8 nibbles.
-__device__ __forceinline__ uint32_t pairs_to_nibbles(uint32_t x)
-{
-    x &= 0xFFFFu;
-    x = (x | (x << 8)) & 0x00FF00FFu;
-    x = (x | (x << 4)) & 0x0F0F0F0Fu;
-    x = (x | (x << 2)) & 0x33333333u;
-    return x;
-}
-
 // Union-find find over a shared-memory parent array (parents never exceed their child), with
 // path halving: each visited entry is pointed at its grandparent.  Every stored value is an
 // ancestor of the entry at the time it was read, so concurrent merges stay correct: a pointer
@@ -396,6 +373,83 @@ __device__ __forceinline__ Img ImgList<Img>::get(int64_t tile) const
 
 using ImgList2D = ImgList<Img2D>;
 using ImgList3D = ImgList<Img3D>;
+
+// ---- Pixel rows as bit words ------------------------------------------------------------------
+// Byte-wise x > thr for four pixels: bit 7 of each byte.  K = 0x7F - (thr & 0x7F) in every byte;
+// `hi` = thr >= 128.  (x & 0x7F) + K carries into bit 7 exactly when the low seven bits exceed
+// thr's; the high bit decides the rest.
+__device__ __forceinline__ uint32_t gt_bytes(uint32_t x, uint32_t K, bool hi)
+{
+    const uint32_t s = (x & 0x7F7F7F7Fu) + K;
+    return (hi ? (x & s) : (x | s)) & 0x80808080u;
+}
+
+// Bits 7, 15, 23, 31 -> bits 0..3 (the four partial products land on distinct bits, no carries).
+__device__ __forceinline__ uint32_t gather4(uint32_t g) { return (g * 0x00204081u) >> 28; }
+
+// 16 pixels of one row -> foreground bits of their even (left) and odd (right) pixels: 8 blocks.
+__device__ __forceinline__ void split16(uint4 v, uint32_t K, bool hi, uint32_t &ev, uint32_t &od)
+{
+    ev = gather4(gt_bytes(__byte_perm(v.x, v.y, 0x6420), K, hi)) |
+         (gather4(gt_bytes(__byte_perm(v.z, v.w, 0x6420), K, hi)) << 4);
+    od = gather4(gt_bytes(__byte_perm(v.x, v.y, 0x7531), K, hi)) |
+         (gather4(gt_bytes(__byte_perm(v.z, v.w, 0x7531), K, hi)) << 4);
+}
+
+// Foreground bits of the n (1..64) pixels at p, split as split16 (bit k of left / right: pixel
+// 2k / 2k + 1), whatever p's alignment: the up to five 16-byte chunks that hold the pixels are
+// loaded whole and the words shifted into place -- an odd offset swaps the even and odd words.  A
+// chunk that would reach outside [lo, hi), the image's bytes, is read byte by byte.  (One byte
+// load per pixel cost a tile kernel 64 dependent load-and-or steps per row for every image whose
+// width is not a multiple of 16.)
+__device__ __forceinline__ void row_bits(const uint8_t *p, int n, const uint8_t *lo, const uint8_t *hi,
+                                         uint32_t K, bool thr_hi, int thr, uint32_t &left, uint32_t &right)
+{
+    const int a = int(reinterpret_cast<uintptr_t>(p) & 15u);
+    const uint8_t *base = p - a;
+    uint4 v[5];
+    uint32_t bytewise = 0;   // chunks to read byte by byte
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        v[i] = make_uint4(0, 0, 0, 0);
+        if (16 * i < a + n) {
+            const uint8_t *c = base + 16 * i;
+            if (c >= lo && c + 16 <= hi) v[i] = __ldg(reinterpret_cast<const uint4 *>(c));
+            else bytewise |= 1u << i;
+        }
+    }
+    uint32_t ev = 0, od = 0, ev4 = 0, od4 = 0;   // even / odd bytes of chunks 0..3, of chunk 4
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        uint32_t e8, o8;
+        split16(v[i], K, thr_hi, e8, o8);
+        if ((bytewise >> i) & 1u) {
+            e8 = o8 = 0;
+#pragma unroll 1
+            for (int k = 0; k < 16; ++k) {
+                const uint8_t *c = base + 16 * i + k;
+                const uint32_t bit = (c >= lo && c < hi && *c > thr) ? 1u << (k >> 1) : 0u;
+                if (k & 1) o8 |= bit;
+                else e8 |= bit;
+            }
+        }
+        if (i < 4) {
+            ev |= e8 << (8 * i);
+            od |= o8 << (8 * i);
+        } else {
+            ev4 = e8;
+            od4 = o8;
+        }
+    }
+    const uint32_t h = uint32_t(a) >> 1;
+    const uint32_t el = __funnelshift_r(ev, ev4, h), ol = __funnelshift_r(od, od4, h);
+    const uint32_t er = __funnelshift_r(ev, ev4, h + 1u);
+    left = (a & 1) ? ol : el;
+    right = (a & 1) ? er : ol;
+    const int nl = (n + 1) >> 1, nr = n >> 1;   // valid left / right pixels
+    left &= 0xFFFFFFFFu >> (32 - nl);
+    right &= nr ? 0xFFFFFFFFu >> (32 - nr) : 0u;
+}
 
 // Programmatic dependent launch (sm_90 and later).  A launch made with programmatic stream
 // serialization may put its CTAs on the SMs while the grid before it in the stream still runs:

@@ -42,27 +42,6 @@ __device__ __forceinline__ bool perim_pos(int p, int nbr, int nbc, int &r, int &
     return r < nbr;
 }
 
-// Byte-wise x > thr for four pixels: bit 7 of each byte.  K = 0x7F - (thr & 0x7F) in every byte;
-// `hi` = thr >= 128.  (x & 0x7F) + K carries into bit 7 exactly when the low seven bits exceed
-// thr's; the high bit decides the rest.
-__device__ __forceinline__ uint32_t gt_bytes(uint32_t x, uint32_t K, bool hi)
-{
-    const uint32_t s = (x & 0x7F7F7F7Fu) + K;
-    return (hi ? (x & s) : (x | s)) & 0x80808080u;
-}
-
-// Bits 7, 15, 23, 31 -> bits 0..3 (the four partial products land on distinct bits, no carries).
-__device__ __forceinline__ uint32_t gather4(uint32_t g) { return (g * 0x00204081u) >> 28; }
-
-// 16 pixels of one row -> foreground bits of their even (left) and odd (right) pixels: 8 blocks.
-__device__ __forceinline__ void split16(uint4 v, uint32_t K, bool hi, uint32_t &ev, uint32_t &od)
-{
-    ev = gather4(gt_bytes(__byte_perm(v.x, v.y, 0x6420), K, hi)) |
-         (gather4(gt_bytes(__byte_perm(v.z, v.w, 0x6420), K, hi)) << 4);
-    od = gather4(gt_bytes(__byte_perm(v.x, v.y, 0x7531), K, hi)) |
-         (gather4(gt_bytes(__byte_perm(v.z, v.w, 0x7531), K, hi)) << 4);
-}
-
 // Bits 0..3 of x -> bit 0 of bytes 0..3.
 __device__ __forceinline__ uint32_t spread4(uint32_t x) { return ((x & 0xFu) * 0x00204081u) & 0x01010101u; }
 
@@ -212,12 +191,9 @@ __global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
                 }
             } else {
                 const int n = min(64, ncp - 64 * q);
-                for (int x = 0; x < n; ++x) {
-                    const uint32_t bt = uint32_t(row0[x] > im.thr) << (x >> 1);
-                    const uint32_t bb = row1 ? uint32_t(row0[im.in_pitch + x] > im.thr) << (x >> 1) : 0u;
-                    if (x & 1) { TRw |= bt; BRw |= bb; }
-                    else { TLw |= bt; BLw |= bb; }
-                }
+                const uint8_t *hi_px = im.in + int64_t(im.rows - 1) * im.in_pitch + im.cols;
+                row_bits(row0, n, im.in, hi_px, K, hi, im.thr, TLw, TRw);
+                if (row1) row_bits(row0 + im.in_pitch, n, im.in, hi_px, K, hi, im.thr, BLw, BRw);
             }
         }
         const uint32_t Lw = TLw | BLw, Rw = TRw | BRw, Tw = TLw | TRw, Fw = Tw | BLw | BRw;
