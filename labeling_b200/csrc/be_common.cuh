@@ -69,8 +69,8 @@ struct Work {
     uint2 *nlink;         // per node, after the merge: x = segment of its global root's first pixel
                           // (kNone when the node is a root itself), y = (root block << 16) | rank
                           // of that first pixel among the roots left in its segment
-    uint32_t *rbits;      // per tile: bitmap of the first pixels (voxels) of the tile's components
-                          // that are still roots (the merge clears the ones it links)
+    uint32_t *rbits;      // per tile: bitmap of the tile's components that are still roots (the merge
+                          // clears the ones it links): 2D a bit per run, 3D a bit per first voxel
     uint8_t *segcnt;      // per segment: number of component roots (uint8, word-padded)
     uint32_t *segpref;    // per segment + 1: exclusive prefix of segcnt over the launch
     uint32_t *chunksum;   // per scan chunk: sum of segcnt
@@ -178,6 +178,54 @@ __device__ __forceinline__ void smerge(uint32_t *P, uint32_t a, uint32_t b)
     }
 }
 
+// Points entries first, first + step, ... below n of a shared-memory parent array straight at their
+// roots while no link happens (a read-only walk, then one store: whatever a walk meets is an
+// ancestor, so any interleaving is right).  Entries are taken in ascending order by all threads at
+// once, so a walk soon meets entries that are done.  (Sweeps of pointer jumping with four entries in
+// flight, and one state machine per lane over its entries, were measured slower: the loop is bound by
+// instruction issue, not by the latency of a walk.)
+__device__ __forceinline__ void sflatten_all(uint32_t *P, uint32_t first, uint32_t step, uint32_t n)
+{
+    for (uint32_t i = first; i < n; i += step) {
+        uint32_t x = P[i];
+        if (x == i) continue;
+        uint32_t y = P[x];
+        if (y == x) continue;   // at its root already
+        while (y != x) {
+            x = y;
+            y = P[x];
+        }
+        P[i] = x;
+    }
+}
+
+// First pass over pairs of a flat parent array (every entry at its root), by one warp over its own
+// part q[0 .. n) of the pairs ((a << 16) | b): pairs of one root are dropped, the others hook the larger
+// root under the smaller (atomicMin) and stay, as roots, at the front of q; returns how many.  A hook
+// can be overwritten by another one, and can land on an entry hooked meanwhile, so after a barrier the
+// pairs that stay are merged for good (smerge) -- by then most are one set already.
+__device__ __forceinline__ uint32_t shook_pairs(uint32_t *P, uint32_t *q, uint32_t n)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t kept = 0;
+    for (uint32_t k = 0; k < n; k += 32) {
+        uint32_t x = 0, y = 0;
+        if (k + lane < n) {
+            const uint32_t e = q[k + lane];
+            x = P[e >> 16];
+            y = P[e & 0xFFFFu];
+        }
+        const uint32_t keep = __ballot_sync(0xFFFFFFFFu, x != y);   // (the pairs of this turn are read)
+        if (x != y) {
+            atomicMin(&P[max(x, y)], min(x, y));
+            q[kept + __popc(keep & ((1u << lane) - 1u))] = (x << 16) | y;
+        }
+        kept += __popc(keep);
+    }
+    __syncwarp();
+    return kept;
+}
+
 // Appends this lane's `n` merge pairs to a shared queue with one atomic per warp; returns the
 // lane's first position (positions >= capacity mean the queue is full for those pairs).
 __device__ __forceinline__ uint32_t warp_reserve(uint32_t *count, uint32_t n)
@@ -211,7 +259,7 @@ __device__ __forceinline__ unsigned long long gentry(uint32_t key, uint32_t id)
 // stands on a root, which is linked (CAS) under the other side's parent -- a node of b's set with
 // a smaller key.  A walk that reaches the common ancestor stops there instead of going on to both
 // roots.  Latency, not work, is the cost: each step is one L2 round trip, and one load gives the
-// parent and its key.  on_link(key) is called with the key of the root that was linked.  (Rem's
+// parent and its key.  on_link(node, key) is called with the root that was linked and its key.  (Rem's
 // splicing -- re-pointing the climbing node at the other side's parent -- was measured: it merged
 // the long paths of one-pixel spirals into deep trees.)
 template <typename OnLink>
@@ -229,7 +277,7 @@ __device__ __forceinline__ void gunion_keyed(unsigned long long *gp, uint32_t a,
         if (pa == a) {   // a root
             const unsigned long long old = atomicCAS(gp + a, ea, eb);
             if (old == ea) {
-                on_link(uint32_t(ea >> 32));
+                on_link(a, uint32_t(ea >> 32));
                 return;
             }
             ea = old;
@@ -241,23 +289,6 @@ __device__ __forceinline__ void gunion_keyed(unsigned long long *gp, uint32_t a,
         a = pa;
         ea = ga;
     }
-}
-
-// Find with path halving after all merges of the launch are complete: no link can happen any more,
-// so every pointer stored is to an ancestor and any interleaving of the stores keeps the trees
-// valid.  The cap only bounds the walk should the forest ever hold a cycle (it cannot).
-__device__ __forceinline__ uint32_t gfind_halve(unsigned long long *gp, uint32_t a)
-{
-    volatile unsigned long long *vp = gp;
-    unsigned long long e = vp[a];
-    for (int it = 0; uint32_t(e) != a && it < (1 << 24); ++it) {
-        const uint32_t p = uint32_t(e);
-        const unsigned long long g = vp[p];
-        if (uint32_t(g) != p) vp[a] = g;
-        a = p;
-        e = g;
-    }
-    return a;
 }
 
 // Root of node x after all merges of the launch are complete, by pointer jumping that writes only
@@ -449,6 +480,42 @@ __device__ __forceinline__ void row_bits(const uint8_t *p, int n, const uint8_t 
     const int nl = (n + 1) >> 1, nr = n >> 1;   // valid left / right pixels
     left &= 0xFFFFFFFFu >> (32 - nl);
     right &= nr ? 0xFFFFFFFFu >> (32 - nr) : 0u;
+}
+
+// Stores one row's labels from a group of W neighbouring lanes, lane g holding the four pixels
+// v of the row at dst (n of them, 0..4, are inside the row; a lane's are full before the next
+// lane has any), with aligned 16-byte stores whatever the row's alignment: when dst is m elements
+// past a 16-byte boundary, each lane stores the quad of the m last pixels of the lane before it
+// and its own first 4 - m; the group's ends and the row's end are stored pixel by pixel.  Every
+// lane of the warp calls this (dst & 15 is the same over a group).
+template <int W>
+__device__ __forceinline__ void store_row(int32_t *dst, int4 v, int n)
+{
+    const uint32_t m = uint32_t(reinterpret_cast<uintptr_t>(dst) >> 2) & 3u;
+    const int py = __shfl_up_sync(0xFFFFFFFFu, v.y, 1, W), pz = __shfl_up_sync(0xFFFFFFFFu, v.z, 1, W);
+    const int pw = __shfl_up_sync(0xFFFFFFFFu, v.w, 1, W), pn = __shfl_up_sync(0xFFFFFFFFu, n, 1, W);
+    const int g = int(threadIdx.x) & (W - 1);
+    int4 q = v;
+    if (m == 1) q = make_int4(pw, v.x, v.y, v.z);
+    else if (m == 2) q = make_int4(pz, pw, v.x, v.y);
+    else if (m == 3) q = make_int4(py, pz, pw, v.x);
+    const int have = g ? max(0, pn - (4 - int(m))) : 0;          // pixels of the lane before in the quad
+    int32_t *d = dst - m;
+    if (have == int(m) && n >= 4 - int(m)) {
+        __stcs(reinterpret_cast<int4 *>(d), q);
+    } else {
+        const int b = g ? 0 : int(m), e = n > 0 ? int(m) + min(n, 4 - int(m)) : have;   // elements [b, e) of the quad
+        if (b <= 0 && 0 < e) d[0] = q.x;
+        if (b <= 1 && 1 < e) d[1] = q.y;
+        if (b <= 2 && 2 < e) d[2] = q.z;
+        if (b <= 3 && 3 < e) d[3] = q.w;
+    }
+    if (g == W - 1 && m) {   // the group's last lane: its own pixels past its quad
+        const int b = 4 - int(m);
+        if (b <= 1 && 1 < n) dst[1] = v.y;
+        if (b <= 2 && 2 < n) dst[2] = v.z;
+        if (b <= 3 && 3 < n) dst[3] = v.w;
+    }
 }
 
 // Programmatic dependent launch (sm_90 and later).  A launch made with programmatic stream

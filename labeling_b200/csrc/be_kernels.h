@@ -9,6 +9,7 @@
 #define T2_TBH 32
 #define T2_NPERIM (2 * (T2_TBW + T2_TBH))
 #define T2_MAXB T2_NPERIM
+#define T2_LAB_BYTES (T2_TBW * T2_TBH / 32 * 8 * 4 + T2_TBW * T2_TBH * 2)
 
 // 3D tile: 8 x 16 x 32 blocks = 16 x 32 x 64 voxels (d0, d1, d2).
 #define T3_TB0 8

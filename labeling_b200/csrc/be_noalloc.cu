@@ -31,9 +31,9 @@ constexpr size_t al256(size_t v) { return (v + 255) / 256 * 256; }
 
 // Upper bound of layout_work() for kMaxTiles / kMaxSegs / one image (checked at set-up).
 constexpr size_t kScratchBytes =
-    al256(kMaxTiles * T2_TBW * T2_TBH * 2) +                      // block labels
+    al256(kMaxTiles * T2_LAB_BYTES) +                             // tile words and run entries
     al256(kMaxTiles * T2_NPERIM * 2) +                            // border entries
-    al256(kMaxTiles * (2 * T2_TBH) * (2 * T2_TBW / 32) * 4) +     // root bitmaps
+    al256(kMaxTiles * T2_TBH * T2_TBW / 8) +                      // root bitmaps
     al256(kMaxTiles * 4) +                                        // node counts
     al256(kMaxTiles * T2_MAXB * 8) +                              // union-find entries
     al256(kMaxTiles * T2_MAXB * 2) +                              // root block

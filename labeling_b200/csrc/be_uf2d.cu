@@ -5,33 +5,26 @@
 // Replaces the reference's LBEQ2_Init / LBEQ2_Scan / LBEQ2_Analyze / LBEQ2_SetFinalLabels
 // (LabelingAlgs.cl:176-319) and their host loop (LabelingAlgs.cpp:989-1084) with four launches:
 //
-//   k_tile_local_2d   one CTA per 64x256-pixel tile: 16-byte coalesced loads, 2x2 block masks,
-//                     runs of blocks and their links by bit operations; each run's first link
-//                     becomes its parent by a plain store (a forest), the other links are
-//                     atomicMin unions in shared memory (smaller key wins), then every run start
-//                     walks to its root;
-//                     write one uint16 per block = (mask << 12) | tile-local root block; count
-//                     roots per segment; mark each component's first pixel in the tile's root
-//                     bitmap; export border components as nodes.
+//   k_tile_local_2d   one CTA per 64x256-pixel tile: 16-byte loads, 2x2 block masks, runs of blocks
+//                     and their links by bit operations; runs numbered in the order of their first
+//                     pixels; each run's first link becomes its parent by a plain store (a forest),
+//                     the other links are unions in shared memory (smaller number wins); writes
+//                     the tile's bit words, the root run of every run, a bitmap of the root runs and
+//                     the root count per segment, and exports border components as nodes.
 //   k_merge_2d        unions nodes across tile borders (global union-find after Rem's
 //                     algorithm, smaller key wins); every root that gets linked leaves its segment
 //                     count and its root bitmap.
 //   k_scan_flatten_2d single-pass exclusive scan of the segment counts (be_scan.cuh) and, in
 //                     the same launch, every linked node pointed at its global root (pointer
 //                     jumping).
-//   k_tile_write_2d   one CTA per tile: resolves each block's canonical label and writes the int32
-//                     labels with 16-byte stores.
+//   k_tile_write_2d   one CTA per tile: the label of every run, then the int32 labels with 16-byte
+//                     stores.
 //
-// Canonical numbering.  A block's key is the raster index of its first foreground pixel.  Blocks
-// are merged so that every component is rooted at its smallest key, i.e. at its first pixel in
-// raster order; its label is 1 + the number of component roots that precede that pixel.  The root
-// counts per segment (image row x tile column) and their exclusive prefix give that number.
-//
-// Shared-memory union-find slots.  Within a tile the union-find runs over "slots" whose order is
-// the key order: slot = r * 2*TBW + t * TBW + c for the block in block-row r, block-column c,
-// where t = 0 when the block has a foreground pixel in its top pixel row and 1 otherwise.  Its
-// first pixel is in pixel row 2r + t, so slot order equals raster order of first pixels, and the
-// atomicMin union keeps the first pixel's block as the root.
+// Canonical numbering.  A component's label is 1 + the number of components whose first pixel in
+// raster order precedes its own.  Within a segment -- the part of a pixel row in one tile -- runs are
+// numbered in the order of their first pixels, and a component's root is the run of its first
+// pixel, so the label is the exclusive prefix of the segments' root counts plus the rank of the root's
+// bit among the segment's bits: no pixel positions are stored or sorted.
 #include "be_common.cuh"
 #include "be_kernels.h"
 #include "be_scan.cuh"

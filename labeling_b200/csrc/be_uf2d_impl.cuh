@@ -8,29 +8,21 @@ constexpr int NBLK = TBW * TBH;                    // blocks per tile (4096)
 constexpr int NPERIM = 2 * (TBW + TBH);            // border positions per tile
 constexpr int MAXB = NPERIM;                       // nodes per tile
 constexpr int WPR = TBW / 32;                      // 32-block words per block row
-constexpr int K1_NT = TBH * WPR;                   // one thread per (block row, word) = NBLK / 32
-constexpr int MQCAP = 608;                         // union-queue capacity (more take further rounds)
-constexpr uint32_t kPass = 0xFFFFu;                // "no run start" in the carry scan
+constexpr int NWORD = NBLK / 32;                   // words per tile
+constexpr int K1_NT = NWORD;                       // one thread per (block row, word)
+constexpr int K1_PER_SM = 7;                       // resident tile CTAs per SM (26 KB of shared memory, 72 registers)
+constexpr int MQCAP = 1024;                        // union-queue capacity (more take further rounds)
+constexpr int RBWORDS = NBLK / 32;                 // root-bitmap words per tile: a bit per run
+// A tile's labels as the write kernel reads them (Work::lab): for each of its 32-block words the four
+// pixel-class words (uint4) and the run words (uint4: starts of the runs with a top pixel, of the
+// others, blocks of the former, runs of either kind before the word), then for every run of the
+// tile its component's root run (uint16, at most NBLK).
+constexpr int kHdr = 8 * NWORD;
+constexpr int kLabWords = kHdr + NBLK / 2;
 
-static_assert(NBLK <= 4096, "tile-local block index must fit 12 bits");
+static_assert(NBLK <= 4096, "a run number must fit 12 bits");
 static_assert(MAXB < 4096, "node index must fit 12 bits");
-static_assert(K1_NT == NBLK / 32 && (WPR & (WPR - 1)) == 0 && WPR <= 32, "thread layout");
-
-// Union-find slot order of a block: r*2*TBW + t*TBW + c with t = 0 when the block has a pixel in
-// its top row.  The order is the raster order of the blocks' first pixels, so the smallest slot
-// of a component is the block holding its first pixel.  Mask bits: 0 = top-left, 1 = top-right,
-// 2 = bottom-left, 3 = bottom-right pixel.
-__device__ __forceinline__ uint32_t key_block(uint32_t key)
-{
-    return (key / (2 * TBW)) * TBW + (key % TBW);
-}
-
-// Pixel offset (row, column) of a block's first foreground pixel, inside the block.
-__device__ __forceinline__ void first_px(uint32_t m, int &dy, int &dx)
-{
-    if (m & 3u) { dy = 0; dx = (m & 1u) ? 0 : 1; }
-    else { dy = 1; dx = (m & 4u) ? 0 : 1; }
-}
+static_assert(K1_NT == 128 && (WPR & (WPR - 1)) == 0 && WPR <= 32, "thread layout");
 
 // Block position of border position p of a tile with nbr x nbc valid blocks.
 __device__ __forceinline__ bool perim_pos(int p, int nbr, int nbc, int &r, int &c)
@@ -42,76 +34,27 @@ __device__ __forceinline__ bool perim_pos(int p, int nbr, int nbc, int &r, int &
     return r < nbr;
 }
 
-// Bits 0..3 of x -> bit 0 of bytes 0..3.
-__device__ __forceinline__ uint32_t spread4(uint32_t x) { return ((x & 0xFu) * 0x00204081u) & 0x01010101u; }
-
 // Highest set bit of x (x != 0).
 __device__ __forceinline__ uint32_t hibit(uint32_t x) { return 31u - __clz(x); }
 
-// Shared-memory position of block x's union-find entry: the low five bits are XOR-ed with the
-// block's 32-block word, so that the 32 lanes of a warp -- 32 different words walking the same
-// bit position -- reach 32 different banks.  Entries still name blocks by their plain index.
-__device__ __forceinline__ uint32_t sw(uint32_t x) { return x ^ ((x >> 5) & 31u); }
+// Global keys.  A component is known by (segment, place of its root run among the segment's runs):
+// segments -- the part of one pixel row that lies in one tile -- are numbered in raster order, and a
+// tile numbers the runs of a segment by their first pixel, so key = segment * seg_width + place orders
+// components as their first pixels do.  A segment has at most seg_width runs, every two of them with
+// a background pixel between, so keys stay below 2^31 with the pixel count.
+__device__ __forceinline__ uint32_t seg_width(const Img2D &im) { return uint32_t(min(im.cols, TW) + 1) >> 1; }
 
-// Union-find over run starts with the slot order carried in the parent entry: P[x] holds
-// (slot << 12) | parent, and a root holds its own (slot << 12) | x.  Entries only ever decrease,
-// so the union (atomicMin of the smaller encoding into the other root, Playne-Hawick style)
-// leaves the run with the smallest slot -- the component's first pixel -- as the root.
-__device__ __forceinline__ uint32_t efind(uint32_t *P, uint32_t x)
+// Set bits of the bitmap b in positions [lo, hi).
+__device__ __forceinline__ uint32_t count_bits(const uint32_t *b, uint32_t lo, uint32_t hi)
 {
-    uint32_t v = P[sw(x)];
-    while ((v & 0xFFFu) != x) {
-        const uint32_t y = v & 0xFFFu;
-        const uint32_t vg = P[sw(y)];
-        if ((vg & 0xFFFu) != y) P[sw(x)] = vg;   // path halving
-        x = y;
-        v = vg;
+    uint32_t n = 0;
+    for (uint32_t i = lo >> 5; 32 * i < hi; ++i) {
+        uint32_t x = __ldcg(b + i);
+        if (i == lo >> 5) x &= ~0u << (lo & 31u);
+        if (32 * i + 32 > hi) x &= (1u << (hi & 31u)) - 1u;
+        n += __popc(x);
     }
-    return x;
-}
-
-__device__ __forceinline__ uint32_t efind_ro(const uint32_t *P, uint32_t x)
-{
-    uint32_t v = P[sw(x)];
-    while ((v & 0xFFFu) != x) {
-        x = v & 0xFFFu;
-        v = P[sw(x)];
-    }
-    return x;
-}
-
-// As efind, also returning the root's own entry as read (the union compares the two).
-__device__ __forceinline__ uint32_t efind_e(uint32_t *P, uint32_t x, uint32_t &ev)
-{
-    uint32_t v = P[sw(x)];
-    while ((v & 0xFFFu) != x) {
-        const uint32_t y = v & 0xFFFu;
-        const uint32_t vg = P[sw(y)];
-        if ((vg & 0xFFFu) != y) P[sw(x)] = vg;
-        x = y;
-        v = vg;
-    }
-    ev = v;
-    return x;
-}
-
-__device__ __forceinline__ void eunion(uint32_t *P, uint32_t a, uint32_t b)
-{
-    for (;;) {
-        uint32_t ea, eb;
-        a = efind_e(P, a, ea);
-        b = efind_e(P, b, eb);
-        if (a == b) return;
-        if (ea < eb) {
-            const uint32_t old = atomicMin(&P[sw(b)], ea);
-            if ((old & 0xFFFu) == b) return;
-            b = old & 0xFFFu;
-        } else {
-            const uint32_t old = atomicMin(&P[sw(a)], eb);
-            if ((old & 0xFFFu) == a) return;
-            a = old & 0xFFFu;
-        }
-    }
+    return n;
 }
 
 }  // namespace
@@ -120,31 +63,35 @@ __device__ __forceinline__ void eunion(uint32_t *P, uint32_t a, uint32_t b)
 // Tile-local labeling.  One thread per 32 blocks of a block row (a "word"): the four pixel
 // classes of the blocks (top-left, top-right, bottom-left, bottom-right) are 32-bit words, so
 // horizontal runs of joined blocks, their starts and the links to the row above are bitwise
-// operations; only runs enter the union-find, and only links between runs that no earlier link
-// already joins are merged.
+// operations.  Runs are numbered 0.. over the tile in the raster order of their first pixels: row by
+// row, in a row the runs with a top pixel ("T runs") first, then those without ("B runs"), each by
+// column.  So the run of a block is `runs of its kind before the word + starts of its kind in the
+// word up to the block - 1` -- one popc, no search -- and the union-find over run numbers in shared
+// memory, where the smaller number wins, leaves the run of a component's first pixel as its root.
+// The loops over runs and links are shared evenly by the CTA's threads, and the tile is handed on as
+// bit words and one number per run, not as an entry per block.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
+__global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L, Work w)
 {
     grid_dep_release();   // the merge launch may take free SMs during this grid's last wave
     if (blockIdx.x == 0 && threadIdx.x == 0) {   // a new epoch for the segment scan of this run
         w.epoch[0] += 1u;
         w.epoch[1] = 0u;
     }
-    __shared__ uint32_t P[NBLK];            // run starts: (slot << 12) | parent
-    __shared__ __align__(16) uint8_t M[NBLK];
-    __shared__ uint32_t WBL[NBLK / 32], WBR[NBLK / 32], WHC[NBLK / 32], WS[NBLK / 32], WCS[NBLK / 32];
-    __shared__ uint32_t RB[TH][TW / 32];
-    __shared__ uint32_t BF[NBLK / 32];
-    __shared__ uint32_t MQ[MQCAP];          // union queue: (block_a << 16) | block_b
-    static_assert(MQCAP >= NBLK / 32, "the node numbering reuses the queue's memory");
-    uint32_t *const BP = MQ;                // node numbering per 32 blocks (after the unions)
+    __shared__ __align__(16) uint32_t P[NBLK];   // per run: parent run
+    __shared__ __align__(16) uint4 CW[NWORD];    // class words: TL, TR, BL, BR
+    __shared__ __align__(16) uint4 WR[NWORD];    // T starts, B starts, blocks of T runs, T | B << 16 runs before
+    __shared__ uint32_t WHC[NWORD];              // joins to the right
+    __shared__ uint32_t MQ[MQCAP];               // union queue: (run_a << 16) | run_b
+    __shared__ uint32_t BF[NWORD];               // runs that are border components
+    __shared__ uint32_t BP[NWORD];               // runs that are roots; then nodes before each word of BF
     __shared__ uint32_t mqn;
-    __shared__ uint32_t tmp[K1_NT / 32 + 1];
+    __shared__ uint32_t wtot[K1_NT / 32], ntot[K1_NT / 32];   // run starts / nodes per warp
     __shared__ uint32_t qslot;
 
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r = tid / WPR, q = tid % WPR;
-    uint16_t *lab = reinterpret_cast<uint16_t *>(w.lab);
+    uint32_t *lab = reinterpret_cast<uint32_t *>(w.lab);
     ItemLoop loop{w.queue ? w.queue + 0 : nullptr, w.n_tiles};
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
         const Img2D im = L.get(t);
@@ -156,11 +103,12 @@ __global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
         const uint32_t K = (0x7Fu - (uint32_t(im.thr) & 0x7Fu)) * 0x01010101u;
         const bool hi = im.thr >= 128;
 
-        for (int i = tid; i < TH * (TW / 32); i += K1_NT) (&RB[0][0])[i] = 0;
-        BF[tid] = 0;
         if (tid == 0) mqn = 0;
+        BF[tid] = 0;
+        for (int i = tid; i < NBLK / 4; i += K1_NT)   // every run its own root
+            reinterpret_cast<uint4 *>(P)[i] = make_uint4(4 * i, 4 * i + 1, 4 * i + 2, 4 * i + 3);
 
-        // Phase A: pixel words, runs, run starts and their slots.
+        // Phase A: pixel words, runs, run starts.
         uint32_t TLw = 0, TRw = 0, BLw = 0, BRw = 0;
         if (r < nbr && 64 * q < ncp) {
             const uint8_t *row0 = im.in + int64_t(y0 + 2 * r) * im.in_pitch + x0 + 64 * q;
@@ -196,7 +144,7 @@ __global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
                 if (row1) row_bits(row0 + im.in_pitch, n, im.in, hi_px, K, hi, im.thr, BLw, BRw);
             }
         }
-        const uint32_t Lw = TLw | BLw, Rw = TRw | BRw, Tw = TLw | TRw, Fw = Tw | BLw | BRw;
+        const uint32_t Lw = TLw | BLw, Rw = TRw | BRw, Tw = TLw | TRw;
         // hc bit k: block k is joined to block k + 1 (a right pixel of k touches a left pixel of
         // k + 1 -- every such pair is 8-adjacent); bit 31 looks at the next word.
         const uint32_t Lnext = __shfl_down_sync(0xFFFFFFFFu, Lw, 1, WPR);
@@ -204,62 +152,85 @@ __global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
         const uint32_t hcprev = __shfl_up_sync(0xFFFFFFFFu, hc, 1, WPR);
         const uint32_t cin = q > 0 ? (hcprev >> 31) : 0u;   // block 0 continues a run from the left
         const uint32_t hl = (hc << 1) | cin;                  // bit k: block k joined to block k - 1
-        const uint32_t S = Fw & ~hl;                          // run starts
-        // Column of the start of the run entering from the left: the last start among the words
-        // before this one (an inclusive "last start" scan over the row's words).
-        uint32_t v = S ? uint32_t(32 * q) + hibit(S) : kPass;
-#pragma unroll
-        for (int o = 1; o < WPR; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, v, o, WPR);
-            if (q >= o && v == kPass) v = u;
-        }
-        const uint32_t vprev = __shfl_up_sync(0xFFFFFFFFu, v, 1, WPR);
-        const uint32_t CSc = cin ? vprev : kPass;
-        const uint32_t rbase = uint32_t(r) * TBW, sbase = uint32_t(r) * (2 * TBW);
-
-        // Block masks as bytes (for the first-pixel lookups and the border entries).
-        uint32_t mw[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int k = 4 * i;
-            mw[i] = spread4(TLw >> k) | (spread4(TRw >> k) << 1) | (spread4(BLw >> k) << 2) |
-                    (spread4(BRw >> k) << 3);
-        }
+        const uint32_t S = (Lw | Rw) & ~hl;                   // run starts
+        // T runs: the starts whose run has a top pixel.  Within the word, from each top pixel a carry
+        // runs down (in reversed bits) to the start it belongs to.  A run that goes on past its word
+        // with no top pixel yet takes it from the words it goes on into.
+        uint32_t ST, CT;
         {
-            uint4 *mdst = reinterpret_cast<uint4 *>(&M[rbase + 32 * q]);
-            mdst[0] = make_uint4(mw[0], mw[1], mw[2], mw[3]);
-            mdst[1] = make_uint4(mw[4], mw[5], mw[6], mw[7]);
-        }
-        WBL[tid] = BLw;
-        WBR[tid] = BRw;
-        WHC[tid] = hc;
-        WS[tid] = S;
-        WCS[tid] = CSc;
-        // Slot keys across words: a run that goes on into later words of its row takes its slot
-        // from the first top pixel there when its own part has none.  Each word reports the first
-        // top pixel of the run carried into it (0xFF: none) and whether that run also goes on past
-        // the word (0x100); the word holding the run's start reads them with shuffles inside the
-        // row's lanes, so every slot is complete when it is first written.
-        const uint32_t cbrk = ~hc;
-        const uint32_t ctm = cin ? (Tw & ((2u << (cbrk ? uint32_t(__ffs(cbrk) - 1) : 31u)) - 1u)) : 0u;
-        const uint32_t mine = (ctm ? uint32_t(32 * q + __ffs(ctm) - 1) : 0xFFu) | ((cin && !cbrk) ? 0x100u : 0u);
-        uint32_t tail = 0xFFu;   // first top pixel of this word's last run in the words after it
-        {
-            bool open = (hc >> 31) & 1u;   // the word's last run goes on into the next word
+            const uint32_t rS = __brev(S), rT = __brev(Tw);
+            ST = __brev(((~rS + (rT & ~rS)) | rT) & rS);
+            const uint32_t cm = (S & (0u - S)) - 1u;   // blocks before the word's first start
+            const uint32_t mine = ((cin && (Tw & cm)) ? 1u : 0u) | ((cin && !S && (hc >> 31)) ? 2u : 0u);
+            const uint32_t last = S ? 0x80000000u >> __clz(S) : 0u;
+            bool open = last && (hc >> 31) && !(ST & last);
 #pragma unroll
             for (int d = 1; d < WPR; ++d) {
                 const uint32_t pj = __shfl_down_sync(0xFFFFFFFFu, mine, d, WPR);
                 if (open && q + d < WPR) {
-                    if ((pj & 0xFFu) != 0xFFu) {
-                        tail = pj & 0xFFu;
-                        open = false;
-                    } else if (!(pj & 0x100u)) {
-                        open = false;
-                    }
+                    if (pj & 1u) ST |= last;
+                    open = pj == 2u;
                 }
             }
+            // Blocks of T runs: from each T start up to the next start; a run carried in has the kind
+            // of the last start before the word.
+            uint32_t v = S ? 2u | ((ST & last) ? 1u : 0u) : 0u;
+#pragma unroll
+            for (int o = 1; o < WPR; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, v, o, WPR);
+                if (q >= o && !v) v = u;
+            }
+            const uint32_t vp = __shfl_up_sync(0xFFFFFFFFu, v, 1, WPR);
+            uint32_t pr = ~S;
+            CT = ST | (q > 0 ? vp & pr & 1u : 0u);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                CT |= (CT << o) & pr;
+                pr &= pr << o;
+            }
         }
+        const uint32_t SB = S & ~ST;
+        // Runs before this word: in its row (T runs in the low half, B runs in the high half), and in
+        // the rows before it -- over the warp here, the warps' totals are added after the barrier.
+        uint32_t bTB, rowsum;
+        {
+            const uint32_t c = __popc(ST) | (__popc(SB) << 16);
+            uint32_t x = c;
+#pragma unroll
+            for (int o = 1; o < WPR; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, x, o, WPR);
+                if (q >= o) x += u;
+            }
+            const uint32_t row = __shfl_sync(0xFFFFFFFFu, x, WPR - 1, WPR);
+            const uint32_t rt = (row & 0xFFFFu) + (row >> 16);
+            rowsum = rt;
+#pragma unroll
+            for (int o = WPR; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, rowsum, o);
+                if (lane >= o) rowsum += u;
+            }
+            bTB = x - c + (row << 16) + (rowsum - rt) * 0x10001u;   // B runs follow the row's T runs
+        }
+        if (lane == 31) wtot[warp] = rowsum;
+        CW[tid] = make_uint4(TLw, TRw, BLw, BRw);
+        WR[tid] = make_uint4(ST, SB, CT, bTB);
+        WHC[tid] = hc;
         __syncthreads();   // words of every row written
+        uint32_t woff = 0, nrun = 0, uoff = 0;
+#pragma unroll
+        for (int i = 0; i < K1_NT / 32; ++i) {
+            const uint32_t n = wtot[i];
+            if (i < warp) woff += n;
+            if (i < int(uint32_t(tid - WPR) >> 5)) uoff += n;
+            nrun += n;
+        }
+        bTB += woff * 0x10001u;
+        const uint32_t bT = bTB & 0xFFFFu, bB = bTB >> 16;   // T, B runs numbered before this word's
+        {
+            uint4 *h = reinterpret_cast<uint4 *>(lab + t * kLabWords);
+            h[tid] = make_uint4(TLw, TRw, BLw, BRw);
+            h[NWORD + tid] = make_uint4(ST, SB, CT, bTB);
+        }
 
         // Phase B: links to the block row above.  For block b of this row: N (straight up, a top
         // pixel over a bottom pixel), NW (top-left pixel to the bottom-right pixel of b - 1 above)
@@ -267,21 +238,36 @@ __global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
         // earlier link (further left, or N before NW / NE at the same block) joins the same two
         // runs; every chain of such reasons ends at a link that is kept.
         uint32_t Nm = 0, NWm = 0, NEm = 0;
-        if (r > 0 && r < nbr) {
+        uint32_t uST = 0, uSB = 0, ubTB = 0;              // the word above: starts, runs before
+        uint32_t uC = 0, uCl = 0, uCr = 0, uSn = 0;       // kind of the block above, above left, above right
+        const bool above = r > 0 && r < nbr;
+        if (above) {
             const int u = tid - WPR;   // same word, row above
-            const uint32_t uBL = WBL[u], uBR = WBR[u];
-            const uint32_t uBRp = q > 0 ? WBR[u - 1] >> 31 : 0u;
-            const uint32_t uBLn = q + 1 < WPR ? WBL[u + 1] & 1u : 0u;
-            const uint32_t N = Tw & (uBL | uBR);
-            const uint32_t NW = TLw & ((uBR << 1) | uBRp);
-            const uint32_t NE = TRw & ((uBL >> 1) | (uBLn << 31));
-            Nm = N; NWm = NW; NEm = NE;
+            const uint32_t uBL = CW[u].z, uBR = CW[u].w;
+            const uint32_t uBRp = q > 0 ? CW[u - 1].w >> 31 : 0u;
+            const uint32_t uBLn = q + 1 < WPR ? CW[u + 1].z & 1u : 0u;
+            const uint4 ur = WR[u];
+            uST = ur.x;
+            uSB = ur.y;
+            uC = ur.z;
+            ubTB = ur.w + uoff * 0x10001u;
+            uCl = uC << 1;
+            uCr = uC >> 1;
+            if (q > 0) uCl |= WR[u - 1].z >> 31;
+            if (q + 1 < WPR) {
+                const uint4 un = WR[u + 1];
+                uCr |= un.z << 31;
+                uSn = (un.x | un.y) & 1u;   // a run starts at the next word's first block
+            }
+            Nm = Tw & (uBL | uBR);
+            NWm = TLw & ((uBR << 1) | uBRp);
+            NEm = TRw & ((uBL >> 1) | (uBLn << 31));
         }
         {
             // bit 31 of the previous word's raw N / NE, for the rules at block 0
             const uint32_t Np = __shfl_up_sync(0xFFFFFFFFu, Nm, 1, WPR);
             const uint32_t NEp = __shfl_up_sync(0xFFFFFFFFu, NEm, 1, WPR);
-            if (r > 0 && r < nbr) {
+            if (above) {
                 const int u = tid - WPR;
                 const uint32_t uhc = WHC[u];
                 const uint32_t uhl = (uhc << 1) | (q > 0 ? WHC[u - 1] >> 31 : 0u);
@@ -293,166 +279,122 @@ __global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
                 NEm = NE & ~((N & uhc) | (hl & NEsh & uhc));
             }
         }
-        // The run start of a block: a start in the block's word at or before it, else the start
-        // carried in from the left.
-        auto start_of = [&](uint32_t blk) -> uint32_t {
-            const uint32_t m = WS[blk >> 5] & ((2u << (blk & 31u)) - 1u);
-            const uint32_t st = m ? (blk & ~31u) + hibit(m) : (blk & ~uint32_t(TBW - 1)) + WCS[blk >> 5];
-            // A start of this tile by construction; the mask only keeps a broken invariant
-            // from leaving the array.
-            (void)GUARD(w, st < uint32_t(NBLK), 112, (uint64_t(blk) << 32) | st);
-            return st & (NBLK - 1);
+        // Takes one kept link of block b off the masks (N, else NW, else NE): its two runs.
+        auto take = [&](uint32_t b, uint32_t &own, uint32_t &up) {
+            const uint32_t bit = 1u << b, upto = (bit << 1) - 1u;
+            const bool tt = CT & bit;
+            own = (tt ? bT : bB) + __popc((tt ? ST : SB) & upto) - 1u;
+            const bool isN = Nm & bit, isW = !isN && (NWm & bit), isE = !isN && !isW;
+            Nm &= isN ? ~bit : ~0u;
+            NWm &= isW ? ~bit : ~0u;
+            NEm &= isE ? ~bit : ~0u;
+            // Blocks of the word above up to the link's (NW at b = 0: none, its block is the last of the
+            // word before; NE at b >= 30: all, at b = 31 and the first block of the word after).
+            const uint32_t m = isN ? upto : isW ? bit - 1u : (bit << 2) - 1u;
+            const bool ut = (isN ? uC : isW ? uCl : uCr) & bit;
+            up = (ut ? ubTB & 0xFFFFu : ubTB >> 16) + __popc((ut ? uST : uSB) & m) + (isE && b == 31u ? uSn : 0u) - 1u;
         };
-        const uint32_t ubase = rbase - TBW + 32 * q, abase = rbase + 32 * q;
-
-        // Every run that starts in this word gets its entry.  A run with a kept link in this word
-        // takes the first one as its parent: the parent is in the row above, whose slots are all
-        // smaller than this row's, so a plain store links it (no atomic, no cycle possible).  Its
-        // entry holds key 0 -- the smallest value, so no atomicMin of a union ever changes it and
-        // unions walk on to the parent; only a root's key is ever compared.  Any other run is a
-        // root for now: (slot << 12) | itself, the slot being its first block with a top pixel
-        // (this word, else the words after it), else its start.  These forest links leave the
-        // queue; the union-find below walks the forest like any other path (path halving), and
-        // the flatten pass compresses it.  (Pointer jumping over the forest first was measured
-        // slower.)
+        // The first link of every run that starts in this word becomes the run's parent by a plain
+        // store: the parent is in the row above, whose numbers are all smaller, so no cycle is
+        // possible and no atomic is needed.  First links by a carry: adding the starts that hold no
+        // link to ~links ripples from each of them to the next link bit and stops there; a start
+        // without any link ripples on into the next start, which absorbs the carry or is itself a link.
         {
-            uint32_t ss = S;
-            while (ss) {
-                const uint32_t s0 = __ffs(ss) - 1;
-                ss &= ss - 1;
-                const uint32_t from = ~0u << s0;
-                const uint32_t brk = ~hc & from;
-                const uint32_t e = brk ? uint32_t(__ffs(brk) - 1) : 31u;
-                const uint32_t span = from & (0xFFFFFFFFu >> (31u - e));
-                const uint32_t lk = (Nm | NWm | NEm) & span;
-                const uint32_t x = abase + s0;
-                if (lk) {
-                    const uint32_t b = __ffs(lk) - 1, bit = 1u << b;
-                    uint32_t tgt;
-                    if (Nm & bit) {
-                        tgt = ubase + b;
-                        Nm &= ~bit;
-                    } else if (NWm & bit) {
-                        tgt = ubase + b - 1;
-                        NWm &= ~bit;
-                    } else {
-                        tgt = ubase + b + 1;
-                        NEm &= ~bit;
-                    }
-                    P[sw(x)] = start_of(tgt);   // key 0
-                } else {
-                    const uint32_t tm = Tw & span;
-                    uint32_t key = sbase + TBW + 32 * q + s0;
-                    if (tm) key = sbase + 32 * q + (__ffs(tm) - 1);
-                    else if (brk == 0 && tail != 0xFFu) key = sbase + tail;
-                    P[sw(x)] = (key << 12) | x;
-                }
+            const uint32_t lk = Nm | NWm | NEm;
+            uint32_t first = lk & ((~lk + (S & ~lk)) | S);
+            while (first) {
+                const uint32_t b = __ffs(first) - 1;
+                first &= first - 1;
+                uint32_t own, up;
+                take(b, own, up);
+                (void)GUARD(w, own < nrun && up < own, 112, (uint64_t(own) << 32) | up);
+                P[own & (NBLK - 1)] = up & (NBLK - 1);
             }
         }
-        // The remaining links are unions.  The queue holds the two blocks of each link; their run
-        // starts are looked up by the merging lanes, which share that work evenly.  Links past the
-        // queue's capacity go in in later rounds.
+        // The remaining links are unions: queued and merged by every lane.
         const uint32_t n = __popc(Nm) + __popc(NWm) + __popc(NEm);
-        const uint32_t pos0 = warp_reserve(&mqn, n);
-        auto each_link = [&](auto &&f) {
-            uint32_t pos = pos0;
-            uint32_t todo = Nm | NWm | NEm;
-            while (todo) {
-                const uint32_t b = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const uint32_t bit = 1u << b;
-                const uint32_t a = abase + b;
-                if (Nm & bit) f(pos++, a, ubase + b);
-                if (NWm & bit) f(pos++, a, ubase + b - 1);   // b = 0: the last block of the word before
-                if (NEm & bit) f(pos++, a, ubase + b + 1);   // b = 31: the first block of the word after
+        uint32_t pos = warp_reserve(&mqn, n);
+        auto push = [&](uint32_t lo, uint32_t end) {   // links at queue positions [lo, end) go in
+            while (pos < end) {
+                const uint32_t b = __ffs(Nm | NWm | NEm);
+                if (!b) break;
+                uint32_t own, up;
+                take(b - 1u, own, up);
+                MQ[pos - lo] = (own << 16) | up;
+                ++pos;
             }
         };
-        if (pos0 < uint32_t(MQCAP))
-            each_link([&](uint32_t pos, uint32_t a, uint32_t b) {
-                if (pos < uint32_t(MQCAP)) MQ[pos] = (a << 16) | b;
-            });
+        push(0u, uint32_t(MQCAP));
         __syncthreads();
-        // Rounds of the queue: the links with positions [base, base + MQCAP) go in, and each thread
-        // takes a contiguous run of them: neighbouring links, mostly of the same rows, are merged
-        // one after another by one thread instead of racing on the same roots.
-        {
-            const uint32_t total = mqn;
-            for (uint32_t base = 0; base < total; base += MQCAP) {
-                if (base) {
-                    if (pos0 + n > base && pos0 < base + MQCAP)
-                        each_link([&](uint32_t pos, uint32_t a, uint32_t b) {
-                            if (pos >= base && pos < base + MQCAP) MQ[pos - base] = (a << 16) | b;
-                        });
-                    __syncthreads();
-                }
-                const uint32_t nq = min(total - base, uint32_t(MQCAP));
-                const uint32_t per = (nq + K1_NT - 1) / K1_NT, lo = min(nq, uint32_t(tid) * per), hi = min(nq, lo + per);
-                for (uint32_t i = lo; i < hi; ++i) eunion(P, start_of(MQ[i] >> 16), start_of(MQ[i] & 0xFFFFu));
+        WR[tid].w = bTB;   // from here on the runs before each word over the whole tile
+        // The forest of first links is as deep as the tile has rows; every run of it is pointed at its
+        // tree's root before the unions, in ascending order, so that a walk meets runs already done.
+        sflatten_all(P, tid, K1_NT, nrun);
+        __syncthreads();
+        // Rounds of the queue, each warp with its quarter.
+        const uint32_t total = mqn;
+        uint32_t kept = 0;
+        for (uint32_t lo = 0; lo < total; lo += MQCAP) {
+            if (lo) {
+                sflatten_all(P, tid, K1_NT, nrun);   // shook_pairs wants every run at its root
+                push(lo, lo + MQCAP);
                 __syncthreads();
             }
+            const uint32_t nq = min(total - lo, uint32_t(MQCAP)), per = (nq + K1_NT / 32 - 1) / (K1_NT / 32);
+            const uint32_t q0 = min(nq, warp * per);
+            kept = shook_pairs(P, MQ + q0, min(nq - q0, per));
+            __syncthreads();
+            for (uint32_t k = lane; k < kept; k += 32) smerge(P, MQ[q0 + k] >> 16, MQ[q0 + k] & 0xFFFFu);
+            __syncthreads();
         }
 
-        // Phase C: every run start of this word is pointed straight at its root (a read-only walk,
-        // then the root's entry stored in the start's own entry; every entry is a run start, so each
-        // is compressed by its own thread, and no link happens any more -- storing the root along
-        // the walked path as well was measured slower: a second dependent walk); roots mark their
-        // first pixel.  Then the block entries: (mask << 12) | root block, two blocks per 32-bit word.
-        {
-            uint32_t ss = S;
-            while (ss) {
-                const uint32_t x = abase + (__ffs(ss) - 1);
-                ss &= ss - 1;
-                uint32_t root = x, ev = P[sw(x)];
-                for (int it = 0; (ev & 0xFFFu) != root && it < NBLK; ++it) {   // acyclic: the cap never binds
-                    root = ev & 0xFFFu;
-                    ev = P[sw(root)];
-                }
-                if (root != x) P[sw(x)] = ev;
-                if (root == x) {
-                    const uint32_t key = ev >> 12;
-                    const uint32_t rb = key_block(key);
-                    int dy, dx;
-                    first_px(M[rb], dy, dx);
-                    const int y = 2 * int(key / (2 * TBW)) + dy, xx = 2 * int(key % TBW) + dx;
-                    atomicOr(&RB[y][xx >> 5], 1u << (xx & 31));
+        // Phase C: what the unions linked is the roots of kept pairs; these are pointed at their roots,
+        // so that every run is at most one step from its own (root_of).  With several rounds of the
+        // queue every run is.  Roots are flagged in bit words.
+        if (total > uint32_t(MQCAP)) {
+            sflatten_all(P, tid, K1_NT, nrun);
+        } else if (total) {
+            const uint32_t per = (total + K1_NT / 32 - 1) / (K1_NT / 32), q0 = min(total, warp * per);
+            for (uint32_t k = lane; k < kept; k += 32) {
+                const uint32_t e = MQ[q0 + k];
+#pragma unroll
+                for (int side = 0; side < 2; ++side) {
+                    const uint32_t i = side ? e & 0xFFFFu : e >> 16;
+                    uint32_t x = i, y = P[i];
+                    while (y != x) {
+                        x = y;
+                        y = P[x];
+                    }
+                    if (x != i) P[i] = x;
                 }
             }
         }
-        {
-            uint32_t cur = 0;
-            if (cin) {   // the run carried in from the left starts in an earlier word of this row
-                uint32_t root = rbase + (CSc & (TBW - 1)), ev = P[sw(root)];
-                for (int it = 0; (ev & 0xFFFu) != root && it < NBLK; ++it) {
-                    root = ev & 0xFFFu;
-                    ev = P[sw(root)];
-                }
-                cur = key_block(ev >> 12);
-            }
-            uint32_t ew[16];
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-                if ((S >> k) & 1u) cur = key_block(P[sw(abase + k)] >> 12);
-                const uint32_t m = (mw[k >> 2] >> (8 * (k & 3))) & 15u;
-                const uint32_t e = m ? (m << 12) | cur : 0u;
-                if (k & 1) ew[k >> 1] |= e << 16;
-                else ew[k >> 1] = e;
-            }
-            uint4 *dst = reinterpret_cast<uint4 *>(lab + t * NBLK + abase);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) dst[i] = make_uint4(ew[4 * i], ew[4 * i + 1], ew[4 * i + 2], ew[4 * i + 3]);
+        for (uint32_t i0 = 32 * warp; i0 < nrun; i0 += K1_NT) {
+            const uint32_t i = i0 + lane;
+            const uint32_t roots = __ballot_sync(0xFFFFFFFFu, i < nrun && P[i] == i);
+            if (lane == 0) BP[i0 >> 5] = roots;
         }
-        __syncthreads();   // root bitmap complete; every run start points at its root
+        __syncthreads();
 
-        // Phase D: root bitmap and segment counts out; border components -> nodes.
-        for (int i = tid; i < TH * (TW / 32); i += K1_NT) w.rbits[t * (TH * (TW / 32)) + i] = (&RB[0][0])[i];
-        if (tid < TH && tid < nrp) {
-            uint32_t cnt = 0;
-#pragma unroll
-            for (int k = 0; k < TW / 32; ++k) cnt += __popc(RB[tid][k]);
-            w.segcnt[im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx] = uint8_t(cnt);
+        // Phase D: every run's root, the tile's root bitmap and the segments' root counts out.
+        auto root_of = [&](uint32_t id) -> uint32_t { return P[P[id & (NBLK - 1)]]; };
+        {
+            uint32_t *rl = lab + t * kLabWords + kHdr;
+            for (uint32_t i = 2 * tid; i < nrun; i += 2 * K1_NT)
+                rl[i >> 1] = root_of(i) | (root_of(i + 1 < nrun ? i + 1 : i) << 16);
         }
-        // Root block of each border position held (plus its mask, and whether this position
-        // claimed the node: the one position that sets the root's bit writes the node's record).
+        w.rbits[t * RBWORDS + tid] = 32u * tid < nrun ? BP[tid] : 0u;
+        if (tid < TH && tid < nrp) {   // runs [s, e) start in pixel row tid
+            const uint32_t b = WR[(tid >> 1) * WPR].w;
+            const uint32_t s = (tid & 1) ? b >> 16 : b & 0xFFFFu;
+            const uint32_t e = !(tid & 1) ? b >> 16 : (tid >> 1) + 1 < TBH ? WR[((tid >> 1) + 1) * WPR].w & 0xFFFFu : nrun;
+            uint32_t c = 0;
+            for (uint32_t i = s >> 5; 32 * i < e; ++i)
+                c += __popc(BP[i] & (i == s >> 5 ? ~0u << (s & 31u) : ~0u) & (32 * i + 32 > e ? (1u << (e & 31u)) - 1u : ~0u));
+            w.segcnt[im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx] = uint8_t(c);
+        }
+        // Border positions: component (root run), mask, and whether this position
+        // claimed the node (the one that sets the component's flag writes the node's record).
         constexpr uint32_t kOwner = 1u << 20;
         uint32_t prb[(NPERIM + K1_NT - 1) / K1_NT];
 #pragma unroll
@@ -461,48 +403,67 @@ __global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
             int br, bc;
             prb[i] = kNone;
             if (p >= NPERIM || !perim_pos(p, nbr, nbc, br, bc)) continue;
-            const uint32_t m = M[br * TBW + bc];
+            const int wi = br * WPR + (bc >> 5), k = bc & 31;
+            const uint4 cw = CW[wi];
+            const uint32_t m = ((cw.x >> k) & 1u) | (((cw.y >> k) & 1u) << 1) | (((cw.z >> k) & 1u) << 2) |
+                               (((cw.w >> k) & 1u) << 3);
             if (!m) continue;
-            const int wi = br * WPR + (bc >> 5);
-            const uint32_t sm = WS[wi] & ((2u << (bc & 31)) - 1u);
-            const uint32_t sc = sm ? uint32_t(bc & ~31) + hibit(sm) : WCS[wi];
-            (void)GUARD(w, sc < uint32_t(TBW), 113, sc);
-            const uint32_t rb = key_block(P[sw(uint32_t(br) * TBW + (sc & (TBW - 1)))] >> 12);
-            const uint32_t bit = 1u << (rb & 31);
-            const uint32_t old = atomicOr(&BF[rb >> 5], bit);
-            prb[i] = rb | (m << 16) | ((old & bit) ? 0u : kOwner);
+            const uint4 wr = WR[wi];
+            const uint32_t upto = (2u << k) - 1u;
+            const uint32_t id = ((wr.z >> k) & 1u ? (wr.w & 0xFFFFu) + __popc(wr.x & upto) : (wr.w >> 16) + __popc(wr.y & upto)) - 1u;
+            (void)GUARD(w, id < nrun, 113, id);
+            const uint32_t c = root_of(id);
+            const uint32_t bit = 1u << (c & 31);
+            const uint32_t old = atomicOr(&BF[c >> 5], bit);
+            prb[i] = c | (m << 16) | ((old & bit) ? 0u : kOwner);
+        }
+        __syncthreads();   // node flags complete
+        {   // nodes before each word of flags, within the warp; the warps' totals beside them
+            const uint32_t c = __popc(BF[tid]);
+            uint32_t x = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= o) x += v;
+            }
+            BP[tid] = x - c;
+            if (lane == 31) ntot[warp] = x;
         }
         __syncthreads();
-        uint32_t nb;
-        const uint32_t pre = block_exscan<K1_NT>(__popc(BF[tid]), tmp, &nb);
-        BP[tid] = pre;
-        __syncthreads();
-            // Every border position writes its entry; the position that claimed its node writes the
+        // Every border position writes its entry; the position that claimed its node writes the
         // node's record.
+        uint32_t noff[K1_NT / 32 + 1];
+        noff[0] = 0;
+#pragma unroll
+        for (int i = 0; i < K1_NT / 32; ++i) noff[i + 1] = noff[i] + ntot[i];
 #pragma unroll
         for (int i = 0; i < (NPERIM + K1_NT - 1) / K1_NT; ++i) {
             const int p = tid + i * K1_NT;
             if (p >= NPERIM) continue;
             uint16_t ent = 0;
             if (prb[i] != kNone) {
-                const uint32_t rb = prb[i] & 0xFFFFu, m = (prb[i] >> 16) & 15u;
-                const uint32_t j = BP[rb >> 5] + __popc(BF[rb >> 5] & ((1u << (rb & 31)) - 1u));
+                const uint32_t c = prb[i] & 0xFFFFu, m = (prb[i] >> 16) & 15u;
+                const uint32_t cw = c >> 5, g = cw >> 5;
+                const uint32_t j = (g == 0 ? noff[0] : g == 1 ? noff[1] : g == 2 ? noff[2] : noff[3]) + BP[cw] +
+                                   __popc(BF[cw] & ((1u << (c & 31)) - 1u));
                 ent = uint16_t((j << 4) | m);
-            }
-            if (prb[i] != kNone && (prb[i] & kOwner)) {
-                const uint32_t rb = prb[i] & 0xFFFFu;
-                const uint32_t j = BP[rb >> 5] + __popc(BF[rb >> 5] & ((1u << (rb & 31)) - 1u));
-                int dy, dx;
-                first_px(M[rb], dy, dx);
-                const int y = 2 * int(rb / TBW) + dy, x = 2 * int(rb % TBW) + dx;
-                const int64_t node = t * MAXB + j;
-                const uint32_t key = uint32_t(int64_t(y0 + y) * im.cols + (x0 + x));
-                w.nroot[node] = uint16_t(rb);
-                w.gp[node] = gentry(key, uint32_t(node));
+                if (prb[i] & kOwner) {
+                    int row = 0;   // the block row of run c
+#pragma unroll
+                    for (int h = TBH / 2; h; h >>= 1)
+                        if ((WR[(row + h) * WPR].w & 0xFFFFu) <= c) row += h;
+                    const uint32_t b = WR[row * WPR].w;
+                    const bool low = c >= b >> 16;   // a run without a top pixel
+                    const uint32_t place = c - (low ? b >> 16 : b & 0xFFFFu);
+                    const int64_t seg = int64_t(y0 + 2 * row + (low ? 1 : 0)) * im.tiles_x + tx;
+                    const int64_t node = t * MAXB + j;
+                    w.nroot[node] = uint16_t(c);
+                    w.gp[node] = gentry(uint32_t(seg) * seg_width(im) + place, uint32_t(node));
+                }
             }
             w.perim[t * NPERIM + p] = ent;
         }
-        if (tid == 0) w.nb[t] = nb;
+        if (tid == 0) w.nb[t] = noff[K1_NT / 32];
         __syncthreads();
     }
 }
@@ -512,23 +473,16 @@ __global__ void __launch_bounds__(K1_NT, 8) k_tile_local_2d(ImgList2D L, Work w)
 // ---------------------------------------------------------------------------------------------
 namespace {
 
-// A root linked under another leaves its segment's root count and the root bitmap of its tile
-// (so that after the merge the bitmaps hold exactly the components' first pixels).
-__device__ __forceinline__ void link_dec(const Img2D &im, Work &w, uint32_t key)
-{
-    const int64_t y = key / uint32_t(im.cols), x = key - y * im.cols;
-    const int64_t ty = y / TH, tx = x / TW;
-    dec_u8(w.segcnt, im.seg_base + y * im.tiles_x + tx);
-    const int ly = int(y - ty * TH), lx = int(x - tx * TW);
-    atomicAnd(w.rbits + (im.tile_base + ty * im.tiles_x + tx) * (TH * (TW / 32)) + ly * (TW / 32) + (lx >> 5),
-              ~(1u << (lx & 31)));
-}
-
 // Union of two nodes of one image; the root with the larger key is linked under the other, and
-// the linked root leaves its segment's root count and its tile's root bitmap.
+// the linked root leaves its segment's root count and its tile's root bitmap (so that after the merge
+// the bitmaps hold exactly the components' root runs).
 __device__ void gunion2d(const Img2D &im, Work &w, uint32_t a, uint32_t b)
 {
-    gunion_keyed(w.gp, a, b, [&](uint32_t key) { link_dec(im, w, key); });
+    gunion_keyed(w.gp, a, b, [&](uint32_t node, uint32_t key) {
+        dec_u8(w.segcnt, im.seg_base + key / seg_width(im));
+        const uint32_t run = w.nroot[node];
+        atomicAnd(w.rbits + int64_t(node / MAXB) * RBWORDS + (run >> 5), ~(1u << (run & 31u)));
+    });
 }
 
 }  // namespace
@@ -735,35 +689,47 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_flatten_2d(Work w)
 // Label resolve and write.
 // ---------------------------------------------------------------------------------------------
 constexpr int K3_NT = 256;
-constexpr int RBWORDS = TH * (TW / 32);   // root-bitmap words per tile
-constexpr int RW = TW / 32;               // root-bitmap words per pixel row
+constexpr int K3_PER_SM = 8;              // resident CTAs per SM
 
-__global__ void __launch_bounds__(K3_NT, 8) k_tile_write_2d(ImgList2D L, Work w)
+__global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L, Work w)
 {
-    __shared__ __align__(16) uint16_t Ls[NBLK];
-    __shared__ uint32_t LT[NBLK];
-    __shared__ uint32_t RB[RBWORDS];
+    __shared__ __align__(16) uint4 H[kHdr / 4];   // class words, then run words
+    __shared__ uint32_t LT[NBLK + 1];     // label of run i at i + 1 (0: the place of "no run yet")
+    constexpr int kStageRuns = 2048;      // run entries staged in shared memory (later ones: from L2)
+    __shared__ __align__(16) uint32_t RB[RBWORDS + 1];
+    __shared__ __align__(16) uint32_t E[kStageRuns / 2];
     __shared__ uint32_t segb[TH];
     __shared__ uint32_t qslot;
 
-    const int tid = threadIdx.x, lane = tid & 31;
-    const uint16_t *lab = reinterpret_cast<const uint16_t *>(w.lab);
-    // Block entries and the root bitmap (first pixels of the components that stayed roots through
+    const int tid = threadIdx.x;
+    const uint32_t *lab = reinterpret_cast<const uint32_t *>(w.lab);
+    // The tile's words and the root bitmap (first pixels of the components that stayed roots through
     // the merge) were final before this grid's predecessor (segment scan and node flatten) started:
     // that grid waits for the merge to complete before it lets this one launch.  So they are read
     // before the wait (through L2), and only the segment prefixes, which the scan writes, after it.
-    // With a fixed tile order (no work queue) the CTA loads the next tile's entries, bitmap and
-    // node count into registers while it writes the current tile's labels.
-    static_assert(NBLK / 8 == 2 * K3_NT && RBWORDS == 2 * K3_NT, "two prefetched words per thread");
-    uint4 nL[2];
-    uint32_t nR[2], nNb = 0;
-    auto fetch = [&](int64_t t) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            nL[i] = __ldcg(reinterpret_cast<const uint4 *>(lab + t * NBLK) + tid + i * K3_NT);
-            nR[i] = __ldcg(w.rbits + t * RBWORDS + tid + i * K3_NT);
-        }
+    // With a fixed tile order (no work queue) the CTA fetches the next tile while it works on the
+    // current one: its words into registers, the root bitmap and run entries into shared memory
+    // (cp.async) as soon as the current tile's are used up.
+    static_assert(TBW % 64 == 0, "a warp's output units lie in one block row");
+    static_assert(kHdr == 4 * K3_NT && 2 * NWORD == K3_NT && kStageRuns == 8 * K3_NT, "prefetched words per thread");
+    uint4 nH;
+    uint32_t nNb = 0;
+    auto fetch_words = [&](int64_t t) {
+        nH = __ldcg(reinterpret_cast<const uint4 *>(lab + t * kLabWords) + tid);
         nNb = __ldcg(w.nb + t);
+    };
+    auto fetch_roots = [&](int64_t t) {
+        if (tid < RBWORDS) cp_async4(&RB[tid], w.rbits + t * RBWORDS + tid);
+        cp_async_commit();
+    };
+    auto fetch_runs = [&](int64_t t) {
+        cp_async16(&E[4 * tid], lab + t * kLabWords + kHdr + 4 * tid);
+        cp_async_commit();
+    };
+    auto fetch = [&](int64_t t) {
+        fetch_words(t);
+        fetch_roots(t);
+        fetch_runs(t);
     };
     const bool fixed_order = w.queue == nullptr;
     ItemLoop loop{w.queue ? w.queue + 4 : nullptr, w.n_tiles};
@@ -776,13 +742,11 @@ __global__ void __launch_bounds__(K3_NT, 8) k_tile_write_2d(ImgList2D L, Work w)
         const int ty = int(lt / im.tiles_x), tx = int(lt - int64_t(ty) * im.tiles_x);
         const int y0 = ty * TH, x0 = tx * TW;
         const int nrp = min(TH, im.rows - y0), ncp = min(TW, im.cols - x0);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            reinterpret_cast<uint4 *>(Ls)[tid + i * K3_NT] = nL[i];
-            RB[tid + i * K3_NT] = nR[i];
-        }
+        H[tid] = nH;
         const uint32_t nb = nNb;
-        if (fixed_order && t + gridDim.x < w.n_tiles) fetch(t + gridDim.x);
+        const int64_t tn = fixed_order && t + gridDim.x < w.n_tiles ? t + gridDim.x : -1;   // next tile
+        if (tn >= 0) fetch_words(tn);
+        cp_async_wait();
         grid_dep_wait();   // segment prefixes from here on (returns at once after the first tile)
         const uint32_t base0 = w.segpref[im.seg_base];
         if (tid < TH && tid < nrp)
@@ -790,25 +754,26 @@ __global__ void __launch_bounds__(K3_NT, 8) k_tile_write_2d(ImgList2D L, Work w)
         if (lt == 0 && tid == 0)
             w.ncomp[im.index] = int64_t(w.segpref[im.seg_base + int64_t(im.rows) * im.tiles_x] - base0);
         __syncthreads();
+        const uint32_t nrun = (H[2 * NWORD - 1].w >> 16) + __popc(H[2 * NWORD - 1].y);   // the last B run is the last run
 
-        // Surviving roots: rank = roots before it in its row segment.  RW consecutive lanes hold
-        // the RW words of one pixel row; a shuffle scan gives each word's prefix.
-        for (int i = tid; i < RBWORDS; i += K3_NT) {
-            const uint32_t word = RB[i];
-            uint32_t pre = __popc(word);
+        // Surviving roots: rank = roots before it in its segment.  One thread per word and kind of run:
+        // WPR consecutive lanes hold a segment's words, a shuffle scan gives each word's prefix, and the
+        // word's runs are consecutive bits of the root bitmap.
+        {
+            const int seg = tid / WPR, wi = (seg >> 1) * WPR + tid % WPR;   // segment = pixel row
+            const uint4 wr = H[NWORD + wi];
+            const uint32_t c = __popc((seg & 1) ? wr.y : wr.x), b = (seg & 1) ? wr.w >> 16 : wr.w & 0xFFFFu;
+            const uint32_t g = b >> 5;   // (RB has a word past its end for g = RBWORDS - 1 and b = NBLK)
+            uint32_t bits = c ? __funnelshift_r(RB[g], RB[min(g + 1, uint32_t(RBWORDS))], b & 31u) & (0xFFFFFFFFu >> (32 - c)) : 0u;
+            uint32_t pre = __popc(bits);
 #pragma unroll
-            for (int o = 1; o < RW; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, pre, o);
-                if ((lane & (RW - 1)) >= o) pre += v;
+            for (int o = 1; o < WPR; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, pre, o, WPR);
+                if (tid % WPR >= o) pre += v;
             }
-            pre -= __popc(word);
-            const int y = i / RW, q = i % RW;
-            const uint32_t base = 1u + segb[y] + pre;
-            uint32_t bits = word;
+            uint32_t label = 1u + segb[seg] + pre - __popc(bits);
             while (bits) {
-                const int b = __ffs(bits) - 1;
-                const int x = 32 * q + b;
-                LT[(y >> 1) * TBW + (x >> 1)] = base + __popc(word & ((1u << b) - 1u));
+                LT[b + __ffs(bits)] = label++;   // run i's place is i + 1
                 bits &= bits - 1;
             }
         }
@@ -816,47 +781,72 @@ __global__ void __launch_bounds__(K3_NT, 8) k_tile_write_2d(ImgList2D L, Work w)
         // segment's prefix plus its rank among the first pixels left in its row of its tile.
         for (uint32_t j = tid; j < nb; j += K3_NT) {
             const int64_t node = t * MAXB + j;
-            if (uint32_t(__ldcg(w.gp + node)) == uint32_t(node)) continue;
-            const uint32_t g = gfind_halve(w.gp, uint32_t(node));
-            const uint32_t kg = uint32_t(__ldcg(w.gp + g) >> 32);
-            const int64_t yg = kg / uint32_t(im.cols), xg = kg - yg * im.cols;
-            const int64_t tyg = yg / TH, txg = xg / TW;
-            const int ly = int(yg - tyg * TH), lx = int(xg - txg * TW);
-            const uint32_t *rw = w.rbits + (im.tile_base + tyg * im.tiles_x + txg) * RBWORDS + ly * RW;
-            uint32_t rank = __popc(__ldcg(rw + (lx >> 5)) & ((1u << (lx & 31)) - 1u));
-            for (int k = 0; k < (lx >> 5); ++k) rank += __popc(__ldcg(rw + k));
-            const uint32_t sb = w.segpref[im.seg_base + yg * im.tiles_x + txg] - base0;
-            LT[__ldcg(w.nroot + node)] = 1u + sb + rank;
+            const unsigned long long e = __ldcg(w.gp + node);   // its root's own entry (flatten_tile_nodes)
+            const uint32_t g = uint32_t(e), kg = uint32_t(e >> 32);
+            if (g == uint32_t(node)) continue;
+            const uint32_t sg = kg / seg_width(im), run = __ldcg(w.nroot + g);
+            const uint32_t rank = count_bits(w.rbits + int64_t(g / MAXB) * RBWORDS, run - (kg - sg * seg_width(im)), run);
+            const uint32_t sb = w.segpref[im.seg_base + sg] - base0;
+            LT[__ldcg(w.nroot + node) + 1u] = 1u + sb + rank;
         }
         __syncthreads();
+        if (tn >= 0) fetch_roots(tn);
+        // Every other run takes the label of its root run.
+        for (uint32_t i = 2 * tid; i < nrun; i += 2 * K3_NT) {
+            const uint32_t e = i < uint32_t(kStageRuns) ? E[i >> 1] : __ldcg(lab + t * kLabWords + kHdr + (i >> 1));
+            const uint32_t a = e & 0xFFFFu, b = e >> 16;
+            if (a != i) LT[i + 1] = LT[a + 1];
+            if (i + 1 < nrun && b != i + 1) LT[i + 2] = LT[b + 1];
+        }
+        __syncthreads();
+        if (tn >= 0) fetch_runs(tn);
 
         // Output: one unit = two horizontally adjacent blocks = 4 pixels in each of 2 rows.
         const bool vec_ok = ((reinterpret_cast<uintptr_t>(im.out) | uintptr_t(im.out_pitch * 4)) & 15) == 0;
-        for (int u = tid; u < NBLK / 2; u += K3_NT) {
-            const int br = u / (TBW / 2), q = u % (TBW / 2);
-            const int y = 2 * br;
-            if (y >= nrp || 4 * q >= ncp) continue;
-            const uint32_t ee = reinterpret_cast<const uint32_t *>(Ls)[u];
-            const uint32_t e0 = ee & 0xFFFFu, e1 = ee >> 16;
-            const uint32_t m0 = e0 >> 12, m1 = e1 >> 12;
-            const int l0 = m0 ? int(LT[e0 & 0xFFFu]) : 0, l1 = m1 ? int(LT[e1 & 0xFFFu]) : 0;
-            int4 a, b;
-            a.x = (m0 & 1u) ? l0 : 0; a.y = (m0 & 2u) ? l0 : 0;
-            a.z = (m1 & 1u) ? l1 : 0; a.w = (m1 & 2u) ? l1 : 0;
-            b.x = (m0 & 4u) ? l0 : 0; b.y = (m0 & 8u) ? l0 : 0;
-            b.z = (m1 & 4u) ? l1 : 0; b.w = (m1 & 8u) ? l1 : 0;
-            int32_t *dst = im.out + int64_t(y0 + y) * im.out_pitch + x0 + 4 * q;
-            const bool row2 = y + 1 < nrp;
-            if (vec_ok && 4 * q + 4 <= ncp) {
-                __stcs(reinterpret_cast<int4 *>(dst), a);
-                if (row2) __stcs(reinterpret_cast<int4 *>(dst + im.out_pitch), b);
-            } else {
-                const int n = min(4, ncp - 4 * q);
-                const int va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
-                for (int k = 0; k < n; ++k) {
-                    dst[k] = va[k];
-                    if (row2) dst[im.out_pitch + k] = vb[k];
+        // A thread keeps its column: unit i is UR block rows further down.
+        constexpr int UPR = TBW / 2, UR = K3_NT / UPR;   // units per block row, block rows per turn
+        const int q = tid % UPR, k = 2 * (q & 15);
+        const uint32_t bit0 = 1u << k, bit1 = 2u << k, upto0 = bit0 | (bit0 - 1u), upto1 = bit1 | (bit1 - 1u);
+        const int n = min(4, max(0, ncp - 4 * q));       // pixels of the thread's column inside the image
+        auto unit = [&](int br, int4 &a, int4 &b) {
+            const int wi = br * WPR + (q >> 4);
+            const uint4 c = H[wi], wr = H[NWORD + wi];
+            const uint32_t bT = wr.w & 0xFFFFu, bB = wr.w >> 16;
+            const bool t0 = wr.z & bit0, t1 = wr.z & bit1;
+            const int l0 = int(LT[(t0 ? bT : bB) + __popc((t0 ? wr.x : wr.y) & upto0)]);
+            const int l1 = int(LT[(t1 ? bT : bB) + __popc((t1 ? wr.x : wr.y) & upto1)]);
+            a.x = (c.x & bit0) ? l0 : 0; a.y = (c.y & bit0) ? l0 : 0;
+            a.z = (c.x & bit1) ? l1 : 0; a.w = (c.y & bit1) ? l1 : 0;
+            b.x = (c.z & bit0) ? l0 : 0; b.y = (c.w & bit0) ? l0 : 0;
+            b.z = (c.z & bit1) ? l1 : 0; b.w = (c.w & bit1) ? l1 : 0;
+        };
+        int32_t *dst = im.out + int64_t(y0 + 2 * (tid / UPR)) * im.out_pitch + x0 + 4 * q;
+        const int64_t turn = 2 * UR * im.out_pitch;
+        if (vec_ok) {
+            if (n > 0)
+                for (int br = tid / UPR; 2 * br < nrp; br += UR, dst += turn) {
+                    int4 a, b;
+                    unit(br, a, b);
+                    const bool row2 = 2 * br + 1 < nrp;
+                    if (n == 4) {
+                        __stcs(reinterpret_cast<int4 *>(dst), a);
+                        if (row2) __stcs(reinterpret_cast<int4 *>(dst + im.out_pitch), b);
+                    } else {
+                        const int va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            if (i >= n) break;
+                            dst[i] = va[i];
+                            if (row2) dst[im.out_pitch + i] = vb[i];
+                        }
+                    }
                 }
+        } else {
+            for (int br = tid / UPR; 2 * br < nrp; br += UR, dst += turn) {   // rows of any alignment (whole warps)
+                int4 a, b;
+                unit(br, a, b);
+                store_row<32>(dst, a, n);
+                if (2 * br + 1 < nrp) store_row<32>(dst + im.out_pitch, b, n);
             }
         }
         __syncthreads();
@@ -869,7 +859,7 @@ __global__ void __launch_bounds__(K3_NT, 8) k_tile_write_2d(ImgList2D L, Work w)
 inline Geometry geometry()
 {
     Geometry g;
-    g.lab_bytes_per_tile = size_t(NBLK) * sizeof(uint16_t);
+    g.lab_bytes_per_tile = size_t(kLabWords) * sizeof(uint32_t);
     g.rbits_bytes_per_tile = size_t(RBWORDS) * sizeof(uint32_t);
     g.nperim = NPERIM;
     g.maxb = MAXB;
@@ -896,15 +886,15 @@ inline cudaError_t launch(const ImgList2D &L, const Work &w, int sms, bool persi
         if (e == cudaSuccess) e = r;
     };
     mark(0);
-    k_tile_local_2d<<<grid(w.n_tiles, 8), K1_NT, 0, s>>>(L, wk);
+    k_tile_local_2d<<<grid(w.n_tiles, K1_PER_SM), K1_NT, 0, s>>>(L, wk);
     keep(cudaGetLastError());
     mark(1);
     keep(launch_k(k_merge_2d, grid(w.n_tiles, K2_PER_SM), K2_NT, s, ov, L, wk));
     mark(2);
     keep(launch_k(k_scan_flatten_2d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, wk));
     mark(3);
-    // The label writes run a fixed tile order over 8 CTAs per SM (they prefetch their next tile).
-    keep(launch_k(k_tile_write_2d, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * 8))),
+    // The label writes run a fixed tile order over K3_PER_SM CTAs per SM (they prefetch their next tile).
+    keep(launch_k(k_tile_write_2d, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * K3_PER_SM))),
                   K3_NT, s, ov, L, wk));
     mark(4);
     return e;

@@ -619,7 +619,7 @@ __device__ __forceinline__ KeyPos key_pos(const Img3D &im, uint32_t key)
 // count and its tile's root bitmap.
 __device__ void gunion3d(const Img3D &im, Work &w, uint32_t a, uint32_t b)
 {
-    gunion_keyed(w.gp, a, b, [&](uint32_t key) {
+    gunion_keyed(w.gp, a, b, [&](uint32_t, uint32_t key) {
         const KeyPos kp = key_pos(im, key);
         dec_u8(w.segcnt, kp.seg);
         atomicAnd(w.rbits + kp.word, ~(1u << kp.bit));
