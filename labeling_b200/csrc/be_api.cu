@@ -195,8 +195,7 @@ cudaError_t launch_uf3d(const ImgList3D &L, const Work &w, int sms, bool persist
         if (e == cudaSuccess) e = r;
     };
     mark(0);
-    k_tile_local_3d<<<grid(w.n_tiles, kT3LocalPerSM), kT3LocalThreads, 0, s>>>(L, wk);
-    keep(cudaGetLastError());
+    keep(launch_k(k_tile_local_3d, grid(w.n_tiles, kT3LocalPerSM), kT3LocalThreads, s, false, L, wk));
     mark(1);
     keep(launch_k(k_merge_3d, grid(w.n_tiles, kT3MergePerSM), kT3MergeThreads, s, ov, L, wk));
     mark(2);

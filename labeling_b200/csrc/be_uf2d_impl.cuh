@@ -886,8 +886,7 @@ inline cudaError_t launch(const ImgList2D &L, const Work &w, int sms, bool persi
         if (e == cudaSuccess) e = r;
     };
     mark(0);
-    k_tile_local_2d<<<grid(w.n_tiles, K1_PER_SM), K1_NT, 0, s>>>(L, wk);
-    keep(cudaGetLastError());
+    keep(launch_k(k_tile_local_2d, grid(w.n_tiles, K1_PER_SM), K1_NT, s, false, L, wk));
     mark(1);
     keep(launch_k(k_merge_2d, grid(w.n_tiles, K2_PER_SM), K2_NT, s, ov, L, wk));
     mark(2);
