@@ -50,11 +50,14 @@ enum {
     BE_ALGO_ITER = 2, /* the paper's iterative scan / analyze, with a device-side change flag */
     BE_ALGO_PIXEL = 3, /* pixel-level label equivalence, the -a lbeq path (LabelingAlgs.cl:31-130,
                           635-734): 2D 4-connectivity for BE_COH_4 / BE_COH_DEFAULT (the reference's
-                          default), 8 for BE_COH_8; 3D 26-connectivity */
+                          default), 8 for BE_COH_8; 3D 26-connectivity.  The components of the
+                          reference's scan / analyze loop over pixels, found by union-find over
+                          pixel runs (4) or blocks (8, 26) */
     BE_ALGO_RUNS = 4   /* 2D run equivalence, the -a runeq -g path (TOCLRunEquivLabeling,
                           LabelingAlgs.cpp:1090-1268, RE* kernels LabelingAlgs.cl:325-616): runs of
                           each row joined by column overlap -- 4-connectivity for BE_COH_4 /
-                          BE_COH_DEFAULT (the reference's runs), 8 for BE_COH_8; 2D only */
+                          BE_COH_DEFAULT (the reference's runs), 8 for BE_COH_8; 2D only.  Resolved by
+                          union-find over the runs of a tile and the nodes between tiles */
 };
 
 /* Connectivity selector, as the reference's TCoherence (LabelingTools.hpp:45-50). */

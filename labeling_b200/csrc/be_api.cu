@@ -37,8 +37,22 @@ int cuda_error(be_ctx *ctx, cudaError_t e, const char *what)
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// The forms that run in the iterative graph (their count and error flag live in wsiter / iter_err).
-static bool iter_family(int algo) { return algo == BE_ALGO_ITER || algo == BE_ALGO_PIXEL || algo == BE_ALGO_RUNS; }
+// Where a form's component count is: the iterative form has its own workspace (and its error flag in
+// iter_err), the pixel and run forms theirs.
+static const int64_t *count_of(const be_ctx *c, int algo, int dims)
+{
+    if (algo == BE_ALGO_ITER) return c->wsiter.w.ncomp;
+    if (algo == BE_ALGO_PIXEL || algo == BE_ALGO_RUNS) return dims == 2 ? c->wsform2d.w.ncomp : c->wsform3d.w.ncomp;
+    return dims == 2 ? c->ws2d.w.ncomp : c->ws3d.w.ncomp;
+}
+
+// The smallest power of two not below v, as a shift.
+static int ceil_log2(int v)
+{
+    int s = 0;
+    while ((1 << s) < v) ++s;
+    return s;
+}
 
 Geometry geometry_2d() { return uf2d_geometry(0); }
 
@@ -66,6 +80,9 @@ size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_img
     const int64_t n_chunks = (n_segs + kScanChunk - 1) / kScanChunk;
     const size_t nodes = size_t(n_tiles) * g.maxb;
     Work t{};
+    // The launch epoch comes first: its place is the same for every size, so it only ever grows, and
+    // status words that launches of other sizes left in the workspace are never taken for this one's.
+    t.epoch = reinterpret_cast<uint32_t *>(take(2 * sizeof(uint32_t)));
     t.lab = take(size_t(n_tiles) * g.lab_bytes_per_tile);
     t.perim = reinterpret_cast<uint16_t *>(take(size_t(n_tiles) * g.nperim * sizeof(uint16_t)));
     t.rbits = reinterpret_cast<uint32_t *>(take(size_t(n_tiles) * g.rbits_bytes_per_tile));
@@ -79,7 +96,6 @@ size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_img
     t.queue = reinterpret_cast<uint32_t *>(take(kQueueWords * sizeof(uint32_t)));
     t.ncomp = reinterpret_cast<int64_t *>(take(size_t(std::max(n_imgs, 1)) * sizeof(int64_t)));
     t.err = reinterpret_cast<uint32_t *>(take(16 * sizeof(uint32_t)));
-    t.epoch = reinterpret_cast<uint32_t *>(take(2 * sizeof(uint32_t)));
     t.scan_status = reinterpret_cast<uint64_t *>(take(size_t(std::max<int64_t>(n_chunks, 1)) * sizeof(uint64_t)));
     t.n_tiles = n_tiles;
     t.n_segs = n_segs;
@@ -143,15 +159,15 @@ void fill_img2d(Img2D &im, const uint8_t *in, int64_t in_pitch, int32_t rows, in
                 int32_t *out, int64_t out_pitch, int64_t tile_base, int64_t seg_base, int index,
                 int shape)
 {
-    const int tbw = kShapes2D[shape].tbw, tbh = kShapes2D[shape].tbh;
+    const int tw = kShapes2D[shape].tw, th = kShapes2D[shape].th;
     im.in = in;
     im.out = out;
     im.in_pitch = in_pitch;
     im.out_pitch = out_pitch;
     im.rows = rows;
     im.cols = cols;
-    im.tiles_x = (cols + 2 * tbw - 1) / (2 * tbw);
-    im.tiles_y = (rows + 2 * tbh - 1) / (2 * tbh);
+    im.tiles_x = (cols + tw - 1) / tw;
+    im.tiles_y = (rows + th - 1) / th;
     im.tile_base = tile_base;
     im.seg_base = seg_base;
     im.thr = thr;
@@ -252,6 +268,8 @@ int be_destroy(be_ctx *c)
     c->ws2d.release();
     c->ws3d.release();
     c->wsiter.release();
+    c->wsform2d.release();
+    c->wsform3d.release();
     for (be_iter_graph &g : c->iter_graph) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
         if (g.graph) cudaGraphDestroy(g.graph);
@@ -329,34 +347,42 @@ int be_label2d(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int
     int rc, shape;
     pick2d(c, rows, cols, algo, &algo, &shape);
     c->last_algo = algo;
-    if (algo == BE_ALGO_PIXEL) {
-        rc = run_lbeq2d(c, in, in_pitch, rows, cols, threshold, coh == BE_COH_8, out, out_pitch, s);
-    } else if (algo == BE_ALGO_RUNS) {
-        rc = run_runeq2d(c, in, in_pitch, rows, cols, threshold, coh == BE_COH_8, out, out_pitch, s);
-    } else if (algo == BE_ALGO_ITER) {
+    const bool form = algo == BE_ALGO_PIXEL || algo == BE_ALGO_RUNS;
+    if (algo == BE_ALGO_ITER) {
         rc = run_iter2d(c, in, in_pitch, rows, cols, threshold, out, out_pitch, s);
     } else {
+        if (form) {
+            // The pixel and run forms give the components of their connectivity in canonical order: 4
+            // by the pipeline on pixel runs, 8 by the block pipeline.  (Sizes as their own key space --
+            // rows of a power of two -- takes them.)
+            if ((int64_t(rows) << ceil_log2(cols)) >= (int64_t(1) << 31))
+                return set_error(c, BE_ERR_INVALID, algo == BE_ALGO_PIXEL ? "label equivalence: %d x %d exceeds its key space"
+                                                                          : "run equivalence: %d x %d exceeds its key space", rows, cols);
+            shape = coh == BE_COH_8 ? 0 : kShapePixel2D;
+        }
+        Workspace &ws = form ? c->wsform2d : c->ws2d;
         Img2D im;
         fill_img2d(im, in, in_pitch, rows, cols, threshold, out, out_pitch, 0, 0, 0, shape);
         const int64_t n_tiles = int64_t(im.tiles_x) * im.tiles_y;
         const int64_t n_segs = int64_t(rows) * im.tiles_x;
-        rc = c->ws2d.ensure(c, uf2d_geometry(shape), n_tiles, n_segs, 1);
+        rc = ws.ensure(c, uf2d_geometry(shape), n_tiles, n_segs, 1);
         if (rc) return rc;
         ImgList2D L{nullptr, 1, im};
 #ifdef BE_BOUNDS_CHECK
-        cudaMemsetAsync(c->ws2d.w.err, 0, 16 * sizeof(uint32_t), s);
+        cudaMemsetAsync(ws.w.err, 0, 16 * sizeof(uint32_t), s);
 #endif
-        e = uf2d_launch(shape, L, c->ws2d.w, c->sms, false, s, c->timing ? c->stage_ev : nullptr);
-        c->timed_stages = c->timing ? kStages2D : 0;
+        const bool timed = c->timing && !form;
+        e = uf2d_launch(shape, L, ws.w, c->sms, false, s, timed ? c->stage_ev : nullptr);
+        c->timed_stages = timed ? kStages2D : 0;
         if (e != cudaSuccess) return cuda_error(c, e, "be_label2d launch");
     }
     if (rc) return rc;
     if (n_components) {
-        const int64_t *src = iter_family(algo) ? c->wsiter.w.ncomp : c->ws2d.w.ncomp;
+        const int64_t *src = count_of(c, algo, 2);
         e = cudaMemcpyAsync(c->h_ncomp, src, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_error(c, e, "be_label2d sync");
-        if (iter_family(algo) && c->iter_err && *c->iter_err)
+        if (algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
             return set_error(c, BE_ERR_NO_CONVERGENCE, "be_label2d: iteration cap reached");
         *n_components = c->h_ncomp[0];
     }
@@ -382,32 +408,35 @@ int be_label3d(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2,
     int rc;
     pick3d(c, int64_t(d0) * d1 * d2, algo, &algo);
     c->last_algo = algo;
-    if (algo == BE_ALGO_PIXEL) {
-        rc = run_lbeq3d(c, in, d0, d1, d2, threshold, out, s);
-    } else if (algo == BE_ALGO_ITER) {
+    const bool form = algo == BE_ALGO_PIXEL;
+    if (algo == BE_ALGO_ITER) {
         rc = run_iter3d(c, in, d0, d1, d2, threshold, out, s);
     } else {
+        if (form && (int64_t(d0) << (ceil_log2(d1) + ceil_log2(d2))) >= (int64_t(1) << 31))   // as in 2D
+            return set_error(c, BE_ERR_INVALID, "label equivalence: volume exceeds its key space");
+        Workspace &ws = form ? c->wsform3d : c->ws3d;
         Img3D im;
         fill_img3d(im, in, d0, d1, d2, threshold, out, 0, 0, 0);
         const int64_t n_tiles = int64_t(im.t0) * im.t1 * im.t2;
         const int64_t n_segs = int64_t(d0) * d1 * im.t2;
-        rc = c->ws3d.ensure(c, geometry_3d(), n_tiles, n_segs, 1);
+        rc = ws.ensure(c, geometry_3d(), n_tiles, n_segs, 1);
         if (rc) return rc;
         ImgList3D L{nullptr, 1, im};
 #ifdef BE_BOUNDS_CHECK
-        cudaMemsetAsync(c->ws3d.w.err, 0, 16 * sizeof(uint32_t), s);
+        cudaMemsetAsync(ws.w.err, 0, 16 * sizeof(uint32_t), s);
 #endif
-        e = launch_uf3d(L, c->ws3d.w, c->sms, false, s, c->timing ? c->stage_ev : nullptr);
-        c->timed_stages = c->timing ? kStages3D : 0;
+        const bool timed = c->timing && !form;
+        e = launch_uf3d(L, ws.w, c->sms, false, s, timed ? c->stage_ev : nullptr);
+        c->timed_stages = timed ? kStages3D : 0;
         if (e != cudaSuccess) return cuda_error(c, e, "be_label3d launch");
     }
     if (rc) return rc;
     if (n_components) {
-        const int64_t *src = iter_family(algo) ? c->wsiter.w.ncomp : c->ws3d.w.ncomp;
+        const int64_t *src = count_of(c, algo, 3);
         e = cudaMemcpyAsync(c->h_ncomp, src, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_error(c, e, "be_label3d sync");
-        if (iter_family(algo) && c->iter_err && *c->iter_err)
+        if (algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
             return set_error(c, BE_ERR_NO_CONVERGENCE, "be_label3d: iteration cap reached");
         *n_components = c->h_ncomp[0];
     }
@@ -462,11 +491,11 @@ int be_label2d_host(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows
     e = cudaMemcpy2DAsync(out, out_pitch * sizeof(int32_t), c->d_out, dpo * sizeof(int32_t),
                           cols * sizeof(int32_t), rows, cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return cuda_error(c, e, "download");
-    const int64_t *src = iter_family(c->last_algo) ? c->wsiter.w.ncomp : c->ws2d.w.ncomp;
+    const int64_t *src = count_of(c, c->last_algo, 2);
     e = cudaMemcpyAsync(c->h_ncomp, src, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_error(c, e, "be_label2d_host sync");
-    if (iter_family(c->last_algo) && c->iter_err && *c->iter_err)
+    if (c->last_algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
         return set_error(c, BE_ERR_NO_CONVERGENCE, "be_label2d_host: iteration cap reached");
     n = c->h_ncomp[0];
     if (n_components) *n_components = n;
@@ -502,11 +531,11 @@ int be_label3d_host(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_
     cudaEventRecord(c->ev1, s);
     e = cudaMemcpyAsync(out, c->d_out, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return cuda_error(c, e, "download");
-    const int64_t *src = iter_family(c->last_algo) ? c->wsiter.w.ncomp : c->ws3d.w.ncomp;
+    const int64_t *src = count_of(c, c->last_algo, 3);
     e = cudaMemcpyAsync(c->h_ncomp, src, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_error(c, e, "be_label3d_host sync");
-    if (iter_family(c->last_algo) && c->iter_err && *c->iter_err)
+    if (c->last_algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
         return set_error(c, BE_ERR_NO_CONVERGENCE, "be_label3d_host: iteration cap reached");
     if (n_components) *n_components = c->h_ncomp[0];
     if (elapsed_us) {

@@ -20,12 +20,14 @@ struct Geometry {
     bool links = false;   // the pipeline resolves node links (Work::nlink) before its label writes
 };
 
-// 2D tile shapes (in 2x2 blocks); shape 0 is the default.
+// 2D tile shapes (in pixels): the block shapes the autotuner chooses between, 0 the default, and the
+// pixel shape of the 4-connected forms.
 struct Shape2D {
-    int tbw, tbh;
+    int tw, th;
 };
 constexpr int kNumShapes2D = 3;
-extern const Shape2D kShapes2D[kNumShapes2D];
+constexpr int kShapePixel2D = kNumShapes2D;
+extern const Shape2D kShapes2D[kNumShapes2D + 1];
 Geometry uf2d_geometry(int shape);
 cudaError_t uf2d_launch(int shape, const ImgList2D &L, const Work &w, int sms, bool persistent,
                         cudaStream_t s, cudaEvent_t *ev = nullptr);
@@ -81,12 +83,6 @@ int run_iter2d(struct ::be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t 
                int thr, int32_t *out, int64_t out_pitch, cudaStream_t s);
 int run_iter3d(struct ::be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2, int thr,
                int32_t *out, cudaStream_t s);
-int run_lbeq2d(struct ::be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int32_t cols, int thr,
-               int conn8, int32_t *out, int64_t out_pitch, cudaStream_t s);
-int run_lbeq3d(struct ::be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2, int thr,
-               int32_t *out, cudaStream_t s);
-int run_runeq2d(struct ::be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int32_t cols, int thr,
-                int conn8, int32_t *out, int64_t out_pitch, cudaStream_t s);
 
 }  // namespace be
 
@@ -103,6 +99,7 @@ struct be_ctx {
     int sms = 148;
     std::string err;
     be::Workspace ws2d, ws3d, wsiter;
+    be::Workspace wsform2d, wsform3d;   // the pixel and run forms (apart: a caller may overlap them with the block form)
     void *iter_base = nullptr;      // iterative-form block arrays
     size_t iter_bytes = 0;
     uint32_t *iter_err = nullptr;   // pinned: iteration-cap flag of the last iterative call
@@ -118,5 +115,5 @@ struct be_ctx {
     cudaEvent_t stage_ev[be::kStages + 1] = {};
     std::vector<be::TuneEntry> tune;  // autotuner decisions
     int last_algo = 1;                // algorithm the last label call actually ran
-    be_iter_graph iter_graph[5];      // iterative form: 2D / 3D blocks, 2D / 3D pixels, 2D runs
+    be_iter_graph iter_graph[2];      // iterative form: 2D / 3D blocks
 };

@@ -427,6 +427,23 @@ __device__ __forceinline__ void split16(uint4 v, uint32_t K, bool hi, uint32_t &
          (gather4(gt_bytes(__byte_perm(v.z, v.w, 0x7531), K, hi)) << 4);
 }
 
+// 16 pixels of one row -> their foreground bits in order.
+__device__ __forceinline__ uint32_t bits16(uint4 v, uint32_t K, bool hi)
+{
+    return gather4(gt_bytes(v.x, K, hi)) | (gather4(gt_bytes(v.y, K, hi)) << 4) | (gather4(gt_bytes(v.z, K, hi)) << 8) |
+           (gather4(gt_bytes(v.w, K, hi)) << 12);
+}
+
+// Bits 0..15 of x -> bits 0, 2, .. 30.
+__device__ __forceinline__ uint32_t spread16(uint32_t x)
+{
+    x &= 0xFFFFu;
+    x = (x | (x << 8)) & 0x00FF00FFu;
+    x = (x | (x << 4)) & 0x0F0F0F0Fu;
+    x = (x | (x << 2)) & 0x33333333u;
+    return (x | (x << 1)) & 0x55555555u;
+}
+
 // Foreground bits of the n (1..64) pixels at p, split as split16 (bit k of left / right: pixel
 // 2k / 2k + 1), whatever p's alignment: the up to five 16-byte chunks that hold the pixels are
 // loaded whole and the words shifted into place -- an odd offset swaps the even and odd words.  A

@@ -1,6 +1,7 @@
 // be_uf2d.cu -- 2D Block-Equivalence labeling, union-find form (8-connectivity, 2x2 blocks).
 // The pipeline itself is in be_uf2d_impl.cuh, instantiated here for three tile shapes
-// (32 x 128, 64 x 64 and 16 x 256 blocks) that the autotuner chooses between.
+// (32 x 128, 64 x 64 and 16 x 256 blocks) that the autotuner chooses between, and once on pixels for
+// 4-connectivity (the pixel label-equivalence and run-equivalence forms).
 //
 // Replaces the reference's LBEQ2_Init / LBEQ2_Scan / LBEQ2_Analyze / LBEQ2_SetFinalLabels
 // (LabelingAlgs.cl:176-319) and their host loop (LabelingAlgs.cpp:989-1084) with four launches:
@@ -36,27 +37,34 @@
 namespace be {
 
 namespace s32x128 {
-constexpr int TBW = 128, TBH = 32;
+constexpr int CELL = 2, TBW = 128, TBH = 32;
 #include "be_uf2d_impl.cuh"
 }  // namespace s32x128
 
 namespace s64x64 {
-constexpr int TBW = 64, TBH = 64;
+constexpr int CELL = 2, TBW = 64, TBH = 64;
 #include "be_uf2d_impl.cuh"
 }  // namespace s64x64
 
 namespace s16x256 {
-constexpr int TBW = 256, TBH = 16;
+constexpr int CELL = 2, TBW = 256, TBH = 16;
 #include "be_uf2d_impl.cuh"
 }  // namespace s16x256
 
-const Shape2D kShapes2D[kNumShapes2D] = {{128, 32}, {64, 64}, {256, 16}};
+// 4-connectivity: pixel cells, 64 x 128 pixels, one thread per 32 pixels (256 threads).
+namespace p64x128 {
+constexpr int CELL = 1, TBW = 128, TBH = 64;
+#include "be_uf2d_impl.cuh"
+}  // namespace p64x128
+
+const Shape2D kShapes2D[kNumShapes2D + 1] = {{256, 64}, {128, 128}, {512, 32}, {128, 64}};
 
 Geometry uf2d_geometry(int shape)
 {
     switch (shape) {
     case 1: return s64x64::geometry();
     case 2: return s16x256::geometry();
+    case kShapePixel2D: return p64x128::geometry();
     default: return s32x128::geometry();
     }
 }
@@ -67,6 +75,7 @@ cudaError_t uf2d_launch(int shape, const ImgList2D &L, const Work &w, int sms, b
     switch (shape) {
     case 1: return s64x64::launch(L, w, sms, persistent, s, ev);
     case 2: return s16x256::launch(L, w, sms, persistent, s, ev);
+    case kShapePixel2D: return p64x128::launch(L, w, sms, persistent, s, ev);
     default: return s32x128::launch(L, w, sms, persistent, s, ev);
     }
 }

@@ -1,28 +1,33 @@
 // be_uf2d_impl.cuh -- the 2D union-find pipeline for one tile shape.  Included by be_uf2d.cu
-// once per supported shape, inside a namespace that defines `TBW` and `TBH` (tile width and
-// height in 2x2 blocks, TBW * TBH <= 4096, TBW a power of two in [64, 256]).
+// once per supported shape, inside a namespace that defines
+//   CELL      2: 2x2 blocks, 8-connectivity; 1: pixels, 4-connectivity
+//   TBW, TBH  tile width and height in cells (TBW a power of two in [64, 256], TBW * TBH / 32 threads)
+// Comments speak of blocks; with CELL 1 a block is one pixel, in pixel row and block row alike, every
+// run is a T run (below), and the only link is the one straight up.
 namespace {
 
-constexpr int TW = 2 * TBW, TH = 2 * TBH;          // tile in pixels
-constexpr int NBLK = TBW * TBH;                    // blocks per tile (4096)
+constexpr int TW = CELL * TBW, TH = CELL * TBH;    // tile in pixels
+constexpr int NBLK = TBW * TBH;                    // blocks per tile
+constexpr int MAXRUN = CELL == 2 ? NBLK : NBLK / 2;   // runs per tile (between two pixel runs is a gap)
 constexpr int NPERIM = 2 * (TBW + TBH);            // border positions per tile
 constexpr int MAXB = NPERIM;                       // nodes per tile
 constexpr int WPR = TBW / 32;                      // 32-block words per block row
 constexpr int NWORD = NBLK / 32;                   // words per tile
 constexpr int K1_NT = NWORD;                       // one thread per (block row, word)
-constexpr int K1_PER_SM = 7;                       // resident tile CTAs per SM (26 KB of shared memory, 72 registers)
+constexpr int K1_PER_SM = CELL == 2 ? 7 : 4;       // resident tile CTAs per SM (26 KB of shared memory, 72 registers)
 constexpr int MQCAP = 1024;                        // union-queue capacity (more take further rounds)
-constexpr int RBWORDS = NBLK / 32;                 // root-bitmap words per tile: a bit per run
+constexpr int RBWORDS = MAXRUN / 32;               // root-bitmap words per tile: a bit per run
 // A tile's labels as the write kernel reads them (Work::lab): for each of its 32-block words the four
 // pixel-class words (uint4) and the run words (uint4: starts of the runs with a top pixel, of the
 // others, blocks of the former, runs of either kind before the word), then for every run of the
-// tile its component's root run (uint16, at most NBLK).
-constexpr int kHdr = 8 * NWORD;
-constexpr int kLabWords = kHdr + NBLK / 2;
+// tile its component's root run (uint16, at most MAXRUN).  With CELL 1 there are no class words, and
+// the run words' second word is the pixels.
+constexpr int kHdr = (CELL == 2 ? 8 : 4) * NWORD;
+constexpr int kLabWords = kHdr + MAXRUN / 2;
 
-static_assert(NBLK <= 4096, "a run number must fit 12 bits");
+static_assert(MAXRUN == 4096, "a run number must fit 12 bits; 128 words of run flags");
 static_assert(MAXB < 4096, "node index must fit 12 bits");
-static_assert(K1_NT == 128 && (WPR & (WPR - 1)) == 0 && WPR <= 32, "thread layout");
+static_assert(K1_NT % 128 == 0 && K1_NT >= RBWORDS && (WPR & (WPR - 1)) == 0 && WPR <= 32, "thread layout");
 
 // Block position of border position p of a tile with nbr x nbc valid blocks.
 __device__ __forceinline__ bool perim_pos(int p, int nbr, int nbc, int &r, int &c)
@@ -43,6 +48,9 @@ __device__ __forceinline__ uint32_t hibit(uint32_t x) { return 31u - __clz(x); }
 // components as their first pixels do.  A segment has at most seg_width runs, every two of them with
 // a background pixel between, so keys stay below 2^31 with the pixel count.
 __device__ __forceinline__ uint32_t seg_width(const Img2D &im) { return uint32_t(min(im.cols, TW) + 1) >> 1; }
+
+// Blocks that n pixels take.
+__device__ __forceinline__ int cells(int n) { return CELL == 2 ? (n + 1) >> 1 : n; }
 
 // Set bits of the bitmap b in positions [lo, hi).
 __device__ __forceinline__ uint32_t count_bits(const uint32_t *b, uint32_t lo, uint32_t hi)
@@ -78,15 +86,16 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
         w.epoch[0] += 1u;
         w.epoch[1] = 0u;
     }
-    __shared__ __align__(16) uint32_t P[NBLK];   // per run: parent run
-    __shared__ __align__(16) uint4 CW[NWORD];    // class words: TL, TR, BL, BR
-    __shared__ __align__(16) uint4 WR[NWORD];    // T starts, B starts, blocks of T runs, T | B << 16 runs before
+    __shared__ __align__(16) uint32_t P[MAXRUN]; // per run: parent run
+    __shared__ __align__(16) uint4 CW[CELL == 2 ? NWORD : 1];   // class words: TL, TR, BL, BR
+    __shared__ __align__(16) uint4 WR[NWORD];    // T starts, B starts (CELL 1: pixels), blocks of T runs,
+                                                 // runs before (T | B << 16)
     __shared__ uint32_t WHC[NWORD];              // joins to the right
     __shared__ uint32_t MQ[MQCAP];               // union queue: (run_a << 16) | run_b
-    __shared__ uint32_t BF[NWORD];               // runs that are border components
-    __shared__ uint32_t BP[NWORD];               // runs that are roots; then nodes before each word of BF
+    __shared__ uint32_t BF[RBWORDS];             // runs that are border components
+    __shared__ uint32_t BP[RBWORDS];             // runs that are roots; then nodes before each word of BF
     __shared__ uint32_t mqn;
-    __shared__ uint32_t wtot[K1_NT / 32], ntot[K1_NT / 32];   // run starts / nodes per warp
+    __shared__ uint32_t wtot[K1_NT / 32], ntot[RBWORDS / 32];   // run starts / nodes per warp
     __shared__ uint32_t qslot;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -99,52 +108,66 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
         const int ty = int(lt / im.tiles_x), tx = int(lt - int64_t(ty) * im.tiles_x);
         const int y0 = ty * TH, x0 = tx * TW;
         const int nrp = min(TH, im.rows - y0), ncp = min(TW, im.cols - x0);
-        const int nbr = (nrp + 1) >> 1, nbc = (ncp + 1) >> 1;
+        const int nbr = cells(nrp), nbc = cells(ncp);
         const uint32_t K = (0x7Fu - (uint32_t(im.thr) & 0x7Fu)) * 0x01010101u;
         const bool hi = im.thr >= 128;
 
         if (tid == 0) mqn = 0;
-        BF[tid] = 0;
-        for (int i = tid; i < NBLK / 4; i += K1_NT)   // every run its own root
+        if (tid < RBWORDS) BF[tid] = 0;
+        for (int i = tid; i < MAXRUN / 4; i += K1_NT)   // every run its own root
             reinterpret_cast<uint4 *>(P)[i] = make_uint4(4 * i, 4 * i + 1, 4 * i + 2, 4 * i + 3);
 
         // Phase A: pixel words, runs, run starts.
-        uint32_t TLw = 0, TRw = 0, BLw = 0, BRw = 0;
-        if (r < nbr && 64 * q < ncp) {
-            const uint8_t *row0 = im.in + int64_t(y0 + 2 * r) * im.in_pitch + x0 + 64 * q;
-            const bool row1 = 2 * r + 1 < nrp;
-            const bool vec = (64 * q + 64 <= ncp) &&
-                             ((reinterpret_cast<uintptr_t>(row0) | uintptr_t(im.in_pitch)) & 15) == 0;
-            if (vec) {
-                const uint4 *p0 = reinterpret_cast<const uint4 *>(row0);
-                uint4 v[4], u[4];
+        uint32_t TLw = 0, TRw = 0, BLw = 0, BRw = 0;   // CELL 2: pixel classes
+        uint32_t F = 0;                                // CELL 1: pixels
+        if constexpr (CELL == 2) {
+            if (r < nbr && 64 * q < ncp) {
+                const uint8_t *row0 = im.in + int64_t(y0 + 2 * r) * im.in_pitch + x0 + 64 * q;
+                const bool row1 = 2 * r + 1 < nrp;
+                const bool vec = (64 * q + 64 <= ncp) &&
+                                 ((reinterpret_cast<uintptr_t>(row0) | uintptr_t(im.in_pitch)) & 15) == 0;
+                if (vec) {
+                    const uint4 *p0 = reinterpret_cast<const uint4 *>(row0);
+                    uint4 v[4], u[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) v[i] = __ldg(p0 + i);
-                if (row1) {
-                    const uint4 *p1 = reinterpret_cast<const uint4 *>(row0 + im.in_pitch);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) u[i] = __ldg(p1 + i);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    uint32_t ev, od;
-                    split16(v[i], K, hi, ev, od);
-                    TLw |= ev << (8 * i);
-                    TRw |= od << (8 * i);
+                    for (int i = 0; i < 4; ++i) v[i] = __ldg(p0 + i);
                     if (row1) {
-                        split16(u[i], K, hi, ev, od);
-                        BLw |= ev << (8 * i);
-                        BRw |= od << (8 * i);
+                        const uint4 *p1 = reinterpret_cast<const uint4 *>(row0 + im.in_pitch);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) u[i] = __ldg(p1 + i);
                     }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        uint32_t ev, od;
+                        split16(v[i], K, hi, ev, od);
+                        TLw |= ev << (8 * i);
+                        TRw |= od << (8 * i);
+                        if (row1) {
+                            split16(u[i], K, hi, ev, od);
+                            BLw |= ev << (8 * i);
+                            BRw |= od << (8 * i);
+                        }
+                    }
+                } else {
+                    const int n = min(64, ncp - 64 * q);
+                    const uint8_t *hi_px = im.in + int64_t(im.rows - 1) * im.in_pitch + im.cols;
+                    row_bits(row0, n, im.in, hi_px, K, hi, im.thr, TLw, TRw);
+                    if (row1) row_bits(row0 + im.in_pitch, n, im.in, hi_px, K, hi, im.thr, BLw, BRw);
                 }
+            }
+        } else if (r < nbr && 32 * q < ncp) {
+            const uint8_t *row = im.in + int64_t(y0 + r) * im.in_pitch + x0 + 32 * q;
+            if (32 * q + 32 <= ncp && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row)), u = __ldg(reinterpret_cast<const uint4 *>(row) + 1);
+                F = bits16(v, K, hi) | (bits16(u, K, hi) << 16);
             } else {
-                const int n = min(64, ncp - 64 * q);
-                const uint8_t *hi_px = im.in + int64_t(im.rows - 1) * im.in_pitch + im.cols;
-                row_bits(row0, n, im.in, hi_px, K, hi, im.thr, TLw, TRw);
-                if (row1) row_bits(row0 + im.in_pitch, n, im.in, hi_px, K, hi, im.thr, BLw, BRw);
+                uint32_t even, odd;
+                row_bits(row, min(32, ncp - 32 * q), im.in, im.in + int64_t(im.rows - 1) * im.in_pitch + im.cols, K, hi,
+                         im.thr, even, odd);
+                F = spread16(even) | (spread16(odd) << 1);
             }
         }
-        const uint32_t Lw = TLw | BLw, Rw = TRw | BRw, Tw = TLw | TRw;
+        const uint32_t Lw = CELL == 2 ? TLw | BLw : F, Rw = CELL == 2 ? TRw | BRw : F, Tw = CELL == 2 ? TLw | TRw : F;
         // hc bit k: block k is joined to block k + 1 (a right pixel of k touches a left pixel of
         // k + 1 -- every such pair is 8-adjacent); bit 31 looks at the next word.
         const uint32_t Lnext = __shfl_down_sync(0xFFFFFFFFu, Lw, 1, WPR);
@@ -156,8 +179,8 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
         // T runs: the starts whose run has a top pixel.  Within the word, from each top pixel a carry
         // runs down (in reversed bits) to the start it belongs to.  A run that goes on past its word
         // with no top pixel yet takes it from the words it goes on into.
-        uint32_t ST, CT;
-        {
+        uint32_t ST = S, CT = ~0u;
+        if constexpr (CELL == 2) {
             const uint32_t rS = __brev(S), rT = __brev(Tw);
             ST = __brev(((~rS + (rT & ~rS)) | rT) & rS);
             const uint32_t cm = (S & (0u - S)) - 1u;   // blocks before the word's first start
@@ -189,7 +212,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
                 pr &= pr << o;
             }
         }
-        const uint32_t SB = S & ~ST;
+        const uint32_t SB = CELL == 2 ? S & ~ST : 0u;
         // Runs before this word: in its row (T runs in the low half, B runs in the high half), and in
         // the rows before it -- over the warp here, the warps' totals are added after the barrier.
         uint32_t bTB, rowsum;
@@ -212,8 +235,8 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
             bTB = x - c + (row << 16) + (rowsum - rt) * 0x10001u;   // B runs follow the row's T runs
         }
         if (lane == 31) wtot[warp] = rowsum;
-        CW[tid] = make_uint4(TLw, TRw, BLw, BRw);
-        WR[tid] = make_uint4(ST, SB, CT, bTB);
+        if constexpr (CELL == 2) CW[tid] = make_uint4(TLw, TRw, BLw, BRw);
+        WR[tid] = make_uint4(ST, CELL == 2 ? SB : F, CT, bTB);
         WHC[tid] = hc;
         __syncthreads();   // words of every row written
         uint32_t woff = 0, nrun = 0, uoff = 0;
@@ -228,8 +251,8 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
         const uint32_t bT = bTB & 0xFFFFu, bB = bTB >> 16;   // T, B runs numbered before this word's
         {
             uint4 *h = reinterpret_cast<uint4 *>(lab + t * kLabWords);
-            h[tid] = make_uint4(TLw, TRw, BLw, BRw);
-            h[NWORD + tid] = make_uint4(ST, SB, CT, bTB);
+            if constexpr (CELL == 2) h[tid] = make_uint4(TLw, TRw, BLw, BRw);
+            h[kHdr / 4 - NWORD + tid] = make_uint4(ST, CELL == 2 ? SB : F, CT, bTB);
         }
 
         // Phase B: links to the block row above.  For block b of this row: N (straight up, a top
@@ -241,47 +264,65 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
         uint32_t uST = 0, uSB = 0, ubTB = 0;              // the word above: starts, runs before
         uint32_t uC = 0, uCl = 0, uCr = 0, uSn = 0;       // kind of the block above, above left, above right
         const bool above = r > 0 && r < nbr;
-        if (above) {
-            const int u = tid - WPR;   // same word, row above
-            const uint32_t uBL = CW[u].z, uBR = CW[u].w;
-            const uint32_t uBRp = q > 0 ? CW[u - 1].w >> 31 : 0u;
-            const uint32_t uBLn = q + 1 < WPR ? CW[u + 1].z & 1u : 0u;
-            const uint4 ur = WR[u];
-            uST = ur.x;
-            uSB = ur.y;
-            uC = ur.z;
-            ubTB = ur.w + uoff * 0x10001u;
-            uCl = uC << 1;
-            uCr = uC >> 1;
-            if (q > 0) uCl |= WR[u - 1].z >> 31;
-            if (q + 1 < WPR) {
-                const uint4 un = WR[u + 1];
-                uCr |= un.z << 31;
-                uSn = (un.x | un.y) & 1u;   // a run starts at the next word's first block
-            }
-            Nm = Tw & (uBL | uBR);
-            NWm = TLw & ((uBR << 1) | uBRp);
-            NEm = TRw & ((uBL >> 1) | (uBLn << 31));
-        }
-        {
-            // bit 31 of the previous word's raw N / NE, for the rules at block 0
-            const uint32_t Np = __shfl_up_sync(0xFFFFFFFFu, Nm, 1, WPR);
-            const uint32_t NEp = __shfl_up_sync(0xFFFFFFFFu, NEm, 1, WPR);
+        if constexpr (CELL == 2) {
             if (above) {
-                const int u = tid - WPR;
-                const uint32_t uhc = WHC[u];
-                const uint32_t uhl = (uhc << 1) | (q > 0 ? WHC[u - 1] >> 31 : 0u);
-                const uint32_t N = Nm, NE = NEm;
-                const uint32_t Nsh = (N << 1) | (q > 0 ? Np >> 31 : 0u);
-                const uint32_t NEsh = (NE << 1) | (q > 0 ? NEp >> 31 : 0u);
-                Nm = N & ~(hl & ((Nsh & uhl) | NEsh));
-                NWm &= ~((N & uhl) | (hl & Nsh));
-                NEm = NE & ~((N & uhc) | (hl & NEsh & uhc));
+                const int u = tid - WPR;   // same word, row above
+                const uint32_t uBL = CW[u].z, uBR = CW[u].w;
+                const uint32_t uBRp = q > 0 ? CW[u - 1].w >> 31 : 0u;
+                const uint32_t uBLn = q + 1 < WPR ? CW[u + 1].z & 1u : 0u;
+                const uint4 ur = WR[u];
+                uST = ur.x;
+                uSB = ur.y;
+                uC = ur.z;
+                ubTB = ur.w + uoff * 0x10001u;
+                uCl = uC << 1;
+                uCr = uC >> 1;
+                if (q > 0) uCl |= WR[u - 1].z >> 31;
+                if (q + 1 < WPR) {
+                    const uint4 un = WR[u + 1];
+                    uCr |= un.z << 31;
+                    uSn = (un.x | un.y) & 1u;   // a run starts at the next word's first block
+                }
+                Nm = Tw & (uBL | uBR);
+                NWm = TLw & ((uBR << 1) | uBRp);
+                NEm = TRw & ((uBL >> 1) | (uBLn << 31));
             }
+            {
+                // bit 31 of the previous word's raw N / NE, for the rules at block 0
+                const uint32_t Np = __shfl_up_sync(0xFFFFFFFFu, Nm, 1, WPR);
+                const uint32_t NEp = __shfl_up_sync(0xFFFFFFFFu, NEm, 1, WPR);
+                if (above) {
+                    const int u = tid - WPR;
+                    const uint32_t uhc = WHC[u];
+                    const uint32_t uhl = (uhc << 1) | (q > 0 ? WHC[u - 1] >> 31 : 0u);
+                    const uint32_t N = Nm, NE = NEm;
+                    const uint32_t Nsh = (N << 1) | (q > 0 ? Np >> 31 : 0u);
+                    const uint32_t NEsh = (NE << 1) | (q > 0 ? NEp >> 31 : 0u);
+                    Nm = N & ~(hl & ((Nsh & uhl) | NEsh));
+                    NWm &= ~((N & uhl) | (hl & Nsh));
+                    NEm = NE & ~((N & uhc) | (hl & NEsh & uhc));
+                }
+            }
+        } else {
+            if (above) {
+                const uint4 ur = WR[tid - WPR];
+                uST = ur.x;
+                ubTB = ur.w + uoff * 0x10001u;
+                Nm = F & ur.y;
+            }
+            // A pixel pair left of another one is joined to it in both rows.
+            const uint32_t Np = __shfl_up_sync(0xFFFFFFFFu, Nm, 1, WPR);
+            Nm &= ~((Nm << 1) | (q > 0 ? Np >> 31 : 0u));
         }
         // Takes one kept link of block b off the masks (N, else NW, else NE): its two runs.
         auto take = [&](uint32_t b, uint32_t &own, uint32_t &up) {
             const uint32_t bit = 1u << b, upto = (bit << 1) - 1u;
+            if constexpr (CELL == 1) {
+                Nm ^= bit;
+                own = bT + __popc(ST & upto) - 1u;
+                up = (ubTB & 0xFFFFu) + __popc(uST & upto) - 1u;
+                return;
+            }
             const bool tt = CT & bit;
             own = (tt ? bT : bB) + __popc((tt ? ST : SB) & upto) - 1u;
             const bool isN = Nm & bit, isW = !isN && (NWm & bit), isE = !isN && !isW;
@@ -308,7 +349,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
                 uint32_t own, up;
                 take(b, own, up);
                 (void)GUARD(w, own < nrun && up < own, 112, (uint64_t(own) << 32) | up);
-                P[own & (NBLK - 1)] = up & (NBLK - 1);
+                P[own & (MAXRUN - 1)] = up & (MAXRUN - 1);
             }
         }
         // The remaining links are unions: queued and merged by every lane.
@@ -377,17 +418,19 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
         __syncthreads();
 
         // Phase D: every run's root, the tile's root bitmap and the segments' root counts out.
-        auto root_of = [&](uint32_t id) -> uint32_t { return P[P[id & (NBLK - 1)]]; };
+        auto root_of = [&](uint32_t id) -> uint32_t { return P[P[id & (MAXRUN - 1)]]; };
         {
             uint32_t *rl = lab + t * kLabWords + kHdr;
             for (uint32_t i = 2 * tid; i < nrun; i += 2 * K1_NT)
                 rl[i >> 1] = root_of(i) | (root_of(i + 1 < nrun ? i + 1 : i) << 16);
         }
-        w.rbits[t * RBWORDS + tid] = 32u * tid < nrun ? BP[tid] : 0u;
+        if (tid < RBWORDS) w.rbits[t * RBWORDS + tid] = 32u * tid < nrun ? BP[tid] : 0u;
         if (tid < TH && tid < nrp) {   // runs [s, e) start in pixel row tid
-            const uint32_t b = WR[(tid >> 1) * WPR].w;
-            const uint32_t s = (tid & 1) ? b >> 16 : b & 0xFFFFu;
-            const uint32_t e = !(tid & 1) ? b >> 16 : (tid >> 1) + 1 < TBH ? WR[((tid >> 1) + 1) * WPR].w & 0xFFFFu : nrun;
+            const int br = tid / CELL;
+            const bool low = CELL == 2 && (tid & 1);
+            const uint32_t b = WR[br * WPR].w;
+            const uint32_t s = low ? b >> 16 : b & 0xFFFFu;
+            const uint32_t e = !low ? b >> 16 : br + 1 < TBH ? WR[(br + 1) * WPR].w & 0xFFFFu : nrun;
             uint32_t c = 0;
             for (uint32_t i = s >> 5; 32 * i < e; ++i)
                 c += __popc(BP[i] & (i == s >> 5 ? ~0u << (s & 31u) : ~0u) & (32 * i + 32 > e ? (1u << (e & 31u)) - 1u : ~0u));
@@ -404,13 +447,17 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
             prb[i] = kNone;
             if (p >= NPERIM || !perim_pos(p, nbr, nbc, br, bc)) continue;
             const int wi = br * WPR + (bc >> 5), k = bc & 31;
-            const uint4 cw = CW[wi];
-            const uint32_t m = ((cw.x >> k) & 1u) | (((cw.y >> k) & 1u) << 1) | (((cw.z >> k) & 1u) << 2) |
-                               (((cw.w >> k) & 1u) << 3);
-            if (!m) continue;
             const uint4 wr = WR[wi];
+            uint32_t m;
+            if constexpr (CELL == 2) {
+                const uint4 cw = CW[wi];
+                m = ((cw.x >> k) & 1u) | (((cw.y >> k) & 1u) << 1) | (((cw.z >> k) & 1u) << 2) | (((cw.w >> k) & 1u) << 3);
+            } else {
+                m = (wr.y >> k) & 1u;
+            }
+            if (!m) continue;
             const uint32_t upto = (2u << k) - 1u;
-            const uint32_t id = ((wr.z >> k) & 1u ? (wr.w & 0xFFFFu) + __popc(wr.x & upto) : (wr.w >> 16) + __popc(wr.y & upto)) - 1u;
+            const uint32_t id = (CELL == 1 || ((wr.z >> k) & 1u) ? (wr.w & 0xFFFFu) + __popc(wr.x & upto) : (wr.w >> 16) + __popc(wr.y & upto)) - 1u;
             (void)GUARD(w, id < nrun, 113, id);
             const uint32_t c = root_of(id);
             const uint32_t bit = 1u << (c & 31);
@@ -418,7 +465,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
             prb[i] = c | (m << 16) | ((old & bit) ? 0u : kOwner);
         }
         __syncthreads();   // node flags complete
-        {   // nodes before each word of flags, within the warp; the warps' totals beside them
+        if (tid < RBWORDS) {   // nodes before each word of flags, within the warp; the warps' totals beside them
             const uint32_t c = __popc(BF[tid]);
             uint32_t x = c;
 #pragma unroll
@@ -432,10 +479,10 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
         __syncthreads();
         // Every border position writes its entry; the position that claimed its node writes the
         // node's record.
-        uint32_t noff[K1_NT / 32 + 1];
+        uint32_t noff[RBWORDS / 32 + 1];
         noff[0] = 0;
 #pragma unroll
-        for (int i = 0; i < K1_NT / 32; ++i) noff[i + 1] = noff[i] + ntot[i];
+        for (int i = 0; i < RBWORDS / 32; ++i) noff[i + 1] = noff[i] + ntot[i];
 #pragma unroll
         for (int i = 0; i < (NPERIM + K1_NT - 1) / K1_NT; ++i) {
             const int p = tid + i * K1_NT;
@@ -453,9 +500,9 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
                     for (int h = TBH / 2; h; h >>= 1)
                         if ((WR[(row + h) * WPR].w & 0xFFFFu) <= c) row += h;
                     const uint32_t b = WR[row * WPR].w;
-                    const bool low = c >= b >> 16;   // a run without a top pixel
+                    const bool low = CELL == 2 && c >= b >> 16;   // a run without a top pixel
                     const uint32_t place = c - (low ? b >> 16 : b & 0xFFFFu);
-                    const int64_t seg = int64_t(y0 + 2 * row + (low ? 1 : 0)) * im.tiles_x + tx;
+                    const int64_t seg = int64_t(y0 + CELL * row + (low ? 1 : 0)) * im.tiles_x + tx;
                     const int64_t node = t * MAXB + j;
                     w.nroot[node] = uint16_t(c);
                     w.gp[node] = gentry(uint32_t(seg) * seg_width(im) + place, uint32_t(node));
@@ -463,7 +510,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
             }
             w.perim[t * NPERIM + p] = ent;
         }
-        if (tid == 0) w.nb[t] = noff[K1_NT / 32];
+        if (tid == 0) w.nb[t] = noff[RBWORDS / 32];
         __syncthreads();
     }
 }
@@ -521,8 +568,8 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
         const Img2D im = L.get(t);
         const int64_t lt = t - im.tile_base;
         const int ty = int(lt / im.tiles_x), tx = int(lt - int64_t(ty) * im.tiles_x);
-        const int nbr = (min(TH, im.rows - ty * TH) + 1) >> 1;
-        const int nbc = (min(TW, im.cols - tx * TW) + 1) >> 1;
+        const int nbr = cells(min(TH, im.rows - ty * TH));
+        const int nbc = cells(min(TW, im.cols - tx * TW));
         const uint16_t *pe = w.perim;
         for (int i = threadIdx.x; i < NLOC2; i += K2_NT) lp[i] = uint32_t(i);
         if (threadIdx.x == 0) nq = 0;
@@ -597,9 +644,10 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
 #pragma unroll
                     for (int d = -1; d <= 1; ++d) {
                         const int rr = p + d;
+                        if (CELL == 1 && d) continue;   // pixels: straight across only
                         if (rr < 0 || rr >= nbr || sid[rr] == kNone) continue;
                         const uint32_t mB = smk[rr];
-                        if (d == 0 ? ((mA & 0xAu) && (mB & 0x5u)) : d < 0 ? ((mA & 2u) && (mB & 4u)) : ((mA & 8u) && (mB & 1u)))
+                        if (CELL == 1 || (d == 0 ? ((mA & 0xAu) && (mB & 0x5u)) : d < 0 ? ((mA & 2u) && (mB & 4u)) : ((mA & 8u) && (mB & 1u))))
                             cb |= 1u << (d + 1);
                     }
                 } else {
@@ -608,9 +656,10 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
 #pragma unroll
                     for (int d = -1; d <= 1; ++d) {
                         const int k = c + d + 1;   // staged bottom index
+                        if (CELL == 1 && d) continue;
                         if (sid[TBH + k] == kNone) continue;
                         const uint32_t mB = smk[TBH + k];
-                        if (d == 0 ? ((mA & 0xCu) && (mB & 0x3u)) : d < 0 ? ((mA & 4u) && (mB & 2u)) : ((mA & 8u) && (mB & 1u)))
+                        if (CELL == 1 || (d == 0 ? ((mA & 0xCu) && (mB & 0x3u)) : d < 0 ? ((mA & 4u) && (mB & 2u)) : ((mA & 8u) && (mB & 1u))))
                             cb |= 1u << (d + 1);
                     }
                 }
@@ -694,7 +743,7 @@ constexpr int K3_PER_SM = 8;              // resident CTAs per SM
 __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L, Work w)
 {
     __shared__ __align__(16) uint4 H[kHdr / 4];   // class words, then run words
-    __shared__ uint32_t LT[NBLK + 1];     // label of run i at i + 1 (0: the place of "no run yet")
+    __shared__ uint32_t LT[MAXRUN + 1];   // label of run i at i + 1 (0: the place of "no run yet")
     constexpr int kStageRuns = 2048;      // run entries staged in shared memory (later ones: from L2)
     __shared__ __align__(16) uint32_t RB[RBWORDS + 1];
     __shared__ __align__(16) uint32_t E[kStageRuns / 2];
@@ -710,8 +759,8 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
     // With a fixed tile order (no work queue) the CTA fetches the next tile while it works on the
     // current one: its words into registers, the root bitmap and run entries into shared memory
     // (cp.async) as soon as the current tile's are used up.
-    static_assert(TBW % 64 == 0, "a warp's output units lie in one block row");
-    static_assert(kHdr == 4 * K3_NT && 2 * NWORD == K3_NT && kStageRuns == 8 * K3_NT, "prefetched words per thread");
+    static_assert(TW % 128 == 0, "a warp's output units lie in one row");
+    static_assert(kHdr == 4 * K3_NT && TH * WPR == K3_NT && kStageRuns == 8 * K3_NT, "prefetched words per thread");
     uint4 nH;
     uint32_t nNb = 0;
     auto fetch_words = [&](int64_t t) {
@@ -754,16 +803,19 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         if (lt == 0 && tid == 0)
             w.ncomp[im.index] = int64_t(w.segpref[im.seg_base + int64_t(im.rows) * im.tiles_x] - base0);
         __syncthreads();
-        const uint32_t nrun = (H[2 * NWORD - 1].w >> 16) + __popc(H[2 * NWORD - 1].y);   // the last B run is the last run
+        const uint4 *HR = H + kHdr / 4 - NWORD;   // run words
+        // The last B run is the last run.
+        const uint32_t nrun = (HR[NWORD - 1].w >> 16) + (CELL == 2 ? __popc(HR[NWORD - 1].y) : 0);
 
         // Surviving roots: rank = roots before it in its segment.  One thread per word and kind of run:
         // WPR consecutive lanes hold a segment's words, a shuffle scan gives each word's prefix, and the
         // word's runs are consecutive bits of the root bitmap.
         {
-            const int seg = tid / WPR, wi = (seg >> 1) * WPR + tid % WPR;   // segment = pixel row
-            const uint4 wr = H[NWORD + wi];
-            const uint32_t c = __popc((seg & 1) ? wr.y : wr.x), b = (seg & 1) ? wr.w >> 16 : wr.w & 0xFFFFu;
-            const uint32_t g = b >> 5;   // (RB has a word past its end for g = RBWORDS - 1 and b = NBLK)
+            const int seg = tid / WPR, wi = (seg / CELL) * WPR + tid % WPR;   // segment = pixel row
+            const bool low = CELL == 2 && (seg & 1);
+            const uint4 wr = HR[wi];
+            const uint32_t c = __popc(low ? wr.y : wr.x), b = low ? wr.w >> 16 : wr.w & 0xFFFFu;
+            const uint32_t g = b >> 5;   // (RB has a word past its end; b = MAXRUN only with c = 0)
             uint32_t bits = c ? __funnelshift_r(RB[g], RB[min(g + 1, uint32_t(RBWORDS))], b & 31u) & (0xFFFFFFFFu >> (32 - c)) : 0u;
             uint32_t pre = __popc(bits);
 #pragma unroll
@@ -801,16 +853,30 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         __syncthreads();
         if (tn >= 0) fetch_runs(tn);
 
-        // Output: one unit = two horizontally adjacent blocks = 4 pixels in each of 2 rows.
+        // Output: one unit = 4 pixels in each row of a block row (two 2x2 blocks, or four pixel cells).
         const bool vec_ok = ((reinterpret_cast<uintptr_t>(im.out) | uintptr_t(im.out_pitch * 4)) & 15) == 0;
         // A thread keeps its column: unit i is UR block rows further down.
-        constexpr int UPR = TBW / 2, UR = K3_NT / UPR;   // units per block row, block rows per turn
-        const int q = tid % UPR, k = 2 * (q & 15);
+        constexpr int UPR = TW / 4, UR = K3_NT / UPR;   // units per block row, block rows per turn
+        constexpr int UPW = CELL == 2 ? 16 : 8;         // units per word
+        const int q = tid % UPR, k = (32 / UPW) * (q % UPW);
         const uint32_t bit0 = 1u << k, bit1 = 2u << k, upto0 = bit0 | (bit0 - 1u), upto1 = bit1 | (bit1 - 1u);
         const int n = min(4, max(0, ncp - 4 * q));       // pixels of the thread's column inside the image
         auto unit = [&](int br, int4 &a, int4 &b) {
-            const int wi = br * WPR + (q >> 4);
-            const uint4 c = H[wi], wr = H[NWORD + wi];
+            const int wi = br * WPR + q / UPW;
+            if constexpr (CELL == 1) {
+                const uint4 wr = HR[wi];
+                const uint32_t st = wr.x >> k, f = wr.y >> k;
+                uint32_t i = (wr.w & 0xFFFFu) + __popc(wr.x & upto0);
+                a.x = (f & 1u) ? int(LT[i]) : 0;
+                i += (st >> 1) & 1u;
+                a.y = (f & 2u) ? int(LT[i]) : 0;
+                i += (st >> 2) & 1u;
+                a.z = (f & 4u) ? int(LT[i]) : 0;
+                i += (st >> 3) & 1u;
+                a.w = (f & 8u) ? int(LT[i]) : 0;
+                return;
+            }
+            const uint4 c = H[wi], wr = HR[wi];
             const uint32_t bT = wr.w & 0xFFFFu, bB = wr.w >> 16;
             const bool t0 = wr.z & bit0, t1 = wr.z & bit1;
             const int l0 = int(LT[(t0 ? bT : bB) + __popc((t0 ? wr.x : wr.y) & upto0)]);
@@ -820,14 +886,14 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             b.x = (c.z & bit0) ? l0 : 0; b.y = (c.w & bit0) ? l0 : 0;
             b.z = (c.z & bit1) ? l1 : 0; b.w = (c.w & bit1) ? l1 : 0;
         };
-        int32_t *dst = im.out + int64_t(y0 + 2 * (tid / UPR)) * im.out_pitch + x0 + 4 * q;
-        const int64_t turn = 2 * UR * im.out_pitch;
+        int32_t *dst = im.out + int64_t(y0 + CELL * (tid / UPR)) * im.out_pitch + x0 + 4 * q;
+        const int64_t turn = CELL * UR * im.out_pitch;
         if (vec_ok) {
             if (n > 0)
-                for (int br = tid / UPR; 2 * br < nrp; br += UR, dst += turn) {
+                for (int br = tid / UPR; CELL * br < nrp; br += UR, dst += turn) {
                     int4 a, b;
                     unit(br, a, b);
-                    const bool row2 = 2 * br + 1 < nrp;
+                    const bool row2 = CELL == 2 && 2 * br + 1 < nrp;
                     if (n == 4) {
                         __stcs(reinterpret_cast<int4 *>(dst), a);
                         if (row2) __stcs(reinterpret_cast<int4 *>(dst + im.out_pitch), b);
@@ -842,11 +908,11 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
                     }
                 }
         } else {
-            for (int br = tid / UPR; 2 * br < nrp; br += UR, dst += turn) {   // rows of any alignment (whole warps)
+            for (int br = tid / UPR; CELL * br < nrp; br += UR, dst += turn) {   // rows of any alignment (whole warps)
                 int4 a, b;
                 unit(br, a, b);
                 store_row<32>(dst, a, n);
-                if (2 * br + 1 < nrp) store_row<32>(dst + im.out_pitch, b, n);
+                if (CELL == 2 && 2 * br + 1 < nrp) store_row<32>(dst + im.out_pitch, b, n);
             }
         }
         __syncthreads();
