@@ -59,9 +59,9 @@ Geometry geometry_2d() { return uf2d_geometry(0); }
 Geometry geometry_3d()
 {
     Geometry g;
-    g.lab_bytes_per_tile = size_t(T3_NBLK) * sizeof(uint32_t);
-    g.rbits_bytes_per_tile = size_t(2 * T3_TB0) * (2 * T3_TB1) * (2 * T3_TB2 / 32) * sizeof(uint32_t);
-    g.nperim = T3_NPERIM;
+    g.lab_bytes_per_tile = size_t(T3_LAB_WORDS) * sizeof(uint32_t);
+    g.rbits_bytes_per_tile = size_t(T3_NROW) * sizeof(uint32_t);
+    g.nperim = T3_EDGE;
     g.maxb = T3_MAXB;
     g.links = true;
     return g;
@@ -217,8 +217,8 @@ cudaError_t launch_uf3d(const ImgList3D &L, const Work &w, int sms, bool persist
     mark(2);
     keep(launch_k(k_scan_link_3d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, L, wk));
     mark(3);
-    // The label writes run a fixed tile order over 5 CTAs per SM (they prefetch their next tile).
-    keep(launch_k(k_tile_write_3d, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * 5))),
+    // The label writes run a fixed tile order over kT3WritePerSM CTAs per SM (they prefetch their next tile).
+    keep(launch_k(k_tile_write_3d, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * kT3WritePerSM))),
                   kT3Threads, s, ov, L, wk));
     mark(4);
     return e;

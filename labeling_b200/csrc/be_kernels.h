@@ -16,8 +16,11 @@
 #define T3_TB1 16
 #define T3_TB2 32
 #define T3_NBLK (T3_TB0 * T3_TB1 * T3_TB2)
+#define T3_NROW (T3_TB0 * T3_TB1)
+#define T3_LAB_WORDS (13 * T3_NROW + T3_NBLK / 2)   // tile words and run entries
 #define T3_NPERIM (2 * (T3_TB0 * T3_TB1 + T3_TB0 * T3_TB2 + T3_TB1 * T3_TB2))
 #define T3_MAXB T3_NPERIM
+#define T3_EDGE (T3_NBLK + 2 * T3_NROW + T3_NROW / 2)   // uint16 words of a tile's border data
 
 namespace be {
 
@@ -33,8 +36,9 @@ constexpr int kPostThreads = 128;   // k_chunk_sums
 constexpr int kT3Threads = 256;
 constexpr int kT3LocalThreads = T3_TB0 * T3_TB1;   // k_tile_local_3d: one thread per block row
 constexpr int kT3LocalPerSM = 7;   // k_tile_local_3d: resident CTAs per SM (31 KB of shared memory each)
+constexpr int kT3WritePerSM = 5;   // k_tile_write_3d: resident CTAs per SM
 constexpr int kT3MergeThreads = 128;   // k_merge_3d threads
-constexpr int kT3MergePerSM = 9;       // k_merge_3d: tiles in flight per SM (23.5 KB of shared memory each)
+constexpr int kT3MergePerSM = 16;      // k_merge_3d: tiles in flight per SM
 constexpr int kScanThreads = 256;
 
 }  // namespace be

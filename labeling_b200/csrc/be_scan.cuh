@@ -145,8 +145,8 @@ __device__ __forceinline__ void flatten_tile_nodes(Work &w, int64_t t, int maxb)
 
 // As flatten_tile_nodes, and resolves each node's link for the label writes: nlink[node] =
 // (segment of the root's first pixel, (node's root block << 16) | rank of that pixel among the
-// roots left in its segment), or x = kNone for a node that is a root.  locate(key, &seg, &rank)
-// finds the segment and the rank of the pixel with raster key `key` from the root bitmaps, which
+// roots left in its segment), or x = kNone for a node that is a root.  locate(root, key, &seg, &rank)
+// finds the segment and the rank of the root node with its key from the root bitmaps, which
 // the merge has left final.  Called by a whole CTA.
 template <typename Locate>
 __device__ __forceinline__ void link_tile_nodes(Work &w, int64_t t, int maxb, Locate locate)
@@ -160,7 +160,7 @@ __device__ __forceinline__ void link_tile_nodes(Work &w, int64_t t, int maxb, Lo
             const unsigned long long re = w.gp[root];
             w.gp[node] = re;
             uint32_t seg, rank;
-            locate(uint32_t(re >> 32), seg, rank);
+            locate(root, uint32_t(re >> 32), seg, rank);
             link = make_uint2(seg, (uint32_t(w.nroot[node]) << 16) | rank);
         }
         w.nlink[node] = link;

@@ -6,17 +6,18 @@
 //
 //   k_tile_local_3d   one CTA per 16 x 32 x 64-voxel tile (8 x 16 x 32 blocks): 16-byte loads,
 //                     voxel-class words per block row, runs along d2 and their links to the four
-//                     preceding rows by bit operations, a shared-memory union-find over runs (the
-//                     run of the component's first voxel stays the root), one uint32 per block,
-//                     segment root counts, a per-tile bitmap of component first voxels, border
-//                     components exported as nodes.
-//   k_merge_3d        global union-find over nodes across the +d0 / +d1 / +d2 tile faces; a root
-//                     linked under another leaves its segment count and its tile's bitmap.
+//                     preceding rows by bit operations, a shared-memory union-find over run numbers
+//                     (the run of the component's first voxel stays the root); writes the tile's bit
+//                     words, the root run of every run, a bitmap of the root runs and the segments'
+//                     root counts, and exports border components as nodes.
+//   k_merge_3d        links of block rows across tile borders, and the global union-find over the nodes
+//                     they join; a root linked under another leaves its segment count and its
+//                     tile's bitmap.
 //   k_scan_link_3d    exclusive scan of the segment counts (single pass, look-back) and, in the
 //                     same launch, every linked node pointed at its global root with the segment
 //                     and in-segment rank of that root's first voxel resolved.
-//   k_tile_write_3d   resolves canonical labels (segment prefix + rank in the bitmap row) and
-//                     writes int32 voxels with 16-byte stores.
+//   k_tile_write_3d   resolves the label of every run (segment prefix + rank among the segment's roots)
+//                     and writes int32 voxels with 16-byte stores.
 //
 // Volume layout is the reference's cv::Mat 3-D order [d0][d1][d2] with d2 fastest
 // (Read3DImage, main.cpp:191-203; kernel addressing x*h*d + y*d + z, LabelingAlgs.cl:974).
@@ -28,9 +29,10 @@
 // 0 of A and offset 1 of B can touch, along an axis with d = 0 every offset can.  This is the
 // predicate the reference evaluates voxel by voxel with TEST_CONN1/2/4 (LabelingAlgs.cl:770-856).
 //
-// Within a tile the union-find entries carry the slot (b0, i, b1, j, b2) of a run's first voxel,
-// whose order is the raster order of first voxels, and the atomicMin union keeps the smaller slot as
-// the root: the root run of a component holds its first voxel.
+// Within a tile runs are numbered by block row; the union-find entries carry the slot (b0, i, b1, j, b2)
+// of a run, (i, j) being the voxel row of its first voxel, whose order is the raster order of first
+// voxels, and the atomicMin union keeps the smaller slot as the root: the root run of a component holds
+// its first voxel.
 #include "be_common.cuh"
 #include "be_kernels.h"
 #include "be_scan.cuh"
@@ -42,52 +44,41 @@ namespace {
 constexpr int TB0 = T3_TB0, TB1 = T3_TB1, TB2 = T3_TB2;   // tile in blocks
 constexpr int TX = 2 * TB0, TY = 2 * TB1, TZ = 2 * TB2;   // tile in voxels
 constexpr int NBLK = T3_NBLK;
-constexpr int NPERIM = T3_NPERIM;
 constexpr int MAXB = T3_MAXB;
 constexpr int NT = kT3Threads;
-constexpr int RBW = TZ / 32;                // root-bitmap words per voxel row
-constexpr uint32_t ROOT_FLAG = 1u << 23;
+constexpr int NROW = T3_NROW;               // block rows along d2 per tile: one 32-bit word each
 
-static_assert(NBLK <= (1 << 13), "tile-local block index must fit the entry payload");
-static_assert(TX * TY * TZ <= (1 << 23), "tile-local key must fit the entry payload");
-static_assert(NPERIM < 65536 && MAXB < 4096, "border encodings");
+static_assert(TB2 == 32, "a block row along d2 is one 32-bit word");
+static_assert(NBLK <= 4096, "a run number must fit 12 bits");
+static_assert(MAXB <= 2048, "node indices of the merge queue");
 
-__device__ __forceinline__ int blk(int b0, int b1, int b2) { return (b0 * TB1 + b1) * TB2 + b2; }
+// A tile's border as the merge kernel reads it (Work::perim, uint16): for every run the node of its
+// component, where that is one (T3_NBLK); for every block row the nodes of its first and last block's
+// runs, low and high half of a word (2 * NROW); and for every block row the voxels of the first block on
+// the - d2 face and of the last block on the + d2 face, as bits 2i + j of the low and high half of a
+// byte (NROW / 2).
+constexpr int kZNode = NBLK, kZFace = NBLK + 2 * NROW;
+static_assert(T3_EDGE == kZFace + NROW / 2 && T3_EDGE % 2 == 0, "border words");
+constexpr uint32_t kNoNode = 0xFFFFu;
 
-// Highest set bit of x (x != 0).
-__device__ __forceinline__ uint32_t hibit3(uint32_t x) { return 31u - __clz(x); }
+// A tile's labels as the write kernel reads them (Work::lab), in 32-bit words: the voxel-class words
+// 0..3 and 4..7 of its block rows (two arrays of uint4), (run starts, runs before, starts whose first
+// voxel is of voxel row (0, 0), of (0, 1)) and the starts of voxel row (1, 0) per row, then the root run
+// of every run (uint16).
+constexpr int kHdr3 = 13 * NROW;
+static_assert(T3_LAB_WORDS == kHdr3 + NBLK / 2, "tile words");
 
-// Tile-local key of the first voxel of a block.
-__device__ __forceinline__ uint32_t local_key(int b, uint32_t m)
+// Of the starts, those of voxel row ij (2i + j) of their block row: the four sets of `first voxel in that
+// voxel row`.
+__device__ __forceinline__ uint32_t starts_of(int ij, uint32_t S, uint32_t S00, uint32_t S01, uint32_t S10)
 {
-    const int v = __ffs(m) - 1;
-    const int b2 = b % TB2, b1 = (b / TB2) % TB1, b0 = b / (TB1 * TB2);
-    const int X = 2 * b0 + (v >> 2), Y = 2 * b1 + ((v >> 1) & 1), Z = 2 * b2 + (v & 1);
-    return uint32_t((X * TY + Y) * TZ + Z);
+    return ij == 0 ? S00 : ij == 1 ? S01 : ij == 2 ? S10 : S & ~(S00 | S01 | S10);
 }
 
-// Border faces: 0 = -d0, 1 = +d0, 2 = -d1, 3 = +d1, 4 = -d2, 5 = +d2.
-__device__ __forceinline__ int face_base(int f)
-{
-    constexpr int sz[6] = {TB1 * TB2, TB1 * TB2, TB0 * TB2, TB0 * TB2, TB0 * TB1, TB0 * TB1};
-    int b = 0;
-    for (int i = 0; i < f; ++i) b += sz[i];
-    return b;
-}
-
-// The four voxels of a block on face f, as bits (a*2 + b) over the two tangent axes in order.
-__device__ __forceinline__ uint32_t face_bits(uint32_t m, int f)
-{
-    // Mask bit v = 4i + 2j + k; the face's four voxels in the order (first tangent, second).
-    const uint32_t s = uint32_t(f & 1);
-    switch (f >> 1) {
-    case 0: return (m >> (4 * s)) & 0xFu;                                          // (j, k)
-    case 1: return ((m >> (2 * s)) & 3u) | (((m >> (4 + 2 * s)) & 3u) << 2);       // (i, k)
-    default:                                                                        // (i, j)
-        return ((m >> s) & 1u) | (((m >> (2 + s)) & 1u) << 1) | (((m >> (4 + s)) & 1u) << 2) |
-               (((m >> (6 + s)) & 1u) << 3);
-    }
-}
+// Global keys: segment (one voxel row inside one tile, numbered in raster order) * seg_width + the place
+// of the root run among the runs whose first voxel is in that segment -- the order of the components'
+// first voxels.
+__device__ __forceinline__ uint32_t seg_width3(const Img3D &im) { return uint32_t(min(im.d2, TZ) + 1) >> 1; }
 
 // Selector over face bits (a*2 + b) for the tangent offsets (da, db).
 __device__ __forceinline__ uint32_t face_sel(int da, int db)
@@ -117,21 +108,6 @@ __device__ __forceinline__ TileGeo tile_geo(const Img3D &im, int64_t t)
     return g;
 }
 
-// Block position of border position p (face f, index q), when valid for this tile.
-__device__ __forceinline__ bool perim_pos3(int p, const TileGeo &g, int &f, int &b0, int &b1, int &b2)
-{
-    constexpr int F0 = TB1 * TB2, F1 = TB0 * TB2;   // positions on a d0 face, on a d1 face
-    int q;
-    if (p < 2 * F0) { f = p >= F0; q = p - f * F0; }
-    else if (p < 2 * F0 + 2 * F1) { const int r = p - 2 * F0; f = 2 + (r >= F1); q = r - (f - 2) * F1; }
-    else { const int r = p - 2 * F0 - 2 * F1; f = 4 + (r >= TB0 * TB1); q = r - (f - 4) * TB0 * TB1; }
-    const int axis = f >> 1, hi = f & 1;
-    if (axis == 0) { b0 = hi ? g.n0 - 1 : 0; b1 = q / TB2; b2 = q % TB2; }
-    else if (axis == 1) { b1 = hi ? g.n1 - 1 : 0; b0 = q / TB2; b2 = q % TB2; }
-    else { b2 = hi ? g.n2 - 1 : 0; b0 = q / TB1; b1 = q % TB1; }
-    return b0 < g.n0 && b1 < g.n1 && b2 < g.n2;
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------
@@ -143,9 +119,10 @@ __device__ __forceinline__ bool perim_pos3(int p, const TileGeo &g, int &f, int 
 namespace {
 
 constexpr int NT1 = kT3LocalThreads;   // threads of the tile-local kernel: one per block row
-constexpr int MQ1 = 1024;          // union-queue capacity (more are merged in place)
-static_assert(TB2 == 32, "a block row along d2 is one 32-bit word");
-static_assert(NBLK <= 4096, "run starts must fit 12 bits");
+static_assert(NT1 == NROW && NT1 == 128, "thread layout");
+constexpr int kRawWords = 3 * 4 * NROW;         // raw links of the rows (three uint4 per row)
+constexpr int MQ1 = 2048;                       // union-queue capacity (more take further rounds)
+static_assert(kRawWords <= MQ1, "the raw links live in the queue's memory");
 
 // Word of the blocks whose side toward (dx, dy, dz) holds a foreground voxel: the OR of the
 // classes with offset 0 along an axis where d < 0, offset 1 where d > 0.
@@ -163,33 +140,24 @@ __device__ __forceinline__ uint32_t face_word(const uint32_t (&c)[8])
     return r;
 }
 
-// Slot of a block with first voxel offsets (i, j): the raster order of first voxels is the order
-// of (b0, i, b1, j, b2) (b2 decides last: blocks of one row and class differ only there).
-__device__ __forceinline__ uint32_t slot3(int b0, int i, int b1, int j, int b2)
+// Slot of the run that starts at block b2 of row (b0, b1) and has its first voxel in the row's voxel
+// row ij = 2i + j: the raster order of first voxels is the order of (b0, i, b1, j) and, in one voxel
+// row, the order of the runs.
+__device__ __forceinline__ uint32_t slot3(uint32_t b0, uint32_t b1, uint32_t ij, uint32_t b2)
 {
-    return uint32_t((((b0 * 2 + i) * TB1 + b1) * 2 + j) * TB2 + b2);
+    return (((b0 * 2 + (ij >> 1)) * TB1 + b1) * 2 + (ij & 1)) * TB2 + b2;
 }
 
-__device__ __forceinline__ uint32_t slot_block(uint32_t slot)
+// Union-find over run numbers, the slot carried in the entry: (slot << 12) | parent, a root holding its
+// own.  The union (atomicMin of the smaller entry into the other root, Playne-Hawick) leaves the run
+// of the first voxel as the root.
+__device__ __forceinline__ uint32_t efind3(uint32_t *P, uint32_t x, uint32_t &ev)
 {
-    const uint32_t b2 = slot % TB2, b1 = (slot / (2 * TB2)) % TB1, b0 = slot / (4 * TB2 * TB1);
-    return (b0 * TB1 + b1) * TB2 + b2;
-}
-
-// Shared-memory position of block x's union-find entry: the low five bits (the block's place along
-// d2) are XOR-ed with its row, so that the 32 lanes of a warp -- 32 rows walking the same position
-// -- reach 32 different banks.  Entries still name blocks by their plain index.
-__device__ __forceinline__ uint32_t sw3(uint32_t x) { return x ^ ((x >> 5) & 31u); }
-
-// Union-find over run starts, the slot carried in the entry: (slot << 12) | parent.  The find
-// (path halving) returns the root and the root's own entry as read (the union compares the two).
-__device__ __forceinline__ uint32_t efind3_e(uint32_t *P, uint32_t x, uint32_t &ev)
-{
-    uint32_t v = P[sw3(x)];
+    uint32_t v = P[x];
     while ((v & 0xFFFu) != x) {
         const uint32_t y = v & 0xFFFu;
-        const uint32_t vg = P[sw3(y)];
-        if ((vg & 0xFFFu) != y) P[sw3(x)] = vg;
+        const uint32_t vg = P[y];
+        if ((vg & 0xFFFu) != y) P[x] = vg;   // path halving
         x = y;
         v = vg;
     }
@@ -201,23 +169,100 @@ __device__ __forceinline__ void eunion3(uint32_t *P, uint32_t a, uint32_t b)
 {
     for (;;) {
         uint32_t ea, eb;
-        a = efind3_e(P, a, ea);
-        b = efind3_e(P, b, eb);
+        a = efind3(P, a, ea);
+        b = efind3(P, b, eb);
         if (a == b) return;
-        if (ea < eb) {
-            const uint32_t old = atomicMin(&P[sw3(b)], ea);
-            if ((old & 0xFFFu) == b) return;
-            b = old & 0xFFFu;
-        } else {
-            const uint32_t old = atomicMin(&P[sw3(a)], eb);
-            if ((old & 0xFFFu) == a) return;
-            a = old & 0xFFFu;
-        }
+        const uint32_t hi = ea < eb ? b : a;
+        const uint32_t old = atomicMin(&P[hi], min(ea, eb)) & 0xFFFu;
+        if (old == hi) return;
+        b = ea < eb ? a : b;
+        a = old;
     }
 }
 
-// Bits 0..3 of x -> bit 0 of bytes 0..3.
-__device__ __forceinline__ uint32_t spread4b(uint32_t x) { return ((x & 0xFu) * 0x00204081u) & 0x01010101u; }
+// As sflatten_all, on entries: every run's entry becomes its root's.
+__device__ __forceinline__ void eflatten3_all(uint32_t *P, uint32_t first, uint32_t step, uint32_t n)
+{
+    for (uint32_t i = first; i < n; i += step) {
+        uint32_t x = P[i] & 0xFFFu;
+        if (x == i) continue;
+        uint32_t v = P[x];
+        while ((v & 0xFFFu) != x) {
+            x = v & 0xFFFu;
+            v = P[x];
+        }
+        P[i] = v;
+    }
+}
+
+// As shook_pairs, on entries.
+__device__ __forceinline__ uint32_t ehook3_pairs(uint32_t *P, uint32_t *q, uint32_t n)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t kept = 0;
+    for (uint32_t k = 0; k < n; k += 32) {
+        uint32_t x = 0, y = 0;
+        if (k + lane < n) {
+            const uint32_t e = q[k + lane];
+            x = P[e >> 16];
+            y = P[e & 0xFFFFu];
+        }
+        const uint32_t keep = __ballot_sync(0xFFFFFFFFu, x != y);
+        if (x != y) {
+            atomicMin(&P[max(x, y) & 0xFFFu], min(x, y));
+            q[kept + __popc(keep & ((1u << lane) - 1u))] = ((x & 0xFFFu) << 16) | (y & 0xFFFu);
+        }
+        kept += __popc(keep);
+    }
+    __syncwarp();
+    return kept;
+}
+
+// Of the run starts S, those whose run holds a bit of x (every bit of x lies in a run): from each bit a
+// carry runs down -- in reversed bits -- to the start it belongs to.
+__device__ __forceinline__ uint32_t starts_with(uint32_t S, uint32_t x)
+{
+    const uint32_t rS = __brev(S), rx = __brev(x);
+    return __brev(((~rS + (rx & ~rS)) | rx) & rS);
+}
+
+// Links of a block row (classes c, joins hz) to its preceding row nr -- 0..2: d0-1 with d1-1 / d1 / d1+1,
+// 3: d0 with d1-1 -- whose classes are ua, ub and joins uhz, at the offsets dz = 0 / -1 / +1 along d2 (n /
+// w / e).  raw: as found.  Returned: without those that an earlier one (further along d2, or dz = 0
+// before dz = +-1 at the same block) stands for because it joins the same two runs.
+struct Links {
+    uint32_t n, w, e;
+};
+__device__ __forceinline__ Links row_links(int nr, const uint32_t (&c)[8], uint32_t hz, uint4 ua, uint4 ub, uint32_t uhz,
+                                           Links &raw)
+{
+    const uint32_t u[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
+    uint32_t A0, Am, Ap, B0, Bm, Bp;   // own sides toward dz = 0/-1/+1, neighbour's opposite sides
+    if (nr == 0) {
+        A0 = face_word<-1, -1, 0>(c); Am = face_word<-1, -1, -1>(c); Ap = face_word<-1, -1, 1>(c);
+        B0 = face_word<1, 1, 0>(u); Bm = face_word<1, 1, 1>(u); Bp = face_word<1, 1, -1>(u);
+    } else if (nr == 1) {
+        A0 = face_word<-1, 0, 0>(c); Am = face_word<-1, 0, -1>(c); Ap = face_word<-1, 0, 1>(c);
+        B0 = face_word<1, 0, 0>(u); Bm = face_word<1, 0, 1>(u); Bp = face_word<1, 0, -1>(u);
+    } else if (nr == 2) {
+        A0 = face_word<-1, 1, 0>(c); Am = face_word<-1, 1, -1>(c); Ap = face_word<-1, 1, 1>(c);
+        B0 = face_word<1, -1, 0>(u); Bm = face_word<1, -1, 1>(u); Bp = face_word<1, -1, -1>(u);
+    } else {
+        A0 = face_word<0, -1, 0>(c); Am = face_word<0, -1, -1>(c); Ap = face_word<0, -1, 1>(c);
+        B0 = face_word<0, 1, 0>(u); Bm = face_word<0, 1, 1>(u); Bp = face_word<0, 1, -1>(u);
+    }
+    const uint32_t hl = hz << 1, uhl = uhz << 1;
+    raw = Links{A0 & B0, Am & (Bm << 1), Ap & (Bp >> 1)};
+    const uint32_t Nsh = raw.n << 1, NEsh = raw.e << 1;
+    return Links{raw.n & ~(hl & ((Nsh & uhl) | NEsh)), raw.w & ~((raw.n & uhl) | (hl & Nsh)),
+                 raw.e & ~((raw.n & uhz) | (hl & NEsh & uhz))};
+}
+
+// Joins along d2 of a row's classes: bit k, block k touches block k + 1.
+__device__ __forceinline__ uint32_t row_joins(const uint32_t (&c)[8])
+{
+    return face_word<0, 0, 1>(c) & (face_word<0, 0, -1>(c) >> 1);
+}
 
 // row_bits out of line: inlined into the four unrolled rows it slowed the aligned path by 1%.
 __device__ __noinline__ uint2 row_bits_call(const uint8_t *p, int n, const uint8_t *lo, const uint8_t *hi,
@@ -237,22 +282,19 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
         w.epoch[0] += 1u;
         w.epoch[1] = 0u;
     }
-    __shared__ uint32_t P[NBLK];               // run starts: (slot << 12) | parent
-    __shared__ __align__(16) uint8_t M[NBLK];  // block masks
-    __shared__ uint32_t CW[8][NT1];            // class words of every row
-    __shared__ uint32_t WHZ[NT1], WS[NT1];     // joins along d2, run starts
-    __shared__ uint32_t BF[NBLK / 32];
-    __shared__ uint32_t BP[NBLK / 32];
-    __shared__ uint32_t MQ[MQ1];               // union queue: (block_a << 16) | block_b
-    static_assert(TX * TY * RBW <= MQ1, "the root bitmap fits the queue's memory");
-    uint32_t *const RB = MQ;                   // root bitmap (after the unions)
-    __shared__ uint32_t mqn[4];                // queue counts of the union rounds
-    __shared__ uint32_t tmp[NT1 / 32 + 1];
+    __shared__ uint32_t P[NBLK];               // per run: (slot << 12) | parent
+    __shared__ __align__(16) uint4 CA[NROW], CB[NROW];   // class words 0..3, 4..7 of every row
+    __shared__ __align__(16) uint4 WR[NROW];   // run starts, joins along d2, runs before, -
+    __shared__ __align__(16) uint32_t MQ[MQ1]; // raw links, then the union queue: (run_a << 16) | run_b
+    __shared__ uint32_t BF[NBLK / 32];         // runs that are border components
+    __shared__ uint32_t BP[NBLK / 32];         // nodes before each word of BF
+    __shared__ uint32_t mqn;
+    __shared__ uint32_t wtot[NT1 / 32], ntot[NBLK / 32 / 32];
     __shared__ uint32_t qslot;
+    uint4 *const RW = reinterpret_cast<uint4 *>(MQ);   // raw links: of row r straight below, below right, beside
 
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b0 = tid / TB1, b1 = tid % TB1;
-    const uint32_t rowb = uint32_t(tid) * TB2;   // block index of the row's first block
     uint32_t *lab = reinterpret_cast<uint32_t *>(w.lab);
     ItemLoop loop{w.queue ? w.queue + 0 : nullptr, w.n_tiles};
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
@@ -263,9 +305,9 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
         const int64_t rs0 = int64_t(im.d1) * im.d2;   // stride of d0 in voxels
 
         BF[tid] = 0;
-        if (tid < 4) mqn[tid] = 0;
+        if (tid == 0) mqn = 0;
 
-        // Phase A: class words, runs along d2, run slots.
+        // Phase A: class words, runs along d2, run numbers.
         uint32_t c[8];
 #pragma unroll
         for (int v = 0; v < 8; ++v) c[v] = 0;
@@ -299,582 +341,446 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
             }
         }
         const uint32_t Fw = c[0] | c[1] | c[2] | c[3] | c[4] | c[5] | c[6] | c[7];
-        const uint32_t hz = face_word<0, 0, 1>(c) & (face_word<0, 0, -1>(c) >> 1);   // k joined to k + 1
+        const uint32_t hz = row_joins(c);                                          // k joined to k + 1
         const uint32_t hl = hz << 1;                                               // k joined to k - 1
         const uint32_t S = Fw & ~hl;
+        // The voxel row of each run's first voxel.
+        const uint32_t S00 = starts_with(S, c[0] | c[1]);
+        const uint32_t S01 = starts_with(S, c[2] | c[3]) & ~S00;
+        const uint32_t S10 = starts_with(S, c[4] | c[5]) & ~(S00 | S01);
+        uint32_t incl = __popc(S);
 #pragma unroll
-        for (int v = 0; v < 8; ++v) CW[v][tid] = c[v];
-        WHZ[tid] = hz;
-        WS[tid] = S;
-        {
-            uint32_t mw[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                uint32_t m = 0;
-#pragma unroll
-                for (int v = 0; v < 8; ++v) m |= spread4b(c[v] >> (4 * q)) << v;
-                mw[q] = m;
-            }
-            uint4 *md = reinterpret_cast<uint4 *>(&M[rowb]);
-            md[0] = make_uint4(mw[0], mw[1], mw[2], mw[3]);
-            md[1] = make_uint4(mw[4], mw[5], mw[6], mw[7]);
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += v;
         }
+        if (lane == 31) wtot[warp] = incl;
+        CA[tid] = make_uint4(c[0], c[1], c[2], c[3]);
+        CB[tid] = make_uint4(c[4], c[5], c[6], c[7]);
+        WR[tid] = make_uint4(S, hz, incl - __popc(S), 0u);
         __syncthreads();
+        uint32_t woff = 0, nrun = 0;
+#pragma unroll
+        for (int i = 0; i < NT1 / 32; ++i) {
+            const uint32_t n = wtot[i];
+            if (i < warp) woff += n;
+            nrun += n;
+        }
+        const uint32_t base = woff + incl - __popc(S);
+        {
+            uint32_t *h = lab + t * T3_LAB_WORDS;
+            reinterpret_cast<uint4 *>(h)[tid] = make_uint4(c[0], c[1], c[2], c[3]);
+            reinterpret_cast<uint4 *>(h)[NROW + tid] = make_uint4(c[4], c[5], c[6], c[7]);
+            reinterpret_cast<uint4 *>(h)[2 * NROW + tid] = make_uint4(S, base, S00, S01);
+            h[12 * NROW + tid] = S10;
+        }
 
-        // Phase B: links to the four preceding rows (d0-1 with d1-1 / d1 / d1+1, and d0 with
-        // d1-1), each with offsets dz = -1 / 0 / +1 along d2.  As in 2D, a link is dropped when
-        // an earlier one (further along d2, or dz = 0 before dz = +-1 at the same block) joins the
-        // same two runs.
+        // Phase B: links to the four preceding rows, as found and with the ones dropped that an earlier
+        // link to the same row stands for.
         uint32_t LN[4], LW[4], LE[4];
-        int UR[4];
+        uint32_t n1 = 0, w1 = 0, e1 = 0, n3 = 0, w3 = 0, e3 = 0;   // as found, straight below and beside
+        uint32_t n2 = 0, w2 = 0, e2 = 0;                           // below right
 #pragma unroll
         for (int nr = 0; nr < 4; ++nr) {
-            const int dx = nr < 3 ? -1 : 0, dy = nr < 3 ? nr - 1 : -1;
-            const int r0 = b0 + dx, r1 = b1 + dy;
-            uint32_t N = 0, NW = 0, NE = 0;
-            int ur = 0;
+            const int r0 = b0 + (nr < 3 ? -1 : 0), r1 = b1 + (nr < 3 ? nr - 1 : -1);
+            Links l{0u, 0u, 0u}, raw{0u, 0u, 0u};
             if (Fw && r0 >= 0 && r1 >= 0 && r1 < TB1) {
-                ur = r0 * TB1 + r1;
-                uint32_t u[8];
-#pragma unroll
-                for (int v = 0; v < 8; ++v) u[v] = CW[v][ur];
-                uint32_t A0, Am, Ap, B0, Bm, Bp;   // own sides toward dz = 0/-1/+1, neighbour's opposite sides
-                if (nr == 0) {
-                    A0 = face_word<-1, -1, 0>(c); Am = face_word<-1, -1, -1>(c); Ap = face_word<-1, -1, 1>(c);
-                    B0 = face_word<1, 1, 0>(u); Bm = face_word<1, 1, 1>(u); Bp = face_word<1, 1, -1>(u);
-                } else if (nr == 1) {
-                    A0 = face_word<-1, 0, 0>(c); Am = face_word<-1, 0, -1>(c); Ap = face_word<-1, 0, 1>(c);
-                    B0 = face_word<1, 0, 0>(u); Bm = face_word<1, 0, 1>(u); Bp = face_word<1, 0, -1>(u);
-                } else if (nr == 2) {
-                    A0 = face_word<-1, 1, 0>(c); Am = face_word<-1, 1, -1>(c); Ap = face_word<-1, 1, 1>(c);
-                    B0 = face_word<1, -1, 0>(u); Bm = face_word<1, -1, 1>(u); Bp = face_word<1, -1, -1>(u);
-                } else {
-                    A0 = face_word<0, -1, 0>(c); Am = face_word<0, -1, -1>(c); Ap = face_word<0, -1, 1>(c);
-                    B0 = face_word<0, 1, 0>(u); Bm = face_word<0, 1, 1>(u); Bp = face_word<0, 1, -1>(u);
-                }
-                const uint32_t uhz = WHZ[ur], uhl = uhz << 1;
-                const uint32_t n0 = A0 & B0, nw = Am & (Bm << 1), ne = Ap & (Bp >> 1);
-                const uint32_t Nsh = n0 << 1, NEsh = ne << 1;
-                N = n0 & ~(hl & ((Nsh & uhl) | NEsh));
-                NW = nw & ~((n0 & uhl) | (hl & Nsh));
-                NE = ne & ~((n0 & uhz) | (hl & NEsh & uhz));
+                const int ur = r0 * TB1 + r1;
+                l = row_links(nr, c, hz, CA[ur], CB[ur], WR[ur].y, raw);
             }
-            LN[nr] = N;
-            LW[nr] = NW;
-            LE[nr] = NE;
-            UR[nr] = ur;
+            if (nr == 1) { n1 = raw.n; w1 = raw.w; e1 = raw.e; }
+            if (nr == 2) { n2 = raw.n; w2 = raw.w; e2 = raw.e; }
+            if (nr == 3) { n3 = raw.n; w3 = raw.w; e3 = raw.e; }
+            LN[nr] = l.n;
+            LW[nr] = l.w;
+            LE[nr] = l.e;
         }
-        auto start_of = [&](uint32_t b) -> uint32_t {
-            return (b & ~31u) + hibit3(WS[b >> 5] & ((2u << (b & 31u)) - 1u));
-        };
-        // Every run of this row gets its entry.  A run with a link into the preceding layer (d0 - 1,
-        // whose slots are all smaller than this row's) takes the first one as its parent by a plain
-        // store; the entry holds key 0, the smallest value, so no atomicMin of a union changes it and
-        // unions walk on to the parent (only a root's key is ever compared).  These links leave the
-        // queue.  Links within the same layer (d1 - 1) may go to larger slots and stay unions.  Any
-        // other run is a root for now: (slot << 12) | itself, the slot being that of its first voxel.
-        // (Pointer jumping over the forest before the unions was measured slower.)
-        {
-            const uint32_t H00 = c[0] | c[1], H01 = c[2] | c[3], H10 = c[4] | c[5], H11 = c[6] | c[7];
-            uint32_t ss = S;
-            while (ss) {
-                const uint32_t s0 = __ffs(ss) - 1;
-                ss &= ss - 1;
-                const uint32_t brk = ~hz & (~0u << s0);
-                const uint32_t e = brk ? uint32_t(__ffs(brk) - 1) : 31u;
-                const uint32_t span = (~0u << s0) & (0xFFFFFFFFu >> (31u - e));
-                const uint32_t x = rowb + s0;
-                bool found = false;
-#pragma unroll
-                for (int nr = 0; nr < 3; ++nr) {
-                    const uint32_t lk = (LN[nr] | LW[nr] | LE[nr]) & span;
-                    if (found || !lk) continue;
-                    found = true;
-                    const uint32_t k = __ffs(lk) - 1, bit = 1u << k;
-                    const uint32_t ubase = uint32_t(UR[nr]) * TB2;
-                    uint32_t tgt;
-                    if (LN[nr] & bit) {
-                        tgt = ubase + k;
-                        LN[nr] &= ~bit;
-                    } else if (LW[nr] & bit) {
-                        tgt = ubase + k - 1;
-                        LW[nr] &= ~bit;
-                    } else {
-                        tgt = ubase + k + 1;
-                        LE[nr] &= ~bit;
-                    }
-                    P[sw3(x)] = start_of(tgt);   // key 0
-                }
-                if (!found) {
-                    int i, j;
-                    uint32_t m;
-                    if (H00 & span) { i = 0; j = 0; m = H00 & span; }
-                    else if (H01 & span) { i = 0; j = 1; m = H01 & span; }
-                    else if (H10 & span) { i = 1; j = 0; m = H10 & span; }
-                    else { i = 1; j = 1; m = H11 & span; }
-                    P[sw3(x)] = (slot3(b0, i, b1, j, __ffs(m) - 1) << 12) | x;
-                }
-            }
-        }
+        RW[tid] = make_uint4(n1, w1, e1, 0u);
+        RW[NROW + tid] = make_uint4(n2, w2, e2, 0u);
+        RW[2 * NROW + tid] = make_uint4(n3, w3, e3, 0u);
         __syncthreads();
-        // The remaining links are unions, queued and merged by every lane, one neighbour row per
-        // round; a round whose links overflow the queue takes further passes through it (the links
-        // with positions [base, base + MQ1) each), so the overflow is shared by every lane too.
+        // A link is also dropped when two others close a triangle with it over a block of the row
+        // straight below, or beside: own - below left over own - below and below - below left, and so
+        // on, all as found, dropped or not.  Every reason uses links of earlier rows, or of this
+        // row to `below` (dropped only by the rules above) or `beside` (dropped only over `below`), so
+        // the reasons of a dropped link end at links that are kept.  This keeps 65% of the links of
+        // Bernoulli 0.3 and 39% of those of 0.5 for about 60 instructions a row.
+        {
+            const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+            const uint4 p = b0 > 0 ? RW[2 * NROW + tid - TB1] : z;                      // below - below left
+            const uint4 r = b0 > 0 && b1 + 1 < TB1 ? RW[2 * NROW + tid - TB1 + 1] : z;   // below right - below
+            const uint4 s = b1 > 0 ? RW[tid - 1] : z;                                   // beside - below left
+            const uint4 v = b1 > 0 ? RW[NROW + tid - 1] : z;                            // beside - below
+            LN[0] &= ~((n1 & p.x) | (n3 & s.x));
+            LW[0] &= ~((n1 & p.y) | (w1 & (p.x << 1)) | (n3 & s.y) | (w3 & (s.x << 1)));
+            LE[0] &= ~((n1 & p.z) | (e1 & (p.x >> 1)) | (n3 & s.z) | (e3 & (s.x >> 1)));
+            LN[2] &= ~(n1 & r.x);
+            LW[2] &= ~((n1 & (r.z << 1)) | (w1 & (r.x << 1)));
+            LE[2] &= ~((n1 & (r.y >> 1)) | (e1 & (r.x >> 1)));
+            LN[3] &= ~(n1 & v.x);
+            LW[3] &= ~((n1 & (v.z << 1)) | (w1 & (v.x << 1)));
+            LE[3] &= ~((n1 & (v.y >> 1)) | (e1 & (v.x >> 1)));
+        }
+        // The first link of a run into the preceding layer (d0 - 1, whose slots are all smaller than
+        // this row's) becomes its parent by a plain store: straight below if it has one there, else
+        // below left, else below right.  Its entry holds key 0, the smallest value.  The other runs are
+        // roots for now, with their slot.  (First links by a carry, as in 2D, from the starts whose run
+        // has a link.)
+        auto up_row = [&](int nr) -> int { return tid + (nr < 3 ? nr - 1 - TB1 : -1); };
+        auto take = [&](int nr, uint32_t uS, uint32_t ubase, uint32_t b, uint32_t &own, uint32_t &up) {
+            const uint32_t bit = 1u << b, upto = (bit << 1) - 1u;
+            own = base + __popc(S & upto) - 1u;
+            const bool isN = LN[nr] & bit, isW = !isN && (LW[nr] & bit), isE = !isN && !isW;
+            LN[nr] &= isN ? ~bit : ~0u;
+            LW[nr] &= isW ? ~bit : ~0u;
+            LE[nr] &= isE ? ~bit : ~0u;
+            up = ubase + __popc(uS & (isN ? upto : isW ? bit - 1u : (bit << 2) - 1u)) - 1u;   // (b = 30: all)
+        };
+        auto warp_base = [&](int row) -> uint32_t {   // runs before the warp of a row
+            uint32_t n = 0;
 #pragma unroll
-        for (int round = 0; round < 4; ++round) {
-            const uint32_t n = __popc(LN[round]) + __popc(LW[round]) + __popc(LE[round]);
-            const uint32_t pos0 = warp_reserve(&mqn[round], n);
-            const uint32_t ubase = uint32_t(UR[round]) * TB2;
-            auto each_link = [&](auto &&fn) {
-                uint32_t pos = pos0;
-                uint32_t todo = LN[round] | LW[round] | LE[round];
-                while (todo) {
-                    const uint32_t k = __ffs(todo) - 1;
-                    todo &= todo - 1;
-                    const uint32_t bit = 1u << k;
-                    const uint32_t a = rowb + k;
-                    if (LN[round] & bit) fn(pos++, a, ubase + k);
-                    if (LW[round] & bit) fn(pos++, a, ubase + k - 1);
-                    if (LE[round] & bit) fn(pos++, a, ubase + k + 1);
+            for (int i = 0; i < NT1 / 32 - 1; ++i)
+                if (i < (row >> 5)) n += wtot[i];
+            return n;
+        };
+        uint32_t rem = S;   // runs without a parent
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+            const int nr = o == 0 ? 1 : o == 1 ? 0 : 2;
+            const uint32_t lk = LN[nr] | LW[nr] | LE[nr];
+            if (!lk) continue;
+            const uint32_t with = starts_with(S, lk) & rem;
+            uint32_t first = lk & ((~lk + (with & ~lk)) | with);
+            rem &= ~with;
+            const int ur = up_row(nr);
+            const uint4 uw = WR[ur];
+            const uint32_t ub = uw.z + warp_base(ur);
+            while (first) {
+                const uint32_t b = __ffs(first) - 1;
+                first &= first - 1;
+                uint32_t own, up;
+                take(nr, uw.x, ub, b, own, up);
+                (void)GUARD(w, own < nrun && up < own, 101, (uint64_t(own) << 32) | up);
+                P[own & (NBLK - 1)] = up & (NBLK - 1);
+            }
+        }
+        for (uint32_t ss = rem; ss; ss &= ss - 1) {
+            const uint32_t b = __ffs(ss) - 1, bit = 1u << b;
+            const uint32_t ij = (S00 & bit) ? 0u : (S01 & bit) ? 1u : (S10 & bit) ? 2u : 3u;
+            const uint32_t id = base + __popc(S & (bit - 1u));
+            P[id] = (slot3(b0, b1, ij, b) << 12) | id;
+        }
+        // The remaining links are unions: queued and merged by every lane.
+        uint32_t n = 0;
+#pragma unroll
+        for (int nr = 0; nr < 4; ++nr) n += __popc(LN[nr]) + __popc(LW[nr]) + __popc(LE[nr]);
+        uint32_t pos = warp_reserve(&mqn, n);
+        auto push = [&](uint32_t lo, uint32_t end) {   // links at queue positions [lo, end) go in
+#pragma unroll
+            for (int nr = 0; nr < 4; ++nr) {
+                if (!(LN[nr] | LW[nr] | LE[nr])) continue;
+                const int ur = up_row(nr);
+                const uint4 uw = WR[ur];
+                const uint32_t ub = uw.z + warp_base(ur);
+                while (pos < end) {
+                    const uint32_t b = __ffs(LN[nr] | LW[nr] | LE[nr]);
+                    if (!b) break;
+                    uint32_t own, up;
+                    take(nr, uw.x, ub, b - 1u, own, up);
+                    MQ[pos - lo] = (own << 16) | up;
+                    ++pos;
                 }
-            };
-            if (pos0 < uint32_t(MQ1))
-                each_link([&](uint32_t pos, uint32_t a, uint32_t b) {
-                    if (pos < uint32_t(MQ1)) MQ[pos] = (a << 16) | b;
-                });
-            __syncthreads();
-            const uint32_t total = mqn[round];
-            for (uint32_t base = 0; base < total; base += MQ1) {
-                if (base) {
-                    if (pos0 + n > base && pos0 < base + MQ1)
-                        each_link([&](uint32_t pos, uint32_t a, uint32_t b) {
-                            if (pos >= base && pos < base + MQ1) MQ[pos - base] = (a << 16) | b;
-                        });
-                    __syncthreads();
-                }
-                const uint32_t nq = min(total - base, uint32_t(MQ1));
-                // Contiguous runs of the queue per thread, as in 2D.
-                const uint32_t per = (nq + NT1 - 1) / NT1, lo = min(nq, uint32_t(tid) * per), hi = min(nq, lo + per);
-                for (uint32_t q = lo; q < hi; ++q) eunion3(P, start_of(MQ[q] >> 16), start_of(MQ[q] & 0xFFFFu));
+            }
+        };
+        __syncthreads();   // the raw links are used up
+        push(0u, uint32_t(MQ1));
+        // The forest of first links is flattened before the unions, as in 2D.
+        eflatten3_all(P, tid, NT1, nrun);
+        __syncthreads();
+        const uint32_t total = mqn;
+        for (uint32_t lo = 0; lo < total; lo += MQ1) {
+            if (lo) {
+                eflatten3_all(P, tid, NT1, nrun);   // ehook3_pairs wants every run at its root
+                push(lo, lo + MQ1);
                 __syncthreads();
             }
+            const uint32_t nq = min(total - lo, uint32_t(MQ1)), per = (nq + NT1 / 32 - 1) / (NT1 / 32);
+            const uint32_t q0 = min(nq, warp * per);
+            const uint32_t kept = ehook3_pairs(P, MQ + q0, min(nq - q0, per));
+            __syncthreads();
+            for (uint32_t k = lane; k < kept; k += 32) eunion3(P, MQ[q0 + k] >> 16, MQ[q0 + k] & 0xFFFFu);
+            __syncthreads();
         }
 
-        // The root bitmap lives in the queue's memory from here on (the unions are done).
-        for (int i = tid; i < TX * TY * RBW; i += NT1) RB[i] = 0;
+        // Phase C: every run's entry becomes its root's.
+        if (total) eflatten3_all(P, tid, NT1, nrun);
         __syncthreads();
-        // Phase C: every run start of this row is pointed straight at its root (a read-only walk,
-        // then the root's entry stored in the start's own entry, as in 2D); roots mark their first
-        // voxel.
-        {
-            uint32_t ss = S;
-            while (ss) {
-                const uint32_t x = rowb + (__ffs(ss) - 1);
-                ss &= ss - 1;
-                uint32_t root = x, ev = P[sw3(x)];
-                for (int it = 0; (ev & 0xFFFu) != root && it < NBLK; ++it) {   // acyclic: the cap never binds
-                    root = ev & 0xFFFu;
-                    ev = P[sw3(root)];
-                }
-                if (root != x) P[sw3(x)] = ev;
-                if (root != x) continue;
-                const uint32_t rb = slot_block(ev >> 12);
-                const uint32_t key = local_key(int(rb), M[rb]);
-                const int Z = key % TZ, Y = (key / TZ) % TY, X = key / (TZ * TY);
-                if (GUARD(w, key < uint32_t(TX * TY * TZ), 101, key))
-                    atomicOr(&RB[(X * TY + Y) * RBW + (Z >> 5)], 1u << (Z & 31));
-            }
+        // Phase D: the root bitmap (a bit per run start, so a word per row) and the segments' root
+        // counts.
+        uint32_t roots = 0;
+        for (uint32_t ss = rem; ss; ss &= ss - 1) {
+            const uint32_t bit = ss & (0u - ss);
+            const uint32_t id = base + __popc(S & (bit - 1u));
+            if ((P[id] & 0xFFFu) == id) roots |= bit;
         }
-        // Block entries: the root block of a component carries ROOT_FLAG | its first-voxel key,
-        // every other block its root block.  (Runs do not cross rows: every start read here is
-        // this thread's own.)
-        {
-            uint32_t cur = 0;
+        w.rbits[t * NROW + tid] = roots;
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                const uint32_t mm = *reinterpret_cast<const uint32_t *>(&M[rowb + 4 * h]);
-                uint32_t e[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int k = 4 * h + q;
-                    if ((S >> k) & 1u) cur = slot_block(P[sw3(rowb + k)] >> 12);
-                    const uint32_t m = (mm >> (8 * q)) & 0xFFu;
-                    uint32_t v = 0;
-                    if (m) {
-                        v = (m << 24) | cur;
-                        if (cur == rowb + uint32_t(k)) v = (m << 24) | ROOT_FLAG | local_key(int(cur), m);
-                    }
-                    e[q] = v;
-                }
-                reinterpret_cast<uint4 *>(lab + t * NBLK + rowb)[h] = make_uint4(e[0], e[1], e[2], e[3]);
-            }
-        }
-        __syncthreads();   // root bitmap complete; every run start points at its root
-
-        // Phase D: root bitmap and segment counts out, border nodes.
-        for (int i = tid; i < TX * TY * RBW; i += NT1) w.rbits[t * (TX * TY * RBW) + i] = RB[i];
-        for (int r = tid; r < TX * TY; r += NT1) {
-            const int X = r / TY, Y = r % TY;
+        for (int ij = 0; ij < 4; ++ij) {
+            const int X = 2 * b0 + (ij >> 1), Y = 2 * b1 + (ij & 1);
             if (X >= g.nx || Y >= g.ny) continue;
-            uint32_t cnt = 0;
-#pragma unroll
-            for (int k = 0; k < RBW; ++k) cnt += __popc(RB[r * RBW + k]);
             const int64_t si = im.seg_base + (int64_t(g.x0 + X) * im.d1 + (g.y0 + Y)) * im.t2 + g.tx2;
-            if (GUARD(w, si >= 0 && si < w.n_segs, 104, si)) w.segcnt[si] = uint8_t(cnt);
+            if (GUARD(w, si >= 0 && si < w.n_segs, 104, si)) w.segcnt[si] = uint8_t(__popc(roots & starts_of(ij, S, S00, S01, S10)));
         }
-        auto root_block = [&](int b) -> uint32_t {
-            const uint32_t row = uint32_t(b) >> 5, k = uint32_t(b) & 31u;
-            const uint32_t st = hibit3(WS[row] & ((2u << k) - 1u));
-            return slot_block(P[sw3((row << 5) + st)] >> 12);
-        };
-        // Each border position's root block and face bits, kept in registers for the entries below
-        // ((root << 4) | face bits, 16 bits each; 0 stands for an empty position -- a root block 0
-        // with no face voxel gives entry 0 as well).
-        constexpr int KP = NPERIM / NT1;
-        static_assert(NPERIM % NT1 == 0, "border positions per thread");
-        uint32_t pc[(KP + 1) / 2];
-#pragma unroll
-        for (int k = 0; k < KP; ++k) {
-            const int p = tid + k * NT1;
-            int f, pb0, pb1, pb2;
-            uint32_t c = 0;
-            if (perim_pos3(p, g, f, pb0, pb1, pb2)) {
-                const int b = blk(pb0, pb1, pb2);
-                const uint32_t m = M[b];
-                if (m) {
-                    const uint32_t rb = root_block(b);
-                    atomicOr(&BF[rb >> 5], 1u << (rb & 31));
-                    c = (rb << 4) | face_bits(m, f);
-                }
-            }
-            if (k & 1) pc[k >> 1] |= c << 16;
-            else pc[k >> 1] = c;
-        }
-        __syncthreads();
-        uint32_t nb;
-        const uint32_t pre = block_exscan<NT1>(__popc(BF[tid]), tmp, &nb);
-        BP[tid] = pre;
-        __syncthreads();
+        // Border components -> nodes: the runs of the rows on a face that has a tile behind it, and the
+        // runs of the first and last blocks of every row where a tile lies behind those.
+        const bool zlo = g.tx2 > 0 && (S & 1u), zhi = g.tx2 + 1 < im.t2 && (Fw >> 31);
         {
-            uint32_t bits = BF[tid];
-            uint32_t j = pre;
-            while (bits) {
-                const int bit = __ffs(bits) - 1;
-                bits &= bits - 1;
-                const uint32_t rb = tid * 32 + bit;
-                const uint32_t key = local_key(int(rb), M[rb]);
-                if (!GUARD(w, key < uint32_t(TX * TY * TZ) && j < uint32_t(MAXB), 102, (uint64_t(j) << 32) | key))
-                    break;
-                const int Z = key % TZ, Y = (key / TZ) % TY, X = key / (TZ * TY);
-                const int64_t node = t * MAXB + j;
-                const uint32_t vkey = uint32_t((int64_t(g.x0 + X) * im.d1 + (g.y0 + Y)) * im.d2 + (g.z0 + Z));
-                w.nroot[node] = uint16_t(rb);
-                w.gp[node] = gentry(vkey, uint32_t(node));
-                ++j;
+            const bool face = (b0 == 0 && g.tx0 > 0) || (b0 == TB0 - 1 && g.tx0 + 1 < im.t0) || (b1 == 0 && g.tx1 > 0) ||
+                              (b1 == TB1 - 1 && g.tx1 + 1 < im.t1);
+            uint32_t ss = face ? S : (zlo ? 1u : 0u) | (zhi ? 0x80000000u >> __clz(S) : 0u);
+            for (; ss; ss &= ss - 1) {
+                const uint32_t id = base + __popc(S & ((ss & (0u - ss)) - 1u));
+                const uint32_t rt = P[id] & 0xFFFu;
+                atomicOr(&BF[rt >> 5], 1u << (rt & 31));
             }
         }
+        __syncthreads();
+        uint32_t nin = __popc(BF[tid]);   // nodes up to this word, within the warp
 #pragma unroll
-        for (int k = 0; k < KP; ++k) {
-            const uint32_t c = (pc[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
-            uint16_t ent = 0;
-            if (c) {
-                const uint32_t rb = c >> 4;
-                const uint32_t j = BP[rb >> 5] + __popc(BF[rb >> 5] & ((1u << (rb & 31)) - 1u));
-                ent = uint16_t((j << 4) | (c & 15u));
-            }
-            w.perim[t * NPERIM + tid + k * NT1] = ent;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, nin, o);
+            if (lane >= o) nin += v;
         }
-        if (tid == 0) w.nb[t] = nb;
+        BP[tid] = nin - __popc(BF[tid]);
+        if (lane == 31) ntot[warp] = nin;
+        __syncthreads();
+        uint32_t noff[NBLK / 32 / 32 + 1];
+        noff[0] = 0;
+#pragma unroll
+        for (int i = 0; i < NBLK / 32 / 32; ++i) noff[i + 1] = noff[i] + ntot[i];
+        auto node_of = [&](uint32_t rt) -> uint32_t {   // node of a root run's component
+            const uint32_t f = BF[rt >> 5], bit = 1u << (rt & 31), q = rt >> 10;
+            if (!(f & bit)) return kNoNode;
+            return (q == 0 ? noff[0] : q == 1 ? noff[1] : q == 2 ? noff[2] : noff[3]) + BP[rt >> 5] + __popc(f & (bit - 1u));
+        };
+        // Node records, by the row of the root run; root and node of every run; the row's ends.
+        for (uint32_t ss = roots; ss; ss &= ss - 1) {
+            const uint32_t bit = ss & (0u - ss), id = base + __popc(S & (bit - 1u));
+            const uint32_t j = node_of(id);
+            if (j == kNoNode) continue;
+            if (!GUARD(w, j < uint32_t(MAXB), 102, j)) break;
+            const uint32_t ij = (S00 & bit) ? 0u : (S01 & bit) ? 1u : (S10 & bit) ? 2u : 3u;
+            const uint32_t place = __popc(starts_of(int(ij), S, S00, S01, S10) & (bit - 1u));
+            const int64_t seg = (int64_t(g.x0 + 2 * b0 + (ij >> 1)) * im.d1 + (g.y0 + 2 * b1 + (ij & 1))) * im.t2 + g.tx2;
+            const int64_t node = t * MAXB + j;
+            w.nroot[node] = uint16_t(tid * TB2 + __ffs(bit) - 1);
+            w.gp[node] = gentry(uint32_t(seg) * seg_width3(im) + place, uint32_t(node));
+        }
+        {
+            uint32_t *rl = lab + t * T3_LAB_WORDS + kHdr3;
+            uint32_t *nl = reinterpret_cast<uint32_t *>(w.perim + t * T3_EDGE);
+            for (uint32_t i = 2 * tid; i < nrun; i += 2 * NT1) {
+                const uint32_t ra = P[i] & 0xFFFu, rb = P[i + 1 < nrun ? i + 1 : i] & 0xFFFu;
+                rl[i >> 1] = ra | (rb << 16);
+                nl[i >> 1] = node_of(ra) | (node_of(rb) << 16);
+            }
+            const uint32_t na = zlo ? node_of(P[base] & 0xFFFu) : kNoNode;
+            const uint32_t nz = zhi ? node_of(P[base + __popc(S) - 1u] & 0xFFFu) : kNoNode;
+            nl[kZNode / 2 + tid] = na | (nz << 16);
+            reinterpret_cast<uint8_t *>(w.perim + t * T3_EDGE + kZFace)[tid] =
+                uint8_t((c[0] & 1u) | ((c[2] & 1u) << 1) | ((c[4] & 1u) << 2) | ((c[6] & 1u) << 3) | ((c[1] >> 31) << 4) |
+                        ((c[3] >> 31) << 5) | ((c[5] >> 31) << 6) | ((c[7] >> 31) << 7));
+        }
+        if (tid == 0) w.nb[t] = noff[NBLK / 32 / 32];
         __syncthreads();
     }
 }
 
 // ---------------------------------------------------------------------------------------------
-// Cross-tile merge over the +d0, +d1 and +d2 faces.
+// Cross-tile merge.
 // ---------------------------------------------------------------------------------------------
 namespace {
-
-// Where the voxel with raster key `key` of image im sits: its tile, the root-bitmap word and bit of
-// it in that tile, and its segment.
-struct KeyPos {
-    int64_t tile, word, seg;
-    uint32_t bit;
-};
-__device__ __forceinline__ KeyPos key_pos(const Img3D &im, uint32_t key)
-{
-    // Keys index one volume (< 2^32 voxels): 32-bit division suffices.
-    const uint32_t row = key / uint32_t(im.d2), Z = key - row * uint32_t(im.d2);
-    const uint32_t X = row / uint32_t(im.d1), Y = row - X * uint32_t(im.d1);
-    const uint32_t q0 = X / TX, q1 = Y / TY, q2 = Z / TZ;
-    KeyPos kp;
-    kp.tile = im.tile_base + (int64_t(q0) * im.t1 + q1) * im.t2 + q2;
-    const uint32_t lx = X % TX, ly = Y % TY, lz = Z % TZ;
-    kp.word = kp.tile * (TX * TY * RBW) + int64_t((lx * TY + ly) * RBW + (lz >> 5));
-    kp.bit = lz & 31u;
-    kp.seg = im.seg_base + int64_t(row) * im.t2 + q2;
-    return kp;
-}
 
 // Union of two nodes of one volume; the root linked under the other leaves its segment's root
 // count and its tile's root bitmap.
 __device__ void gunion3d(const Img3D &im, Work &w, uint32_t a, uint32_t b)
 {
-    gunion_keyed(w.gp, a, b, [&](uint32_t, uint32_t key) {
-        const KeyPos kp = key_pos(im, key);
-        dec_u8(w.segcnt, kp.seg);
-        atomicAnd(w.rbits + kp.word, ~(1u << kp.bit));
+    gunion_keyed(w.gp, a, b, [&](uint32_t node, uint32_t key) {
+        dec_u8(w.segcnt, im.seg_base + key / seg_width3(im));
+        const uint32_t blk = w.nroot[node];
+        atomicAnd(w.rbits + int64_t(node / MAXB) * NROW + blk / TB2, ~(1u << (blk % TB2)));
     });
 }
 
 }  // namespace
 
-// Cross-tile merge over the +d0, +d1 and +d2 faces.  The border entries of the blocks across
-// each + face (the next tile's - face, widened by one block on every side into the diagonal
-// tiles) are staged in shared memory once per tile, so each face block checks its nine
-// neighbours without index arithmetic or global loads.  A CTA-local union-find over this tile's
-// nodes and the staged positions then filters the pairs: only a pair that joins two local sets
-// goes on to the global union-find (from a shared queue, once the tile's pairs are all seen); a
-// dense volume that crosses a face with one component in hundreds of blocks costs a handful of
-// global unions.
-constexpr int kGQ3 = 256;    // queued global unions per tile (more are done at once)
-constexpr int kPL3 = 576;    // listed face pairs per tile (more are checked where they are found)
-constexpr int PF0 = (TB1 + 2) * (TB2 + 2);   // staged entries across the +d0 face
-constexpr int PF1 = (TB0 + 2) * (TB2 + 2);   // +d1
-constexpr int PF2 = (TB0 + 2) * (TB1 + 2);   // +d2
-constexpr int NPF = PF0 + PF1 + PF2;
-constexpr int NPLUS = TB1 * TB2 + TB0 * TB2 + TB0 * TB1;
-constexpr int NSROWS = (TB1 + 2) + (TB0 + 2) + (TB0 + 2);   // staged rows over the three faces
-
-// Face geometry along axis AX (compile-time, so nothing is indexed at run time): the two tangent
-// axes in order, their tile sizes, the staged array's offset and pitch.
-template <int AX> struct FaceAx {
-    static constexpr int A1 = AX == 0 ? 1 : 0, A2 = AX == 2 ? 1 : 2;
-    static constexpr int TA = A1 == 0 ? TB0 : TB1, TBb = A2 == 1 ? TB1 : TB2;
-    static constexpr int TAX = AX == 0 ? TB0 : AX == 1 ? TB1 : TB2;
-    static constexpr int EBASE = AX == 0 ? 0 : AX == 1 ? PF0 : PF0 + PF1;
-    static constexpr int PITCH = TBb + 2;
-    static constexpr int NPOS = TA * TBb;
-    static constexpr int PBASE = AX == 0 ? 0 : AX == 1 ? TB1 * TB2 : TB1 * TB2 + TB0 * TB2;
-};
-
-__device__ __forceinline__ int pick3(int a0, int a1, int a2, int i) { return i == 0 ? a0 : i == 1 ? a1 : a2; }
-
-// Stage entry e (0 <= e < (TA+2) * (TBb+2)) of the face along AX.
-template <int AX>
-__device__ __forceinline__ void stage_face(const Img3D &im, const TileGeo &g, Work &w, int e, uint32_t *nbid,
-                                           uint8_t *nbf)
-{
-    using F = FaceAx<AX>;
-    const int iu = e / F::PITCH, iv = e % F::PITCH;
-    const int tcx = pick3(g.tx0, g.tx1, g.tx2, AX), tnx = pick3(im.t0, im.t1, im.t2, AX);
-    const int tc1 = pick3(g.tx0, g.tx1, g.tx2, F::A1), tc2 = pick3(g.tx0, g.tx1, g.tx2, F::A2);
-    const int nb1 = (pick3(im.d0, im.d1, im.d2, F::A1) + 1) >> 1, nb2 = (pick3(im.d0, im.d1, im.d2, F::A2) + 1) >> 1;
-    const int g1 = tc1 * F::TA + iu - 1, g2 = tc2 * F::TBb + iv - 1;
-    uint32_t id = kNone, fb = 0;
-    if (tcx + 1 < tnx && g1 >= 0 && g1 < nb1 && g2 >= 0 && g2 < nb2) {
-        const int t1 = g1 / F::TA, l1 = g1 - t1 * F::TA, t2 = g2 / F::TBb, l2 = g2 - t2 * F::TBb;
-        int tt0, tt1, tt2;
-        if (AX == 0) { tt0 = tcx + 1; tt1 = t1; tt2 = t2; }
-        else if (AX == 1) { tt0 = t1; tt1 = tcx + 1; tt2 = t2; }
-        else { tt0 = t1; tt1 = t2; tt2 = tcx + 1; }
-        const int64_t t2i = im.tile_base + (int64_t(tt0) * im.t1 + tt1) * im.t2 + tt2;
-        const int qb = l1 * F::TBb + l2;   // position on the - face: (first tangent, second tangent)
-        if (GUARD(w, t2i >= 0 && t2i < w.n_tiles && qb >= 0 && qb < NPERIM, 201, t2i)) {
-            const uint32_t B = w.perim[t2i * NPERIM + face_base(2 * AX) + qb];
-            if (B && GUARD(w, (B >> 4) < w.nb[t2i], 203, (uint64_t(t2i) << 16) | (B >> 4))) {
-                id = uint32_t(t2i * MAXB + (B >> 4));
-                fb = B & 15u;
-            }
-        }
-    }
-    nbid[F::EBASE + e] = id;
-    nbf[F::EBASE + e] = uint8_t(fb);
-}
-
-// This tile's + face entry at position q of the face along AX (0 when the face has no neighbour).
-template <int AX>
-__device__ __forceinline__ uint32_t plus_entry(const Img3D &im, const TileGeo &g, const Work &w, int64_t t, int q,
-                                               int &u, int &v)
-{
-    using F = FaceAx<AX>;
-    u = q / F::TBb;
-    v = q % F::TBb;
-    const int tcx = pick3(g.tx0, g.tx1, g.tx2, AX), tnx = pick3(im.t0, im.t1, im.t2, AX);
-    const int n1 = pick3(g.n0, g.n1, g.n2, F::A1), n2 = pick3(g.n0, g.n1, g.n2, F::A2);
-    if (tcx + 1 >= tnx || u >= n1 || v >= n2) return 0u;
-    return w.perim[t * NPERIM + face_base(2 * AX + 1) + q];
-}
-
-// Tangent coordinates of position q of this tile's + face along AX.
-template <int AX>
-__device__ __forceinline__ void plus_uv(int q, int &u, int &v)
-{
-    using F = FaceAx<AX>;
-    u = q / F::TBb;
-    v = q % F::TBb;
-}
-
-// Staged position e of the face along AX -> (iu, iv) in the staged grid, or false when e lies in
-// another face's range.
-template <int AX>
-__device__ __forceinline__ bool staged_pos(int e, int &iu, int &iv)
-{
-    using F = FaceAx<AX>;
-    const int k = e - F::EBASE;
-    if (k < 0 || k >= (F::TA + 2) * F::PITCH) return false;
-    iu = k / F::PITCH;
-    iv = k % F::PITCH;
-    return true;
-}
+// Cross-tile merge.  One CTA per tile, one thread per block row: the row's links to those of its four
+// preceding rows that lie in other tiles, by the same bit operations as inside a tile (row_links), and
+// its first and last block's links across d2 to the tiles beside (one byte of face voxels per row and
+// two nodes, written by the tile kernel).  The links go through a shared queue, so that the rows on a
+// face, which have most of them, are shared by all lanes; a pair of nodes that the CTA has just seen
+// -- most links join the same few large components -- is dropped by a small table, and the others
+// are unions, whose walks (dependent loads through L2) end as soon as the two sides have one parent.
+constexpr int kMQ3 = 1024;     // queued links (more take further rounds)
+constexpr int kSeen3 = 256;    // table of node pairs seen
 
 __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(ImgList3D L, Work w)
 {
     grid_dep_wait();
     grid_dep_release();
-    __shared__ uint32_t qslot;
-    __shared__ uint32_t lp[MAXB + NPF];   // local union-find: this tile's nodes, then staged positions
-    __shared__ uint32_t nbid[NPF];        // global node id across the face, kNone = none
-    __shared__ uint8_t nbf[NPF];          // its face bits
-    __shared__ uint2 gq[kGQ3];
+    __shared__ uint32_t Q[kMQ3];
+    __shared__ unsigned long long seen[kSeen3];
     __shared__ uint32_t nq;
-    __shared__ uint32_t pl[kPL3];         // listed pairs: (node << 16) | staged position
-    __shared__ uint32_t npl;
-    __shared__ uint16_t own[NPLUS];       // this tile's + face entries (staged with the others)
+    __shared__ uint32_t qslot;
+    static_assert(kT3MergeThreads == NROW, "one thread per block row");
+    const int tid = threadIdx.x;
+    const int b0 = tid / TB1, b1 = tid % TB1;
+    const uint32_t *lab = reinterpret_cast<const uint32_t *>(w.lab);
     ItemLoop loop{w.queue ? w.queue + 1 : nullptr, w.n_tiles};
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
         const Img3D im = L.get(t);
         const TileGeo g = tile_geo(im, t);
-        for (int i = threadIdx.x; i < MAXB + NPF; i += kT3MergeThreads) lp[i] = uint32_t(i);
-        if (threadIdx.x == 0) {
-            nq = 0;
-            npl = 0;
-        }
-        for (int e = threadIdx.x; e < PF0; e += kT3MergeThreads) stage_face<0>(im, g, w, e, nbid, nbf);
-        for (int e = threadIdx.x; e < PF1; e += kT3MergeThreads) stage_face<1>(im, g, w, e, nbid, nbf);
-        for (int e = threadIdx.x; e < PF2; e += kT3MergeThreads) stage_face<2>(im, g, w, e, nbid, nbf);
-        for (int q = threadIdx.x; q < NPLUS; q += kT3MergeThreads) {
-            int u, v;
-            if (q < FaceAx<0>::NPOS) own[q] = uint16_t(plus_entry<0>(im, g, w, t, q, u, v));
-            else if (q < FaceAx<0>::NPOS + FaceAx<1>::NPOS) own[q] = uint16_t(plus_entry<1>(im, g, w, t, q - FaceAx<1>::PBASE, u, v));
-            else own[q] = uint16_t(plus_entry<2>(im, g, w, t, q - FaceAx<2>::PBASE, u, v));
-        }
+        for (int i = tid; i < kSeen3; i += kT3MergeThreads) seen[i] = ~0ull;
+        if (tid == 0) nq = 0;
         __syncthreads();
-        // Staged positions of the same node that touch on the face are one element from here on
-        // (a component crosses a face as a patch, not as scattered blocks): runs along each staged
-        // row point at their first position, runs of neighbouring rows are merged where one of
-        // them starts, and every staged position is then pointed straight at its root.
-        for (int row = threadIdx.x; row < NSROWS; row += kT3MergeThreads) {
-            int e0, n;
-            if (row < FaceAx<0>::TA + 2) { e0 = FaceAx<0>::EBASE + row * FaceAx<0>::PITCH; n = FaceAx<0>::PITCH; }
-            else if (row < FaceAx<0>::TA + FaceAx<1>::TA + 4) {
-                e0 = FaceAx<1>::EBASE + (row - FaceAx<0>::TA - 2) * FaceAx<1>::PITCH; n = FaceAx<1>::PITCH;
-            } else {
-                e0 = FaceAx<2>::EBASE + (row - FaceAx<0>::TA - FaceAx<1>::TA - 4) * FaceAx<2>::PITCH; n = FaceAx<2>::PITCH;
-            }
-            uint32_t prev = kNone, start = 0;
-            for (int k = 0; k < n; ++k) {
-                const uint32_t id = nbid[e0 + k];
-                if (id != prev) start = uint32_t(MAXB + e0 + k);
-                lp[MAXB + e0 + k] = start;
-                prev = id;
-            }
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < NPF; e += kT3MergeThreads) {
-            const uint32_t id = nbid[e];
-            if (id == kNone) continue;
-            int iu, iv, pitch;
-            if (staged_pos<0>(e, iu, iv)) pitch = FaceAx<0>::PITCH;
-            else if (staged_pos<1>(e, iu, iv)) pitch = FaceAx<1>::PITCH;
-            else { staged_pos<2>(e, iu, iv); pitch = FaceAx<2>::PITCH; }
-            if (iu == 0 || nbid[e - pitch] != id) continue;
-            // One link per pair of overlapping runs: at the overlap's first column, where one of
-            // the two runs starts.
-            const bool xs = iv == 0 || nbid[e - 1] != id, ys = iv == 0 || nbid[e - pitch - 1] != id;
-            if (xs || ys) smerge(lp, uint32_t(MAXB + e), uint32_t(MAXB + e - pitch));
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < NPF; e += kT3MergeThreads)
-            if (nbid[e] != kNone) sflatten(lp, uint32_t(MAXB + e));
-        __syncthreads();
-        // Pairs: every face position lists its connected neighbours (a bit test each) in one pass
-        // over the three faces, then all lanes check the listed pairs; a pair whose two elements are
-        // already one local set is implied by pairs queued before it (smerge_joined).  Pairs past
-        // the list's capacity are checked by the lane that finds them.  The rest are unioned
-        // globally at the end.
-        auto check_pair = [&](uint32_t ja2, uint32_t e) {
-            if (!smerge_joined(lp, ja2, uint32_t(MAXB) + e)) return;
-            const uint32_t nA = uint32_t(t * MAXB + ja2), id = nbid[e];
-            const uint32_t slot = atomicAdd(&nq, 1u);
-            if (slot < uint32_t(kGQ3)) gq[slot] = make_uint2(nA, id);
-            else gunion3d(im, w, nA, id);
+
+        // Preceding row nr: its row in its tile, and that tile's offset code 4 * (o0 + 1) + (o1 + 1)
+        // with o0 in {-1, 0}; 16 when there is no such tile.
+        auto preceding = [&](int nr, int &rr) -> int {
+            const int r0 = b0 + (nr < 3 ? -1 : 0), r1 = b1 + (nr < 3 ? nr - 1 : -1);
+            const int o0 = r0 < 0 ? -1 : 0, o1 = r1 < 0 ? -1 : r1 >= TB1 ? 1 : 0;
+            rr = (r0 & (TB0 - 1)) * TB1 + (r1 & (TB1 - 1));
+            if (g.tx0 + o0 < 0 || g.tx1 + o1 < 0 || g.tx1 + o1 >= im.t1) return 16;
+            return 4 * (o0 + 1) + (o1 + 1);
         };
-        const uint32_t nbt = w.nb[t];   // (read by the bounds checks of checked builds)
-        (void)nbt;
-        for (int base = 0; base < NPLUS; base += kT3MergeThreads) {
-            const int p = base + int(threadIdx.x);
-            int u = 0, v = 0, ebase = 0, pitch = 1;
-            uint32_t A = 0;
-            if (p < FaceAx<0>::NPOS) {
-                plus_uv<0>(p, u, v);
-                ebase = FaceAx<0>::EBASE; pitch = FaceAx<0>::PITCH;
-            } else if (p < FaceAx<0>::NPOS + FaceAx<1>::NPOS) {
-                plus_uv<1>(p - FaceAx<1>::PBASE, u, v);
-                ebase = FaceAx<1>::EBASE; pitch = FaceAx<1>::PITCH;
-            } else if (p < NPLUS) {
-                plus_uv<2>(p - FaceAx<2>::PBASE, u, v);
-                ebase = FaceAx<2>::EBASE; pitch = FaceAx<2>::PITCH;
-            }
-            if (p < NPLUS) A = own[p];
-            if (A && !GUARD(w, (A >> 4) < nbt && (A >> 4) < uint32_t(MAXB), 204, (uint64_t(t) << 16) | (A >> 4)))
-                A = 0;
-            const uint32_t fa = A & 15u, ja = A >> 4;
-            uint32_t hit = 0;   // bit 3 * (da + 1) + (db + 1): connected neighbour
-            if (A) {
+        auto tile_at = [&](int code, int o2) -> int64_t {
+            return t + (int64_t((code >> 2) - 1) * im.t1 + (code & 3) - 1) * im.t2 + o2;
+        };
+        constexpr int kOwn = 5;   // code of the row's own tile
+        // Links to rows of other tiles.
+        uint32_t LN[4] = {0u, 0u, 0u, 0u}, LW[4] = {0u, 0u, 0u, 0u}, LE[4] = {0u, 0u, 0u, 0u};
+        uint32_t S = 0, base = 0;
+        const bool inside = b0 < g.n0 && b1 < g.n1;
+        if (inside && ((b0 == 0 && g.tx0 > 0) || (b1 == 0 && g.tx1 > 0) || (b1 == TB1 - 1 && g.tx1 + 1 < im.t1))) {
+            const uint4 *h = reinterpret_cast<const uint4 *>(lab + t * T3_LAB_WORDS);
+            const uint4 ca = __ldcg(h + tid), cb = __ldcg(h + NROW + tid), rw = __ldcg(h + 2 * NROW + tid);
+            const uint32_t c[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+            S = rw.x;
+            base = rw.y;
+            const uint32_t hz = row_joins(c);
+            if (S) {
 #pragma unroll
-                for (int da = -1; da <= 1; ++da) {
-#pragma unroll
-                    for (int db = -1; db <= 1; ++db) {
-                        if (!(fa & face_sel(da, db))) continue;
-                        const int e = ebase + (u + 1 + da) * pitch + (v + 1 + db);
-                        if (nbid[e] != kNone && (nbf[e] & face_sel(-da, -db))) hit |= 1u << (3 * (da + 1) + (db + 1));
-                    }
+                for (int nr = 0; nr < 4; ++nr) {
+                    int rr;
+                    const int code = preceding(nr, rr);
+                    if (code == kOwn || code == 16) continue;
+                    const uint4 *uh = reinterpret_cast<const uint4 *>(lab + tile_at(code, 0) * T3_LAB_WORDS);
+                    const uint4 ua = __ldcg(uh + rr), ub = __ldcg(uh + NROW + rr);
+                    const uint32_t u[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
+                    Links raw;
+                    const Links l = row_links(nr, c, hz, ua, ub, row_joins(u), raw);
+                    LN[nr] = l.n;
+                    LW[nr] = l.w;
+                    LE[nr] = l.e;
                 }
             }
-            // Neighbours whose staged positions already share a local parent are one local set
-            // (mostly one node's patch across the face): the first of them stands for the others.
-            uint32_t keep = 0;
-            {
-                uint32_t h = hit, last0 = kNone, last1 = kNone;
-                while (h) {
-                    const int k = __ffs(h) - 1;
-                    h &= h - 1;
-                    const uint32_t a = lp[MAXB + ebase + (u + k / 3) * pitch + (v + k % 3)];
-                    if (a == last0 || a == last1) continue;
-                    last1 = last0;
-                    last0 = a;
-                    keep |= 1u << k;
+        }
+        // Links across d2: bits 0..3, own first block to preceding row nr of the tiles before; bit 4, to
+        // the same row; bits 5..8, own last block to preceding row nr of the tiles after.
+        auto zface = [&](int64_t tt, int row) -> uint32_t {
+            return __ldcg(reinterpret_cast<const uint8_t *>(w.perim + tt * T3_EDGE + kZFace) + row);
+        };
+        uint32_t zm = 0;
+        if (inside) {
+            const uint32_t f = zface(t, tid);
+            const uint32_t lo = g.tx2 > 0 ? f & 15u : 0u, hi = g.tx2 + 1 < im.t2 ? f >> 4 : 0u;
+            if (lo && (zface(t - 1, tid) >> 4)) zm |= 16u;
+            if (lo | hi) {
+#pragma unroll
+                for (int nr = 0; nr < 4; ++nr) {
+                    int rr;
+                    const int code = preceding(nr, rr);
+                    if (code == 16) continue;
+                    const int dx = nr < 3 ? -1 : 0, dy = nr < 3 ? nr - 1 : -1;
+                    const uint32_t own = face_sel(dx, dy), opp = face_sel(-dx, -dy);
+                    if ((lo & own) && ((zface(tile_at(code, -1), rr) >> 4) & opp)) zm |= 1u << nr;
+                    if ((hi & own) && (zface(tile_at(code, 1), rr) & opp)) zm |= 32u << nr;
                 }
             }
-            uint32_t pos = warp_reserve(&npl, __popc(keep));
-            while (keep) {
-                const int k = __ffs(keep) - 1;
-                keep &= keep - 1;
-                const uint32_t e = uint32_t(ebase + (u + k / 3) * pitch + (v + k % 3));
-                if (pos < uint32_t(kPL3)) pl[pos] = (ja << 16) | e;
-                else check_pair(ja, e);
-                ++pos;
+        }
+        // Queue entries: run links, own run | other run << 12 | code << 24; links across d2, own node |
+        // other node << 11 | code << 24 | (o2 < 0: 1, o2 > 0: 2) << 29.
+        uint32_t n = __popc(zm);
+#pragma unroll
+        for (int nr = 0; nr < 4; ++nr) n += __popc(LN[nr]) + __popc(LW[nr]) + __popc(LE[nr]);
+        uint32_t pos = warp_reserve(&nq, n);
+        auto push = [&](uint32_t from, uint32_t end) {   // links at queue positions [from, end) go in
+#pragma unroll
+            for (int nr = 0; nr < 4; ++nr) {
+                if (!(LN[nr] | LW[nr] | LE[nr]) || pos >= end) continue;
+                int rr;
+                const int code = preceding(nr, rr);
+                const uint4 uw = __ldcg(reinterpret_cast<const uint4 *>(lab + tile_at(code, 0) * T3_LAB_WORDS) + 2 * NROW + rr);
+                while (pos < end) {
+                    const uint32_t f = __ffs(LN[nr] | LW[nr] | LE[nr]);
+                    if (!f) break;
+                    const uint32_t b = f - 1, bit = 1u << b, upto = (bit << 1) - 1u;
+                    const bool isN = LN[nr] & bit, isW = !isN && (LW[nr] & bit), isE = !isN && !isW;
+                    LN[nr] &= isN ? ~bit : ~0u;
+                    LW[nr] &= isW ? ~bit : ~0u;
+                    LE[nr] &= isE ? ~bit : ~0u;
+                    const uint32_t own = base + __popc(S & upto) - 1u;
+                    const uint32_t up = uw.y + __popc(uw.x & (isN ? upto : isW ? bit - 1u : (bit << 2) - 1u)) - 1u;
+                    Q[pos++ - from] = own | (up << 12) | (uint32_t(code) << 24);
+                }
             }
+            if (zm && pos < end) {
+                auto znodes = [&](int64_t tt, int row) -> uint32_t {
+                    return __ldcg(reinterpret_cast<const uint32_t *>(w.perim + tt * T3_EDGE + kZNode) + row);
+                };
+                const uint32_t zo = znodes(t, tid);
+                while (zm && pos < end) {
+                    const int k = __ffs(zm) - 1;
+                    zm &= zm - 1;
+                    int rr = tid, code = kOwn;
+                    if (k != 4) code = preceding(k < 4 ? k : k - 5, rr);
+                    const uint32_t zu = znodes(tile_at(code, k < 5 ? -1 : 1), rr);
+                    const uint32_t a = k < 5 ? zo & 0xFFFFu : zo >> 16, b = k < 5 ? zu >> 16 : zu & 0xFFFFu;
+                    Q[pos++ - from] = a | (b << 11) | (uint32_t(code) << 24) | (k < 5 ? 1u << 29 : 2u << 29);
+                }
+            }
+        };
+        push(0u, uint32_t(kMQ3));
+        __syncthreads();
+        const uint32_t total = nq;
+        for (uint32_t from = 0; from < total; from += kMQ3) {
+            if (from) {
+                push(from, from + kMQ3);
+                __syncthreads();
+            }
+            const uint32_t cnt = min(total - from, uint32_t(kMQ3));
+            for (uint32_t i = tid; i < cnt; i += kT3MergeThreads) {
+                const uint32_t e = Q[i], z = e >> 29;
+                const int64_t tt = tile_at(int(e >> 24) & 31, z == 0 ? 0 : z == 1 ? -1 : 1);
+                uint32_t a, b;
+                if (z) {
+                    a = e & 0x7FFu;
+                    b = (e >> 11) & 0x7FFu;
+                } else {
+                    a = __ldcg(w.perim + t * T3_EDGE + (e & 0xFFFu));
+                    b = __ldcg(w.perim + tt * T3_EDGE + ((e >> 12) & 0xFFFu));
+                }
+                if (!GUARD(w, a < w.nb[t] && b < w.nb[tt], 204, (uint64_t(tt) << 32) | e)) continue;
+                const uint32_t nA = uint32_t(t * MAXB + a), nB = uint32_t(tt * MAXB + b);
+                const unsigned long long key = (static_cast<unsigned long long>(nA) << 32) | nB;
+                const uint32_t slot = (nA * 0x9E3779B1u ^ nB * 0x85EBCA77u) >> 24;
+                static_assert(kSeen3 == 256, "eight hash bits");
+                if (atomicExch(&seen[slot], key) == key) continue;   // the lane that put it there unites the two
+                gunion3d(im, w, nA, nB);
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        {
-            const uint32_t n = min(npl, uint32_t(kPL3));
-            for (uint32_t i = threadIdx.x; i < n; i += kT3MergeThreads) check_pair(pl[i] >> 16, pl[i] & 0xFFFFu);
-        }
-        __syncthreads();
-        const uint32_t nqt = min(nq, uint32_t(kGQ3));
-        for (uint32_t i = threadIdx.x; i < nqt; i += kT3MergeThreads) gunion3d(im, w, gq[i].x, gq[i].y);
-        __syncthreads();
+        __syncthreads();   // every lane has read this tile's count
     }
 }
 
@@ -900,12 +806,17 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_link_3d(ImgList3D L, Work
         }
         const int64_t t = it - w.n_chunks;
         const Img3D im = L.get(t);
-        link_tile_nodes(w, t, MAXB, [&](uint32_t key, uint32_t &seg, uint32_t &rank) {
-            const KeyPos kp = key_pos(im, key);
-            const uint32_t *rw = w.rbits + (kp.word & ~int64_t(RBW - 1));
-            rank = __popc(rw[kp.word & (RBW - 1)] & ((1u << kp.bit) - 1u));
-            for (int k = 0; k < int(kp.word & (RBW - 1)); ++k) rank += __popc(rw[k]);
-            seg = uint32_t(kp.seg);
+        link_tile_nodes(w, t, MAXB, [&](uint32_t root, uint32_t key, uint32_t &seg, uint32_t &rank) {
+            // The root's segment, and the roots left in it before the root.
+            const uint32_t sg = key / seg_width3(im), line = sg / uint32_t(im.t2);   // line = X * d1 + Y
+            const uint32_t X = line / uint32_t(im.d1), Y = line - X * uint32_t(im.d1);
+            const uint32_t blk = w.nroot[root], row = blk / TB2;
+            const int64_t tile = root / MAXB;
+            const uint32_t *h = reinterpret_cast<const uint32_t *>(w.lab) + tile * T3_LAB_WORDS;
+            const uint4 rw = reinterpret_cast<const uint4 *>(h)[2 * NROW + row];
+            const uint32_t st = starts_of(int(X & 1) * 2 + int(Y & 1), rw.x, rw.z, rw.w, h[12 * NROW + row]);
+            rank = __popc(w.rbits[tile * NROW + row] & st & ((1u << (blk % TB2)) - 1u));
+            seg = uint32_t(im.seg_base) + sg;
         });
     }
 }
@@ -913,33 +824,42 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_link_3d(ImgList3D L, Work
 // ---------------------------------------------------------------------------------------------
 // Label resolve and write.
 // ---------------------------------------------------------------------------------------------
-constexpr int kNLCap = 512;   // node links a write CTA stages in shared memory (later ones: from L2)
+constexpr int kNLCap = 512;        // node links a write CTA stages in shared memory (later ones: from L2)
+constexpr int kStageRuns3 = 2048;  // run entries likewise
 
-__global__ void __launch_bounds__(NT, 5) k_tile_write_3d(ImgList3D L, Work w)
+__global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L, Work w)
 {
-    __shared__ __align__(16) uint32_t Ls[NBLK];
-    __shared__ uint32_t LT[NBLK];
-    __shared__ __align__(16) uint32_t RB[TX * TY * RBW];
+    __shared__ __align__(16) uint4 H[3 * NROW];   // class words 0..3, 4..7, (starts, runs before, S00, S01)
+    __shared__ uint32_t H10[NROW];
+    __shared__ uint32_t LT[NBLK + 1];             // label of run i at i + 1
+    __shared__ uint32_t RB[NROW];                 // roots left, a bit per run start
     __shared__ uint32_t segb[TX * TY + 1];   // segment prefixes of the tile's voxel rows; [TX * TY]: the volume's first
     __shared__ __align__(16) uint2 NL[kNLCap];
+    __shared__ __align__(16) uint32_t E[kStageRuns3 / 2];
     __shared__ uint32_t snb;
     __shared__ uint32_t qslot;
 
     const int tid = threadIdx.x;
     const uint32_t *lab = reinterpret_cast<const uint32_t *>(w.lab);
-    static_assert(NBLK / 4 == 4 * NT && TX * TY * RBW == 4 * NT, "four prefetched words per thread");
-    static_assert(TX * TY == 2 * NT && kNLCap == 2 * NT, "two segment prefixes and two node links per thread");
-    // Block entries, root bitmaps and node counts were final before this grid's predecessor (the
+    static_assert(3 * NROW <= 2 * NT && NROW <= NT, "tile words per thread");
+    static_assert(TX * TY == 2 * NT && kNLCap == 2 * NT && kStageRuns3 == 8 * NT, "fetched words per thread");
+    // The tile's words, root bitmaps and node counts were final before this grid's predecessor (the
     // scan and link pass) started: that grid waits for the merge to complete before it lets this
-    // one launch.  So they are read before the wait -- the entries into registers, the bitmap and
-    // count into shared memory (cp.async) -- and the segment prefixes and node links, which the
-    // predecessor writes, are copied after it.  With a fixed tile order (no work queue) the next
-    // tile's fetches are issued before the current tile's labels are written.
-    uint4 nL[4];
+    // one launch.  So they are read before the wait -- the words into registers, the rest into shared
+    // memory (cp.async) -- and the segment prefixes and node links, which the predecessor writes, are
+    // copied after it.  With a fixed tile order (no work queue) the next tile's fetches are issued
+    // before the current tile's labels are written.
+    uint4 nH[2];
+    uint32_t n10 = 0;
     auto fetch = [&](int64_t t) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) nL[i] = __ldcg(reinterpret_cast<const uint4 *>(lab + t * NBLK) + tid + i * NT);
-        cp_async16(&RB[4 * tid], w.rbits + t * (TX * TY * RBW) + 4 * tid);
+        const uint32_t *h = lab + t * T3_LAB_WORDS;
+        nH[0] = __ldcg(reinterpret_cast<const uint4 *>(h) + tid);
+        if (tid + NT < 3 * NROW) nH[1] = __ldcg(reinterpret_cast<const uint4 *>(h) + tid + NT);
+        if (tid < NROW) {
+            n10 = __ldcg(h + 12 * NROW + tid);
+            cp_async4(&RB[tid], w.rbits + t * NROW + tid);
+        }
+        cp_async16(&E[4 * tid], h + kHdr3 + 4 * tid);
         if (tid == NT - 1) cp_async4(&snb, w.nb + t);
         cp_async_commit();
     };
@@ -968,72 +888,83 @@ __global__ void __launch_bounds__(NT, 5) k_tile_write_3d(ImgList3D L, Work w)
         const Img3D im = L.get(t);
         const TileGeo g = tile_geo(im, t);
         const int64_t rs0 = int64_t(im.d1) * im.d2;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) reinterpret_cast<uint4 *>(Ls)[tid + i * NT] = nL[i];
+        H[tid] = nH[0];
+        if (tid + NT < 3 * NROW) H[tid + NT] = nH[1];
+        if (tid < NROW) H10[tid] = n10;
         cp_async_wait();
         __syncthreads();
         const uint32_t nb = snb, base0 = segb[TX * TY];
+        const uint4 *HR = H + 2 * NROW;
+        const uint32_t nrun = HR[NROW - 1].y + __popc(HR[NROW - 1].x);
         if (t == im.tile_base && tid == 0)
             w.ncomp[im.index] = int64_t(w.segpref[im.seg_base + int64_t(im.d0) * im.d1 * im.t2] - base0);
-        for (int b = tid; b < NBLK; b += NT) {
-            const uint32_t e = Ls[b];
-            if (!(e & ROOT_FLAG)) continue;
-            const uint32_t key = e & (ROOT_FLAG - 1);
-            const int Z = key % TZ, Y = (key / TZ) % TY, X = key / (TZ * TY);
-            const uint32_t *row = &RB[(X * TY + Y) * RBW];
-            uint32_t rank = __popc(row[Z >> 5] & ((1u << (Z & 31)) - 1u));
-            for (int k = 0; k < (Z >> 5); ++k) rank += __popc(row[k]);
-            LT[b] = 1u + (segb[X * TY + Y] - base0) + rank;
+        // Surviving roots, by block row and voxel row: rank = roots before it in its segment.
+#pragma unroll
+        for (int i = 0; i < 4 * NROW / NT; ++i) {
+            const int u = tid + i * NT, row = u / 4, ij = u % 4;
+            const uint4 rw = HR[row];
+            uint32_t bits = RB[row] & starts_of(ij, rw.x, rw.z, rw.w, H10[row]);
+            uint32_t label = 1u + segb[(2 * (row / TB1) + (ij >> 1)) * TY + 2 * (row % TB1) + (ij & 1)] - base0;
+            while (bits) {
+                const uint32_t bit = bits & (0u - bits);
+                LT[rw.y + __popc(rw.x & (bit | (bit - 1u)))] = label++;
+                bits &= bits - 1;
+            }
         }
-        __syncthreads();
         // Border components linked under another tile's component: the label of that root, its
-        // segment's prefix plus its rank among the first voxels left there (both resolved by the
-        // link pass).
+        // segment's prefix plus its rank among the roots left there (both resolved by the link pass).
         for (uint32_t j = tid; j < nb; j += NT) {
             const uint2 e = j < uint32_t(kNLCap) ? NL[j] : __ldcg(w.nlink + t * MAXB + j);
             if (e.x == kNone) continue;
-            const uint32_t nr = e.y >> 16;
-            if (GUARD(w, nr < uint32_t(NBLK) && e.x < w.n_segs, 402, t * MAXB + j))
-                LT[nr] = 1u + (__ldcg(w.segpref + e.x) - base0) + (e.y & 0xFFFFu);
+            const uint32_t blk = e.y >> 16;
+            if (GUARD(w, blk < uint32_t(NBLK) && e.x < w.n_segs, 402, t * MAXB + j)) {
+                const uint4 rw = HR[blk / TB2];
+                LT[rw.y + __popc(rw.x & ((2u << (blk % TB2)) - 1u))] = 1u + (__ldcg(w.segpref + e.x) - base0) + (e.y & 0xFFFFu);
+            }
         }
         __syncthreads();
-        if (fixed_order && t + gridDim.x < w.n_tiles) {   // RB, NL, segb and snb are free now
+        // Every other run takes the label of its root run.
+        for (uint32_t i = 2 * tid; i < nrun; i += 2 * NT) {
+            const uint32_t e = i < uint32_t(kStageRuns3) ? E[i >> 1] : __ldcg(lab + t * T3_LAB_WORDS + kHdr3 + (i >> 1));
+            const uint32_t a = e & 0xFFFFu, b = e >> 16;
+            if (!GUARD(w, a < nrun && (i + 1 >= nrun || b < nrun), 403, e)) continue;
+            if (a != i) LT[i + 1] = LT[a + 1];
+            if (i + 1 < nrun && b != i + 1) LT[i + 2] = LT[b + 1];
+        }
+        __syncthreads();
+        if (fixed_order && t + gridDim.x < w.n_tiles) {   // RB, NL, E, segb and snb are free now
             fetch(t + gridDim.x);
             fetch_links(t + gridDim.x);
         }
 
-        // Output: one unit = two blocks along d2 in all four voxel rows (X, Y) they cover: the two
-        // entries and labels are looked up once for four 16-byte stores.
-        for (int u = tid; u < TB0 * TB1 * (TB2 / 2); u += NT) {
-            const int q = u % (TB2 / 2), r = u / (TB2 / 2);
-            const int b0 = r / TB1, b1 = r % TB1;
-            if (2 * b0 >= g.nx || 2 * b1 >= g.ny || 4 * q >= g.nz) continue;
-            const int bb = blk(b0, b1, 2 * q);
-            const uint32_t e0 = Ls[bb], e1 = Ls[bb + 1];
-            const uint32_t m0 = e0 >> 24, m1 = e1 >> 24;
-            if (!GUARD(w, !m0 || (e0 & ROOT_FLAG) || (Ls[(e0 & 0x7FFFFFu) % NBLK] & ROOT_FLAG && (e0 & 0x7FFFFFu) < NBLK), 403, e0)) continue;
-            const uint32_t l0 = m0 ? ((e0 & ROOT_FLAG) ? LT[bb] : LT[e0 & 0x7FFFFFu]) : 0u;
-            const uint32_t l1 = m1 ? ((e1 & ROOT_FLAG) ? LT[bb + 1] : LT[e1 & 0x7FFFFFu]) : 0u;
-            const bool full = 4 * q + 4 <= g.nz;
+        // Output: one unit = two blocks along d2 in all four voxel rows (X, Y) they cover: the
+        // labels are looked up once for four 16-byte stores.  A thread keeps its place along d2.
+        const bool vec_ok = ((reinterpret_cast<uintptr_t>(im.out) | (uintptr_t(im.d2) * 4)) & 15) == 0;
+        const int q = tid % (TB2 / 2);
+        const uint32_t bit0 = 1u << (2 * q), bit1 = 2u << (2 * q), upto0 = bit0 | (bit0 - 1u);
+        const int n = min(4, max(0, g.nz - 4 * q));   // voxels of the thread's place inside the volume
+        for (int row = tid / (TB2 / 2); row < NROW; row += NT / (TB2 / 2)) {
+            const int b0 = row / TB1, b1 = row % TB1;
+            if (vec_ok && (n == 0 || 2 * b0 >= g.nx || 2 * b1 >= g.ny)) continue;
+            const uint4 a = H[row], b = H[NROW + row], rw = HR[row];
+            const uint32_t i0 = rw.y + __popc(rw.x & upto0);
+            const uint32_t l0 = LT[i0], l1 = LT[i0 + ((rw.x & bit1) ? 1u : 0u)];
 #pragma unroll
             for (int ij = 0; ij < 4; ++ij) {
                 const int X = 2 * b0 + (ij >> 1), Y = 2 * b1 + (ij & 1);
-                if (X >= g.nx || Y >= g.ny) continue;
-                const int sh = 2 * ij;   // mask bit of voxel (i, j, k) is 4i + 2j + k
+                const uint32_t ce = ij == 0 ? a.x : ij == 1 ? a.z : ij == 2 ? b.x : b.z;   // even, odd voxels
+                const uint32_t co = ij == 0 ? a.y : ij == 1 ? a.w : ij == 2 ? b.y : b.w;
                 int4 v;
-                v.x = ((m0 >> sh) & 1u) ? int(l0) : 0;
-                v.y = ((m0 >> (sh + 1)) & 1u) ? int(l0) : 0;
-                v.z = ((m1 >> sh) & 1u) ? int(l1) : 0;
-                v.w = ((m1 >> (sh + 1)) & 1u) ? int(l1) : 0;
+                v.x = (ce & bit0) ? int(l0) : 0;
+                v.y = (co & bit0) ? int(l0) : 0;
+                v.z = (ce & bit1) ? int(l1) : 0;
+                v.w = (co & bit1) ? int(l1) : 0;
                 int32_t *dst = im.out + (g.x0 + X) * rs0 + int64_t(g.y0 + Y) * im.d2 + g.z0 + 4 * q;
-                if (full && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+                const bool in = X < g.nx && Y < g.ny;
+                if (!vec_ok) {   // rows of any alignment: 16-byte stores across the row's lanes
+                    store_row<TB2 / 2>(dst, v, in ? n : 0);
+                } else if (in) {   // (vec_ok: d2 is a multiple of 4, so is every row's end)
                     __stcs(reinterpret_cast<int4 *>(dst), v);
-                } else {
-                    const int n = min(4, g.nz - 4 * q);
-                    dst[0] = v.x;
-                    if (n > 1) dst[1] = v.y;
-                    if (n > 2) dst[2] = v.z;
-                    if (n > 3) dst[3] = v.w;
                 }
             }
         }
