@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
         const Img2D im = L.get(t);
         const int64_t lt = t - im.tile_base;
-        const int ty = int(lt / im.tiles_x), tx = int(lt - int64_t(ty) * im.tiles_x);
+        const int ty = int(uint32_t(lt) / uint32_t(im.tiles_x)), tx = int(uint32_t(lt) - uint32_t(ty) * uint32_t(im.tiles_x));
         const int y0 = ty * TH, x0 = tx * TW;
         const int nrp = min(TH, im.rows - y0), ncp = min(TW, im.cols - x0);
         const int nbr = cells(nrp), nbc = cells(ncp);
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
         const Img2D im = L.get(t);
         const int64_t lt = t - im.tile_base;
-        const int ty = int(lt / im.tiles_x), tx = int(lt - int64_t(ty) * im.tiles_x);
+        const int ty = int(uint32_t(lt) / uint32_t(im.tiles_x)), tx = int(uint32_t(lt) - uint32_t(ty) * uint32_t(im.tiles_x));
         const int nbr = cells(min(TH, im.rows - ty * TH));
         const int nbc = cells(min(TW, im.cols - tx * TW));
         const uint16_t *pe = w.perim;
@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         if (!fixed_order && !first) fetch(t);   // a work queue gives the next tile only now
         const Img2D im = L.get(t);
         const int64_t lt = t - im.tile_base;
-        const int ty = int(lt / im.tiles_x), tx = int(lt - int64_t(ty) * im.tiles_x);
+        const int ty = int(uint32_t(lt) / uint32_t(im.tiles_x)), tx = int(uint32_t(lt) - uint32_t(ty) * uint32_t(im.tiles_x));
         const int y0 = ty * TH, x0 = tx * TW;
         const int nrp = min(TH, im.rows - y0), ncp = min(TW, im.cols - x0);
         H[tid] = nH;

@@ -98,10 +98,11 @@ struct TileGeo {
 __device__ __forceinline__ TileGeo tile_geo(const Img3D &im, int64_t t)
 {
     TileGeo g;
-    const int64_t lt = t - im.tile_base;
-    g.tx2 = int(lt % im.t2);
-    g.tx1 = int((lt / im.t2) % im.t1);
-    g.tx0 = int(lt / (int64_t(im.t2) * im.t1));
+    const uint32_t lt = uint32_t(t - im.tile_base);   // (an image has fewer than 2^31 tiles)
+    const uint32_t l12 = lt / uint32_t(im.t2);
+    g.tx2 = int(lt - l12 * uint32_t(im.t2));
+    g.tx0 = int(l12 / uint32_t(im.t1));
+    g.tx1 = int(l12 - uint32_t(g.tx0) * uint32_t(im.t1));
     g.x0 = g.tx0 * TX; g.y0 = g.tx1 * TY; g.z0 = g.tx2 * TZ;
     g.nx = min(TX, im.d0 - g.x0); g.ny = min(TY, im.d1 - g.y0); g.nz = min(TZ, im.d2 - g.z0);
     g.n0 = (g.nx + 1) >> 1; g.n1 = (g.ny + 1) >> 1; g.n2 = (g.nz + 1) >> 1;
