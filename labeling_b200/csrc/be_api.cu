@@ -87,6 +87,7 @@ size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_img
     t.perim = reinterpret_cast<uint16_t *>(take(size_t(n_tiles) * g.nperim * sizeof(uint16_t)));
     t.rbits = reinterpret_cast<uint32_t *>(take(size_t(n_tiles) * g.rbits_bytes_per_tile));
     t.nb = reinterpret_cast<uint32_t *>(take(size_t(n_tiles) * sizeof(uint32_t)));
+    t.timg = reinterpret_cast<uint32_t *>(take(n_imgs > 1 ? size_t(n_tiles) * sizeof(uint32_t) : 0));
     t.gp = reinterpret_cast<unsigned long long *>(take(nodes * sizeof(unsigned long long)));
     t.nroot = reinterpret_cast<uint16_t *>(take(nodes * sizeof(uint16_t)));
     t.nlink = g.links ? reinterpret_cast<uint2 *>(take(nodes * sizeof(uint2))) : nullptr;
@@ -189,39 +190,6 @@ void fill_img3d(Img3D &im, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2
     im.seg_base = seg_base;
     im.thr = thr;
     im.index = index;
-}
-
-cudaError_t launch_uf3d(const ImgList3D &L, const Work &w, int sms, bool persistent, cudaStream_t s,
-                        cudaEvent_t *ev)
-{
-    auto mark = [&](int i) {
-        if (ev) cudaEventRecord(ev[i], s);
-    };
-    auto grid = [&](int64_t items, int per_sm) -> unsigned {
-        int64_t g = persistent ? std::min<int64_t>(items, int64_t(sms) * per_sm) : items;
-        return unsigned(std::max<int64_t>(g, 1));
-    };
-    Work wk = w;
-    if (!persistent) wk.queue = nullptr;
-    // The launches after the first overlap their start with the tail of the one before (they
-    // wait for it on the device); not when events are recorded between them.
-    const bool ov = !persistent && !ev;
-    cudaError_t e = cudaSuccess;
-    auto keep = [&](cudaError_t r) {
-        if (e == cudaSuccess) e = r;
-    };
-    mark(0);
-    keep(launch_k(k_tile_local_3d, grid(w.n_tiles, kT3LocalPerSM), kT3LocalThreads, s, false, L, wk));
-    mark(1);
-    keep(launch_k(k_merge_3d, grid(w.n_tiles, kT3MergePerSM), kT3MergeThreads, s, ov, L, wk));
-    mark(2);
-    keep(launch_k(k_scan_link_3d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, L, wk));
-    mark(3);
-    // The label writes run a fixed tile order over kT3WritePerSM CTAs per SM (they prefetch their next tile).
-    keep(launch_k(k_tile_write_3d, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * kT3WritePerSM))),
-                  kT3Threads, s, ov, L, wk));
-    mark(4);
-    return e;
 }
 
 }  // namespace be

@@ -54,7 +54,8 @@ struct ImgList {
     const Img *ptr;
     int n;
     Img one;
-    __device__ __forceinline__ Img get(int64_t tile) const;
+    __device__ __forceinline__ Img find(int64_t tile, uint32_t *timg) const;
+    __device__ __forceinline__ Img get(int64_t tile, const uint32_t *timg) const;
 };
 
 // Global scratch of one pipeline launch ("workspace").  Sizes are per tile so that every tile
@@ -63,6 +64,7 @@ struct Work {
     void *lab;            // per-block tile-local labels: uint16 (2D) / uint32 (3D), NBLK per tile
     uint16_t *perim;      // per tile NPERIM border entries: (node << 4) | side bits, 0 = empty
     uint32_t *nb;         // per tile: number of nodes
+    uint32_t *timg;       // per tile: its image's place in the launch's list (launches of several images)
     unsigned long long *gp;   // per node (tile * MAXB + j): union-find entry (key of the parent << 32) |
                               // parent (global node id); see gentry
     uint16_t *nroot;      // per node: tile-local block index of the node's root block
@@ -396,10 +398,20 @@ __device__ __forceinline__ int find_img_tile(const Img *imgs, int n, int64_t t)
     return lo;
 }
 
+// The image of a tile: by search in the first launch, which leaves its index for the later ones.
 template <class Img>
-__device__ __forceinline__ Img ImgList<Img>::get(int64_t tile) const
+__device__ __forceinline__ Img ImgList<Img>::find(int64_t tile, uint32_t *timg) const
 {
-    return n == 1 ? one : ptr[find_img_tile(ptr, n, tile)];
+    if (n == 1) return one;
+    const int i = find_img_tile(ptr, n, tile);
+    if (threadIdx.x == 0) timg[tile] = uint32_t(i);
+    return ptr[i];
+}
+
+template <class Img>
+__device__ __forceinline__ Img ImgList<Img>::get(int64_t tile, const uint32_t *timg) const
+{
+    return n == 1 ? one : ptr[__ldcg(timg + tile)];
 }
 
 using ImgList2D = ImgList<Img2D>;
@@ -590,24 +602,36 @@ inline cudaError_t launch_k(void (*k)(P...), unsigned grid, unsigned block, cuda
     return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
-// Work distribution: with a queue counter every CTA pulls items until none are left (persistent
-// launch); without one, CTA b takes items b, b + grid, ...
+// Work distribution: with a queue (Q) every CTA pulls items from a counter until none are left
+// (persistent launch); without one, CTA b takes items b, b + grid, ...  The counter's answer takes an L2
+// round trip, so a CTA asks for its next item (request) while it still works on the current one and
+// reads the answer (next) after the barrier that ends it -- or an earlier one, where it prefetches.
+template <bool Q>
 struct ItemLoop {
     uint32_t *queue;
-    int64_t n;
+    uint32_t ticket = 0;   // thread 0: the item asked for
     __device__ __forceinline__ int64_t first(uint32_t *slot)
     {
-        if (!queue) return blockIdx.x;
+        if (!Q) return blockIdx.x;
         if (threadIdx.x == 0) *slot = atomicAdd(queue, 1u);
         __syncthreads();
-        int64_t v = *slot;
+        const int64_t v = *slot;
         __syncthreads();
         return v;
     }
-    __device__ __forceinline__ int64_t next(int64_t cur, uint32_t *slot)
+    __device__ __forceinline__ void request()
     {
-        if (!queue) return cur + gridDim.x;
-        return first(slot);
+        if (Q && threadIdx.x == 0) ticket = atomicAdd(queue, 1u);
+    }
+    // Publishes the answer; a barrier goes between this and next(), and another between next() and the
+    // following publish().
+    __device__ __forceinline__ void publish(uint32_t *slot)
+    {
+        if (Q && threadIdx.x == 0) *slot = ticket;
+    }
+    __device__ __forceinline__ int64_t next(int64_t cur, const uint32_t *slot) const
+    {
+        return Q ? int64_t(*slot) : cur + gridDim.x;
     }
 };
 

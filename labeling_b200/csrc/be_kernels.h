@@ -24,11 +24,6 @@
 
 namespace be {
 
-__global__ void k_tile_local_3d(ImgList3D L, Work w);
-__global__ void k_merge_3d(ImgList3D L, Work w);
-__global__ void k_scan_link_3d(ImgList3D L, Work w);
-__global__ void k_tile_write_3d(ImgList3D L, Work w);
-
 __global__ void k_segscan(Work w);
 __global__ void k_chunk_sums(Work w);
 

@@ -79,6 +79,7 @@ __device__ __forceinline__ uint32_t count_bits(const uint32_t *b, uint32_t lo, u
 // The loops over runs and links are shared evenly by the CTA's threads, and the tile is handed on as
 // bit words and one number per run, not as an entry per block.
 // ---------------------------------------------------------------------------------------------
+template <bool Q>
 __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L, Work w)
 {
     grid_dep_release();   // the merge launch may take free SMs during this grid's last wave
@@ -101,9 +102,9 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r = tid / WPR, q = tid % WPR;
     uint32_t *lab = reinterpret_cast<uint32_t *>(w.lab);
-    ItemLoop loop{w.queue ? w.queue + 0 : nullptr, w.n_tiles};
+    ItemLoop<Q> loop{w.queue + 0};
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
-        const Img2D im = L.get(t);
+        const Img2D im = L.find(t, w.timg);
         const int64_t lt = t - im.tile_base;
         const int ty = int(uint32_t(lt) / uint32_t(im.tiles_x)), tx = int(uint32_t(lt) - uint32_t(ty) * uint32_t(im.tiles_x));
         const int y0 = ty * TH, x0 = tx * TW;
@@ -417,6 +418,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
         }
         __syncthreads();
 
+        loop.request();
         // Phase D: every run's root, the tile's root bitmap and the segments' root counts out.
         auto root_of = [&](uint32_t id) -> uint32_t { return P[P[id & (MAXRUN - 1)]]; };
         {
@@ -511,6 +513,8 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
             w.perim[t * NPERIM + p] = ent;
         }
         if (tid == 0) w.nb[t] = noff[RBWORDS / 32];
+        if (!Q) break;   // one tile per CTA
+        loop.publish(&qslot);
         __syncthreads();
     }
 }
@@ -551,6 +555,7 @@ constexpr int NLOC2 = MAXB + TBH + TBW + 2;    // local union-find size
 // union-find, from a shared queue once all of the tile's pairs are seen.  The merge is bound by
 // the latency of those global unions (dependent L2 round trips), so a CTA is two warps that loop
 // over the positions: many tiles are in flight on each SM at once.
+template <bool Q>
 __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work w)
 {
     grid_dep_wait();
@@ -563,9 +568,10 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
     __shared__ uint8_t cm[K2_NP];             // connected staged neighbours of each position
     __shared__ uint2 gq[kGQ2];
     __shared__ uint32_t nq;
-    ItemLoop loop{w.queue ? w.queue + 1 : nullptr, w.n_tiles};
+    ItemLoop<Q> loop{w.queue + 1};
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
-        const Img2D im = L.get(t);
+        const Img2D im = L.get(t, w.timg);
+        loop.request();
         const int64_t lt = t - im.tile_base;
         const int ty = int(uint32_t(lt) / uint32_t(im.tiles_x)), tx = int(uint32_t(lt) - uint32_t(ty) * uint32_t(im.tiles_x));
         const int nbr = cells(min(TH, im.rows - ty * TH));
@@ -706,6 +712,8 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
         __syncthreads();
         const uint32_t nqt = min(nq, uint32_t(kGQ2));
         for (uint32_t i = threadIdx.x; i < nqt; i += K2_NT) gunion2d(im, w, gq[i].x, gq[i].y);
+        if (!Q) break;   // one tile per CTA
+        loop.publish(&qslot);
         __syncthreads();
     }
 }
@@ -722,10 +730,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_flatten_2d(Work w)
     grid_dep_release();   // after the wait: the label-write launch relies on it
     __shared__ uint32_t tmp[kScanThreads / 32 + 1];
     __shared__ uint32_t sh[2];
-    __shared__ uint32_t qslot;
     const int64_t n = int64_t(w.n_chunks) + w.n_tiles;
-    ItemLoop loop{w.queue ? w.queue + 2 : nullptr, n};
-    for (int64_t it = loop.first(&qslot); it < n; it = loop.next(it, &qslot)) {
+    for (int64_t it = blockIdx.x; it < n; it += gridDim.x) {   // (in a fixed order: the items are short)
         if (it < w.n_chunks) {
             segscan_lb_chunk<kScanThreads>(w, tmp, sh);
             continue;
@@ -740,6 +746,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_flatten_2d(Work w)
 constexpr int K3_NT = 256;
 constexpr int K3_PER_SM = 8;              // resident CTAs per SM
 
+template <bool Q>
 __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L, Work w)
 {
     __shared__ __align__(16) uint4 H[kHdr / 4];   // class words, then run words
@@ -756,9 +763,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
     // the merge) were final before this grid's predecessor (segment scan and node flatten) started:
     // that grid waits for the merge to complete before it lets this one launch.  So they are read
     // before the wait (through L2), and only the segment prefixes, which the scan writes, after it.
-    // With a fixed tile order (no work queue) the CTA fetches the next tile while it works on the
-    // current one: its words into registers, the root bitmap and run entries into shared memory
-    // (cp.async) as soon as the current tile's are used up.
+    // The words go into registers, the root bitmap and run entries into shared memory (cp.async).
     static_assert(TW % 128 == 0, "a warp's output units lie in one row");
     static_assert(kHdr == 4 * K3_NT && TH * WPR == K3_NT && kStageRuns == 8 * K3_NT, "prefetched words per thread");
     uint4 nH;
@@ -780,21 +785,22 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         fetch_roots(t);
         fetch_runs(t);
     };
-    const bool fixed_order = w.queue == nullptr;
-    ItemLoop loop{w.queue ? w.queue + 4 : nullptr, w.n_tiles};
+    ItemLoop<Q> loop{w.queue + 4};
     int64_t t = loop.first(&qslot);
     if (t < w.n_tiles) fetch(t);
-    for (bool first = true; t < w.n_tiles; t = loop.next(t, &qslot), first = false) {
-        if (!fixed_order && !first) fetch(t);   // a work queue gives the next tile only now
-        const Img2D im = L.get(t);
+    while (t < w.n_tiles) {
+        loop.request();
+        const Img2D im = L.get(t, w.timg);
         const int64_t lt = t - im.tile_base;
         const int ty = int(uint32_t(lt) / uint32_t(im.tiles_x)), tx = int(uint32_t(lt) - uint32_t(ty) * uint32_t(im.tiles_x));
         const int y0 = ty * TH, x0 = tx * TW;
         const int nrp = min(TH, im.rows - y0), ncp = min(TW, im.cols - x0);
         H[tid] = nH;
         const uint32_t nb = nNb;
-        const int64_t tn = fixed_order && t + gridDim.x < w.n_tiles ? t + gridDim.x : -1;   // next tile
-        if (tn >= 0) fetch_words(tn);
+        // The next tile's data come while this one's labels are worked out and written, each part as soon
+        // as its place is free -- and the tile is known, which with a work queue is before the writes.
+        int64_t tn = Q ? w.n_tiles : t + gridDim.x;
+        if (tn < w.n_tiles) fetch_words(tn);
         cp_async_wait();
         grid_dep_wait();   // segment prefixes from here on (returns at once after the first tile)
         const uint32_t base0 = w.segpref[im.seg_base];
@@ -842,7 +848,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             LT[__ldcg(w.nroot + node) + 1u] = 1u + sb + rank;
         }
         __syncthreads();
-        if (tn >= 0) fetch_roots(tn);
+        if (tn < w.n_tiles) fetch_roots(tn);
         // Every other run takes the label of its root run.
         for (uint32_t i = 2 * tid; i < nrun; i += 2 * K3_NT) {
             const uint32_t e = i < uint32_t(kStageRuns) ? E[i >> 1] : __ldcg(lab + t * kLabWords + kHdr + (i >> 1));
@@ -850,8 +856,14 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             if (a != i) LT[i + 1] = LT[a + 1];
             if (i + 1 < nrun && b != i + 1) LT[i + 2] = LT[b + 1];
         }
+        loop.publish(&qslot);
         __syncthreads();
-        if (tn >= 0) fetch_runs(tn);
+        if (Q) {
+            tn = loop.next(t, &qslot);
+            if (tn < w.n_tiles) fetch(tn);
+        } else if (tn < w.n_tiles) {
+            fetch_runs(tn);
+        }
 
         // Output: one unit = 4 pixels in each row of a block row (two 2x2 blocks, or four pixel cells).
         const bool vec_ok = ((reinterpret_cast<uintptr_t>(im.out) | uintptr_t(im.out_pitch * 4)) & 15) == 0;
@@ -916,6 +928,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             }
         }
         __syncthreads();
+        t = tn;
     }
 }
 
@@ -942,8 +955,6 @@ inline cudaError_t launch(const ImgList2D &L, const Work &w, int sms, bool persi
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
     };
-    Work wk = w;
-    if (!persistent) wk.queue = nullptr;
     // The launches after the first overlap their start with the tail of the one before (they
     // wait for it on the device); not when events are recorded between them.
     const bool ov = !persistent && !ev;
@@ -952,15 +963,15 @@ inline cudaError_t launch(const ImgList2D &L, const Work &w, int sms, bool persi
         if (e == cudaSuccess) e = r;
     };
     mark(0);
-    keep(launch_k(k_tile_local_2d, grid(w.n_tiles, K1_PER_SM), K1_NT, s, false, L, wk));
+    keep(launch_k(persistent ? k_tile_local_2d<true> : k_tile_local_2d<false>, grid(w.n_tiles, K1_PER_SM), K1_NT, s, false, L, w));
     mark(1);
-    keep(launch_k(k_merge_2d, grid(w.n_tiles, K2_PER_SM), K2_NT, s, ov, L, wk));
+    keep(launch_k(persistent ? k_merge_2d<true> : k_merge_2d<false>, grid(w.n_tiles, K2_PER_SM), K2_NT, s, ov, L, w));
     mark(2);
-    keep(launch_k(k_scan_flatten_2d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, wk));
+    keep(launch_k(k_scan_flatten_2d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, w));
     mark(3);
     // The label writes run a fixed tile order over K3_PER_SM CTAs per SM (they prefetch their next tile).
-    keep(launch_k(k_tile_write_2d, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * K3_PER_SM))),
-                  K3_NT, s, ov, L, wk));
+    keep(launch_k(persistent ? k_tile_write_2d<true> : k_tile_write_2d<false>, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * K3_PER_SM))),
+                  K3_NT, s, ov, L, w));
     mark(4);
     return e;
 }

@@ -37,6 +37,10 @@
 #include "be_kernels.h"
 #include "be_scan.cuh"
 
+#include "be_api_internal.h"
+
+#include <algorithm>
+
 namespace be {
 
 namespace {
@@ -276,6 +280,7 @@ __device__ __noinline__ uint2 row_bits_call(const uint8_t *p, int n, const uint8
 
 }  // namespace
 
+template <bool Q>
 __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D L, Work w)
 {
     grid_dep_release();   // the merge launch may take free SMs during this grid's last wave
@@ -297,9 +302,9 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b0 = tid / TB1, b1 = tid % TB1;
     uint32_t *lab = reinterpret_cast<uint32_t *>(w.lab);
-    ItemLoop loop{w.queue ? w.queue + 0 : nullptr, w.n_tiles};
+    ItemLoop<Q> loop{w.queue + 0};
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
-        const Img3D im = L.get(t);
+        const Img3D im = L.find(t, w.timg);
         const TileGeo g = tile_geo(im, t);
         const uint32_t K = (0x7Fu - (uint32_t(im.thr) & 0x7Fu)) * 0x01010101u;
         const bool hi = im.thr >= 128;
@@ -516,6 +521,7 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
         // Phase C: every run's entry becomes its root's.
         if (total) eflatten3_all(P, tid, NT1, nrun);
         __syncthreads();
+        loop.request();
         // Phase D: the root bitmap (a bit per run start, so a word per row) and the segments' root
         // counts.
         uint32_t roots = 0;
@@ -593,6 +599,8 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
                         ((c[3] >> 31) << 5) | ((c[5] >> 31) << 6) | ((c[7] >> 31) << 7));
         }
         if (tid == 0) w.nb[t] = noff[NBLK / 32 / 32];
+        if (!Q) break;   // one tile per CTA
+        loop.publish(&qslot);
         __syncthreads();
     }
 }
@@ -625,11 +633,12 @@ __device__ void gunion3d(const Img3D &im, Work &w, uint32_t a, uint32_t b)
 constexpr int kMQ3 = 1024;     // queued links (more take further rounds)
 constexpr int kSeen3 = 256;    // table of node pairs seen
 
+template <bool Q>
 __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(ImgList3D L, Work w)
 {
     grid_dep_wait();
     grid_dep_release();
-    __shared__ uint32_t Q[kMQ3];
+    __shared__ uint32_t LQ[kMQ3];
     __shared__ unsigned long long seen[kSeen3];
     __shared__ uint32_t nq;
     __shared__ uint32_t qslot;
@@ -637,9 +646,10 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
     const int tid = threadIdx.x;
     const int b0 = tid / TB1, b1 = tid % TB1;
     const uint32_t *lab = reinterpret_cast<const uint32_t *>(w.lab);
-    ItemLoop loop{w.queue ? w.queue + 1 : nullptr, w.n_tiles};
+    ItemLoop<Q> loop{w.queue + 1};
     for (int64_t t = loop.first(&qslot); t < w.n_tiles; t = loop.next(t, &qslot)) {
-        const Img3D im = L.get(t);
+        const Img3D im = L.get(t, w.timg);
+        loop.request();
         const TileGeo g = tile_geo(im, t);
         for (int i = tid; i < kSeen3; i += kT3MergeThreads) seen[i] = ~0ull;
         if (tid == 0) nq = 0;
@@ -732,7 +742,7 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
                     LE[nr] &= isE ? ~bit : ~0u;
                     const uint32_t own = base + __popc(S & upto) - 1u;
                     const uint32_t up = uw.y + __popc(uw.x & (isN ? upto : isW ? bit - 1u : (bit << 2) - 1u)) - 1u;
-                    Q[pos++ - from] = own | (up << 12) | (uint32_t(code) << 24);
+                    LQ[pos++ - from] = own | (up << 12) | (uint32_t(code) << 24);
                 }
             }
             if (zm && pos < end) {
@@ -747,7 +757,7 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
                     if (k != 4) code = preceding(k < 4 ? k : k - 5, rr);
                     const uint32_t zu = znodes(tile_at(code, k < 5 ? -1 : 1), rr);
                     const uint32_t a = k < 5 ? zo & 0xFFFFu : zo >> 16, b = k < 5 ? zu >> 16 : zu & 0xFFFFu;
-                    Q[pos++ - from] = a | (b << 11) | (uint32_t(code) << 24) | (k < 5 ? 1u << 29 : 2u << 29);
+                    LQ[pos++ - from] = a | (b << 11) | (uint32_t(code) << 24) | (k < 5 ? 1u << 29 : 2u << 29);
                 }
             }
         };
@@ -761,7 +771,7 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
             }
             const uint32_t cnt = min(total - from, uint32_t(kMQ3));
             for (uint32_t i = tid; i < cnt; i += kT3MergeThreads) {
-                const uint32_t e = Q[i], z = e >> 29;
+                const uint32_t e = LQ[i], z = e >> 29;
                 const int64_t tt = tile_at(int(e >> 24) & 31, z == 0 ? 0 : z == 1 ? -1 : 1);
                 uint32_t a, b;
                 if (z) {
@@ -781,6 +791,8 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
             }
             __syncthreads();
         }
+        if (!Q) break;   // one tile per CTA
+        loop.publish(&qslot);
         __syncthreads();   // every lane has read this tile's count
     }
 }
@@ -797,16 +809,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_link_3d(ImgList3D L, Work
     grid_dep_release();   // after the wait: the label-write launch relies on it
     __shared__ uint32_t tmp[kScanThreads / 32 + 1];
     __shared__ uint32_t sh[2];
-    __shared__ uint32_t qslot;
     const int64_t n = int64_t(w.n_chunks) + w.n_tiles;
-    ItemLoop loop{w.queue ? w.queue + 2 : nullptr, n};
-    for (int64_t it = loop.first(&qslot); it < n; it = loop.next(it, &qslot)) {
+    for (int64_t it = blockIdx.x; it < n; it += gridDim.x) {   // (in a fixed order: the items are short)
         if (it < w.n_chunks) {
             segscan_lb_chunk<kScanThreads>(w, tmp, sh);
             continue;
         }
         const int64_t t = it - w.n_chunks;
-        const Img3D im = L.get(t);
+        const Img3D im = L.get(t, w.timg);
         link_tile_nodes(w, t, MAXB, [&](uint32_t root, uint32_t key, uint32_t &seg, uint32_t &rank) {
             // The root's segment, and the roots left in it before the root.
             const uint32_t sg = key / seg_width3(im), line = sg / uint32_t(im.t2);   // line = X * d1 + Y
@@ -828,6 +838,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_link_3d(ImgList3D L, Work
 constexpr int kNLCap = 512;        // node links a write CTA stages in shared memory (later ones: from L2)
 constexpr int kStageRuns3 = 2048;  // run entries likewise
 
+template <bool Q>
 __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L, Work w)
 {
     __shared__ __align__(16) uint4 H[3 * NROW];   // class words 0..3, 4..7, (starts, runs before, S00, S01)
@@ -848,8 +859,7 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
     // scan and link pass) started: that grid waits for the merge to complete before it lets this
     // one launch.  So they are read before the wait -- the words into registers, the rest into shared
     // memory (cp.async) -- and the segment prefixes and node links, which the predecessor writes, are
-    // copied after it.  With a fixed tile order (no work queue) the next tile's fetches are issued
-    // before the current tile's labels are written.
+    // copied after it.  The next tile's fetches are issued before the current tile's labels are written.
     uint4 nH[2];
     uint32_t n10 = 0;
     auto fetch = [&](int64_t t) {
@@ -865,7 +875,7 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
         cp_async_commit();
     };
     auto fetch_links = [&](int64_t t) {
-        const Img3D im = L.get(t);
+        const Img3D im = L.get(t, w.timg);
         const TileGeo g = tile_geo(im, t);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -878,15 +888,16 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
         if (tid == 0) cp_async4(&segb[TX * TY], w.segpref + im.seg_base);
         cp_async_commit();
     };
-    const bool fixed_order = w.queue == nullptr;
-    ItemLoop loop{w.queue ? w.queue + 4 : nullptr, w.n_tiles};
+    ItemLoop<Q> loop{w.queue + 4};
     int64_t t = loop.first(&qslot);
     if (t < w.n_tiles) fetch(t);
-    for (bool first = true; t < w.n_tiles; t = loop.next(t, &qslot), first = false) {
-        if (!fixed_order && !first) fetch(t);   // a work queue gives the next tile only now
-        if (first) grid_dep_wait();   // segment prefixes and node links from here on
-        if (first || !fixed_order) fetch_links(t);
-        const Img3D im = L.get(t);
+    if (t < w.n_tiles) {
+        grid_dep_wait();   // segment prefixes and node links from here on
+        fetch_links(t);
+    }
+    while (t < w.n_tiles) {
+        loop.request();
+        const Img3D im = L.get(t, w.timg);
         const TileGeo g = tile_geo(im, t);
         const int64_t rs0 = int64_t(im.d1) * im.d2;
         H[tid] = nH[0];
@@ -932,10 +943,12 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
             if (a != i) LT[i + 1] = LT[a + 1];
             if (i + 1 < nrun && b != i + 1) LT[i + 2] = LT[b + 1];
         }
+        loop.publish(&qslot);
         __syncthreads();
-        if (fixed_order && t + gridDim.x < w.n_tiles) {   // RB, NL, E, segb and snb are free now
-            fetch(t + gridDim.x);
-            fetch_links(t + gridDim.x);
+        const int64_t tn = loop.next(t, &qslot);   // the next tile's data come while this one's labels go
+        if (tn < w.n_tiles) {   // RB, NL, E, segb and snb are free now
+            fetch(tn);
+            fetch_links(tn);
         }
 
         // Output: one unit = two blocks along d2 in all four voxel rows (X, Y) they cover: the
@@ -970,7 +983,42 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
             }
         }
         __syncthreads();
+        t = tn;
     }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Launch sequence.
+// ---------------------------------------------------------------------------------------------
+cudaError_t launch_uf3d(const ImgList3D &L, const Work &w, int sms, bool persistent, cudaStream_t s,
+                        cudaEvent_t *ev)
+{
+    auto mark = [&](int i) {
+        if (ev) cudaEventRecord(ev[i], s);
+    };
+    auto grid = [&](int64_t items, int per_sm) -> unsigned {
+        int64_t g = persistent ? std::min<int64_t>(items, int64_t(sms) * per_sm) : items;
+        return unsigned(std::max<int64_t>(g, 1));
+    };
+    // The launches after the first overlap their start with the tail of the one before (they
+    // wait for it on the device); not when events are recorded between them.
+    const bool ov = !persistent && !ev;
+    cudaError_t e = cudaSuccess;
+    auto keep = [&](cudaError_t r) {
+        if (e == cudaSuccess) e = r;
+    };
+    mark(0);
+    keep(launch_k(persistent ? k_tile_local_3d<true> : k_tile_local_3d<false>, grid(w.n_tiles, kT3LocalPerSM), kT3LocalThreads, s, false, L, w));
+    mark(1);
+    keep(launch_k(persistent ? k_merge_3d<true> : k_merge_3d<false>, grid(w.n_tiles, kT3MergePerSM), kT3MergeThreads, s, ov, L, w));
+    mark(2);
+    keep(launch_k(k_scan_link_3d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, L, w));
+    mark(3);
+    // The label writes run a fixed tile order over kT3WritePerSM CTAs per SM (they prefetch their next tile).
+    keep(launch_k(persistent ? k_tile_write_3d<true> : k_tile_write_3d<false>, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * kT3WritePerSM))),
+                  kT3Threads, s, ov, L, w));
+    mark(4);
+    return e;
 }
 
 }  // namespace be
