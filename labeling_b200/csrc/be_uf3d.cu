@@ -623,13 +623,14 @@ __device__ void gunion3d(const Img3D &im, Work &w, uint32_t a, uint32_t b)
 
 }  // namespace
 
-// Cross-tile merge.  One CTA per tile, one thread per block row: the row's links to those of its four
-// preceding rows that lie in other tiles, by the same bit operations as inside a tile (row_links), and
-// its first and last block's links across d2 to the tiles beside (one byte of face voxels per row and
-// two nodes, written by the tile kernel).  The links go through a shared queue, so that the rows on a
-// face, which have most of them, are shared by all lanes; a pair of nodes that the CTA has just seen
-// -- most links join the same few large components -- is dropped by a small table, and the others
-// are unions, whose walks (dependent loads through L2) end as soon as the two sides have one parent.
+// Cross-tile merge.  One CTA per tile: the links of its block rows to those of their four preceding rows
+// that lie in other tiles, by the same bit operations as inside a tile (row_links), and the links of
+// their first and last blocks across d2 to the tiles beside (one byte of face voxels per row and two
+// nodes, written by the tile kernel).  Of the 512 (row, preceding row) pairs only 70 leave the tile: one
+// warp takes those of one direction, a lane a pair.  The links go through a shared queue and are shared
+// by all lanes; a pair of nodes that the CTA has just seen -- most links join the same few large
+// components -- is dropped by a small table, and the others are unions, whose walks (dependent loads
+// through L2) end as soon as the two sides have one parent.
 constexpr int kMQ3 = 1024;     // queued links (more take further rounds)
 constexpr int kSeen3 = 256;    // table of node pairs seen
 
@@ -642,8 +643,8 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
     __shared__ unsigned long long seen[kSeen3];
     __shared__ uint32_t nq;
     __shared__ uint32_t qslot;
-    static_assert(kT3MergeThreads == NROW, "one thread per block row");
-    const int tid = threadIdx.x;
+    static_assert(kT3MergeThreads == NROW && TB1 + TB0 - 1 <= 32, "one thread per block row; a warp's lanes take a direction");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b0 = tid / TB1, b1 = tid % TB1;
     const uint32_t *lab = reinterpret_cast<const uint32_t *>(w.lab);
     ItemLoop<Q> loop{w.queue + 1};
@@ -655,10 +656,10 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
         if (tid == 0) nq = 0;
         __syncthreads();
 
-        // Preceding row nr: its row in its tile, and that tile's offset code 4 * (o0 + 1) + (o1 + 1)
-        // with o0 in {-1, 0}; 16 when there is no such tile.
-        auto preceding = [&](int nr, int &rr) -> int {
-            const int r0 = b0 + (nr < 3 ? -1 : 0), r1 = b1 + (nr < 3 ? nr - 1 : -1);
+        // Preceding row nr of row (a, b): its row in its tile, and that tile's offset code
+        // 4 * (o0 + 1) + (o1 + 1) with o0 in {-1, 0}; 16 when there is no such tile.
+        auto preceding = [&](int a, int b, int nr, int &rr) -> int {
+            const int r0 = a + (nr < 3 ? -1 : 0), r1 = b + (nr < 3 ? nr - 1 : -1);
             const int o0 = r0 < 0 ? -1 : 0, o1 = r1 < 0 ? -1 : r1 >= TB1 ? 1 : 0;
             rr = (r0 & (TB0 - 1)) * TB1 + (r1 & (TB1 - 1));
             if (g.tx0 + o0 < 0 || g.tx1 + o1 < 0 || g.tx1 + o1 >= im.t1) return 16;
@@ -668,31 +669,60 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
             return t + (int64_t((code >> 2) - 1) * im.t1 + (code & 3) - 1) * im.t2 + o2;
         };
         constexpr int kOwn = 5;   // code of the row's own tile
-        // Links to rows of other tiles.
-        uint32_t LN[4] = {0u, 0u, 0u, 0u}, LW[4] = {0u, 0u, 0u, 0u}, LE[4] = {0u, 0u, 0u, 0u};
-        uint32_t S = 0, base = 0;
-        const bool inside = b0 < g.n0 && b1 < g.n1;
-        if (inside && ((b0 == 0 && g.tx0 > 0) || (b1 == 0 && g.tx1 > 0) || (b1 == TB1 - 1 && g.tx1 + 1 < im.t1))) {
-            const uint4 *h = reinterpret_cast<const uint4 *>(lab + t * T3_LAB_WORDS);
-            const uint4 ca = __ldcg(h + tid), cb = __ldcg(h + NROW + tid), rw = __ldcg(h + 2 * NROW + tid);
-            const uint32_t c[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-            S = rw.x;
-            base = rw.y;
-            const uint32_t hz = row_joins(c);
-            if (S) {
-#pragma unroll
-                for (int nr = 0; nr < 4; ++nr) {
-                    int rr;
-                    const int code = preceding(nr, rr);
-                    if (code == kOwn || code == 16) continue;
-                    const uint4 *uh = reinterpret_cast<const uint4 *>(lab + tile_at(code, 0) * T3_LAB_WORDS);
-                    const uint4 ua = __ldcg(uh + rr), ub = __ldcg(uh + NROW + rr);
-                    const uint32_t u[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
-                    Links raw;
-                    const Links l = row_links(nr, c, hz, ua, ub, row_joins(u), raw);
-                    LN[nr] = l.n;
-                    LW[nr] = l.w;
-                    LE[nr] = l.e;
+        // Links to rows of other tiles: warp 0 straight below (the rows of the first layer), warp 1 below
+        // left (the first layer; the others' first row), warp 2 below right (.. last row), warp 3 beside
+        // (every layer's first row).
+        const int nr = warp == 0 ? 1 : warp == 1 ? 0 : warp;
+        const int ra = nr == 3 ? lane : lane < TB1 ? 0 : lane - TB1 + 1;
+        const int rb = nr == 3 ? 0 : lane < TB1 ? lane : nr == 0 ? 0 : TB1 - 1;
+        Links lk{0u, 0u, 0u};
+        uint32_t S = 0, base = 0, uS = 0, ubase = 0;
+        int code = 16;
+        if (ra < g.n0 && rb < g.n1 && lane < (nr == 1 ? TB1 : nr == 3 ? TB0 : TB1 + TB0 - 1)) {
+            int rr;
+            code = preceding(ra, rb, nr, rr);
+            if (code != kOwn && code != 16) {
+                const uint4 *h = reinterpret_cast<const uint4 *>(lab + t * T3_LAB_WORDS);
+                const uint4 *uh = reinterpret_cast<const uint4 *>(lab + tile_at(code, 0) * T3_LAB_WORDS);
+                const int row = ra * TB1 + rb;
+                const uint4 ca = __ldcg(h + row), cb = __ldcg(h + NROW + row), rw = __ldcg(h + 2 * NROW + row);
+                const uint4 ua = __ldcg(uh + rr), ub = __ldcg(uh + NROW + rr), uw = __ldcg(uh + 2 * NROW + rr);
+                // Below left / right: also the row straight below, over which most of them are dropped.
+                uint4 va = make_uint4(0, 0, 0, 0), vb = va;
+                if (nr == 0 || nr == 2) {
+                    int r1;
+                    const int c1 = preceding(ra, rb, 1, r1);
+                    if (c1 != 16) {
+                        const uint4 *vh = reinterpret_cast<const uint4 *>(lab + tile_at(c1, 0) * T3_LAB_WORDS);
+                        va = __ldcg(vh + r1);
+                        vb = __ldcg(vh + NROW + r1);
+                    }
+                }
+                const uint32_t c[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+                const uint32_t u[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
+                const uint32_t v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+                const uint32_t hz = row_joins(c), uhz = row_joins(u);
+                S = rw.x;
+                base = rw.y;
+                uS = uw.x;
+                ubase = uw.y;
+                Links raw, r1, p;
+                if (nr == 1) lk = row_links(1, c, hz, ua, ub, uhz, raw);
+                else if (nr == 3) lk = row_links(3, c, hz, ua, ub, uhz, raw);
+                else if (nr == 0) {   // the triangle rule of the tile kernel over own - below - below left
+                    lk = row_links(0, c, hz, ua, ub, uhz, raw);
+                    row_links(1, c, hz, va, vb, 0u, r1);
+                    row_links(3, v, 0u, ua, ub, 0u, p);
+                    lk.n &= ~(r1.n & p.n);
+                    lk.w &= ~((r1.n & p.w) | (r1.w & (p.n << 1)));
+                    lk.e &= ~((r1.n & p.e) | (r1.e & (p.n >> 1)));
+                } else {              // over own - below - below right
+                    lk = row_links(2, c, hz, ua, ub, uhz, raw);
+                    row_links(1, c, hz, va, vb, 0u, r1);
+                    row_links(3, u, 0u, va, vb, 0u, p);
+                    lk.n &= ~(r1.n & p.n);
+                    lk.w &= ~((r1.n & (p.e << 1)) | (r1.w & (p.n << 1)));
+                    lk.e &= ~((r1.n & (p.w >> 1)) | (r1.e & (p.n >> 1)));
                 }
             }
         }
@@ -702,48 +732,38 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
             return __ldcg(reinterpret_cast<const uint8_t *>(w.perim + tt * T3_EDGE + kZFace) + row);
         };
         uint32_t zm = 0;
-        if (inside) {
+        if (b0 < g.n0 && b1 < g.n1) {
             const uint32_t f = zface(t, tid);
             const uint32_t lo = g.tx2 > 0 ? f & 15u : 0u, hi = g.tx2 + 1 < im.t2 ? f >> 4 : 0u;
             if (lo && (zface(t - 1, tid) >> 4)) zm |= 16u;
             if (lo | hi) {
 #pragma unroll
-                for (int nr = 0; nr < 4; ++nr) {
+                for (int k = 0; k < 4; ++k) {
                     int rr;
-                    const int code = preceding(nr, rr);
-                    if (code == 16) continue;
-                    const int dx = nr < 3 ? -1 : 0, dy = nr < 3 ? nr - 1 : -1;
+                    const int cd = preceding(b0, b1, k, rr);
+                    if (cd == 16) continue;
+                    const int dx = k < 3 ? -1 : 0, dy = k < 3 ? k - 1 : -1;
                     const uint32_t own = face_sel(dx, dy), opp = face_sel(-dx, -dy);
-                    if ((lo & own) && ((zface(tile_at(code, -1), rr) >> 4) & opp)) zm |= 1u << nr;
-                    if ((hi & own) && (zface(tile_at(code, 1), rr) & opp)) zm |= 32u << nr;
+                    if ((lo & own) && ((zface(tile_at(cd, -1), rr) >> 4) & opp)) zm |= 1u << k;
+                    if ((hi & own) && (zface(tile_at(cd, 1), rr) & opp)) zm |= 32u << k;
                 }
             }
         }
         // Queue entries: run links, own run | other run << 12 | code << 24; links across d2, own node |
         // other node << 11 | code << 24 | (o2 < 0: 1, o2 > 0: 2) << 29.
-        uint32_t n = __popc(zm);
-#pragma unroll
-        for (int nr = 0; nr < 4; ++nr) n += __popc(LN[nr]) + __popc(LW[nr]) + __popc(LE[nr]);
-        uint32_t pos = warp_reserve(&nq, n);
+        uint32_t pos = warp_reserve(&nq, __popc(zm) + __popc(lk.n) + __popc(lk.w) + __popc(lk.e));
         auto push = [&](uint32_t from, uint32_t end) {   // links at queue positions [from, end) go in
-#pragma unroll
-            for (int nr = 0; nr < 4; ++nr) {
-                if (!(LN[nr] | LW[nr] | LE[nr]) || pos >= end) continue;
-                int rr;
-                const int code = preceding(nr, rr);
-                const uint4 uw = __ldcg(reinterpret_cast<const uint4 *>(lab + tile_at(code, 0) * T3_LAB_WORDS) + 2 * NROW + rr);
-                while (pos < end) {
-                    const uint32_t f = __ffs(LN[nr] | LW[nr] | LE[nr]);
-                    if (!f) break;
-                    const uint32_t b = f - 1, bit = 1u << b, upto = (bit << 1) - 1u;
-                    const bool isN = LN[nr] & bit, isW = !isN && (LW[nr] & bit), isE = !isN && !isW;
-                    LN[nr] &= isN ? ~bit : ~0u;
-                    LW[nr] &= isW ? ~bit : ~0u;
-                    LE[nr] &= isE ? ~bit : ~0u;
-                    const uint32_t own = base + __popc(S & upto) - 1u;
-                    const uint32_t up = uw.y + __popc(uw.x & (isN ? upto : isW ? bit - 1u : (bit << 2) - 1u)) - 1u;
-                    LQ[pos++ - from] = own | (up << 12) | (uint32_t(code) << 24);
-                }
+            while (pos < end) {
+                const uint32_t f = __ffs(lk.n | lk.w | lk.e);
+                if (!f) break;
+                const uint32_t b = f - 1, bit = 1u << b, upto = (bit << 1) - 1u;
+                const bool isN = lk.n & bit, isW = !isN && (lk.w & bit), isE = !isN && !isW;
+                lk.n &= isN ? ~bit : ~0u;
+                lk.w &= isW ? ~bit : ~0u;
+                lk.e &= isE ? ~bit : ~0u;
+                const uint32_t own = base + __popc(S & upto) - 1u;
+                const uint32_t up = ubase + __popc(uS & (isN ? upto : isW ? bit - 1u : (bit << 2) - 1u)) - 1u;
+                LQ[pos++ - from] = own | (up << 12) | (uint32_t(code) << 24);
             }
             if (zm && pos < end) {
                 auto znodes = [&](int64_t tt, int row) -> uint32_t {
@@ -753,11 +773,11 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
                 while (zm && pos < end) {
                     const int k = __ffs(zm) - 1;
                     zm &= zm - 1;
-                    int rr = tid, code = kOwn;
-                    if (k != 4) code = preceding(k < 4 ? k : k - 5, rr);
-                    const uint32_t zu = znodes(tile_at(code, k < 5 ? -1 : 1), rr);
+                    int rr = tid, cd = kOwn;
+                    if (k != 4) cd = preceding(b0, b1, k < 4 ? k : k - 5, rr);
+                    const uint32_t zu = znodes(tile_at(cd, k < 5 ? -1 : 1), rr);
                     const uint32_t a = k < 5 ? zo & 0xFFFFu : zo >> 16, b = k < 5 ? zu >> 16 : zu & 0xFFFFu;
-                    LQ[pos++ - from] = a | (b << 11) | (uint32_t(code) << 24) | (k < 5 ? 1u << 29 : 2u << 29);
+                    LQ[pos++ - from] = a | (b << 11) | (uint32_t(cd) << 24) | (k < 5 ? 1u << 29 : 2u << 29);
                 }
             }
         };
