@@ -735,7 +735,10 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
         if (b0 < g.n0 && b1 < g.n1) {
             const uint32_t f = zface(t, tid);
             const uint32_t lo = g.tx2 > 0 ? f & 15u : 0u, hi = g.tx2 + 1 < im.t2 ? f >> 4 : 0u;
-            if (lo && (zface(t - 1, tid) >> 4)) zm |= 16u;
+            // The same row beside: a link before (after, one that the tile there makes), over which those
+            // to the preceding rows that its face voxels touch too are dropped.
+            const uint32_t before = lo ? zface(t - 1, tid) >> 4 : 0u, after = hi ? zface(t + 1, tid) & 15u : 0u;
+            if (before) zm |= 16u;
             if (lo | hi) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -744,8 +747,8 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
                     if (cd == 16) continue;
                     const int dx = k < 3 ? -1 : 0, dy = k < 3 ? k - 1 : -1;
                     const uint32_t own = face_sel(dx, dy), opp = face_sel(-dx, -dy);
-                    if ((lo & own) && ((zface(tile_at(cd, -1), rr) >> 4) & opp)) zm |= 1u << k;
-                    if ((hi & own) && (zface(tile_at(cd, 1), rr) & opp)) zm |= 32u << k;
+                    if ((lo & own) && !(before & own) && ((zface(tile_at(cd, -1), rr) >> 4) & opp)) zm |= 1u << k;
+                    if ((hi & own) && !(after & own) && (zface(tile_at(cd, 1), rr) & opp)) zm |= 32u << k;
                 }
             }
         }
