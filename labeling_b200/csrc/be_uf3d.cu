@@ -269,6 +269,74 @@ __device__ __forceinline__ uint32_t row_joins(const uint32_t (&c)[8])
     return face_word<0, 0, 1>(c) & (face_word<0, 0, -1>(c) >> 1);
 }
 
+// Class words of the CTA's block rows of a tile whose rows are whole and 16-byte aligned (p: its first
+// voxel; rs0, rs1: strides of d0 and d1; nx, ny: voxels inside the volume).  A warp instruction reads
+// whole 64-byte rows, four lanes a row -- with each thread reading its own four rows every load touched
+// 32 cache lines, and those lookups took 60% of the load / store unit's time.  Lane 4 Y' + j of a warp loads
+// chunk j of row Y of every plane X; two exchanges inside the four lanes leave lane j the words of planes
+// 4 j .. 4 j + 3, and one with the lanes of row Y ^ 1 leaves it the two planes of block row (load_b0(tid),
+// load_b1(tid)) in both rows.
+__device__ __forceinline__ int load_b0(int tid) { return 2 * (tid & 3) + ((tid >> 2) & 1); }
+__device__ __forceinline__ int load_b1(int tid) { return tid >> 3; }
+static_assert(TB0 == 8 && TY * 4 == NT1, "the load's lanes");
+__device__ __forceinline__ void load_rows(const uint8_t *p, int64_t rs0, int64_t rs1, int nx, int ny, uint32_t K, bool hi,
+                                          uint32_t (&c)[8])
+{
+    const int Y = int(threadIdx.x) >> 2, j = int(threadIdx.x) & 3, s = Y & 1;
+    const uint4 *q = reinterpret_cast<const uint4 *>(p + Y * rs1) + j;
+    const int64_t step = rs0 / 16;
+    uint32_t r[8];   // bytes: even and odd bits of plane k, of plane k + 8
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = 8 * h + k < nx && Y < ny ? __ldg(q + (8 * h + k) * step) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            uint32_t ev, od;
+            split16(v[k], K, hi, ev, od);
+            if (8 * h + k >= nx || Y >= ny) ev = od = 0;
+            const uint32_t x = ev | (od << 8);
+            r[k] = h ? r[k] | (x << 16) : x;
+        }
+    }
+    // Lanes 0, 1 of the four keep planes 0..7, lanes 2, 3 planes 8..15.
+    uint32_t own[4], oth[4];   // planes 2 m, 2 m + 1 of the kept eight: chunk j, chunk j ^ 2
+    const bool up = j & 2;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        own[m] = __byte_perm(r[2 * m], r[2 * m + 1], up ? 0x7632 : 0x5410);
+        oth[m] = __shfl_xor_sync(0xFFFFFFFFu, __byte_perm(r[2 * m], r[2 * m + 1], up ? 0x5410 : 0x7632), 2);
+    }
+    // Then lanes 0, 2 the first four of their eight planes, lanes 1, 3 the others.
+    const bool hi2 = j & 1;
+    uint32_t W[4][2];   // planes 4 j + 0..3: even, odd words
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const uint32_t a = hi2 ? own[m + 2] : own[m], b = hi2 ? oth[m + 2] : oth[m];                 // chunks j, j ^ 2
+        const uint32_t x = __shfl_xor_sync(0xFFFFFFFFu, hi2 ? own[m] : own[m + 2], 1);               // chunk j ^ 1
+        const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, hi2 ? oth[m] : oth[m + 2], 1);               // chunk j ^ 3
+        const uint32_t a0 = hi2 ? x : a, a1 = hi2 ? a : x, b0 = hi2 ? y : b, b1 = hi2 ? b : y;
+        const uint32_t k0 = up ? b0 : a0, k1 = up ? b1 : a1, k2 = up ? a0 : b0, k3 = up ? a1 : b1;   // chunks 0..3
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t lo = __byte_perm(k0, k1, h ? 0x7362 : 0x5140), hi4 = __byte_perm(k2, k3, h ? 0x7362 : 0x5140);
+            W[2 * m + h][0] = __byte_perm(lo, hi4, 0x5410);
+            W[2 * m + h][1] = __byte_perm(lo, hi4, 0x7632);
+        }
+    }
+    // Planes 2 s, 2 s + 1 of the four stay, the others go to the lane of the row beside.
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t keep = s ? W[2 + i][k] : W[i][k];
+            const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, s ? W[i][k] : W[2 + i][k], 4);
+            c[4 * i + k] = s ? got : keep;        // row 2 b1
+            c[4 * i + 2 + k] = s ? keep : got;    // row 2 b1 + 1
+        }
+}
+
 // row_bits out of line: inlined into the four unrolled rows it slowed the aligned path by 1%.
 __device__ __noinline__ uint2 row_bits_call(const uint8_t *p, int n, const uint8_t *lo, const uint8_t *hi,
                                             uint32_t K, bool thr_hi, int thr)
@@ -317,33 +385,25 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
         uint32_t c[8];
 #pragma unroll
         for (int v = 0; v < 8; ++v) c[v] = 0;
-        if (b0 < g.n0 && b1 < g.n1) {
+        if (g.nz == TZ && ((reinterpret_cast<uintptr_t>(im.in) | uintptr_t(im.d2)) & 15) == 0) {
+            // The lanes that loaded a row are not those that go on with it: through shared memory.
+            load_rows(im.in + g.x0 * rs0 + int64_t(g.y0) * im.d2 + g.z0, rs0, im.d2, g.nx, g.ny, K, hi, c);
+            const int row = load_b0(tid) * TB1 + load_b1(tid);
+            CA[row] = make_uint4(c[0], c[1], c[2], c[3]);
+            CB[row] = make_uint4(c[4], c[5], c[6], c[7]);
+            __syncthreads();
+            const uint4 ca = CA[tid], cb = CB[tid];
+            c[0] = ca.x; c[1] = ca.y; c[2] = ca.z; c[3] = ca.w;
+            c[4] = cb.x; c[5] = cb.y; c[6] = cb.z; c[7] = cb.w;
+        } else if (b0 < g.n0 && b1 < g.n1) {
 #pragma unroll
             for (int ij = 0; ij < 4; ++ij) {
-                const int i = ij >> 1, j = ij & 1;
-                const int X = 2 * b0 + i, Y = 2 * b1 + j;
+                const int X = 2 * b0 + (ij >> 1), Y = 2 * b1 + (ij & 1);
                 if (X >= g.nx || Y >= g.ny) continue;
                 const uint8_t *row = im.in + (g.x0 + X) * rs0 + int64_t(g.y0 + Y) * im.d2 + g.z0;
-                uint32_t ev = 0, od = 0;
-                if (g.nz == TZ && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
-                    const uint4 *pv = reinterpret_cast<const uint4 *>(row);
-                    uint4 q[4];
-#pragma unroll
-                    for (int h = 0; h < 4; ++h) q[h] = __ldg(pv + h);
-#pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        uint32_t e8, o8;
-                        split16(q[h], K, hi, e8, o8);
-                        ev |= e8 << (8 * h);
-                        od |= o8 << (8 * h);
-                    }
-                } else {
-                    const uint2 eo = row_bits_call(row, g.nz, im.in, im.in + im.d0 * rs0, K, hi, im.thr);
-                    ev = eo.x;
-                    od = eo.y;
-                }
-                c[4 * i + 2 * j] = ev;
-                c[4 * i + 2 * j + 1] = od;
+                const uint2 eo = row_bits_call(row, g.nz, im.in, im.in + im.d0 * rs0, K, hi, im.thr);
+                c[2 * ij] = eo.x;
+                c[2 * ij + 1] = eo.y;
             }
         }
         const uint32_t Fw = c[0] | c[1] | c[2] | c[3] | c[4] | c[5] | c[6] | c[7];
