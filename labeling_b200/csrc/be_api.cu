@@ -340,14 +340,16 @@ int be_label2d(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int
         cudaMemsetAsync(ws.w.err, 0, 16 * sizeof(uint32_t), s);
 #endif
         const bool timed = c->timing && !form;
-        e = uf2d_launch(shape, L, ws.w, c->sms, false, s, timed ? c->stage_ev : nullptr);
+        Work w = ws.w;
+        w.host_count = n_components ? c->h_ncomp : nullptr;   // the count straight to the host, no copy after
+        e = uf2d_launch(shape, L, w, c->sms, false, s, timed ? c->stage_ev : nullptr);
         c->timed_stages = timed ? kStages2D : 0;
         if (e != cudaSuccess) return cuda_error(c, e, "be_label2d launch");
     }
     if (rc) return rc;
     if (n_components) {
-        const int64_t *src = count_of(c, algo, 2);
-        e = cudaMemcpyAsync(c->h_ncomp, src, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+        if (algo == BE_ALGO_ITER)
+            e = cudaMemcpyAsync(c->h_ncomp, count_of(c, algo, 2), sizeof(int64_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_error(c, e, "be_label2d sync");
         if (algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
@@ -394,14 +396,16 @@ int be_label3d(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2,
         cudaMemsetAsync(ws.w.err, 0, 16 * sizeof(uint32_t), s);
 #endif
         const bool timed = c->timing && !form;
-        e = launch_uf3d(L, ws.w, c->sms, false, s, timed ? c->stage_ev : nullptr);
+        Work w = ws.w;
+        w.host_count = n_components ? c->h_ncomp : nullptr;   // as in 2D
+        e = launch_uf3d(L, w, c->sms, false, s, timed ? c->stage_ev : nullptr);
         c->timed_stages = timed ? kStages3D : 0;
         if (e != cudaSuccess) return cuda_error(c, e, "be_label3d launch");
     }
     if (rc) return rc;
     if (n_components) {
-        const int64_t *src = count_of(c, algo, 3);
-        e = cudaMemcpyAsync(c->h_ncomp, src, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+        if (algo == BE_ALGO_ITER)
+            e = cudaMemcpyAsync(c->h_ncomp, count_of(c, algo, 3), sizeof(int64_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_error(c, e, "be_label3d sync");
         if (algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)

@@ -78,6 +78,7 @@ struct Work {
     uint32_t *chunksum;   // per scan chunk: sum of segcnt
     uint32_t *queue;      // work-queue counters (persistent mode); zeroed before a launch
     int64_t *ncomp;       // per image: number of components
+    int64_t *host_count;  // the first image's count once more, in pinned host memory (or null)
     uint32_t *err;        // error flags (bounded waits / iteration caps)
     uint32_t *epoch;      // [0] launch epoch (+1 per pipeline run), [1] scan ticket counter
     uint64_t *scan_status;  // per scan chunk: (epoch << 34 | state << 32) | prefix value

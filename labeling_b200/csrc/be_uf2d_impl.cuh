@@ -746,7 +746,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_flatten_2d(Work w)
 constexpr int K3_NT = 256;
 constexpr int K3_PER_SM = 8;              // resident CTAs per SM
 
-template <bool Q>
+// ONE (a plain launch of one tile): the tile kernel's launch goes straight before this one -- there is
+// nothing to merge and no prefix beyond the tile's own rows, which the CTA sums itself -- so that the
+// smallest images take two launches: 16^2 17.4 -> 13.1 us, 64^2 18.5 -> 16.1 us.  (Doing without the scan
+// launch for images of several tiles, every CTA scanning the counts, was slower: 2048^2 43.0 -> 44.7 us.)
+template <bool Q, bool ONE>
 __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L, Work w)
 {
     __shared__ __align__(16) uint4 H[kHdr / 4];   // class words, then run words
@@ -787,6 +791,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
     };
     ItemLoop<Q> loop{w.queue + 4};
     int64_t t = loop.first(&qslot);
+    if (ONE) grid_dep_wait();   // the tile kernel is this grid's predecessor
     if (t < w.n_tiles) fetch(t);
     while (t < w.n_tiles) {
         loop.request();
@@ -802,12 +807,38 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         int64_t tn = Q ? w.n_tiles : t + gridDim.x;
         if (tn < w.n_tiles) fetch_words(tn);
         cp_async_wait();
-        grid_dep_wait();   // segment prefixes from here on (returns at once after the first tile)
-        const uint32_t base0 = w.segpref[im.seg_base];
-        if (tid < TH && tid < nrp)
-            segb[tid] = w.segpref[im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx] - base0;
-        if (lt == 0 && tid == 0)
-            w.ncomp[im.index] = int64_t(w.segpref[im.seg_base + int64_t(im.rows) * im.tiles_x] - base0);
+        auto put_count = [&](int64_t n) {
+            w.ncomp[im.index] = n;
+            if (w.host_count) *w.host_count = n;
+        };
+        uint32_t base0 = 0;
+        if (ONE) {
+            constexpr int PER = TH / 32;
+            if (tid < 32) {
+                uint32_t c[PER], sum = 0;
+#pragma unroll
+                for (int i = 0; i < PER; ++i) sum += c[i] = PER * tid + i < nrp ? w.segcnt[PER * tid + i] : 0u;
+                uint32_t x = sum;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                    if (tid >= o) x += v;
+                }
+                if (tid == 31) put_count(int64_t(x));
+                x -= sum;
+#pragma unroll
+                for (int i = 0; i < PER; ++i) {
+                    segb[PER * tid + i] = x;
+                    x += c[i];
+                }
+            }
+        } else {
+            grid_dep_wait();   // segment prefixes from here on (returns at once after the first tile)
+            base0 = w.segpref[im.seg_base];
+            if (tid < TH && tid < nrp)
+                segb[tid] = w.segpref[im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx] - base0;
+            if (lt == 0 && tid == 0) put_count(int64_t(w.segpref[im.seg_base + int64_t(im.rows) * im.tiles_x] - base0));
+        }
         __syncthreads();
         const uint4 *HR = H + kHdr / 4 - NWORD;   // run words
         // The last B run is the last run.
@@ -837,7 +868,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         }
         // Border components linked under another tile's component: the label of that root, its
         // segment's prefix plus its rank among the first pixels left in its row of its tile.
-        for (uint32_t j = tid; j < nb; j += K3_NT) {
+        for (uint32_t j = tid; !ONE && j < nb; j += K3_NT) {
             const int64_t node = t * MAXB + j;
             const unsigned long long e = __ldcg(w.gp + node);   // its root's own entry (flatten_tile_nodes)
             const uint32_t g = uint32_t(e), kg = uint32_t(e >> 32);
@@ -965,13 +996,14 @@ inline cudaError_t launch(const ImgList2D &L, const Work &w, int sms, bool persi
     mark(0);
     keep(launch_k(persistent ? k_tile_local_2d<true> : k_tile_local_2d<false>, grid(w.n_tiles, K1_PER_SM), K1_NT, s, false, L, w));
     mark(1);
-    keep(launch_k(persistent ? k_merge_2d<true> : k_merge_2d<false>, grid(w.n_tiles, K2_PER_SM), K2_NT, s, ov, L, w));
+    const bool one = !persistent && w.n_tiles == 1;
+    if (!one) keep(launch_k(persistent ? k_merge_2d<true> : k_merge_2d<false>, grid(w.n_tiles, K2_PER_SM), K2_NT, s, ov, L, w));
     mark(2);
-    keep(launch_k(k_scan_flatten_2d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, w));
+    if (!one) keep(launch_k(k_scan_flatten_2d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, w));
     mark(3);
     // The label writes run a fixed tile order over K3_PER_SM CTAs per SM (they prefetch their next tile).
-    keep(launch_k(persistent ? k_tile_write_2d<true> : k_tile_write_2d<false>, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * K3_PER_SM))),
-                  K3_NT, s, ov, L, w));
+    keep(launch_k(persistent ? k_tile_write_2d<true, false> : one ? k_tile_write_2d<false, true> : k_tile_write_2d<false, false>,
+                  unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * K3_PER_SM))), K3_NT, s, ov, L, w));
     mark(4);
     return e;
 }

@@ -991,8 +991,11 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
         const uint32_t nb = snb, base0 = segb[TX * TY];
         const uint4 *HR = H + 2 * NROW;
         const uint32_t nrun = HR[NROW - 1].y + __popc(HR[NROW - 1].x);
-        if (t == im.tile_base && tid == 0)
-            w.ncomp[im.index] = int64_t(w.segpref[im.seg_base + int64_t(im.d0) * im.d1 * im.t2] - base0);
+        if (t == im.tile_base && tid == 0) {
+            const int64_t n = int64_t(w.segpref[im.seg_base + int64_t(im.d0) * im.d1 * im.t2] - base0);
+            w.ncomp[im.index] = n;
+            if (w.host_count) *w.host_count = n;
+        }
         // Surviving roots, by block row and voxel row: rank = roots before it in its segment.
 #pragma unroll
         for (int i = 0; i < 4 * NROW / NT; ++i) {
