@@ -134,33 +134,6 @@ __device__ __forceinline__ uint32_t sfind(uint32_t *P, uint32_t a)
     return a;
 }
 
-// Find without writes, for the flatten pass after all merges: no link can happen any more, so the
-// entry reached is the true root.  (Path halving is not allowed there: a halving store that lands
-// after the entry's owner wrote its root would point the entry back at an inner node.)
-__device__ __forceinline__ uint32_t sfind_ro(const uint32_t *P, uint32_t a)
-{
-    uint32_t p = P[a];
-    while (p != a) {
-        a = p;
-        p = P[a];
-    }
-    return a;
-}
-
-// Root of `a` after all merges, pointing every entry on the path straight at it.  Safe while
-// other threads do the same: all of them store the same final root into shared entries.
-__device__ __forceinline__ uint32_t sflatten(uint32_t *P, uint32_t a)
-{
-    const uint32_t r = sfind_ro(P, a);
-    uint32_t x = a;
-    while (x != r) {
-        const uint32_t nx = P[x];
-        P[x] = r;
-        x = nx;
-    }
-    return r;
-}
-
 // Merge of two shared-memory union-find trees that keeps the smaller index as the root
 // (the atomicMin formulation of Playne & Hawick's union-find, safe under concurrent merges).
 __device__ __forceinline__ void smerge(uint32_t *P, uint32_t a, uint32_t b)
@@ -294,6 +267,16 @@ __device__ __forceinline__ void gunion_keyed(unsigned long long *gp, uint32_t a,
     }
 }
 
+// Points node x at its parent's parent (one jump; a root and a root's child stay).
+__device__ __forceinline__ void gjump(unsigned long long *gp, uint32_t x)
+{
+    volatile unsigned long long *vp = gp;
+    const uint32_t p = uint32_t(vp[x]);
+    if (p == x) return;
+    const unsigned long long ep = vp[p];
+    if (uint32_t(ep) != p) vp[x] = ep;
+}
+
 // Root of node x after all merges of the launch are complete, by pointer jumping that writes only
 // x's own entry: each step x is pointed at its parent's parent as that entry reads now.  When every
 // node of a deep tree runs this at once, each read lands on an entry that its own thread has
@@ -313,39 +296,6 @@ __device__ __forceinline__ uint32_t gfind_jump(unsigned long long *gp, uint32_t 
         p = g;
     }
     return p;
-}
-
-// ---- Border-merge filter ---------------------------------------------------------------------
-// The cross-tile merge kernels see the same pair of border components over and over (every face
-// position of a large component yields one).  Before a pair costs a global union (dependent loads
-// through L2), it is merged in a small shared-memory union-find over the tile's nodes and the
-// staged neighbour positions: only a pair that joins two different local sets goes on to the
-// global union-find; a pair already connected by earlier local merges is implied by the global
-// unions those merges queued.
-// Local merge of the sets of slots a and b (smaller slot wins, as smerge); false only when the
-// two were already one set and this call changed no parent.  An atomicMin that lands on an entry
-// another thread has just linked still rewrites that entry's parent (it moves the entry's subtree
-// under `a`), so a call that changed anything reports true: every local link then has a pair
-// that goes on to the global union-find, and local connectivity never runs ahead of the global.
-__device__ __forceinline__ bool smerge_joined(uint32_t *P, uint32_t a, uint32_t b)
-{
-    bool changed = false;
-    for (;;) {
-        a = sfind(P, a);
-        b = sfind(P, b);
-        if (a == b) return changed;
-        if (a < b) {
-            const uint32_t old = atomicMin(&P[b], a);
-            if (old == b) return true;
-            changed |= old > a;
-            b = old;
-        } else {
-            const uint32_t old = atomicMin(&P[a], b);
-            if (old == a) return true;
-            changed |= old > b;
-            a = old;
-        }
-    }
 }
 
 // Decrement a uint8 counter packed in a 32-bit word (the counter is >= 1 when this is called).

@@ -39,9 +39,6 @@ __device__ __forceinline__ bool perim_pos(int p, int nbr, int nbc, int &r, int &
     return r < nbr;
 }
 
-// Highest set bit of x (x != 0).
-__device__ __forceinline__ uint32_t hibit(uint32_t x) { return 31u - __clz(x); }
-
 // Global keys.  A component is known by (segment, place of its root run among the segment's runs):
 // segments -- the part of one pixel row that lies in one tile -- are numbered in raster order, and a
 // tile numbers the runs of a segment by their first pixel, so key = segment * seg_width + place orders
@@ -542,30 +539,27 @@ constexpr int K2_NP = TBH + TBW;               // border positions a merge CTA l
 constexpr int K2_NT = 64;                      // threads of a merge CTA (small: many tiles per SM)
 constexpr int K2_PER_SM = 28;                  // resident merge CTAs per SM
 constexpr int kGQ2 = 256;                      // queued global unions per tile (more are done at once)
-constexpr int SR = MAXB;                       // local index of the staged right column
-constexpr int SD = MAXB + TBH;                 // local index of the staged bottom row (column -1 first)
-constexpr int NLOC2 = MAXB + TBH + TBW + 2;    // local union-find size
+constexpr int kSeen2 = 256;                    // table of pairs seen
 
 // Positions p < TBH are the right border's rows, the others the bottom border's columns
 // (p - TBH).  The border entries across the right border (the next tile's left column) and the
 // bottom border (the top row of the tile below, widened by one block into the two diagonal tiles)
-// are staged in shared memory with the global node id they belong to.  A CTA-local union-find over
-// this tile's nodes and the staged positions (neighbouring staged positions of one node merged
-// first) filters the pairs: only a pair that joins two local sets goes on to the global
-// union-find, from a shared queue once all of the tile's pairs are seen.  The merge is bound by
-// the latency of those global unions (dependent L2 round trips), so a CTA is two warps that loop
-// over the positions: many tiles are in flight on each SM at once.
+// are staged in shared memory.  Most links join the same few pairs of border components; a table
+// of the pairs seen lets one link of each through, to a shared queue that both warps empty by global
+// unions once all of the tile's links are seen.  The merge is bound by the latency of those unions
+// (dependent L2 round trips), so a CTA is two warps that loop over the positions: many tiles are in
+// flight on each SM at once.  Measured (this launch, us; a CTA-local union-find before the queue ->
+// the table; 8192^2 noise of density 0.6: 29.0 -> 24.4, 0.1: 19.4 -> 14.6; 2048^2 disks 19.0 -> 16.4),
+// and with the jumps after the unions 25.7, 15.7 and 16.6 -- for an 8192^2 spiral 101 -> 54, for a
+// 2048^2 one 31 -> 22.
 template <bool Q>
 __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work w)
 {
     grid_dep_wait();
     grid_dep_release();
     __shared__ uint32_t qslot;
-    __shared__ uint32_t lp[NLOC2];
-    __shared__ uint32_t sid[TBH + TBW + 2];   // staged global node ids (kNone = none)
-    __shared__ uint8_t smk[TBH + TBW + 2];    // staged masks
-    __shared__ uint16_t own[K2_NP];           // this tile's own border entries
-    __shared__ uint8_t cm[K2_NP];             // connected staged neighbours of each position
+    __shared__ uint16_t st[TBH + TBW + 2];    // staged border entries (0 = background)
+    __shared__ uint32_t seen[kSeen2];
     __shared__ uint2 gq[kGQ2];
     __shared__ uint32_t nq;
     ItemLoop<Q> loop{w.queue + 1};
@@ -577,141 +571,86 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
         const int nbr = cells(min(TH, im.rows - ty * TH));
         const int nbc = cells(min(TW, im.cols - tx * TW));
         const uint16_t *pe = w.perim;
-        for (int i = threadIdx.x; i < NLOC2; i += K2_NT) lp[i] = uint32_t(i);
+        for (int i = threadIdx.x; i < kSeen2; i += K2_NT) seen[i] = kNone;
         if (threadIdx.x == 0) nq = 0;
         // Stage: position p < TBH stages right-column row p; the others bottom-row column p - TBH,
         // and the first two of those also columns -1 and TBW.  Each position's own entry is loaded
         // with the staging loads.
-        auto stage = [&](int k, int64_t t2, int pos) {
-            const uint32_t B = pe[t2 * NPERIM + pos];
-            sid[k] = B ? uint32_t(t2 * MAXB + (B >> 4)) : kNone;
-            smk[k] = uint8_t(B & 15u);
-        };
-        for (int p = threadIdx.x; p < K2_NP; p += K2_NT) {
-            uint16_t A = 0;
+        constexpr int NI = (K2_NP + K2_NT - 1) / K2_NT;
+        uint32_t own[NI];
+        const bool right = tx + 1 < im.tiles_x, below = ty + 1 < im.tiles_y;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int p = threadIdx.x + i * K2_NT;
+            own[i] = 0;
             if (p < TBH) {
-                if (p < nbr && tx + 1 < im.tiles_x) {
-                    A = pe[t * NPERIM + 2 * TBW + TBH + p];
-                    stage(p, t + 1, 2 * TBW + p);
-                } else {
-                    sid[p] = kNone;
-                    smk[p] = 0;
+                uint16_t B = 0;
+                if (p < nbr && right) {
+                    own[i] = pe[t * NPERIM + 2 * TBW + TBH + p];
+                    B = pe[(t + 1) * NPERIM + 2 * TBW + p];
                 }
-            } else {
+                st[p] = B;
+            } else if (p < K2_NP) {
                 const int c = p - TBH;
-                const int k = TBH + 1 + c;
-                if (c < nbc && ty + 1 < im.tiles_y) {
-                    A = pe[t * NPERIM + TBW + c];
-                    stage(k, t + im.tiles_x, c);
-                } else {
-                    sid[k] = kNone;
-                    smk[k] = 0;
+                uint16_t B = 0;
+                if (c < nbc && below) {
+                    own[i] = pe[t * NPERIM + TBW + c];
+                    B = pe[(t + im.tiles_x) * NPERIM + c];
                 }
-                if (c == 0) {
-                    if (tx > 0 && ty + 1 < im.tiles_y) stage(TBH, t + im.tiles_x - 1, TBW - 1);
-                    else { sid[TBH] = kNone; smk[TBH] = 0; }
-                }
-                if (c == 1) {
-                    // column TBW: block 0 of the tile below-right (a tile with a right neighbour is
-                    // full-width; a narrower tile's column nbc is staged empty by its own position)
-                    if (nbc == TBW && tx + 1 < im.tiles_x && ty + 1 < im.tiles_y)
-                        stage(TBH + TBW + 1, t + im.tiles_x + 1, 0);
-                    else { sid[TBH + TBW + 1] = kNone; smk[TBH + TBW + 1] = 0; }
-                }
+                st[p + 1] = B;
+                if (c == 0) st[TBH] = tx > 0 && below ? pe[(t + im.tiles_x - 1) * NPERIM + TBW - 1] : uint16_t(0);
+                // column TBW: block 0 of the tile below-right (a tile with a right neighbour is
+                // full-width; a narrower tile's column nbc is staged empty by its own position)
+                if (c == 1) st[TBH + TBW + 1] = nbc == TBW && right && below ? pe[(t + im.tiles_x + 1) * NPERIM] : uint16_t(0);
             }
-            own[p] = A;
         }
         __syncthreads();
-        // Neighbouring staged positions of one node are one element: every position of a run of
-        // equal node ids along the staged column (warp 0) or row (warp 1) points at the run's first
-        // position, found by ballots 32 positions at a time (no merging, no chains).
-        {
-            const int lane = threadIdx.x & 31;
-            const int lo = threadIdx.x < 32 ? 0 : TBH, n = threadIdx.x < 32 ? TBH : TBW + 2;
-            uint32_t carry = 0;
-            for (int c0 = 0; c0 < n; c0 += 32) {
-                const int k = c0 + lane;
-                const bool valid = k < n;
-                const bool start = valid && (k == 0 || sid[lo + k] != sid[lo + k - 1]);
-                const uint32_t below = __ballot_sync(0xFFFFFFFFu, start) & (0xFFFFFFFFu >> (31 - lane));
-                const uint32_t st = below ? uint32_t(c0) + hibit(below) : carry;
-                if (valid) lp[MAXB + lo + k] = uint32_t(MAXB + lo) + st;
-                carry = __shfl_sync(0xFFFFFFFFu, st, 31);
-            }
-        }
-        // Connected neighbours of every position: bit d + 1 for the staged neighbour at offset d.
-        for (int p = threadIdx.x; p < K2_NP; p += K2_NT) {
-            const uint32_t A = own[p];
-            uint32_t cb = 0;
-            if (A) {
-                const uint32_t mA = A & 15u;
-                if (p < TBH) {
-                    // Right border: neighbours in the tile to the right, same tile row.
+        // Links of every position to the staged positions at offsets -1, 0, 1.  Neighbouring staged
+        // positions of one node need one link; a pair of nodes in the table has its union queued.
 #pragma unroll
-                    for (int d = -1; d <= 1; ++d) {
-                        const int rr = p + d;
-                        if (CELL == 1 && d) continue;   // pixels: straight across only
-                        if (rr < 0 || rr >= nbr || sid[rr] == kNone) continue;
-                        const uint32_t mB = smk[rr];
-                        if (CELL == 1 || (d == 0 ? ((mA & 0xAu) && (mB & 0x5u)) : d < 0 ? ((mA & 2u) && (mB & 4u)) : ((mA & 8u) && (mB & 1u))))
-                            cb |= 1u << (d + 1);
-                    }
-                } else {
-                    // Bottom border: neighbours in the tile row below (including the diagonal tiles).
-                    const int c = p - TBH;
+        for (int i = 0; i < NI; ++i) {
+            const int p = threadIdx.x + i * K2_NT;
+            const uint32_t A = own[i];
+            if (!A) continue;
+            const uint32_t ja = A >> 4;
+            const bool col = p < TBH;            // right border: the same rows of the tile to the right
+            const int k0 = col ? p : p + 1;      // staged position straight across
+            uint32_t last = kNone;
 #pragma unroll
-                    for (int d = -1; d <= 1; ++d) {
-                        const int k = c + d + 1;   // staged bottom index
-                        if (CELL == 1 && d) continue;
-                        if (sid[TBH + k] == kNone) continue;
-                        const uint32_t mB = smk[TBH + k];
-                        if (CELL == 1 || (d == 0 ? ((mA & 0xCu) && (mB & 0x3u)) : d < 0 ? ((mA & 4u) && (mB & 2u)) : ((mA & 8u) && (mB & 1u))))
-                            cb |= 1u << (d + 1);
-                    }
+            for (int dd = 0; dd < (CELL == 1 ? 1 : 3); ++dd) {
+                const int d = dd == 0 ? 0 : dd == 1 ? -1 : 1, k = k0 + d;
+                if (d < 0 && col && p == 0) continue;
+                if (d > 0 && col && p == TBH - 1) continue;
+                const uint32_t B = st[k];
+                if constexpr (CELL == 2) {
+                    const uint32_t a = col ? (d == 0 ? 0xAu : d < 0 ? 2u : 8u) : (d == 0 ? 0xCu : d < 0 ? 4u : 8u);
+                    const uint32_t b = col ? (d == 0 ? 0x5u : d < 0 ? 4u : 1u) : (d == 0 ? 0x3u : d < 0 ? 2u : 1u);
+                    if (!(A & a) || !(B & b)) continue;
+                } else if (!B) {
+                    continue;
                 }
-            }
-            cm[p] = uint8_t(cb);
-        }
-        __syncthreads();
-        // Pairs.  Staged index of a position's neighbour at offset d: p + d on the right border,
-        // TBH + c + d + 1 on the bottom border.  A pair is skipped when the position before (same
-        // border, same own node) touches the same staged run: that position's pair stands for it.
-        // A pair that passes goes through the CTA-local union-find, and only one that joins two
-        // local sets goes on to the global union-find.
-        auto pair = [&](uint32_t ja, uint32_t nA, uint32_t le, uint32_t nB) {
-            if (!smerge_joined(lp, ja, le)) return;
-            const uint32_t slot = atomicAdd(&nq, 1u);
-            if (slot < uint32_t(kGQ2)) gq[slot] = make_uint2(nA, nB);
-            else gunion2d(im, w, nA, nB);
-        };
-        for (int p = threadIdx.x; p < K2_NP; p += K2_NT) {
-            const uint32_t A = own[p];
-            uint32_t cb = cm[p];
-            if (!A || !cb) continue;
-            const uint32_t ja = A >> 4, nA = uint32_t(t * MAXB + ja);
-            const int i0 = p < TBH ? p : p + 1;   // staged index of the neighbour at offset d: i0 + d
-            // the position before on the same border, when it belongs to the same own node
-            const bool prev = p != 0 && p != TBH && own[p - 1] && (own[p - 1] >> 4) == ja;
-            const uint32_t cbp = prev ? cm[p - 1] : 0u;
-            uint32_t lastB = kNone;   // a node already paired with this one needs no second pair
-            while (cb) {
-                const int d = __ffs(cb) - 2;
-                cb &= cb - 1;
-                const int i = i0 + d;
-                const uint32_t nB = sid[i], rs = lp[MAXB + i];
-                if (nB == lastB) continue;
-                bool seen = false;
-#pragma unroll
-                for (int dp = -1; dp <= 1; ++dp)
-                    if ((cbp >> (dp + 1)) & 1u) seen |= lp[MAXB + i0 - 1 + dp] == rs;
-                if (seen) continue;
-                pair(ja, nA, rs, nB);
-                lastB = nB;
+                // the staged position's tile: to the right, below left, below, below right
+                const uint32_t side = col ? 0u : k == TBH ? 1u : k <= TBH + TBW ? 2u : 3u;
+                const uint32_t key = (side << 24) | ((B >> 4) << 12) | ja;
+                if (key == last) continue;
+                last = key;
+                if (atomicExch(&seen[(key * 0x9E3779B1u) >> 24], key) == key) continue;
+                const uint32_t nA = uint32_t(t * MAXB + ja);
+                const uint32_t nB = uint32_t((col ? t + 1 : t + im.tiles_x + int(side) - 2) * MAXB + (B >> 4));
+                const uint32_t slot = atomicAdd(&nq, 1u);
+                if (slot < uint32_t(kGQ2)) gq[slot] = make_uint2(nA, nB);
+                else gunion2d(im, w, nA, nB);
             }
         }
         __syncthreads();
         const uint32_t nqt = min(nq, uint32_t(kGQ2));
+        const uint32_t nb = w.nb[t];
         for (uint32_t i = threadIdx.x; i < nqt; i += K2_NT) gunion2d(im, w, gq[i].x, gq[i].y);
+        __syncthreads();
+        // Every node of the tile then jumps to its parent's parent, all tiles at once: a component that
+        // winds through many tiles is a path as long as the tiles it crosses, and the union that closes
+        // it climbs what nobody has shortened.
+        for (uint32_t j = threadIdx.x; j < nb; j += K2_NT) gjump(w.gp, uint32_t(t * MAXB + j));
         if (!Q) break;   // one tile per CTA
         loop.publish(&qslot);
         __syncthreads();

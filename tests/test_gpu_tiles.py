@@ -54,3 +54,24 @@ def test_forms_of_one_context_keep_apart(ctx):
             k = be.label2d(ctx, src, out, algo=algo, coh=coh)
             ref, kr = O.ccl2d(img, 0, conn8)
             assert k == kr and np.array_equal(out.cpu().numpy(), ref), (i, h, w, algo, coh)
+
+
+@pytest.mark.parametrize("conn8", [True, False])
+@pytest.mark.parametrize("size", [(257, 1025), (400, 777)])
+def test_links_across_tile_borders(ctx, size, conn8):
+    """One path through every tile many times, and separate components that touch on both diagonals
+    across every tile border."""
+    import torch
+    import labeling_b200 as be
+    h, w = size
+    y, x = np.indices((h, w))
+    snake = (y % 2 == 0) | ((x == 0) & (y % 4 == 1)) | ((x == w - 1) & (y % 4 == 3))
+    weave = np.where(y // 2 % 2 == 0, x % 4 < 2, x % 4 >= 2)
+    for name, mask in (("snake", snake), ("snake back", snake[::-1, ::-1]), ("weave", weave), ("thin weave", weave & (y % 2 == 1))):
+        img = (mask * 255).astype(np.uint8)
+        ref, k = O.ccl2d(img, 0, conn8)
+        src = torch.from_numpy(img).cuda()
+        out = torch.full(size, -1, dtype=torch.int32, device="cuda")
+        algo, coh = (be.ALGO_UF, be.COH_8) if conn8 else (be.ALGO_PIXEL, be.COH_4)
+        assert be.label2d(ctx, src, out, algo=algo, coh=coh) == k, name
+        assert np.array_equal(out.cpu().numpy(), ref), name
