@@ -683,15 +683,19 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_flatten_2d(Work w)
 // Label resolve and write.
 // ---------------------------------------------------------------------------------------------
 constexpr int K3_NT = 256;
+// CTAs per SM up to which CTAs share a tile's rows: with 4, a 2048^2 call (256 tiles) is 0.5 us slower, and
+// none is faster than with 2.
+constexpr int kSplitPerSM2 = 2;
 constexpr int K3_PER_SM = 8;              // resident CTAs per SM
 
 // ONE (a plain launch of one tile): the tile kernel's launch goes straight before this one -- there is
 // nothing to merge and no prefix beyond the tile's own rows, which the CTA sums itself -- so that the
 // smallest images take two launches: 16^2 17.4 -> 13.1 us, 64^2 18.5 -> 16.1 us.  (Doing without the scan
 // launch for images of several tiles, every CTA scanning the counts, was slower: 2048^2 43.0 -> 44.7 us.)
-template <bool Q, bool ONE>
+template <bool Q, WriteForm F>
 __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L, Work w)
 {
+    constexpr bool ONE = F == kWriteOne, SHARED = F != kWriteTiles;
     __shared__ __align__(16) uint4 H[kHdr / 4];   // class words, then run words
     __shared__ uint32_t LT[MAXRUN + 1];   // label of run i at i + 1 (0: the place of "no run yet")
     constexpr int kStageRuns = 2048;      // run entries staged in shared memory (later ones: from L2)
@@ -730,6 +734,12 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
     };
     ItemLoop<Q> loop{w.queue + 4};
     int64_t t = loop.first(&qslot);
+    int part = 0, split = 1;   // of the tile's rows
+    if (SHARED) {
+        split = int(gridDim.x / uint32_t(w.n_tiles));
+        part = int(blockIdx.x % uint32_t(split));
+        t = blockIdx.x / uint32_t(split);
+    }
     if (ONE) grid_dep_wait();   // the tile kernel is this grid's predecessor
     if (t < w.n_tiles) fetch(t);
     while (t < w.n_tiles) {
@@ -743,7 +753,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         const uint32_t nb = nNb;
         // The next tile's data come while this one's labels are worked out and written, each part as soon
         // as its place is free -- and the tile is known, which with a work queue is before the writes.
-        int64_t tn = Q ? w.n_tiles : t + gridDim.x;
+        int64_t tn = Q || SHARED ? w.n_tiles : t + gridDim.x;
         if (tn < w.n_tiles) fetch_words(tn);
         cp_async_wait();
         auto put_count = [&](int64_t n) {
@@ -763,7 +773,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
                     const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, x, o);
                     if (tid >= o) x += v;
                 }
-                if (tid == 31) put_count(int64_t(x));
+                if (tid == 31 && part == 0) put_count(int64_t(x));
                 x -= sum;
 #pragma unroll
                 for (int i = 0; i < PER; ++i) {
@@ -776,7 +786,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             base0 = w.segpref[im.seg_base];
             if (tid < TH && tid < nrp)
                 segb[tid] = w.segpref[im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx] - base0;
-            if (lt == 0 && tid == 0) put_count(int64_t(w.segpref[im.seg_base + int64_t(im.rows) * im.tiles_x] - base0));
+            if (lt == 0 && tid == 0 && part == 0) put_count(int64_t(w.segpref[im.seg_base + int64_t(im.rows) * im.tiles_x] - base0));
         }
         __syncthreads();
         const uint4 *HR = H + kHdr / 4 - NWORD;   // run words
@@ -868,11 +878,12 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             b.x = (c.z & bit0) ? l0 : 0; b.y = (c.w & bit0) ? l0 : 0;
             b.z = (c.z & bit1) ? l1 : 0; b.w = (c.w & bit1) ? l1 : 0;
         };
-        int32_t *dst = im.out + int64_t(y0 + CELL * (tid / UPR)) * im.out_pitch + x0 + 4 * q;
-        const int64_t turn = CELL * UR * im.out_pitch;
+        const int br0 = tid / UPR + UR * part, brs = UR * split;
+        int32_t *dst = im.out + int64_t(y0 + CELL * br0) * im.out_pitch + x0 + 4 * q;
+        const int64_t turn = CELL * brs * im.out_pitch;
         if (vec_ok) {
             if (n > 0)
-                for (int br = tid / UPR; CELL * br < nrp; br += UR, dst += turn) {
+                for (int br = br0; CELL * br < nrp; br += brs, dst += turn) {
                     int4 a, b;
                     unit(br, a, b);
                     const bool row2 = CELL == 2 && 2 * br + 1 < nrp;
@@ -890,7 +901,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
                     }
                 }
         } else {
-            for (int br = tid / UPR; CELL * br < nrp; br += UR, dst += turn) {   // rows of any alignment (whole warps)
+            for (int br = br0; CELL * br < nrp; br += brs, dst += turn) {   // rows of any alignment (whole warps)
                 int4 a, b;
                 unit(br, a, b);
                 store_row<32>(dst, a, n);
@@ -940,9 +951,13 @@ inline cudaError_t launch(const ImgList2D &L, const Work &w, int sms, bool persi
     mark(2);
     if (!one) keep(launch_k(k_scan_flatten_2d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, w));
     mark(3);
+    const int64_t ctas = int64_t(sms) * K3_PER_SM;
+    const int split = persistent ? 1 : write_split(w.n_tiles, int64_t(sms) * kSplitPerSM2);
     // The label writes run a fixed tile order over K3_PER_SM CTAs per SM (they prefetch their next tile).
-    keep(launch_k(persistent ? k_tile_write_2d<true, false> : one ? k_tile_write_2d<false, true> : k_tile_write_2d<false, false>,
-                  unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * K3_PER_SM))), K3_NT, s, ov, L, w));
+    const auto write = persistent ? k_tile_write_2d<true, kWriteTiles>
+                       : one ? k_tile_write_2d<false, kWriteOne>
+                       : split > 1 ? k_tile_write_2d<false, kWriteShared> : k_tile_write_2d<false, kWriteTiles>;
+    keep(launch_k(write, unsigned(std::max<int64_t>(1, std::min(w.n_tiles * split, ctas))), K3_NT, s, ov, L, w));
     mark(4);
     return e;
 }

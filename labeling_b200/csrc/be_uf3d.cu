@@ -918,10 +918,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_link_3d(ImgList3D L, Work
 // ---------------------------------------------------------------------------------------------
 // Label resolve and write.
 // ---------------------------------------------------------------------------------------------
+// CTAs per SM up to which CTAs share a tile's rows (191x223x157, 252 tiles: one CTA a tile 68.3 us, two
+// 65.8; 200^3, 364 tiles: the same with 2 to 5).
+constexpr int kSplitPerSM3 = 4;
 constexpr int kNLCap = 512;        // node links a write CTA stages in shared memory (later ones: from L2)
 constexpr int kStageRuns3 = 2048;  // run entries likewise
 
-template <bool Q>
+template <bool Q, bool SHARED>
 __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L, Work w)
 {
     __shared__ __align__(16) uint4 H[3 * NROW];   // class words 0..3, 4..7, (starts, runs before, S00, S01)
@@ -973,6 +976,12 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
     };
     ItemLoop<Q> loop{w.queue + 4};
     int64_t t = loop.first(&qslot);
+    int part = 0, split = 1;   // of the tile's rows
+    if (SHARED) {
+        split = int(gridDim.x / uint32_t(w.n_tiles));
+        part = int(blockIdx.x % uint32_t(split));
+        t = blockIdx.x / uint32_t(split);
+    }
     if (t < w.n_tiles) fetch(t);
     if (t < w.n_tiles) {
         grid_dep_wait();   // segment prefixes and node links from here on
@@ -991,7 +1000,7 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
         const uint32_t nb = snb, base0 = segb[TX * TY];
         const uint4 *HR = H + 2 * NROW;
         const uint32_t nrun = HR[NROW - 1].y + __popc(HR[NROW - 1].x);
-        if (t == im.tile_base && tid == 0) {
+        if (t == im.tile_base && tid == 0 && part == 0) {
             const int64_t n = int64_t(w.segpref[im.seg_base + int64_t(im.d0) * im.d1 * im.t2] - base0);
             w.ncomp[im.index] = n;
             if (w.host_count) *w.host_count = n;
@@ -1031,7 +1040,7 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
         }
         loop.publish(&qslot);
         __syncthreads();
-        const int64_t tn = loop.next(t, &qslot);   // the next tile's data come while this one's labels go
+        const int64_t tn = SHARED ? w.n_tiles : loop.next(t, &qslot);   // the next tile's data come while this one's labels go
         if (tn < w.n_tiles) {   // RB, NL, E, segb and snb are free now
             fetch(tn);
             fetch_links(tn);
@@ -1043,7 +1052,7 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
         const int q = tid % (TB2 / 2);
         const uint32_t bit0 = 1u << (2 * q), bit1 = 2u << (2 * q), upto0 = bit0 | (bit0 - 1u);
         const int n = min(4, max(0, g.nz - 4 * q));   // voxels of the thread's place inside the volume
-        for (int row = tid / (TB2 / 2); row < NROW; row += NT / (TB2 / 2)) {
+        for (int row = tid / (TB2 / 2) + NT / (TB2 / 2) * part; row < NROW; row += NT / (TB2 / 2) * split) {
             const int b0 = row / TB1, b1 = row % TB1;
             if (vec_ok && (n == 0 || 2 * b0 >= g.nx || 2 * b1 >= g.ny)) continue;
             const uint4 a = H[row], b = H[NROW + row], rw = HR[row];
@@ -1100,9 +1109,11 @@ cudaError_t launch_uf3d(const ImgList3D &L, const Work &w, int sms, bool persist
     mark(2);
     keep(launch_k(k_scan_link_3d, grid(int64_t(w.n_chunks) + w.n_tiles, 8), kScanThreads, s, ov, L, w));
     mark(3);
+    const int64_t ctas = int64_t(sms) * kT3WritePerSM;
+    const int split = persistent ? 1 : write_split(w.n_tiles, int64_t(sms) * kSplitPerSM3);
     // The label writes run a fixed tile order over kT3WritePerSM CTAs per SM (they prefetch their next tile).
-    keep(launch_k(persistent ? k_tile_write_3d<true> : k_tile_write_3d<false>, unsigned(std::max<int64_t>(1, std::min<int64_t>(w.n_tiles, int64_t(sms) * kT3WritePerSM))),
-                  kT3Threads, s, ov, L, w));
+    const auto write = persistent ? k_tile_write_3d<true, false> : split > 1 ? k_tile_write_3d<false, true> : k_tile_write_3d<false, false>;
+    keep(launch_k(write, unsigned(std::max<int64_t>(1, std::min(w.n_tiles * split, ctas))), kT3Threads, s, ov, L, w));
     mark(4);
     return e;
 }

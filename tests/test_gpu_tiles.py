@@ -75,3 +75,17 @@ def test_links_across_tile_borders(ctx, size, conn8):
         algo, coh = (be.ALGO_UF, be.COH_8) if conn8 else (be.ALGO_PIXEL, be.COH_4)
         assert be.label2d(ctx, src, out, algo=algo, coh=coh) == k, name
         assert np.array_equal(out.cpu().numpy(), ref), name
+
+
+@pytest.mark.parametrize("tiles", [2, 37, 38, 98, 99, 148, 149])
+def test_rows_of_a_tile_shared_by_ctas(ctx, tiles):
+    """Numbers of tiles on both sides of the lines where fewer CTAs share a tile's rows (148 SMs)."""
+    import torch
+    import labeling_b200 as be
+    img = ((np.random.default_rng(tiles).random((64 * tiles - 3, 45)) < 0.5) * 255).astype(np.uint8)
+    src = torch.from_numpy(img).cuda()
+    for algo, coh, conn8 in ((be.ALGO_UF, be.COH_8, True), (be.ALGO_PIXEL, be.COH_4, False)):
+        ref, k = O.ccl2d(img, 0, conn8)
+        out = torch.full(img.shape, -1, dtype=torch.int32, device="cuda")
+        assert be.label2d(ctx, src, out, algo=algo, coh=coh) == k
+        assert np.array_equal(out.cpu().numpy(), ref)

@@ -43,3 +43,15 @@ def test_tile_edges_and_capacities_3d(ctx, shape):
         assert b.counts() == [k, k], name
         assert all(np.array_equal(o.cpu().numpy(), ref) for o in outs), name
         b.close()
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 74, 75, 197, 198, 296, 297])
+def test_rows_of_a_tile_shared_by_ctas(ctx, tiles):
+    """Numbers of tiles on both sides of the lines where fewer CTAs share a tile's rows (148 SMs)."""
+    import torch
+    import labeling_b200 as be
+    vol = (np.random.default_rng(tiles).random((16 * tiles - 5, 31, 13)) < 0.25).astype(np.uint8)
+    ref, k = O.ccl3d(vol)
+    out = torch.full(vol.shape, -1, dtype=torch.int32, device="cuda")
+    assert be.label3d(ctx, torch.from_numpy(vol).cuda(), out) == k
+    assert np.array_equal(out.cpu().numpy(), ref)
