@@ -14,7 +14,7 @@ constexpr int MAXB = NPERIM;                       // nodes per tile
 constexpr int WPR = TBW / 32;                      // 32-block words per block row
 constexpr int NWORD = NBLK / 32;                   // words per tile
 constexpr int K1_NT = NWORD;                       // one thread per (block row, word)
-constexpr int K1_PER_SM = CELL == 2 ? 7 : 4;       // resident tile CTAs per SM (26 KB of shared memory, 72 registers)
+constexpr int K1_PER_SM = CELL == 2 ? 7 : 4;       // resident tile CTAs per SM (26 KB of shared memory, 66 registers)
 constexpr int MQCAP = 1024;                        // union-queue capacity (more take further rounds)
 constexpr int RBWORDS = MAXRUN / 32;               // root-bitmap words per tile: a bit per run
 // A tile's labels as the write kernel reads them (Work::lab): for each of its 32-block words the four
@@ -75,6 +75,13 @@ __device__ __forceinline__ uint32_t count_bits(const uint32_t *b, uint32_t lo, u
 // memory, where the smaller number wins, leaves the run of a component's first pixel as its root.
 // The loops over runs and links are shared evenly by the CTA's threads, and the tile is handed on as
 // bit words and one number per run, not as an entry per block.
+//
+// Bound by instruction issue (65% of the issue slots, four instructions of a 32-lane warp per block) and
+// the latency of shared-memory chains behind it, not by the image's bytes (67 MB of an 8192^2 image, 10
+// us).  Measured (this launch on 8192^2, us; one thread's serial loops over its word's runs, entries per
+// block -> this form): noise of density 0.6 150 -> 88, 0.4 158 -> 94, 0.1 73 -> 59, spiral 129 -> 87.
+// The 64 x 256 tile and 7 CTAs of 128 threads are what its 26 KB and 66 registers leave room for; the
+// pixel form (256 threads of 32 pixels) runs 4.
 // ---------------------------------------------------------------------------------------------
 template <bool Q>
 __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L, Work w)
@@ -686,9 +693,21 @@ constexpr int K3_NT = 256;
 // CTAs per SM up to which CTAs share a tile's rows: with 4, a 2048^2 call (256 tiles) is 0.5 us slower, and
 // none is faster than with 2.
 constexpr int kSplitPerSM2 = 2;
-constexpr int K3_PER_SM = 8;              // resident CTAs per SM
+// Resident CTAs per SM.  Fewer have registers for rows of any alignment (48 instead of 32 a thread), and
+// four to five full of stores keep the memory as busy as eight: 8 / 7 / 6 / 5 / 4 take 58.0 / 59.0 / 59.5 /
+// 57.5 / 61.3 us for 8192^2 noise, 83.0 / 85.4 / 82.2 / 79.9 / 84.7 for 8191x8189, 12.3 / 12.4 / 10.3 / 10.3 / 10.2
+// for 1021x1787.
+constexpr int K3_PER_SM = 5;
 
-// ONE (a plain launch of one tile): the tile kernel's launch goes straight before this one -- there is
+// A CTA works out the label of every run (roots by rank in their segment, linked border components
+// through their global root, the others through their root run), then writes the rows; with a fixed tile
+// order it fetches its next tile's words while it writes.  Bound by the stores: of 57 us for the 268 MB
+// of an 8192^2 image a bare kernel that stores the same tiles takes 44 (6.1 TB/s); the rest is the first
+// tile's set-up and the last, half-full round of tiles.  Copying the segment prefixes and node entries
+// ahead too, and starting an SM's CTAs apart, changed nothing.  Four pixels a thread and row,
+// as one 16-byte store; rows of any other alignment go through store_row.
+//
+// kWriteOne (a plain launch of one tile): the tile kernel's launch goes straight before this one -- there is
 // nothing to merge and no prefix beyond the tile's own rows, which the CTA sums itself -- so that the
 // smallest images take two launches: 16^2 17.4 -> 13.1 us, 64^2 18.5 -> 16.1 us.  (Doing without the scan
 // launch for images of several tiles, every CTA scanning the counts, was slower: 2048^2 43.0 -> 44.7 us.)

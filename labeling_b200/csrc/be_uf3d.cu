@@ -348,6 +348,13 @@ __device__ __noinline__ uint2 row_bits_call(const uint8_t *p, int n, const uint8
 
 }  // namespace
 
+// One thread per block row (32 blocks along d2, one word per voxel class).  Bound by instruction issue
+// and shared-memory latency: of a tile's time on noise of density 0.3, 13% are the loads, 16% links and
+// first links, 18% queueing the other links and flattening, 38% the unions of about 700 kept links, 10%
+// nodes and border data; on smooth fields (long runs) the loads are a third.  Measured (this launch on
+// 512^3, us; slots of first voxels as run numbers and every link a union -> dense run numbers, links that
+// close a triangle dropped, hooking before the unions, whole-row loads): density 0.3 390 -> 199, smooth
+// half-full fields 196 -> 87.  128 threads, 31 KB and 72 registers: 7 CTAs per SM.
 template <bool Q>
 __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D L, Work w)
 {
@@ -690,7 +697,10 @@ __device__ void gunion3d(const Img3D &im, Work &w, uint32_t a, uint32_t b)
 // warp takes those of one direction, a lane a pair.  The links go through a shared queue and are shared
 // by all lanes; a pair of nodes that the CTA has just seen -- most links join the same few large
 // components -- is dropped by a small table, and the others are unions, whose walks (dependent loads
-// through L2) end as soon as the two sides have one parent.
+// through L2) end as soon as the two sides have one parent.  Bound by the latency of its loads: 16 tiles
+// in flight per SM (8 / 12 / 16: 127 / 110 / 107 us before the direction split).  Measured (this launch on
+// 512^3, us; voxel pairs through a CTA-local union-find -> this): density 0.3 150 -> 68, smooth fields
+// 143 -> 44, density 0.1 79 -> 70.
 constexpr int kMQ3 = 1024;     // queued links (more take further rounds)
 constexpr int kSeen3 = 256;    // table of node pairs seen
 
@@ -918,6 +928,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_link_3d(ImgList3D L, Work
 // ---------------------------------------------------------------------------------------------
 // Label resolve and write.
 // ---------------------------------------------------------------------------------------------
+// As k_tile_write_2d, with the nodes' links resolved by the launch before and one lookup per block pair for
+// its four voxel rows.  Bound by the stores: of 111 us for the 537 MB of a 512^3 volume a bare kernel that
+// stores the same tiles takes 87.  4 CTAs of 256 threads per SM, for their 64 registers: with 6 / 5 / 4 / 3
+// a 512^3 volume takes 121 / 114 / 111 / 110 us, a 511x511x509 one, whose rows have every alignment, - /
+// 243 / 181 / 177, and 191x223x157 - / 24.5 / 18.6 / 24.
 // CTAs per SM up to which CTAs share a tile's rows (191x223x157, 252 tiles: one CTA a tile 68.3 us, two
 // 65.8; 200^3, 364 tiles: the same with 2 to 5).
 constexpr int kSplitPerSM3 = 4;
