@@ -89,3 +89,17 @@ def test_rows_of_a_tile_shared_by_ctas(ctx, tiles):
         out = torch.full(img.shape, -1, dtype=torch.int32, device="cuda")
         assert be.label2d(ctx, src, out, algo=algo, coh=coh) == k
         assert np.array_equal(out.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("sides", [[(128, 128), (130, 120), (1, 1)], [(64, 256), (60, 500), (3, 129)], [(65, 128), (64, 256)]])
+def test_batch_tile_shape_by_tiles(ctx, sides):
+    """Batches that square tiles cover with fewer, with more and with as many tiles as the default's."""
+    import torch
+    import labeling_b200 as be
+    rng = np.random.default_rng(len(sides))
+    imgs = [((rng.random(s) < 0.5) * 255).astype(np.uint8) for s in sides]
+    dev = [(torch.from_numpy(i).cuda(), torch.full(i.shape, -1, dtype=torch.int32, device="cuda"), 0) for i in imgs]
+    be.Batch(ctx, dev).run()
+    torch.cuda.synchronize()
+    for img, (_, out, _) in zip(imgs, dev):
+        assert np.array_equal(out.cpu().numpy(), O.ccl2d(img, 0, True)[0])
