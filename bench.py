@@ -56,17 +56,20 @@ ALGO_BYTES = {"k_tile_local_2d": 1.0, "k_tile_write_2d": 4.0, "k_tile_local_3d":
 
 # Bytes the union-find pipeline itself moves per pixel / voxel, by array (reads and writes of the
 # pipeline's launches, counted from the kernels' loads and stores; node records of border components,
-# at most a few bytes per border pixel, are left out).  2D tile 64 x 256 px, 3D tile 16 x 32 x 64.
+# at most a few bytes per border pixel, are left out).  2D tile 64 x 256 px, 3D tile 16 x 32 x 64; root
+# runs at the 2048 of a tile that the write kernels fetch (4 KB).
 IMPL_BYTES = {
     "2d": {"input read": 1.0, "labels written": 4.0,
-           "block entries written + read (uint16 per 2x2 block)": 2 * 0.5,
-           "root bitmap written + read (1 bit per pixel)": 2 * 0.125,
-           "border entries written + read twice": 3 * 640 / 16384,
+           "class and run words written + read (4 KB per tile)": 2 * 4096 / 16384,
+           "root runs written + read (uint16 per run)": 2 * 4096 / 16384,
+           "root bitmap written + read (1 bit per run)": 2 * 512 / 16384,
+           "border entries written + read": 2 * 640 / 16384,
            "segment counts + prefix": (1 + 1 + 4 + 4) / 256},
     "3d": {"input read": 1.0, "labels written": 4.0,
-           "block entries written + read (uint32 per 2x2x2 block)": 2 * 0.5,
-           "root bitmap written + read (1 bit per voxel)": 2 * 0.125,
-           "border entries written + read twice": 3 * 2 * (8 * 16 + 8 * 32 + 16 * 32) * 2 / 32768,
+           "class and run words written + read, again for the rows on a border": (2 * 6656 + 210 * 48) / 32768,
+           "root runs written + read (uint16 per run)": 2 * 4096 / 32768,
+           "root bitmap written + read (1 bit per run)": 2 * 512 / 32768,
+           "border data (uint16 per run, 640 B of faces) written + read": 2 * (4096 + 640) / 32768,
            "segment counts + prefix": (1 + 1 + 4 + 4) / 64},
 }
 
@@ -536,7 +539,7 @@ def bench_plain(args, rank, world, local_rank, workload):
         "config": {**headline_config(workload, [n for n, _ in inputs], inputs[0][1].shape, world),
                    "form": form},
         "e2e": e2e, "roofline": roofline, "roofline_kernels": kernels,
-        "gpu_launches": (len(stages) * steps) if algo == be.ALGO_UF else None, "clocks": clocks,
+        "gpu_launches": (len(stages) * steps) if algo != be.ALGO_ITER else None, "clocks": clocks,
         "components": {n: c for (n, _), c in zip(inputs, counts)},
         "per_image_ms": per_image,
         "per_image_stage_ms": {k: [round(float(x), 4) for x in np.mean(v, axis=0)] for k, v in per_stage.items()},
