@@ -67,22 +67,48 @@ Geometry geometry_3d()
     return g;
 }
 
-// Carves the workspace of a launch with n_tiles tiles, n_segs segments and n_imgs images out of
-// one allocation (or only computes its size when base == nullptr).
-size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs, char *base, Work *w)
+// The head of a workspace: launch epoch, error flags and the status words of the segment scan.  A status word
+// is taken for this launch's when it carries its epoch, so whatever else may be in the scratch, these words
+// must never be anything but status words: the head comes first and has one size for all the launches that
+// use an allocation.
+static size_t take_head(int64_t chunks, char *base, Work &t)
 {
     size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char *p = base ? base + off : nullptr;
+        off = align_up(off + bytes, 256);
+        return p;
+    };
+    t.epoch = reinterpret_cast<uint32_t *>(take(2 * sizeof(uint32_t)));
+    t.err = reinterpret_cast<uint32_t *>(take(16 * sizeof(uint32_t)));
+    t.scan_status = reinterpret_cast<uint64_t *>(take(size_t(std::max<int64_t>(chunks, 1)) * sizeof(uint64_t)));
+    return off;
+}
+
+size_t head_bytes(int64_t chunks)
+{
+    Work t{};
+    return take_head(chunks, nullptr, t);
+}
+
+// A segment takes at least five bytes of a launch's arrays, its count and its prefix.
+int64_t max_chunks(size_t bytes) { return int64_t(bytes / (5 * size_t(kScanChunk))) + 1; }
+
+// Carves the workspace of a launch with n_tiles tiles, n_segs segments and n_imgs images out of
+// one allocation (or only computes its size when base == nullptr).  head_chunks: the scan chunks that the
+// allocation's head holds (0: as many as this launch has).
+size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs, char *base, Work *w,
+                   int64_t head_chunks)
+{
+    const int64_t n_chunks = (n_segs + kScanChunk - 1) / kScanChunk;
+    Work t{};
+    size_t off = take_head(head_chunks ? head_chunks : n_chunks, base, t);
     auto take = [&](size_t bytes) {
         size_t o = off;
         off = align_up(off + bytes, 256);
         return base ? base + o : nullptr;
     };
-    const int64_t n_chunks = (n_segs + kScanChunk - 1) / kScanChunk;
     const size_t nodes = size_t(n_tiles) * g.maxb;
-    Work t{};
-    // The launch epoch comes first: its place is the same for every size, so it only ever grows, and
-    // status words that launches of other sizes left in the workspace are never taken for this one's.
-    t.epoch = reinterpret_cast<uint32_t *>(take(2 * sizeof(uint32_t)));
     t.lab = take(size_t(n_tiles) * g.lab_bytes_per_tile);
     t.perim = reinterpret_cast<uint16_t *>(take(size_t(n_tiles) * g.nperim * sizeof(uint16_t)));
     t.rbits = reinterpret_cast<uint32_t *>(take(size_t(n_tiles) * g.rbits_bytes_per_tile));
@@ -96,8 +122,6 @@ size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_img
     t.chunksum = reinterpret_cast<uint32_t *>(take(size_t(std::max<int64_t>(n_chunks, 1)) * sizeof(uint32_t)));
     t.queue = reinterpret_cast<uint32_t *>(take(kQueueWords * sizeof(uint32_t)));
     t.ncomp = reinterpret_cast<int64_t *>(take(size_t(std::max(n_imgs, 1)) * sizeof(int64_t)));
-    t.err = reinterpret_cast<uint32_t *>(take(16 * sizeof(uint32_t)));
-    t.scan_status = reinterpret_cast<uint64_t *>(take(size_t(std::max<int64_t>(n_chunks, 1)) * sizeof(uint64_t)));
     t.n_tiles = n_tiles;
     t.n_segs = n_segs;
     t.n_chunks = int32_t(n_chunks);
@@ -117,27 +141,29 @@ int Workspace::ensure(be_ctx *ctx, const Geometry &g, int64_t n_tiles, int64_t n
 {
     // Node links name a segment in 32 bits.
     if (n_segs >= int64_t(kNone)) return set_error(ctx, BE_ERR_TOO_LARGE, "more than 2^32 - 2 image rows in one launch");
-    const size_t need = layout_work(g, n_tiles, n_segs, n_imgs, nullptr, nullptr);
-    if (!base || need > bytes) {
+    if (!base || layout_work(g, n_tiles, n_segs, n_imgs, nullptr, nullptr, cap_chunks) > bytes) {
         if (base) {
             cudaError_t e = cudaFree(base);
             base = nullptr;
             bytes = 0;
             if (e != cudaSuccess) return cuda_error(ctx, e, "cudaFree(workspace)");
         }
-        const size_t grow = need + need / 4;   // headroom for slightly larger later calls
-        cudaError_t e = cudaMalloc(&base, grow);
+        const size_t need = layout_work(g, n_tiles, n_segs, n_imgs, nullptr, nullptr);
+        const size_t body = need + need / 4;   // headroom for slightly larger later calls
+        const size_t head = head_bytes(max_chunks(body));
+        cudaError_t e = cudaMalloc(&base, head + body);
         if (e != cudaSuccess) {
             base = nullptr;
             return cuda_error(ctx, e, "cudaMalloc(workspace)");
         }
         // The scan's status words and the launch epoch start at zero once; every later run tells
         // its own status words from older ones by the epoch it increments.
-        e = cudaMemset(base, 0, grow);
+        e = cudaMemset(base, 0, head);
         if (e != cudaSuccess) return cuda_error(ctx, e, "cudaMemset(workspace)");
-        bytes = grow;
+        bytes = head + body;
+        cap_chunks = max_chunks(body);   // of any launch whose arrays fit beside the head
     }
-    layout_work(g, n_tiles, n_segs, n_imgs, static_cast<char *>(base), &w);
+    layout_work(g, n_tiles, n_segs, n_imgs, static_cast<char *>(base), &w, cap_chunks);
     cap_tiles = n_tiles;
     cap_segs = n_segs;
     cap_imgs = n_imgs;

@@ -34,14 +34,19 @@ cudaError_t uf2d_launch(int shape, const ImgList2D &L, const Work &w, int sms, b
 
 Geometry geometry_2d();   // shape 0
 Geometry geometry_3d();
-size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs, char *base, Work *w);
+size_t head_bytes(int64_t chunks);      // size of a workspace's head that holds this many scan chunks
+int64_t max_chunks(size_t bytes);       // scan chunks of a launch whose arrays take at most this many bytes
+size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs, char *base, Work *w,
+                   int64_t head_chunks = 0);
 // Zeroes a workspace's launch epoch and scan status words (memory that was not zeroed before).
 cudaError_t reset_scan_state(const Work &w, cudaStream_t s);
 
-// One growable device allocation holding a Work.
+// One growable device allocation holding a Work.  Launches of any sizes and geometries are laid out in it one
+// after the other; its head stays where it is.
 struct Workspace {
     void *base = nullptr;
     size_t bytes = 0;
+    int64_t cap_chunks = 0;   // scan chunks its head holds
     int64_t cap_tiles = 0, cap_segs = 0;
     int cap_imgs = 0;
     Work w{};
