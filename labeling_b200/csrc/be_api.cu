@@ -117,7 +117,7 @@ size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_img
     t.gp = reinterpret_cast<unsigned long long *>(take(nodes * sizeof(unsigned long long)));
     t.nroot = reinterpret_cast<uint16_t *>(take(nodes * sizeof(uint16_t)));
     t.nlink = g.links ? reinterpret_cast<uint2 *>(take(nodes * sizeof(uint2))) : nullptr;
-    t.segcnt = reinterpret_cast<uint8_t *>(take(align_up(size_t(n_segs), 16) + 16));
+    t.segcnt = reinterpret_cast<uint8_t *>(take(align_up(size_t(n_segs) * g.seg_bytes, 16) + 16));
     t.segpref = reinterpret_cast<uint32_t *>(take((size_t(n_segs) + 1) * sizeof(uint32_t)));
     t.chunksum = reinterpret_cast<uint32_t *>(take(size_t(std::max<int64_t>(n_chunks, 1)) * sizeof(uint32_t)));
     t.queue = reinterpret_cast<uint32_t *>(take(kQueueWords * sizeof(uint32_t)));

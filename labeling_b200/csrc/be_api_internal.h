@@ -17,6 +17,7 @@ struct Geometry {
     size_t rbits_bytes_per_tile;
     int nperim;
     int maxb;
+    int seg_bytes = 1;    // bytes of a segment's root count
     bool links = false;   // the pipeline resolves node links (Work::nlink) before its label writes
 };
 

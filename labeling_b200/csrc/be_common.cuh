@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <type_traits>
 #include <utility>
 
 namespace be {
@@ -74,7 +75,8 @@ struct Work {
                           // of that first pixel among the roots left in its segment
     uint32_t *rbits;      // per tile: bitmap of the tile's components that are still roots (the merge
                           // clears the ones it links): 2D a bit per run, 3D a bit per first voxel
-    uint8_t *segcnt;      // per segment: number of component roots (uint8, word-padded)
+    uint8_t *segcnt;      // per segment: number of component roots (uint8, or uint16 in a pipeline whose segments
+                          // can hold more than 255; word-padded)
     uint32_t *segpref;    // per segment + 1: exclusive prefix of segcnt over the launch
     uint32_t *chunksum;   // per scan chunk: sum of segcnt
     uint32_t *queue;      // work-queue counters (persistent mode); zeroed before a launch
@@ -299,11 +301,13 @@ __device__ __forceinline__ uint32_t gfind_jump(unsigned long long *gp, uint32_t 
     return p;
 }
 
-// Decrement a uint8 counter packed in a 32-bit word (the counter is >= 1 when this is called).
-__device__ __forceinline__ void dec_u8(uint8_t *base, int64_t idx)
+// Decrement a uint8 or uint16 counter packed in a 32-bit word (the counter is >= 1 when this is called).
+template <class Count>
+__device__ __forceinline__ void dec_count(uint8_t *base, int64_t idx)
 {
-    uint32_t *w = reinterpret_cast<uint32_t *>(base + (idx & ~int64_t(3)));
-    atomicSub(w, 1u << (8 * (idx & 3)));
+    const int64_t at = idx * int64_t(sizeof(Count));
+    uint32_t *w = reinterpret_cast<uint32_t *>(base + (at & ~int64_t(3)));
+    atomicSub(w, 1u << (8 * (at & 3)));
 }
 
 // Block-wide exclusive scan of one uint32 per thread; returns the thread's prefix and writes the

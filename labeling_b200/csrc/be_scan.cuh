@@ -1,7 +1,7 @@
 // be_scan.cuh -- the segment-count scan and the node-link pass shared by the 2D and 3D pipelines.
 //
-// Segment counts are uint8 (at most half a segment's pixels can start a component).  The
-// union-find pipelines scan them in one launch (segscan_lb_chunk, a single-pass scan with a
+// At most half a segment's pixels can start a component, so segment counts are uint8 -- except in the 2D
+// tiles of 512 pixels' width, whose 256 take uint16.  The union-find pipelines scan them in one launch (segscan_lb_chunk, a single-pass scan with a
 // decoupled look-back) beside the node pass (flatten_tile_nodes in 2D, link_tile_nodes in 3D);
 // the iterative forms use the two-launch scan of be_scan.cu (k_chunk_sums with chunk_sum below,
 // then k_segscan).
@@ -37,7 +37,7 @@ __device__ __forceinline__ void chunk_sum(Work &w, int64_t c, uint32_t *tmp)
 // never need clearing between runs.  Waits are bounded: a wait that runs out sets w.err[3] and the
 // chunk goes on with what it has (the labels are then wrong, the device stays usable).
 // Called by a whole CTA of NT threads; tmp holds NT / 32 + 1 words, sh two.
-template <int NT>
+template <int NT, class Count = uint8_t>
 __device__ __forceinline__ void segscan_lb_chunk(Work &w, uint32_t *tmp, uint32_t *sh)
 {
     constexpr int PER = kScanChunk / NT;
@@ -50,21 +50,24 @@ __device__ __forceinline__ void segscan_lb_chunk(Work &w, uint32_t *tmp, uint32_
 
     const int64_t lo = c * kScanChunk + int64_t(threadIdx.x) * PER;
     const int64_t hi = min(w.n_segs, lo + PER);
-    uint32_t v[PER / 4];
+    constexpr int CW = 4 / sizeof(Count);   // counts in a word
+    const Count *cnt = reinterpret_cast<const Count *>(w.segcnt);
+    uint32_t v[PER / CW];
     uint32_t s = 0;
 #pragma unroll
-    for (int q = 0; q < PER / 4; ++q) {
-        const int64_t i = lo + 4 * q;
+    for (int q = 0; q < PER / CW; ++q) {
+        const int64_t i = lo + CW * q;
         uint32_t x = 0;
-        if (i + 4 <= hi) {
-            x = *reinterpret_cast<const uint32_t *>(w.segcnt + i);
+        if (i + CW <= hi) {
+            x = *reinterpret_cast<const uint32_t *>(cnt + i);
         } else {
-            for (int k = 0; k < 4; ++k)
-                if (i + k < hi) x |= uint32_t(w.segcnt[i + k]) << (8 * k);
+            for (int k = 0; k < CW; ++k)
+                if (i + k < hi) x |= uint32_t(cnt[i + k]) << (32 / CW * k);
         }
         v[q] = x;
-        s += __vsadu4(x, 0u);
+        s += CW == 4 ? __vsadu4(x, 0u) : (x & 0xFFFFu) + (x >> 16);
     }
+    auto count = [&](int j) -> uint32_t { return (v[j / CW] >> (32 / CW * (j % CW))) & ((1u << (32 / CW)) - 1u); };
     uint32_t ctot;
     uint32_t pre = block_exscan<NT>(s, tmp, &ctot);
     volatile unsigned long long *st = reinterpret_cast<volatile unsigned long long *>(w.scan_status);
@@ -114,10 +117,10 @@ __device__ __forceinline__ void segscan_lb_chunk(Work &w, uint32_t *tmp, uint32_
     for (int q = 0; q < PER / 4; ++q) {
         const int64_t i = lo + 4 * q;
         uint4 o;
-        o.x = pre; pre += v[q] & 0xFF;
-        o.y = pre; pre += (v[q] >> 8) & 0xFF;
-        o.z = pre; pre += (v[q] >> 16) & 0xFF;
-        o.w = pre; pre += v[q] >> 24;
+        o.x = pre; pre += count(4 * q);
+        o.y = pre; pre += count(4 * q + 1);
+        o.z = pre; pre += count(4 * q + 2);
+        o.w = pre; pre += count(4 * q + 3);
         if (i + 4 <= hi) {
             *reinterpret_cast<uint4 *>(w.segpref + i) = o;
         } else {

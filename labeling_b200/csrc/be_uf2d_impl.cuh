@@ -25,6 +25,10 @@ constexpr int RBWORDS = MAXRUN / 32;               // root-bitmap words per tile
 constexpr int kHdr = (CELL == 2 ? 8 : 4) * NWORD;
 constexpr int kLabWords = kHdr + MAXRUN / 2;
 
+// Roots of a segment: at most its runs, every two of them with a background pixel between.
+using SegCount = std::conditional_t<TW / 2 <= 255, uint8_t, uint16_t>;
+static_assert(TW / 2 <= 0xFFFF, "a segment's root count fits");
+
 static_assert(MAXRUN == 4096, "a run number must fit 12 bits; 128 words of run flags");
 static_assert(MAXB < 4096, "node index must fit 12 bits");
 static_assert(K1_NT % 128 == 0 && K1_NT >= RBWORDS && (WPR & (WPR - 1)) == 0 && WPR <= 32, "thread layout");
@@ -440,7 +444,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
             uint32_t c = 0;
             for (uint32_t i = s >> 5; 32 * i < e; ++i)
                 c += __popc(BP[i] & (i == s >> 5 ? ~0u << (s & 31u) : ~0u) & (32 * i + 32 > e ? (1u << (e & 31u)) - 1u : ~0u));
-            w.segcnt[im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx] = uint8_t(c);
+            reinterpret_cast<SegCount *>(w.segcnt)[im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx] = SegCount(c);
         }
         // Border positions: component (root run), mask, and whether this position
         // claimed the node (the one that sets the component's flag writes the node's record).
@@ -534,7 +538,7 @@ namespace {
 __device__ void gunion2d(const Img2D &im, Work &w, uint32_t a, uint32_t b)
 {
     gunion_keyed(w.gp, a, b, [&](uint32_t node, uint32_t key) {
-        dec_u8(w.segcnt, im.seg_base + key / seg_width(im));
+        dec_count<SegCount>(w.segcnt, im.seg_base + key / seg_width(im));
         const uint32_t run = w.nroot[node];
         atomicAnd(w.rbits + int64_t(node / MAXB) * RBWORDS + (run >> 5), ~(1u << (run & 31u)));
     });
@@ -679,7 +683,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_flatten_2d(Work w)
     const int64_t n = int64_t(w.n_chunks) + w.n_tiles;
     for (int64_t it = blockIdx.x; it < n; it += gridDim.x) {   // (in a fixed order: the items are short)
         if (it < w.n_chunks) {
-            segscan_lb_chunk<kScanThreads>(w, tmp, sh);
+            segscan_lb_chunk<kScanThreads, SegCount>(w, tmp, sh);
             continue;
         }
         flatten_tile_nodes(w, it - w.n_chunks, MAXB);
@@ -785,7 +789,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             if (tid < 32) {
                 uint32_t c[PER], sum = 0;
 #pragma unroll
-                for (int i = 0; i < PER; ++i) sum += c[i] = PER * tid + i < nrp ? w.segcnt[PER * tid + i] : 0u;
+                for (int i = 0; i < PER; ++i) sum += c[i] = PER * tid + i < nrp ? reinterpret_cast<const SegCount *>(w.segcnt)[PER * tid + i] : 0u;
                 uint32_t x = sum;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
@@ -941,6 +945,7 @@ inline Geometry geometry()
     g.lab_bytes_per_tile = size_t(kLabWords) * sizeof(uint32_t);
     g.rbits_bytes_per_tile = size_t(RBWORDS) * sizeof(uint32_t);
     g.nperim = NPERIM;
+    g.seg_bytes = int(sizeof(SegCount));
     g.maxb = MAXB;
     return g;
 }

@@ -71,6 +71,7 @@ constexpr uint32_t kNoNode = 0xFFFFu;
 // of every run (uint16).
 constexpr int kHdr3 = 13 * NROW;
 static_assert(T3_LAB_WORDS == kHdr3 + NBLK / 2, "tile words");
+static_assert(TZ / 2 <= 0xFF, "a segment's root count fits its uint8");
 
 // Of the starts, those of voxel row ij (2i + j) of their block row: the four sets of `first voxel in that
 // voxel row`.
@@ -682,7 +683,7 @@ namespace {
 __device__ void gunion3d(const Img3D &im, Work &w, uint32_t a, uint32_t b)
 {
     gunion_keyed(w.gp, a, b, [&](uint32_t node, uint32_t key) {
-        dec_u8(w.segcnt, im.seg_base + key / seg_width3(im));
+        dec_count<uint8_t>(w.segcnt, im.seg_base + key / seg_width3(im));
         const uint32_t blk = w.nroot[node];
         atomicAnd(w.rbits + int64_t(node / MAXB) * NROW + blk / TB2, ~(1u << (blk % TB2)));
     });
