@@ -285,8 +285,9 @@ int be_slab_reserve(be_ctx *ctx, int64_t max_count, int64_t max_joined);
 
 /* Report of the bounds-checked debug build (-DBE_BOUNDS_CHECK; no counterpart in the
  * reference): out3 = {site, value low, value high} of the first failed index check of the last
- * 2D (dims = 2) or 3D (dims = 3) union-find call, all zero when none failed.  Normal builds
- * perform no checks and always report zeros. */
+ * 2D (dims = 2) or 3D (dims = 3) union-find call, the pixel and run forms' among them, all zero when
+ * none failed.  Normal builds perform no index checks.  Site 300, in any build: a bounded wait of the
+ * segment scan ran out, in that call or (normal builds) an earlier one of the same form. */
 int be_check_status(be_ctx *ctx, int dims, uint32_t *out3);
 
 /* Per-launch timing of plain calls (no counterpart in the reference, whose stopwatch covers the

@@ -287,10 +287,13 @@ int be_check_status(be_ctx *c, int dims, uint32_t *out3)
 {
     if (!c || !out3 || (dims != 2 && dims != 3)) return BE_ERR_INVALID;
     out3[0] = out3[1] = out3[2] = 0;
-    const Work &w = dims == 2 ? c->ws2d.w : c->ws3d.w;
-    if (!w.err) return BE_OK;
-    cudaError_t e = cudaMemcpy(out3, w.err, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost);
+    const Workspace *ws = c->last_ws[dims - 2];
+    if (!ws || !ws->base) return BE_OK;
+    uint32_t err[4] = {};
+    cudaError_t e = cudaMemcpy(err, ws->w.err, sizeof(err), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_error(c, e, "be_check_status");
+    std::copy(err, err + 3, out3);
+    if (!out3[0] && err[3]) out3[0] = kSiteScanWait;
     return BE_OK;
 }
 
@@ -359,6 +362,7 @@ int be_label2d(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int
         fill_img2d(im, in, in_pitch, rows, cols, threshold, out, out_pitch, 0, 0, 0, shape);
         const int64_t n_tiles = int64_t(im.tiles_x) * im.tiles_y;
         const int64_t n_segs = int64_t(rows) * im.tiles_x;
+        c->last_ws[0] = &ws;
         rc = ws.ensure(c, uf2d_geometry(shape), n_tiles, n_segs, 1);
         if (rc) return rc;
         ImgList2D L{nullptr, 1, im};
@@ -415,6 +419,7 @@ int be_label3d(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2,
         fill_img3d(im, in, d0, d1, d2, threshold, out, 0, 0, 0);
         const int64_t n_tiles = int64_t(im.t0) * im.t1 * im.t2;
         const int64_t n_segs = int64_t(d0) * d1 * im.t2;
+        c->last_ws[1] = &ws;
         rc = ws.ensure(c, geometry_3d(), n_tiles, n_segs, 1);
         if (rc) return rc;
         ImgList3D L{nullptr, 1, im};

@@ -9,6 +9,7 @@
 
 namespace be {
 
+constexpr uint32_t kSiteScanWait = 300;   // be_check_status: a wait of the segment scan ran out
 constexpr int kQueueWords = 16;   // work-queue counters per workspace (one per kernel)
 
 // Per-tile sizes of a pipeline's workspace.
@@ -105,6 +106,7 @@ struct be_ctx {
     int sms = 148;
     std::string err;
     be::Workspace ws2d, ws3d, wsiter;
+    const be::Workspace *last_ws[2] = {};   // workspace of the last union-find call, 2D / 3D
     be::Workspace wsform2d, wsform3d;   // the pixel and run forms (apart: a caller may overlap them with the block form)
     void *iter_base = nullptr;      // iterative-form block arrays
     size_t iter_bytes = 0;
