@@ -132,15 +132,23 @@ __device__ __forceinline__ void segscan_lb_chunk(Work &w, uint32_t *tmp, uint32_
     if (c == w.n_chunks - 1 && threadIdx.x == 0) w.segpref[w.n_segs] = sh_excl + ctot;
 }
 
+// Nodes of tile t.
+__device__ __forceinline__ uint32_t tile_nodes(const Work &w, int64_t t, int maxb)
+{
+    const uint32_t nb = w.nb[t];
+    return GUARD(w, nb <= uint32_t(maxb), 301, nb) ? nb : 0u;
+}
+
 // Points every linked node of tile t at its global root (gfind_jump: the nodes of all tiles jump
 // at once, each writing only its own entry, so deep trees take logarithmic walks).  Called by a
 // whole CTA.
 __device__ __forceinline__ void flatten_tile_nodes(Work &w, int64_t t, int maxb)
 {
-    const uint32_t nb = w.nb[t];
+    const uint32_t nb = tile_nodes(w, t, maxb);
     for (uint32_t j = threadIdx.x; j < nb; j += blockDim.x) {
         const uint32_t node = uint32_t(t * maxb + j);
         if (uint32_t(w.gp[node]) == node) continue;
+        if (!GUARD(w, uint32_t(w.gp[node]) < w.n_tiles * maxb, 302, node)) continue;
         const uint32_t root = gfind_jump(w.gp, node);
         w.gp[node] = w.gp[root];
     }
@@ -154,11 +162,11 @@ __device__ __forceinline__ void flatten_tile_nodes(Work &w, int64_t t, int maxb)
 template <typename Locate>
 __device__ __forceinline__ void link_tile_nodes(Work &w, int64_t t, int maxb, Locate locate)
 {
-    const uint32_t nb = w.nb[t];
+    const uint32_t nb = tile_nodes(w, t, maxb);
     for (uint32_t j = threadIdx.x; j < nb; j += blockDim.x) {
         const uint32_t node = uint32_t(t * maxb + j);
         uint2 link = make_uint2(kNone, 0u);
-        if (uint32_t(w.gp[node]) != node) {
+        if (uint32_t(w.gp[node]) != node && GUARD(w, uint32_t(w.gp[node]) < w.n_tiles * maxb, 302, node)) {
             const uint32_t root = gfind_jump(w.gp, node);
             const unsigned long long re = w.gp[root];
             w.gp[node] = re;

@@ -357,8 +357,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
                 first &= first - 1;
                 uint32_t own, up;
                 take(b, own, up);
-                (void)GUARD(w, own < nrun && up < own, 112, (uint64_t(own) << 32) | up);
-                P[own & (MAXRUN - 1)] = up & (MAXRUN - 1);
+                if (GUARD(w, own < nrun && up < own, 112, (uint64_t(own) << 32) | up)) P[own & (MAXRUN - 1)] = up & (MAXRUN - 1);
             }
         }
         // The remaining links are unions: queued and merged by every lane.
@@ -370,7 +369,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
                 if (!b) break;
                 uint32_t own, up;
                 take(b - 1u, own, up);
-                MQ[pos - lo] = (own << 16) | up;
+                MQ[pos - lo] = GUARD(w, own < nrun && up < own, 114, (uint64_t(own) << 32) | up) ? (own << 16) | up : 0u;
                 ++pos;
             }
         };
@@ -444,7 +443,8 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
             uint32_t c = 0;
             for (uint32_t i = s >> 5; 32 * i < e; ++i)
                 c += __popc(BP[i] & (i == s >> 5 ? ~0u << (s & 31u) : ~0u) & (32 * i + 32 > e ? (1u << (e & 31u)) - 1u : ~0u));
-            reinterpret_cast<SegCount *>(w.segcnt)[im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx] = SegCount(c);
+            const int64_t si = im.seg_base + int64_t(y0 + tid) * im.tiles_x + tx;
+            if (GUARD(w, si >= 0 && si < w.n_segs, 116, si)) reinterpret_cast<SegCount *>(w.segcnt)[si] = SegCount(c);
         }
         // Border positions: component (root run), mask, and whether this position
         // claimed the node (the one that sets the component's flag writes the node's record).
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
             if (!m) continue;
             const uint32_t upto = (2u << k) - 1u;
             const uint32_t id = (CELL == 1 || ((wr.z >> k) & 1u) ? (wr.w & 0xFFFFu) + __popc(wr.x & upto) : (wr.w >> 16) + __popc(wr.y & upto)) - 1u;
-            (void)GUARD(w, id < nrun, 113, id);
+            if (!GUARD(w, id < nrun, 113, id)) continue;
             const uint32_t c = root_of(id);
             const uint32_t bit = 1u << (c & 31);
             const uint32_t old = atomicOr(&BF[c >> 5], bit);
@@ -503,8 +503,9 @@ __global__ void __launch_bounds__(K1_NT, K1_PER_SM) k_tile_local_2d(ImgList2D L,
                 const uint32_t cw = c >> 5, g = cw >> 5;
                 const uint32_t j = (g == 0 ? noff[0] : g == 1 ? noff[1] : g == 2 ? noff[2] : noff[3]) + BP[cw] +
                                    __popc(BF[cw] & ((1u << (c & 31)) - 1u));
-                ent = uint16_t((j << 4) | m);
-                if (prb[i] & kOwner) {
+                const bool ok = GUARD(w, j < uint32_t(MAXB), 115, j);
+                ent = ok ? uint16_t((j << 4) | m) : uint16_t(0);
+                if ((prb[i] & kOwner) && ok) {
                     int row = 0;   // the block row of run c
 #pragma unroll
                     for (int h = TBH / 2; h; h >>= 1)
@@ -589,7 +590,8 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
         // with the staging loads.
         constexpr int NI = (K2_NP + K2_NT - 1) / K2_NT;
         uint32_t own[NI];
-        const bool right = tx + 1 < im.tiles_x, below = ty + 1 < im.tiles_y;
+        bool right = tx + 1 < im.tiles_x, below = ty + 1 < im.tiles_y;
+        if (!GUARD(w, t + (below ? im.tiles_x : 0) + (right ? 1 : 0) < w.n_tiles, 201, t)) right = below = false;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
             const int p = threadIdx.x + i * K2_NT;
@@ -646,8 +648,10 @@ __global__ void __launch_bounds__(K2_NT, K2_PER_SM) k_merge_2d(ImgList2D L, Work
                 if (key == last) continue;
                 last = key;
                 if (atomicExch(&seen[(key * 0x9E3779B1u) >> 24], key) == key) continue;
+                const int64_t tB = col ? t + 1 : t + im.tiles_x + int(side) - 2;
+                if (!GUARD(w, ja < w.nb[t] && (B >> 4) < w.nb[tB], 203, (uint64_t(tB) << 32) | (B << 16) | A)) continue;
                 const uint32_t nA = uint32_t(t * MAXB + ja);
-                const uint32_t nB = uint32_t((col ? t + 1 : t + im.tiles_x + int(side) - 2) * MAXB + (B >> 4));
+                const uint32_t nB = uint32_t(tB * MAXB + (B >> 4));
                 const uint32_t slot = atomicAdd(&nq, 1u);
                 if (slot < uint32_t(kGQ2)) gq[slot] = make_uint2(nA, nB);
                 else gunion2d(im, w, nA, nB);
@@ -814,7 +818,8 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         __syncthreads();
         const uint4 *HR = H + kHdr / 4 - NWORD;   // run words
         // The last B run is the last run.
-        const uint32_t nrun = (HR[NWORD - 1].w >> 16) + (CELL == 2 ? __popc(HR[NWORD - 1].y) : 0);
+        uint32_t nrun = (HR[NWORD - 1].w >> 16) + (CELL == 2 ? __popc(HR[NWORD - 1].y) : 0);
+        if (!GUARD(w, nrun <= uint32_t(MAXRUN), 404, nrun)) nrun = MAXRUN;
 
         // Surviving roots: rank = roots before it in its segment.  One thread per word and kind of run:
         // WPR consecutive lanes hold a segment's words, a shuffle scan gives each word's prefix, and the
@@ -834,6 +839,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             }
             uint32_t label = 1u + segb[seg] + pre - __popc(bits);
             while (bits) {
+                if (!GUARD(w, b + __ffs(bits) <= uint32_t(MAXRUN), 401, b)) break;
                 LT[b + __ffs(bits)] = label++;   // run i's place is i + 1
                 bits &= bits - 1;
             }
@@ -845,7 +851,9 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
             const unsigned long long e = __ldcg(w.gp + node);   // its root's own entry (flatten_tile_nodes)
             const uint32_t g = uint32_t(e), kg = uint32_t(e >> 32);
             if (g == uint32_t(node)) continue;
-            const uint32_t sg = kg / seg_width(im), run = __ldcg(w.nroot + g);
+            const uint32_t sg = kg / seg_width(im);
+            if (!GUARD(w, g < w.n_tiles * MAXB && sg < uint32_t(im.rows) * uint32_t(im.tiles_x), 402, e)) continue;
+            const uint32_t run = __ldcg(w.nroot + g);
             const uint32_t rank = count_bits(w.rbits + int64_t(g / MAXB) * RBWORDS, run - (kg - sg * seg_width(im)), run);
             const uint32_t sb = w.segpref[im.seg_base + sg] - base0;
             LT[__ldcg(w.nroot + node) + 1u] = 1u + sb + rank;
@@ -856,6 +864,7 @@ __global__ void __launch_bounds__(K3_NT, K3_PER_SM) k_tile_write_2d(ImgList2D L,
         for (uint32_t i = 2 * tid; i < nrun; i += 2 * K3_NT) {
             const uint32_t e = i < uint32_t(kStageRuns) ? E[i >> 1] : __ldcg(lab + t * kLabWords + kHdr + (i >> 1));
             const uint32_t a = e & 0xFFFFu, b = e >> 16;
+            if (!GUARD(w, a < nrun && (i + 1 >= nrun || b < nrun), 403, e)) continue;
             if (a != i) LT[i + 1] = LT[a + 1];
             if (i + 1 < nrun && b != i + 1) LT[i + 2] = LT[b + 1];
         }

@@ -534,8 +534,7 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
                 first &= first - 1;
                 uint32_t own, up;
                 take(nr, uw.x, ub, b, own, up);
-                (void)GUARD(w, own < nrun && up < own, 101, (uint64_t(own) << 32) | up);
-                P[own & (NBLK - 1)] = up & (NBLK - 1);
+                if (GUARD(w, own < nrun && up < own, 101, (uint64_t(own) << 32) | up)) P[own & (NBLK - 1)] = up & (NBLK - 1);
             }
         }
         for (uint32_t ss = rem; ss; ss &= ss - 1) {
@@ -561,7 +560,7 @@ __global__ void __launch_bounds__(NT1, kT3LocalPerSM) k_tile_local_3d(ImgList3D 
                     if (!b) break;
                     uint32_t own, up;
                     take(nr, uw.x, ub, b - 1u, own, up);
-                    MQ[pos - lo] = (own << 16) | up;
+                    MQ[pos - lo] = GUARD(w, own < nrun && up < own, 103, (uint64_t(own) << 32) | up) ? (own << 16) | up : 0u;
                     ++pos;
                 }
             }
@@ -737,7 +736,8 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
             return 4 * (o0 + 1) + (o1 + 1);
         };
         auto tile_at = [&](int code, int o2) -> int64_t {
-            return t + (int64_t((code >> 2) - 1) * im.t1 + (code & 3) - 1) * im.t2 + o2;
+            const int64_t tt = t + (int64_t((code >> 2) - 1) * im.t1 + (code & 3) - 1) * im.t2 + o2;
+            return GUARD(w, tt >= im.tile_base && tt < w.n_tiles, 201, tt) ? tt : t;
         };
         constexpr int kOwn = 5;   // code of the row's own tile
         // Links to rows of other tiles: warp 0 straight below (the rows of the first layer), warp 1 below
@@ -872,6 +872,7 @@ __global__ void __launch_bounds__(kT3MergeThreads, kT3MergePerSM) k_merge_3d(Img
                     a = e & 0x7FFu;
                     b = (e >> 11) & 0x7FFu;
                 } else {
+                    if (!GUARD(w, (e & 0xFFFu) < uint32_t(NBLK) && ((e >> 12) & 0xFFFu) < uint32_t(NBLK), 203, e)) continue;
                     a = __ldcg(w.perim + t * T3_EDGE + (e & 0xFFFu));
                     b = __ldcg(w.perim + tt * T3_EDGE + ((e >> 12) & 0xFFFu));
                 }
@@ -1030,6 +1031,7 @@ __global__ void __launch_bounds__(NT, kT3WritePerSM) k_tile_write_3d(ImgList3D L
             uint32_t label = 1u + segb[(2 * (row / TB1) + (ij >> 1)) * TY + 2 * (row % TB1) + (ij & 1)] - base0;
             while (bits) {
                 const uint32_t bit = bits & (0u - bits);
+                if (!GUARD(w, rw.y + __popc(rw.x) <= uint32_t(NBLK), 401, rw.y)) break;
                 LT[rw.y + __popc(rw.x & (bit | (bit - 1u)))] = label++;
                 bits &= bits - 1;
             }
