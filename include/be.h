@@ -52,12 +52,17 @@ enum {
                           635-734): 2D 4-connectivity for BE_COH_4 / BE_COH_DEFAULT (the reference's
                           default), 8 for BE_COH_8; 3D 26-connectivity.  The components of the
                           reference's scan / analyze loop over pixels, found by union-find over
-                          pixel runs (4) or blocks (8, 26) */
+                          pixel runs (4) or blocks (8, 26).  Scratch: about 2.2 bytes a pixel, in whole
+                          tiles (64 x 128 pixels, 16 x 32 x 64 voxels); images of at most about four rows
+                          or columns (or that thin volumes) whose tiles would take more than 512 MiB, and
+                          calls whose tiles' scratch cannot be allocated, run the scan / analyze loop
+                          itself, in 4 to 10 bytes a pixel */
     BE_ALGO_RUNS = 4   /* 2D run equivalence, the -a runeq -g path (TOCLRunEquivLabeling,
                           LabelingAlgs.cpp:1090-1268, RE* kernels LabelingAlgs.cl:325-616): runs of
                           each row joined by column overlap -- 4-connectivity for BE_COH_4 /
                           BE_COH_DEFAULT (the reference's runs), 8 for BE_COH_8; 2D only.  Resolved by
-                          union-find over the runs of a tile and the nodes between tiles */
+                          union-find over the runs of a tile and the nodes between tiles; thin images as
+                          BE_ALGO_PIXEL */
 };
 
 /* Connectivity selector, as the reference's TCoherence (LabelingTools.hpp:45-50). */

@@ -37,15 +37,6 @@ int cuda_error(be_ctx *ctx, cudaError_t e, const char *what)
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Where a form's component count is: the iterative form has its own workspace (and its error flag in
-// iter_err), the pixel and run forms theirs.
-static const int64_t *count_of(const be_ctx *c, int algo, int dims)
-{
-    if (algo == BE_ALGO_ITER) return c->wsiter.w.ncomp;
-    if (algo == BE_ALGO_PIXEL || algo == BE_ALGO_RUNS) return dims == 2 ? c->wsform2d.w.ncomp : c->wsform3d.w.ncomp;
-    return dims == 2 ? c->ws2d.w.ncomp : c->ws3d.w.ncomp;
-}
-
 // The smallest power of two not below v, as a shift.
 static int ceil_log2(int v)
 {
@@ -149,11 +140,17 @@ int Workspace::ensure(be_ctx *ctx, const Geometry &g, int64_t n_tiles, int64_t n
             if (e != cudaSuccess) return cuda_error(ctx, e, "cudaFree(workspace)");
         }
         const size_t need = layout_work(g, n_tiles, n_segs, n_imgs, nullptr, nullptr);
-        const size_t body = need + need / 4;   // headroom for slightly larger later calls
+        size_t body = need + need / 4;   // headroom for slightly larger later calls
+        cudaError_t e = cudaMalloc(&base, head_bytes(max_chunks(body)) + body);
+        if (e == cudaErrorMemoryAllocation) {   // without it
+            cudaGetLastError();
+            body = need;
+            e = cudaMalloc(&base, head_bytes(max_chunks(body)) + body);
+        }
         const size_t head = head_bytes(max_chunks(body));
-        cudaError_t e = cudaMalloc(&base, head + body);
         if (e != cudaSuccess) {
             base = nullptr;
+            cudaGetLastError();
             return cuda_error(ctx, e, "cudaMalloc(workspace)");
         }
         // The scan's status words and the launch epoch start at zero once; every later run tells
@@ -216,6 +213,77 @@ void fill_img3d(Img3D &im, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2
     im.seg_base = seg_base;
     im.thr = thr;
     im.index = index;
+}
+
+// Whether the pixel and run forms leave an image of n pixels to the iterative forms, which give the same
+// labels with about 4.5 bytes of scratch a pixel: the tile pipeline's is a fixed 17 KB a tile, whatever part
+// of the tile the image fills.  Images of up to four rows or columns take more than 32 bytes a pixel so; where
+// that comes to more than half a gigabyte, it is not taken.  Measured, 4-connected, by tiles / iterative: 1 x 2^25
+// pixels, half of them set, 3404 us and 5.4 GB / 1402 us and 0.17 GB, nearly all set 3501 / 5766 us; 2^23 x 1
+// 2813 us and 2.8 GB / 345 us and 0.04 GB, nearly all set 3057 / 1490 us; but 8 x 2^22 617 us and 0.7 GB / 2992
+// us and 0.17 GB.
+constexpr size_t kThinBytes = size_t(1) << 29;
+static bool tiles_nearly_empty(size_t bytes, int64_t n) { return bytes > kThinBytes && bytes > 32 * size_t(n); }
+
+// The tile pipeline on one image, in the context's workspace of the block form or of the others.
+// BE_ERR_OOM when there is no memory for its scratch, or `form` has a better use for it.
+static int run_tiles2d(be_ctx *c, bool form, int shape, const Img2D &im, bool count, cudaStream_t s)
+{
+    const Geometry g = uf2d_geometry(shape);
+    const int64_t n_tiles = int64_t(im.tiles_x) * im.tiles_y, n_segs = int64_t(im.rows) * im.tiles_x;
+    if (form && tiles_nearly_empty(layout_work(g, n_tiles, n_segs, 1, nullptr, nullptr), int64_t(im.rows) * im.cols)) return BE_ERR_OOM;
+    Workspace &ws = form ? c->wsform2d : c->ws2d;
+    c->last_ws[0] = &ws;
+    int rc = ws.ensure(c, g, n_tiles, n_segs, 1);
+    if (rc) return rc;
+    ImgList2D L{nullptr, 1, im};
+#ifdef BE_BOUNDS_CHECK
+    cudaMemsetAsync(ws.w.err, 0, 16 * sizeof(uint32_t), s);
+#endif
+    const bool timed = c->timing && !form;
+    Work w = ws.w;
+    w.host_count = count ? c->h_ncomp : nullptr;   // the count straight to the host, no copy after
+    const cudaError_t e = uf2d_launch(shape, L, w, c->sms, false, s, timed ? c->stage_ev : nullptr);
+    c->timed_stages = timed ? kStages2D : 0;
+    c->last_ncomp = ws.w.ncomp;
+    return e == cudaSuccess ? BE_OK : cuda_error(c, e, "be_label2d launch");
+}
+
+static int run_tiles3d(be_ctx *c, bool form, const Img3D &im, bool count, cudaStream_t s)
+{
+    const Geometry g = geometry_3d();
+    const int64_t n_tiles = int64_t(im.t0) * im.t1 * im.t2, n_segs = int64_t(im.d0) * im.d1 * im.t2;
+    if (form && tiles_nearly_empty(layout_work(g, n_tiles, n_segs, 1, nullptr, nullptr), int64_t(im.d0) * im.d1 * im.d2)) return BE_ERR_OOM;
+    Workspace &ws = form ? c->wsform3d : c->ws3d;
+    c->last_ws[1] = &ws;
+    int rc = ws.ensure(c, g, n_tiles, n_segs, 1);
+    if (rc) return rc;
+    ImgList3D L{nullptr, 1, im};
+#ifdef BE_BOUNDS_CHECK
+    cudaMemsetAsync(ws.w.err, 0, 16 * sizeof(uint32_t), s);
+#endif
+    const bool timed = c->timing && !form;
+    Work w = ws.w;
+    w.host_count = count ? c->h_ncomp : nullptr;   // as in 2D
+    const cudaError_t e = launch_uf3d(L, w, c->sms, false, s, timed ? c->stage_ev : nullptr);
+    c->timed_stages = timed ? kStages3D : 0;
+    c->last_ncomp = ws.w.ncomp;
+    return e == cudaSuccess ? BE_OK : cuda_error(c, e, "be_label3d launch");
+}
+
+// The end of a label call: notes what ran and, where the caller wants the count, waits for it.
+static int finish_label(be_ctx *c, bool iter, int64_t *n_components, const char *what, cudaStream_t s)
+{
+    c->last_iter = iter;
+    if (iter) c->last_ncomp = c->wsiter.w.ncomp;
+    if (!n_components) return BE_OK;
+    cudaError_t e = cudaSuccess;
+    if (iter) e = cudaMemcpyAsync(c->h_ncomp, c->last_ncomp, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_error(c, e, what);
+    if (iter && c->iter_err && *c->iter_err) return set_error(c, BE_ERR_NO_CONVERGENCE, "%s: iteration cap reached", what);
+    *n_components = c->h_ncomp[0];
+    return BE_OK;
 }
 
 }  // namespace be
@@ -341,52 +409,33 @@ int be_label2d(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int
     cudaError_t e = cudaSetDevice(c->device);
     if (e != cudaSuccess) return cuda_error(c, e, "cudaSetDevice");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int rc, shape;
+    int rc = BE_OK, shape;
     pick2d(c, rows, cols, algo, &algo, &shape);
-    c->last_algo = algo;
     const bool form = algo == BE_ALGO_PIXEL || algo == BE_ALGO_RUNS;
-    if (algo == BE_ALGO_ITER) {
-        rc = run_iter2d(c, in, in_pitch, rows, cols, threshold, out, out_pitch, s);
-    } else {
-        if (form) {
-            // The pixel and run forms give the components of their connectivity in canonical order: 4
-            // by the pipeline on pixel runs, 8 by the block pipeline.  (Sizes as their own key space --
-            // rows of a power of two -- takes them.)
-            if ((int64_t(rows) << ceil_log2(cols)) >= (int64_t(1) << 31))
-                return set_error(c, BE_ERR_INVALID, algo == BE_ALGO_PIXEL ? "label equivalence: %d x %d exceeds its key space"
-                                                                          : "run equivalence: %d x %d exceeds its key space", rows, cols);
-            shape = coh == BE_COH_8 ? 0 : kShapePixel2D;
-        }
-        Workspace &ws = form ? c->wsform2d : c->ws2d;
+    bool iter = algo == BE_ALGO_ITER;
+    if (form) {
+        // The pixel and run forms give the components of their connectivity in canonical order: 4
+        // by the pipeline on pixel runs, 8 by the block pipeline.  (Sizes as their own key space --
+        // rows of a power of two -- takes them.)
+        if ((int64_t(rows) << ceil_log2(cols)) >= (int64_t(1) << 31))
+            return set_error(c, BE_ERR_INVALID, algo == BE_ALGO_PIXEL ? "label equivalence: %d x %d exceeds its key space"
+                                                                      : "run equivalence: %d x %d exceeds its key space", rows, cols);
+        shape = coh == BE_COH_8 ? 0 : kShapePixel2D;
+    }
+    if (!iter) {
         Img2D im;
         fill_img2d(im, in, in_pitch, rows, cols, threshold, out, out_pitch, 0, 0, 0, shape);
-        const int64_t n_tiles = int64_t(im.tiles_x) * im.tiles_y;
-        const int64_t n_segs = int64_t(rows) * im.tiles_x;
-        c->last_ws[0] = &ws;
-        rc = ws.ensure(c, uf2d_geometry(shape), n_tiles, n_segs, 1);
+        rc = run_tiles2d(c, form, shape, im, n_components != nullptr, s);
+        if (rc && !(form && rc == BE_ERR_OOM)) return rc;
+        iter = rc != BE_OK;   // scratch refused: the same components with less of it
+    }
+    if (iter) {
+        c->err.clear();
+        rc = form && coh != BE_COH_8 ? run_lbeq2d(c, in, in_pitch, rows, cols, threshold, out, out_pitch, s)
+                                     : run_iter2d(c, in, in_pitch, rows, cols, threshold, out, out_pitch, s);
         if (rc) return rc;
-        ImgList2D L{nullptr, 1, im};
-#ifdef BE_BOUNDS_CHECK
-        cudaMemsetAsync(ws.w.err, 0, 16 * sizeof(uint32_t), s);
-#endif
-        const bool timed = c->timing && !form;
-        Work w = ws.w;
-        w.host_count = n_components ? c->h_ncomp : nullptr;   // the count straight to the host, no copy after
-        e = uf2d_launch(shape, L, w, c->sms, false, s, timed ? c->stage_ev : nullptr);
-        c->timed_stages = timed ? kStages2D : 0;
-        if (e != cudaSuccess) return cuda_error(c, e, "be_label2d launch");
     }
-    if (rc) return rc;
-    if (n_components) {
-        if (algo == BE_ALGO_ITER)
-            e = cudaMemcpyAsync(c->h_ncomp, count_of(c, algo, 2), sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return cuda_error(c, e, "be_label2d sync");
-        if (algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
-            return set_error(c, BE_ERR_NO_CONVERGENCE, "be_label2d: iteration cap reached");
-        *n_components = c->h_ncomp[0];
-    }
-    return BE_OK;
+    return finish_label(c, iter, n_components, "be_label2d", s);
 }
 
 int be_label3d(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2, int threshold,
@@ -405,45 +454,25 @@ int be_label3d(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2,
     cudaError_t e = cudaSetDevice(c->device);
     if (e != cudaSuccess) return cuda_error(c, e, "cudaSetDevice");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int rc;
+    int rc = BE_OK;
     pick3d(c, int64_t(d0) * d1 * d2, algo, &algo);
-    c->last_algo = algo;
     const bool form = algo == BE_ALGO_PIXEL;
-    if (algo == BE_ALGO_ITER) {
-        rc = run_iter3d(c, in, d0, d1, d2, threshold, out, s);
-    } else {
-        if (form && (int64_t(d0) << (ceil_log2(d1) + ceil_log2(d2))) >= (int64_t(1) << 31))   // as in 2D
-            return set_error(c, BE_ERR_INVALID, "label equivalence: volume exceeds its key space");
-        Workspace &ws = form ? c->wsform3d : c->ws3d;
+    bool iter = algo == BE_ALGO_ITER;
+    if (form && (int64_t(d0) << (ceil_log2(d1) + ceil_log2(d2))) >= (int64_t(1) << 31))   // as in 2D
+        return set_error(c, BE_ERR_INVALID, "label equivalence: volume exceeds its key space");
+    if (!iter) {
         Img3D im;
         fill_img3d(im, in, d0, d1, d2, threshold, out, 0, 0, 0);
-        const int64_t n_tiles = int64_t(im.t0) * im.t1 * im.t2;
-        const int64_t n_segs = int64_t(d0) * d1 * im.t2;
-        c->last_ws[1] = &ws;
-        rc = ws.ensure(c, geometry_3d(), n_tiles, n_segs, 1);
+        rc = run_tiles3d(c, form, im, n_components != nullptr, s);
+        if (rc && !(form && rc == BE_ERR_OOM)) return rc;
+        iter = rc != BE_OK;   // as in 2D
+    }
+    if (iter) {
+        c->err.clear();
+        rc = run_iter3d(c, in, d0, d1, d2, threshold, out, s);
         if (rc) return rc;
-        ImgList3D L{nullptr, 1, im};
-#ifdef BE_BOUNDS_CHECK
-        cudaMemsetAsync(ws.w.err, 0, 16 * sizeof(uint32_t), s);
-#endif
-        const bool timed = c->timing && !form;
-        Work w = ws.w;
-        w.host_count = n_components ? c->h_ncomp : nullptr;   // as in 2D
-        e = launch_uf3d(L, w, c->sms, false, s, timed ? c->stage_ev : nullptr);
-        c->timed_stages = timed ? kStages3D : 0;
-        if (e != cudaSuccess) return cuda_error(c, e, "be_label3d launch");
     }
-    if (rc) return rc;
-    if (n_components) {
-        if (algo == BE_ALGO_ITER)
-            e = cudaMemcpyAsync(c->h_ncomp, count_of(c, algo, 3), sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return cuda_error(c, e, "be_label3d sync");
-        if (algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
-            return set_error(c, BE_ERR_NO_CONVERGENCE, "be_label3d: iteration cap reached");
-        *n_components = c->h_ncomp[0];
-    }
-    return BE_OK;
+    return finish_label(c, iter, n_components, "be_label3d", s);
 }
 
 static int ensure_staging(be_ctx *c, size_t in_bytes, size_t out_bytes)
@@ -501,11 +530,10 @@ int be_label2d_host(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows
                           : cudaMemcpy2DAsync(out, out_pitch * sizeof(int32_t), c->d_out, dpo * sizeof(int32_t),
                                               cols * sizeof(int32_t), rows, cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return cuda_error(c, e, "download");
-    const int64_t *src = count_of(c, c->last_algo, 2);
-    e = cudaMemcpyAsync(c->h_ncomp, src, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(c->h_ncomp, c->last_ncomp, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_error(c, e, "be_label2d_host sync");
-    if (c->last_algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
+    if (c->last_iter && c->iter_err && *c->iter_err)
         return set_error(c, BE_ERR_NO_CONVERGENCE, "be_label2d_host: iteration cap reached");
     n = c->h_ncomp[0];
     if (n_components) *n_components = n;
@@ -541,11 +569,10 @@ int be_label3d_host(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_
     cudaEventRecord(c->ev1, s);
     e = cudaMemcpyAsync(out, c->d_out, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return cuda_error(c, e, "download");
-    const int64_t *src = count_of(c, c->last_algo, 3);
-    e = cudaMemcpyAsync(c->h_ncomp, src, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(c->h_ncomp, c->last_ncomp, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_error(c, e, "be_label3d_host sync");
-    if (c->last_algo == BE_ALGO_ITER && c->iter_err && *c->iter_err)
+    if (c->last_iter && c->iter_err && *c->iter_err)
         return set_error(c, BE_ERR_NO_CONVERGENCE, "be_label3d_host: iteration cap reached");
     if (n_components) *n_components = c->h_ncomp[0];
     if (elapsed_us) {

@@ -88,6 +88,9 @@ cudaError_t launch_uf3d(const ImgList3D &L, const Work &w, int sms, bool persist
 
 int run_iter2d(struct ::be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int32_t cols,
                int thr, int32_t *out, int64_t out_pitch, cudaStream_t s);
+// 4-connectivity, on pixels (BE_ALGO_PIXEL and BE_ALGO_RUNS where tiles would be nearly empty).
+int run_lbeq2d(struct ::be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int32_t cols, int thr,
+               int32_t *out, int64_t out_pitch, cudaStream_t s);
 int run_iter3d(struct ::be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2, int thr,
                int32_t *out, cudaStream_t s);
 
@@ -122,6 +125,7 @@ struct be_ctx {
     int timed_stages = 0;
     cudaEvent_t stage_ev[be::kStages + 1] = {};
     std::vector<be::TuneEntry> tune;  // autotuner decisions
-    int last_algo = 1;                // algorithm the last label call actually ran
-    be_iter_graph iter_graph[2];      // iterative form: 2D / 3D blocks
+    bool last_iter = false;                // whether the last label call ran in the iterative graph
+    const int64_t *last_ncomp = nullptr;   // its component count on the device
+    be_iter_graph iter_graph[3];      // iterative form: 2D / 3D blocks, 2D pixels
 };

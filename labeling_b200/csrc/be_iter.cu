@@ -332,6 +332,94 @@ __global__ void it_ncomp(Work w, const uint32_t *ctl, uint32_t *err_out)
     *err_out = ctl[2];
 }
 
+// ---- 4-connected pixels -------------------------------------------------------------------------
+// The reference's DistrInit / Scan / Analize (LabelingAlgs.cl:31-130): every foreground pixel starts with
+// its own label, and the loop of the block form runs on pixels.  For images whose tiles would be nearly
+// empty (one row, one column): the tile pipeline's scratch is a fixed 17 KB per 64 x 128 pixels, this form's
+// about 4.5 bytes a pixel.
+struct Lq2 {
+    const uint8_t *in;
+    int64_t pitch;
+    int32_t *out;
+    int64_t opitch;
+    int rows, cols, sx, thr;
+    uint32_t *lab;
+    uint32_t *rbits;
+    uint32_t *ctl;
+    Work w;
+};
+
+__device__ __forceinline__ int64_t lq_pix2(const Lq2 &g, uint32_t key)
+{
+    return int64_t(key >> g.sx) * g.cols + (key & ((1u << g.sx) - 1u));
+}
+
+__global__ void __launch_bounds__(NT) lq_init_2d(Lq2 g)
+{
+    const int64_t p = int64_t(blockIdx.x) * NT + threadIdx.x;
+    if (p >= int64_t(g.rows) * g.cols) return;
+    const int y = int(p / g.cols), x = int(p - int64_t(y) * g.cols);
+    g.lab[p] = g.in[int64_t(y) * g.pitch + x] > g.thr ? ((uint32_t(y) << g.sx) | uint32_t(x)) + 1u : 0u;
+}
+
+__global__ void __launch_bounds__(NT) lq_scan_2d(Lq2 g)
+{
+    const int64_t p = int64_t(blockIdx.x) * NT + threadIdx.x;
+    if (p >= int64_t(g.rows) * g.cols) return;
+    const uint32_t label = g.lab[p];
+    if (!label) return;
+    const int y = int(p / g.cols), x = int(p - int64_t(y) * g.cols);
+    // The smallest label beside: 0 (background, or outside) wraps to the largest.
+    uint32_t m = (x > 0 ? g.lab[p - 1] : 0u) - 1u;
+    m = min(m, (x + 1 < g.cols ? g.lab[p + 1] : 0u) - 1u);
+    m = min(m, (y > 0 ? g.lab[p - g.cols] : 0u) - 1u);
+    m = min(m, (y + 1 < g.rows ? g.lab[p + g.cols] : 0u) - 1u) + 1u;
+    if (!m) return;
+    if (m < label) {
+        atomicMin(&g.lab[lq_pix2(g, label - 1)], m);
+        g.ctl[0] = 1;
+    }
+}
+
+__global__ void __launch_bounds__(NT) lq_analyze_2d(Lq2 g)
+{
+    const int64_t p = int64_t(blockIdx.x) * NT + threadIdx.x;
+    if (p >= int64_t(g.rows) * g.cols) return;
+    uint32_t label = g.lab[p];
+    if (!label) return;
+    for (int step = 0;; ++step) {
+        const uint32_t nxt = g.lab[lq_pix2(g, label - 1)];
+        if (nxt == label) break;
+        if (step == kChaseCap) { g.ctl[2] = 1; break; }
+        label = nxt;
+    }
+    g.lab[p] = label;
+}
+
+__global__ void __launch_bounds__(NT) lq_mark_2d(Lq2 g)
+{
+    const int64_t p = int64_t(blockIdx.x) * NT + threadIdx.x;
+    if (p >= int64_t(g.rows) * g.cols) return;
+    const uint32_t label = g.lab[p];
+    if (!label || lq_pix2(g, label - 1) != p) return;
+    const uint32_t k = label - 1;
+    atomicOr(&g.rbits[k >> 5], 1u << (k & 31));
+}
+
+__global__ void __launch_bounds__(NT) lq_final_2d(Lq2 g)
+{
+    const int64_t p = int64_t(blockIdx.x) * NT + threadIdx.x;
+    if (p >= int64_t(g.rows) * g.cols) return;
+    const int y = int(p / g.cols), x = int(p - int64_t(y) * g.cols);
+    const uint32_t label = g.lab[p];
+    int32_t l = 0;
+    if (label) {
+        const uint32_t k = label - 1;
+        l = int32_t(1u + g.w.segpref[k >> 5] + __popc(g.rbits[k >> 5] & ((1u << (k & 31)) - 1u)));
+    }
+    g.out[int64_t(y) * g.opitch + x] = l;
+}
+
 unsigned nblk(int64_t n) { return unsigned((n + NT - 1) / NT); }
 
 int ceil_log2(int v)
@@ -388,6 +476,7 @@ int iter_scratch(be_ctx *c, int64_t nblocks, size_t conn_bytes, int64_t nwords, 
 // blanked for the graph cache's key.
 void blank_io(It2 &g) { g.in = nullptr; g.out = nullptr; g.pitch = g.opitch = 0; g.thr = 0; }
 void blank_io(It3 &g) { g.in = nullptr; g.out = nullptr; g.thr = 0; }
+void blank_io(Lq2 &g) { g.in = nullptr; g.out = nullptr; g.pitch = g.opitch = 0; g.thr = 0; }
 
 template <class G>
 cudaError_t set_kernel_args(cudaGraphExec_t exec, cudaGraphNode_t node, void *fn, unsigned grid, G &g)
@@ -402,7 +491,7 @@ cudaError_t set_kernel_args(cudaGraphExec_t exec, cudaGraphNode_t node, void *fn
     return cudaGraphExecKernelNodeSetParams(exec, node, &p);
 }
 
-// Builds and launches the graph: memsets, init, conn, WHILE{scan, analyze, cond}, mark, count,
+// Builds and launches the graph: memsets, init, conn (may be null), WHILE{scan, analyze, cond}, mark, count,
 // chunk sums, segment scan, final, count/flag copy-out.  The instantiated graph is kept in the
 // context (one per form) and launched again, with only the init and final nodes' arguments
 // updated, while the sizes and scratch buffers stay the same.
@@ -460,7 +549,7 @@ int run_graph(be_ctx *c, int kind, G g, int64_t nblocks, int64_t nfinal, int64_t
     }
     if (e == cudaSuccess) e = chain(add_kernel(graph, &n, prev, f_init, nblk(nblocks), NT, g));
     if (e == cudaSuccess) n_init = n;
-    if (e == cudaSuccess) e = chain(add_kernel(graph, &n, prev, f_conn, nblk(nblocks), NT, g));
+    if (e == cudaSuccess && f_conn) e = chain(add_kernel(graph, &n, prev, f_conn, nblk(nblocks), NT, g));
     cudaGraphConditionalHandle h;
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault);
     if (e == cudaSuccess) {
@@ -566,6 +655,31 @@ int run_iter3d(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2,
     g.w.queue = nullptr;
     return run_graph(c, 1, g, nblocks, int64_t(d0) * d1 * d2, nwords, it_init_3d, it_conn_3d, it_scan_3d,
                      it_analyze_3d, it_mark_3d, it_final_3d, s);
+}
+
+int run_lbeq2d(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int32_t cols, int thr,
+               int32_t *out, int64_t out_pitch, cudaStream_t s)
+{
+    Lq2 g{};
+    g.in = in; g.pitch = in_pitch; g.out = out; g.opitch = out_pitch;
+    g.rows = rows; g.cols = cols; g.thr = thr;
+    g.sx = ceil_log2(cols);
+    const int64_t keyspace = int64_t(rows) << g.sx;
+    if (keyspace >= (int64_t(1) << 31))
+        return set_error(c, BE_ERR_INVALID, "label equivalence: %d x %d exceeds its key space", rows, cols);
+    const int64_t n = int64_t(rows) * cols, nwords = (keyspace + 31) / 32;
+    char *lab, *mk, *conn, *rb, *ctl;
+    int rc = iter_scratch(c, n, 0, nwords, &lab, &mk, &conn, &rb, &ctl);
+    if (rc) return rc;
+    rc = c->wsiter.ensure(c, geometry_2d(), 0, nwords, 1);
+    if (rc) return rc;
+    g.lab = reinterpret_cast<uint32_t *>(lab); g.rbits = reinterpret_cast<uint32_t *>(rb);
+    g.ctl = reinterpret_cast<uint32_t *>(ctl);
+    g.w = c->wsiter.w;
+    g.w.n_tiles = 0;
+    g.w.queue = nullptr;
+    return run_graph(c, 2, g, n, n, nwords, lq_init_2d, (void (*)(Lq2)) nullptr, lq_scan_2d, lq_analyze_2d,
+                     lq_mark_2d, lq_final_2d, s);
 }
 
 }  // namespace be
