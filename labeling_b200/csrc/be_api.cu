@@ -37,14 +37,6 @@ int cuda_error(be_ctx *ctx, cudaError_t e, const char *what)
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// The smallest power of two not below v, as a shift.
-static int ceil_log2(int v)
-{
-    int s = 0;
-    while ((1 << s) < v) ++s;
-    return s;
-}
-
 Geometry geometry_2d() { return uf2d_geometry(0); }
 
 Geometry geometry_3d()

@@ -34,6 +34,14 @@ Geometry uf2d_geometry(int shape);
 cudaError_t uf2d_launch(int shape, const ImgList2D &L, const Work &w, int sms, bool persistent,
                         cudaStream_t s, cudaEvent_t *ev = nullptr);
 
+// The smallest power of two not below v (any positive int), as a shift.
+inline int ceil_log2(int v)
+{
+    int s = 0;
+    while ((int64_t(1) << s) < v) ++s;
+    return s;
+}
+
 Geometry geometry_2d();   // shape 0
 Geometry geometry_3d();
 size_t head_bytes(int64_t chunks);      // size of a workspace's head that holds this many scan chunks

@@ -422,13 +422,6 @@ __global__ void __launch_bounds__(NT) lq_final_2d(Lq2 g)
 
 unsigned nblk(int64_t n) { return unsigned((n + NT - 1) / NT); }
 
-int ceil_log2(int v)
-{
-    int s = 0;
-    while ((1 << s) < v) ++s;
-    return s;
-}
-
 // Adds a kernel node with the given arguments to `graph` after `dep` (may be null).
 template <class... A>
 cudaError_t add_kernel(cudaGraph_t graph, cudaGraphNode_t *node, cudaGraphNode_t dep, void (*fn)(A...),
