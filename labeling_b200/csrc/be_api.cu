@@ -120,7 +120,7 @@ cudaError_t reset_scan_state(const Work &w, cudaStream_t s)
     return e;
 }
 
-int Workspace::ensure(be_ctx *ctx, const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs)
+int Workspace::ensure(be_ctx *ctx, const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs, cudaStream_t s)
 {
     // Node links name a segment in 32 bits.
     if (n_segs >= int64_t(kNone)) return set_error(ctx, BE_ERR_TOO_LARGE, "more than 2^32 - 2 image rows in one launch");
@@ -146,9 +146,10 @@ int Workspace::ensure(be_ctx *ctx, const Geometry &g, int64_t n_tiles, int64_t n
             return cuda_error(ctx, e, "cudaMalloc(workspace)");
         }
         // The scan's status words and the launch epoch start at zero once; every later run tells
-        // its own status words from older ones by the epoch it increments.
-        e = cudaMemset(base, 0, head);
-        if (e != cudaSuccess) return cuda_error(ctx, e, "cudaMemset(workspace)");
+        // its own status words from older ones by the epoch it increments.  (On the call's stream: a clear on the
+        // default stream does not hold up a non-blocking one, and could come after its first kernels.)
+        e = cudaMemsetAsync(base, 0, head, s);
+        if (e != cudaSuccess) return cuda_error(ctx, e, "cudaMemsetAsync(workspace)");
         bytes = head + body;
         cap_chunks = max_chunks(body);   // of any launch whose arrays fit beside the head
     }
@@ -226,7 +227,7 @@ static int run_tiles2d(be_ctx *c, bool form, int shape, const Img2D &im, bool co
     if (form && tiles_nearly_empty(layout_work(g, n_tiles, n_segs, 1, nullptr, nullptr), int64_t(im.rows) * im.cols)) return BE_ERR_OOM;
     Workspace &ws = form ? c->wsform2d : c->ws2d;
     c->last_ws[0] = &ws;
-    int rc = ws.ensure(c, g, n_tiles, n_segs, 1);
+    int rc = ws.ensure(c, g, n_tiles, n_segs, 1, s);
     if (rc) return rc;
     ImgList2D L{nullptr, 1, im};
 #ifdef BE_BOUNDS_CHECK
@@ -248,7 +249,7 @@ static int run_tiles3d(be_ctx *c, bool form, const Img3D &im, bool count, cudaSt
     if (form && tiles_nearly_empty(layout_work(g, n_tiles, n_segs, 1, nullptr, nullptr), int64_t(im.d0) * im.d1 * im.d2)) return BE_ERR_OOM;
     Workspace &ws = form ? c->wsform3d : c->ws3d;
     c->last_ws[1] = &ws;
-    int rc = ws.ensure(c, g, n_tiles, n_segs, 1);
+    int rc = ws.ensure(c, g, n_tiles, n_segs, 1, s);
     if (rc) return rc;
     ImgList3D L{nullptr, 1, im};
 #ifdef BE_BOUNDS_CHECK

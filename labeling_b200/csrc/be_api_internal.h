@@ -60,7 +60,7 @@ struct Workspace {
     int64_t cap_tiles = 0, cap_segs = 0;
     int cap_imgs = 0;
     Work w{};
-    int ensure(struct ::be_ctx *ctx, const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs);
+    int ensure(struct ::be_ctx *ctx, const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs, cudaStream_t s);
     void release();
 };
 

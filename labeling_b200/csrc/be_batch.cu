@@ -91,6 +91,7 @@ int build(be_batch *b)
     if (!d2.empty()) e = cudaMemcpy(base + o_d2, d2.data(), d2.size() * sizeof(Img2D), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !d3.empty())
         e = cudaMemcpy(base + o_d3, d3.data(), d3.size() * sizeof(Img3D), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // cleared and uploaded for any stream that runs the batch
     if (e != cudaSuccess) return cuda_error(c, e, "be_batch: descriptor upload");
     Work W2{}, W3{};
     if (!d2.empty()) {

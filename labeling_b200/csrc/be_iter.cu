@@ -612,7 +612,7 @@ int run_iter2d(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int
     char *lab, *mk, *conn, *rb, *ctl;
     int rc = iter_scratch(c, nblocks, 1, nwords, &lab, &mk, &conn, &rb, &ctl);
     if (rc) return rc;
-    rc = c->wsiter.ensure(c, geometry_2d(), 0, nwords, 1);
+    rc = c->wsiter.ensure(c, geometry_2d(), 0, nwords, 1, s);
     if (rc) return rc;
     g.lab = reinterpret_cast<uint32_t *>(lab); g.mk = reinterpret_cast<uint8_t *>(mk);
     g.conn = reinterpret_cast<uint8_t *>(conn); g.rbits = reinterpret_cast<uint32_t *>(rb);
@@ -638,7 +638,7 @@ int run_iter3d(be_ctx *c, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2,
     char *lab, *mk, *conn, *rb, *ctl;
     int rc = iter_scratch(c, nblocks, 4, nwords, &lab, &mk, &conn, &rb, &ctl);
     if (rc) return rc;
-    rc = c->wsiter.ensure(c, geometry_2d(), 0, nwords, 1);
+    rc = c->wsiter.ensure(c, geometry_2d(), 0, nwords, 1, s);
     if (rc) return rc;
     g.lab = reinterpret_cast<uint32_t *>(lab); g.mk = reinterpret_cast<uint8_t *>(mk);
     g.conn = reinterpret_cast<uint32_t *>(conn); g.rbits = reinterpret_cast<uint32_t *>(rb);
@@ -664,7 +664,7 @@ int run_lbeq2d(be_ctx *c, const uint8_t *in, int64_t in_pitch, int32_t rows, int
     char *lab, *mk, *conn, *rb, *ctl;
     int rc = iter_scratch(c, n, 0, nwords, &lab, &mk, &conn, &rb, &ctl);
     if (rc) return rc;
-    rc = c->wsiter.ensure(c, geometry_2d(), 0, nwords, 1);
+    rc = c->wsiter.ensure(c, geometry_2d(), 0, nwords, 1, s);
     if (rc) return rc;
     g.lab = reinterpret_cast<uint32_t *>(lab); g.rbits = reinterpret_cast<uint32_t *>(rb);
     g.ctl = reinterpret_cast<uint32_t *>(ctl);
