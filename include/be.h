@@ -40,7 +40,9 @@ typedef enum be_status {
     BE_ERR_BUSY = 6,           /* admission refused: not enough free device memory or slots */
     BE_ERR_CANCELLED = 7,      /* the request was cancelled before it completed */
     BE_ERR_TOO_LARGE = 8       /* the image exceeds the fixed scratch of be_label2d_noalloc, or one
-                                  launch holds more than 2^32 - 2 image rows (voxel rows) */
+                                  launch holds more than 2^32 - 2 image rows (voxel rows), or more tiles
+                                  than 32-bit ids of border components reach (2.4 million 3D tiles, 7.9
+                                  million 2D tiles of the widest shape) */
 } be_status;
 
 /* Merge algorithm. */

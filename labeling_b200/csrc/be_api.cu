@@ -122,6 +122,7 @@ cudaError_t reset_scan_state(const Work &w, cudaStream_t s)
 
 int Workspace::ensure(be_ctx *ctx, const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs, cudaStream_t s)
 {
+    if (!node_ids_fit(g, n_tiles)) return set_error(ctx, BE_ERR_TOO_LARGE, "more than 2^32 - 2 tile border components in one launch");
     // Node links name a segment in 32 bits.
     if (n_segs >= int64_t(kNone)) return set_error(ctx, BE_ERR_TOO_LARGE, "more than 2^32 - 2 image rows in one launch");
     if (!base || layout_work(g, n_tiles, n_segs, n_imgs, nullptr, nullptr, cap_chunks) > bytes) {

@@ -44,6 +44,8 @@ inline int ceil_log2(int v)
 
 Geometry geometry_2d();   // shape 0
 Geometry geometry_3d();
+// Whether a launch's node ids (tile * maxb + node) fit the 32 bits that the union-find entries give them.
+inline bool node_ids_fit(const Geometry &g, int64_t n_tiles) { return n_tiles * g.maxb < int64_t(kNone); }
 size_t head_bytes(int64_t chunks);      // size of a workspace's head that holds this many scan chunks
 int64_t max_chunks(size_t bytes);       // scan chunks of a launch whose arrays take at most this many bytes
 size_t layout_work(const Geometry &g, int64_t n_tiles, int64_t n_segs, int n_imgs, char *base, Work *w,

@@ -71,6 +71,7 @@ int build(be_batch *b)
         s3 += int64_t(im.dims[0]) * im.dims[1] * d3[i].t2;
     }
     const Geometry g2 = uf2d_geometry(b->shape), g3 = geometry_3d();
+    if (!node_ids_fit(g2, t2) || !node_ids_fit(g3, t3)) return set_error(c, BE_ERR_TOO_LARGE, "be_batch: too many tiles in one launch");
     const size_t w2 = d2.empty() ? 0 : layout_work(g2, t2, s2, b->n, nullptr, nullptr);
     const size_t w3 = d3.empty() ? 0 : layout_work(g3, t3, s3, b->n, nullptr, nullptr);
     const size_t o_d2 = 0, o_d3 = al256(d2.size() * sizeof(Img2D));

@@ -224,7 +224,8 @@ bool be_server::launch(Lane &ln, std::vector<Req *> &batch)
     const size_t o_w3 = o_w2 + al256(w2);
     const size_t total = o_w3 + al256(w3);
     int st = BE_OK;
-    ln.d_work = alloc(total, s, &st);
+    if (node_ids_fit(g2, t2) && node_ids_fit(g3, t3)) ln.d_work = alloc(total, s, &st);
+    else st = BE_ERR_TOO_LARGE;
     auto fail_all = [&](int code) {
         for (Req *q : ok) {
             q->status = code;
