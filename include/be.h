@@ -56,7 +56,7 @@ enum {
                           reference's scan / analyze loop over pixels, found by union-find over
                           pixel runs (4) or blocks (8, 26).  Scratch: about 2.2 bytes a pixel, in whole
                           tiles (64 x 128 pixels, 16 x 32 x 64 voxels); images of at most about four rows
-                          or columns (or that thin volumes) whose tiles would take more than 512 MiB, and
+                          or eight columns (or volumes that thin) whose tiles would take more than 512 MiB, and
                           calls whose tiles' scratch cannot be allocated, run the scan / analyze loop
                           itself, in 4 to 10 bytes a pixel */
     BE_ALGO_RUNS = 4   /* 2D run equivalence, the -a runeq -g path (TOCLRunEquivLabeling,

@@ -211,11 +211,11 @@ void fill_img3d(Img3D &im, const uint8_t *in, int32_t d0, int32_t d1, int32_t d2
 
 // Whether the pixel and run forms leave an image of n pixels to the iterative forms, which give the same
 // labels with about 4.5 bytes of scratch a pixel: the tile pipeline's is a fixed 17 KB a tile, whatever part
-// of the tile the image fills.  Images of up to four rows or columns take more than 32 bytes a pixel so; where
+// of the tile the image fills.  Images of up to four rows or eight columns take more than 32 bytes a pixel so; where
 // that comes to more than half a gigabyte, it is not taken.  Measured, 4-connected, by tiles / iterative: 1 x 2^25
 // pixels, half of them set, 3404 us and 5.4 GB / 1402 us and 0.17 GB, nearly all set 3501 / 5766 us; 2^23 x 1
-// 2813 us and 2.8 GB / 345 us and 0.04 GB, nearly all set 3057 / 1490 us; but 8 x 2^22 617 us and 0.7 GB / 2992
-// us and 0.17 GB.
+// 2813 us and 2.8 GB / 345 us and 0.04 GB, nearly all set 3057 / 1490 us; 4 x 2^22 574 us and 0.7 GB / 1171 us
+// and 0.09 GB; but 8 x 2^22 617 us and 0.7 GB / 2992 us and 0.17 GB.
 constexpr size_t kThinBytes = size_t(1) << 29;
 static bool tiles_nearly_empty(size_t bytes, int64_t n) { return bytes > kThinBytes && bytes > 32 * size_t(n); }
 
